@@ -441,7 +441,7 @@ int apply_T(pw_ctx *c, int ik, int ispin, const void *psi, void *Hpsi, int64_t l
             CK(c, umma_gemm<double2>(kd.beta_tn, B, c->nbeta, nb, c->P.p, c->nbeta, 0, (float *)c->um_ws.p, c->d_err, st));
             c->launches += 2 + (umma_splits(kd.beta_tn.rows, nb, kd.beta_tn.Kp) > 1 ? 1 : 0);
         } else {
-            if ((s = ensure(c, c->gemm_ws, gemm_tn_ws_bytes(kd.Ngw, c->nbeta, nb)))) return s;
+            if ((s = ensure(c, c->gemm_ws, gemm_tn_ws_bytes((int)sizeof(T), kd.Ngw, c->nbeta, nb)))) return s;
             CK(c, (gemm_tn<T>(kd.Ngw, c->nbeta, nb, beta, kd.Ngw, psi, ld, (double2 *)c->P.p, c->nbeta, 0, c->gemm_ws.p, st)));
             c->launches += 2;
         }
@@ -1096,9 +1096,11 @@ extern "C" int pw_gram(pw_ctx *c, int dtype, int64_t K, int m, int n, const void
         return fail(c, PW_ERR_ARG, "bad gram arguments");
     CK(c, cudaSetDevice(c->device));
     if (dtype == PW_C64 && c->use_umma) return umma_tn<double2>(c, K, m, n, A, lda, B, ldb, C, ldc, accumulate);
-    if ((s = ensure(c, c->gemm_ws, gemm_tn_ws_bytes(K, m, n)))) return s;
+    // A^H A: one triangle is formed, the other is its conjugate
+    const int same = dtype == PW_C128 && A == B && lda == ldb && m == n ? 2 : 0;
+    if ((s = ensure(c, c->gemm_ws, gemm_tn_ws_bytes(dtype == PW_C128 ? 8 : 4, K, m, n, same)))) return s;
     if (dtype == PW_C128)
-        CK(c, gemm_tn<double>(K, m, n, A, lda, B, ldb, (double2 *)C, ldc, accumulate, c->gemm_ws.p, c->stream));
+        CK(c, gemm_tn<double>(K, m, n, A, lda, B, ldb, (double2 *)C, ldc, accumulate, c->gemm_ws.p, c->stream, same));
     else
         CK(c, gemm_tn<float>(K, m, n, A, lda, B, ldb, (double2 *)C, ldc, accumulate, c->gemm_ws.p, c->stream));
     c->launches += 2;
@@ -1117,7 +1119,7 @@ int pwk_gram_upper(pw_ctx *c, int dtype, int64_t K, int m, const void *A, int64_
     if (!A || !B || !C || K <= 0 || m <= 0 || lda < K || ldb < K || ldc < m) return fail(c, PW_ERR_ARG, "bad gram arguments");
     CK(c, cudaSetDevice(c->device));
     if (dtype == PW_C64 && c->use_umma) return umma_tn<double2>(c, K, m, m, A, lda, B, ldb, C, ldc, 0, 1);
-    if ((s = ensure(c, c->gemm_ws, gemm_tn_ws_bytes(K, m, m)))) return s;
+    if ((s = ensure(c, c->gemm_ws, gemm_tn_ws_bytes(dtype == PW_C128 ? 8 : 4, K, m, m, 1)))) return s;
     if (dtype == PW_C128)
         CK(c, gemm_tn<double>(K, m, m, A, lda, B, ldb, (double2 *)C, ldc, 0, c->gemm_ws.p, c->stream, 1));
     else
@@ -1304,7 +1306,7 @@ int pwk_beta_dot(pw_ctx *c, int ik, int dtype, const void *psi, int64_t ld, int 
         CK(c, umma_gemm<double2>(kd.beta_tn, B, c->nbeta, nb, out, c->nbeta, 0, (float *)c->um_ws.p, c->d_err, st));
         c->launches += 2 + (umma_splits(kd.beta_tn.rows, nb, kd.beta_tn.Kp) > 1 ? 1 : 0);
     } else {
-        if ((s = ensure(c, c->gemm_ws, gemm_tn_ws_bytes(kd.Ngw, c->nbeta, nb)))) return s;
+        if ((s = ensure(c, c->gemm_ws, gemm_tn_ws_bytes(dtype == PW_C128 ? 8 : 4, kd.Ngw, c->nbeta, nb)))) return s;
         if (dtype == PW_C128)
             CK(c, (gemm_tn<double>(kd.Ngw, c->nbeta, nb, beta, kd.Ngw, psi, ld, out, c->nbeta, 0, c->gemm_ws.p, st)));
         else

@@ -1,5 +1,6 @@
-// Complex GEMMs on CUDA cores for the FP64 path (and the reference for the
-// tensor-core kernels):
+// Complex GEMMs of the FP64 path, on the FP64 tensor cores (mma.sync
+// m8n8k4, exact FP64 products and sums; tcgen05 has no FP64 kind), and FP32
+// CUDA-core versions of the same products (PW_GEMM=cuda):
 //   gemm_tn  C = A^H B      projections betaNL' psi (PsPotNL.jl:252) and the
 //                           Rayleigh-Ritz Gram matrices X'HX, Q'HQ, Q'Q
 //                           (diag_LOBPCG.jl:85,152-153,183-184); long K =
@@ -7,6 +8,9 @@
 //                           reduction in FP64).
 //   gemm_nn  C (+)= A B     betaNL * (D * P) (op_V_Ps_nloc.jl:59-76) and the
 //                           subspace rotations Q*U, HQ*U (diag_LOBPCG.jl:188-194)
+#include <algorithm>
+#include <cmath>
+
 #include "pw_launch.h"
 
 namespace pwk {
@@ -60,48 +64,264 @@ k_gemm_tn(int64_t K, int m, int n, const Cx<T> *__restrict__ A, int64_t lda, con
         }
 }
 
+// ------------------------------------------------------- FP64, tensor cores
+// One CTA of four warps (2 x 2) forms a 16 WM x 16 WN tile of C, each warp
+// WM x WN blocks of 8 x 8 complex values in registers: per step of four k it
+// reads WM + WN fragments of 16 bytes a lane (one complex value) and issues
+// 4 WM WN m8n8k4 products (Re Re, Im Im, Re Im, Im Re), so shared memory
+// serves at most 0.4 of the time the FP64 pipe needs (64 multiply-adds a
+// clock and SM).  Operands come in BK = 8 steps through a ring of three
+// cp.async stages.  Rows are padded to 12 (k-contiguous operands) or 16 WM + 2
+// (row-contiguous ones) complex values, which puts the eight lanes of each
+// 128-byte phase of a fragment read on different banks.
+// TN: C = A^H B, A and B k-contiguous.  NN: C = A B, A row-contiguous.
+// Bound by the FP64 pipe (36.9 TFLOP/s measured for a loop of nothing else).
+// The 32 x 32 CUDA-core tiles before it were bound by shared-memory reads
+// (two 16-byte reads per complex multiply-add and thread).  Measured, 480
+// columns over K = 23,871 (Q'HQ, Q'Q and Q U of 160 bands together):
+// 6.66 -> 3.07 ms, 26 TFLOP/s; op_H of 32 atoms (81 bands) 664 -> 546 us.
+constexpr int ZBK = 8, ZST = 3, ZKP = ZBK + 4;
+template <int WM, int WN, bool TN> constexpr size_t zgemm_smem() {
+    return (size_t)ZST * ((TN ? 16 * WM * ZKP : ZBK * (16 * WM + 2)) + 16 * WN * ZKP) * sizeof(double2);
+}
+
+__device__ __forceinline__ void cp16(double2 *smem, const double2 *g, bool in) {
+    const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
+    const int n = in ? 16 : 0;   // 0: the 16 bytes are zero-filled, nothing is read
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(sa), "l"(g), "r"(n) : "memory");
+}
+__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                 : "+d"(c[0]), "+d"(c[1])
+                 : "d"(a), "d"(b));
+}
+
+// k range of the CTA: [kbeg, kend).  direct: C is written (or added to)
+// here, else the partial sums go to C[z][n][m] (ld m) for k_splitk_reduce.
+// upper (TN): tiles strictly below the diagonal are skipped.  tri (NN):
+// triangular structure the caller guarantees (the k-loop skips the zero
+// blocks, whole tiles are skipped where no needed output lies):
+//   1  A lower triangular (A[g][l] = 0 for l > g)
+//   2  B upper triangular (B[l][j] = 0 for l > j) and only C[g][j], g <= j,
+//      needed (tiles entirely below the diagonal are not formed)
+//   3  A upper triangular (A[g][l] = 0 for l < g)
+template <int WM, int WN, bool TN>
+__global__ void __launch_bounds__(128, WM *WN >= 12 ? 2 : (WM * WN >= 6 ? 3 : 4))
+k_zgemm(int64_t K, int64_t m, int n, const double2 *__restrict__ A, int64_t lda, const double2 *__restrict__ B,
+        int64_t ldb, double2 *__restrict__ C, int64_t ldc, int64_t kchunk, int direct, int accumulate, int upper, int tri) {
+    constexpr int BM = 16 * WM, BN = 16 * WN;
+    constexpr int AP = TN ? ZKP : BM + 2;                       // row pitch of the A stage
+    constexpr int ASZ = TN ? BM * ZKP : ZBK * (BM + 2), BSZ = BN * ZKP;
+    extern __shared__ __align__(16) unsigned char zsm[];
+    double2 *As = reinterpret_cast<double2 *>(zsm), *Bs = As + ZST * ASZ;
+    const int64_t m0 = (int64_t)blockIdx.x * BM;
+    const int n0 = blockIdx.y * BN;
+    if (upper && m0 > n0 + BN - 1) return;
+    if (!TN && tri == 2 && m0 > n0 + BN - 1) return;
+    int64_t kbeg = (int64_t)blockIdx.z * kchunk, kend = min(K, kbeg + kchunk);
+    if (!TN && tri == 1) kend = min(kend, m0 + BM);
+    if (!TN && tri == 2) kend = min(kend, (int64_t)n0 + BN);
+    if (!TN && tri == 3) kbeg = min(K, m0);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int wm = (warp & 1) * 8 * WM, wn = (warp >> 1) * 8 * WN;
+    const int g = lane >> 2, t = lane & 3;
+
+    const int nk = kend > kbeg ? (int)((kend - kbeg + ZBK - 1) / ZBK) : 0;
+    const int ck = tid & 7, cc = tid >> 3;                      // k-contiguous operands: 8 k x 16 columns a round
+    auto load = [&](int it) {
+        const int64_t k0 = kbeg + (int64_t)it * ZBK;
+        double2 *as = As + (it % ZST) * ASZ, *bs = Bs + (it % ZST) * BSZ;
+        const bool kin = k0 + ck < kend;
+        if constexpr (TN) {
+#pragma unroll
+            for (int u = 0; u < WM; ++u) {
+                const int64_t r = m0 + cc + 16 * u;
+                const bool in = kin && r < m;
+                cp16(&as[(cc + 16 * u) * ZKP + ck], in ? &A[(size_t)r * lda + k0 + ck] : A, in);
+            }
+        } else {
+#pragma unroll
+            for (int u = 0; u < WM; ++u) {
+                const int e = tid + 128 * u, kk = e / BM, r = e - kk * BM;
+                const bool in = k0 + kk < kend && m0 + r < m;
+                cp16(&as[kk * AP + r], in ? &A[(size_t)(k0 + kk) * lda + m0 + r] : A, in);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < WN; ++u) {
+            const int c = n0 + cc + 16 * u;
+            const bool in = kin && c < n;
+            cp16(&bs[(cc + 16 * u) * ZKP + ck], in ? &B[(size_t)c * ldb + k0 + ck] : B, in);
+        }
+    };
+
+    double re[WM][WN][2], im[WM][WN][2];
+#pragma unroll
+    for (int i = 0; i < WM; ++i)
+#pragma unroll
+        for (int j = 0; j < WN; ++j) re[i][j][0] = re[i][j][1] = im[i][j][0] = im[i][j][1] = 0.0;
+#pragma unroll
+    for (int p = 0; p < ZST - 1; ++p) {
+        if (p < nk) load(p);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    for (int it = 0; it < nk; ++it) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(ZST - 2) : "memory");
+        __syncthreads();   // stage it has landed for every thread, and everyone is done with stage it - 1
+        if (it + ZST - 1 < nk) load(it + ZST - 1);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        const double2 *as = As + (it % ZST) * ASZ, *bs = Bs + (it % ZST) * BSZ;
+#pragma unroll
+        for (int kk = 0; kk < ZBK; kk += 4) {
+            double2 a[WM], b[WN];
+#pragma unroll
+            for (int i = 0; i < WM; ++i)
+                a[i] = TN ? as[(wm + 8 * i + g) * ZKP + kk + t] : as[(kk + t) * AP + wm + 8 * i + g];
+#pragma unroll
+            for (int j = 0; j < WN; ++j) b[j] = bs[(wn + 8 * j + g) * ZKP + kk + t];
+#pragma unroll
+            for (int i = 0; i < WM; ++i) {
+                const double an = -a[i].y;
+#pragma unroll
+                for (int j = 0; j < WN; ++j) {
+                    dmma(re[i][j], a[i].x, b[j].x);
+                    dmma(im[i][j], a[i].x, b[j].y);
+                    dmma(re[i][j], TN ? a[i].y : an, b[j].y);
+                    dmma(im[i][j], TN ? an : a[i].y, b[j].x);
+                }
+            }
+        }
+    }
+    if (!direct) C += (size_t)blockIdx.z * m * n;
+#pragma unroll
+    for (int i = 0; i < WM; ++i) {
+        const int64_t mm = m0 + wm + 8 * i + g;
+#pragma unroll
+        for (int j = 0; j < WN; ++j)
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const int nn = n0 + wn + 8 * j + 2 * t + q;
+                if (mm < m && nn < n) {
+                    double2 *p = direct ? &C[(size_t)nn * ldc + mm] : &C[(size_t)nn * m + mm];
+                    double2 v = make_double2(re[i][j][q], im[i][j][q]);
+                    if (direct && accumulate) v = cadd(*p, v);
+                    if (!(direct && upper && mm > nn)) *p = v;
+                }
+            }
+    }
+}
+
+// Tile and split-K count of a product: the candidate with the shortest
+// modelled time in clocks.  A CTA's tile costs 16 WM WN clocks of its SM's
+// FP64 pipe per k, plus about 32 k for filling the ring and storing; the SM
+// with the most CTAs decides; a split adds the partial sums' trip through L2
+// (about 2400 bytes a clock) and the reduction's launch (4000 clocks).
+// (480 x 480 over K = 23,871: 48 x 80 tiles, 0 % padding, against 14 % with
+// 64 x 64.)  Splitting stops at four CTAs an SM, which also bounds the workspace
+// (592 tiles: 49 MB).
+struct ZPlan {
+    int wm, wn, S;
+    int64_t kchunk;
+};
+ZPlan zplan(int64_t K, int64_t m, int n, bool tn, int upper) {
+    ZPlan best{2, 2, 1, K};
+    double tbest = 1e300;
+    for (int wm = 2; wm <= 4; ++wm)
+        for (int wn = 1; wn <= 5; ++wn) {
+            if (!tn && wm == 3) continue;
+            const int64_t tm = (m + 16 * wm - 1) / (16 * wm), tc = (n + 16 * wn - 1) / (16 * wn);
+            if (tc > 65535 || (tn && tm > 65535)) continue;
+            double tiles = (double)tm * (double)tc;
+            if (upper) {
+                tiles = 0;
+                for (int64_t c = 0; c < tc; ++c) tiles += (double)std::min<int64_t>(tm, (c * 16 * wn + 16 * wn - 1) / (16 * wm) + 1);
+            }
+            // splits that fill whole rounds of the 148 SMs
+            for (int w = 0; w <= (tn ? 4 : 0); ++w) {
+                const int S = w == 0 ? 1 : (int)(148.0 * w / tiles);
+                if (w > 0 && (S < 2 || (int64_t)S * 64 > K)) continue;
+                const double kc = (double)((K + S - 1) / S);
+                const double per = std::ceil(tiles * S / 148.0);
+                double t = per * 16.0 * wm * wn * (kc + 32.0) * (per < 1.5 ? 1.15 : 1.0);
+                if (S > 1) t += 4000.0 + (double)S * m * n * 32.0 / 2400.0;
+                if (t < tbest * (1.0 - 1e-9)) {
+                    tbest = t;
+                    best = ZPlan{wm, wn, S, K};
+                }
+            }
+        }
+    const int64_t kc = (K + best.S - 1) / best.S;
+    best.kchunk = (kc + ZBK - 1) / ZBK * ZBK;
+    return best;
+}
+
+template <int WM, int WN, bool TN>
+cudaError_t launch_z(const ZPlan &p, int64_t K, int64_t m, int n, const double2 *A, int64_t lda, const double2 *B,
+                     int64_t ldb, double2 *C, int64_t ldc, int direct, int accumulate, int upper, int tri, cudaStream_t st) {
+    constexpr size_t smem = zgemm_smem<WM, WN, TN>();
+    if (smem > 48 * 1024) {
+        cudaError_t e = cudaFuncSetAttribute(k_zgemm<WM, WN, TN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+    }
+    const dim3 grid((unsigned)((m + 16 * WM - 1) / (16 * WM)), (n + 16 * WN - 1) / (16 * WN), p.S);
+    k_zgemm<WM, WN, TN><<<grid, 128, smem, st>>>(K, m, n, A, lda, B, ldb, C, ldc, p.kchunk, direct, accumulate, upper, tri);
+    return cudaGetLastError();
+}
+template <bool TN>
+cudaError_t launch_zgemm(const ZPlan &p, int64_t K, int64_t m, int n, const void *A, int64_t lda, const void *B, int64_t ldb,
+                         double2 *C, int64_t ldc, int direct, int accumulate, int upper, int tri, cudaStream_t st) {
+    const double2 *a = (const double2 *)A, *b = (const double2 *)B;
+#define PW_Z(WM, WN)               \
+    if (p.wm == WM && p.wn == WN) \
+        return launch_z<WM, WN, TN>(p, K, m, n, a, lda, b, ldb, C, ldc, direct, accumulate, upper, tri, st);
+#define PW_ZR(WM) PW_Z(WM, 1) PW_Z(WM, 2) PW_Z(WM, 3) PW_Z(WM, 4) PW_Z(WM, 5)
+    PW_ZR(2)
+    PW_ZR(4)
+    if constexpr (TN) {
+        PW_ZR(3)
+    }
+#undef PW_ZR
+#undef PW_Z
+    return cudaErrorInvalidValue;
+}
+
+// C[j ldc + i] (+)= sum over the S partial sums W[z][j][i].  upper: 1 = only
+// i <= j is formed and written, 2 = only i <= j was formed and the other
+// triangle gets its conjugate transpose (A^H A).
 __global__ void k_splitk_reduce(const double2 *__restrict__ W, int S, int m, int n, double2 *__restrict__ C, int64_t ldc,
                                 int accumulate, int upper) {
     const size_t total = (size_t)m * n;
     for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
         const int nn = (int)(t / m), mm = (int)(t - (size_t)nn * m);
         if (upper && mm > nn) continue;
-        double2 s = accumulate ? C[(size_t)nn * ldc + mm] : make_double2(0.0, 0.0);
-        for (int z = 0; z < S; ++z) {
-            const double2 v = W[(size_t)z * total + t];
-            s.x += v.x;
-            s.y += v.y;
+        double2 s = make_double2(0.0, 0.0);
+#pragma unroll 4
+        for (int z = 0; z < S; ++z) s = cadd(s, W[(size_t)z * total + t]);
+        double2 *p = &C[(size_t)nn * ldc + mm];
+        *p = accumulate ? cadd(*p, s) : s;
+        if (upper == 2 && mm < nn) {
+            double2 *q = &C[(size_t)mm * ldc + nn];
+            const double2 h = make_double2(s.x, -s.y);
+            *q = accumulate ? cadd(*q, h) : h;
         }
-        C[(size_t)nn * ldc + mm] = s;
     }
 }
 
 constexpr int NN_BM = 64, NN_BN = 32, NN_BK = 16;
 
-// tri: triangular structure the caller guarantees (the k-loop skips the
-// zero blocks, whole tiles are skipped where no needed output lies):
-//   1  A lower triangular (A[g][l] = 0 for l > g)
-//   2  B upper triangular (B[l][j] = 0 for l > j) and only C[g][j], g <= j,
-//      needed (tiles entirely below the diagonal are not formed)
-//   3  A upper triangular (A[g][l] = 0 for l < g)
 template <typename T>
 __global__ void __launch_bounds__(256)
 k_gemm_nn(int64_t M, int n, int k, const Cx<T> *__restrict__ A, int64_t lda, const double2 *__restrict__ B, int64_t ldb,
-          Cx<T> *__restrict__ C, int64_t ldc, int accumulate, int tri) {
+          Cx<T> *__restrict__ C, int64_t ldc, int accumulate) {
     __shared__ Cx<T> As[NN_BK][NN_BM];
     __shared__ Cx<T> Bs[NN_BK][NN_BN];
     const int64_t g0 = (int64_t)blockIdx.x * NN_BM;
     const int n0 = blockIdx.y * NN_BN;
-    if (tri == 2 && g0 > n0 + NN_BN - 1) return;   // the whole CTA: before any barrier
-    int jbeg = 0, jend = k;
-    if (tri == 1) jend = (int)min((int64_t)k, g0 + NN_BM);
-    if (tri == 2) jend = min(k, n0 + NN_BN);
-    if (tri == 3) jbeg = (int)min((int64_t)k, (g0 / NN_BK) * NN_BK);
     const int tg = threadIdx.x & 63, tn = threadIdx.x >> 6;  // 64 rows x 4 column groups of 8
     Cx<T> acc[8];
 #pragma unroll
     for (int q = 0; q < 8; ++q) acc[q] = cmake((T)0, (T)0);
-    for (int j0 = jbeg; j0 < jend; j0 += NN_BK) {
+    for (int j0 = 0; j0 < k; j0 += NN_BK) {
         for (int e = threadIdx.x; e < NN_BK * NN_BM; e += 256) {
             const int gg = e % NN_BM, jj = e / NN_BM;
             As[jj][gg] = (g0 + gg < M && j0 + jj < k) ? A[(size_t)(j0 + jj) * lda + g0 + gg] : cmake((T)0, (T)0);
@@ -182,21 +402,32 @@ int splitk_count(int64_t K, int m, int n) {
 
 }  // namespace
 
-size_t gemm_tn_ws_bytes(int64_t K, int m, int n) {
-    return (size_t)splitk_count(K, m, n) * m * n * sizeof(double2);
+size_t gemm_tn_ws_bytes(int dtype, int64_t K, int m, int n, int upper) {
+    const size_t S = dtype == 8 ? zplan(K, m, n, true, upper).S : splitk_count(K, m, n);
+    return S * m * n * sizeof(double2);
 }
 
 template <typename T>
 cudaError_t gemm_tn(int64_t K, int m, int n, const void *A, int64_t lda, const void *B, int64_t ldb, double2 *C,
                     int64_t ldc, int accumulate, void *ws, cudaStream_t st, int upper) {
     if (m <= 0 || n <= 0) return cudaSuccess;
-    const int S = splitk_count(K, m, n);
-    int64_t kchunk = (K + S - 1) / S;
-    kchunk = ((kchunk + TN_BK - 1) / TN_BK) * TN_BK;
-    dim3 grid((m + TN_BM - 1) / TN_BM, (n + TN_BN - 1) / TN_BN, S);
-    k_gemm_tn<T><<<grid, 256, 0, st>>>(K, m, n, (const Cx<T> *)A, lda, (const Cx<T> *)B, ldb, (double2 *)ws, kchunk, upper);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
+    int S;
+    cudaError_t e;
+    if constexpr (sizeof(T) == 8) {
+        const ZPlan p = zplan(K, m, n, true, upper);
+        S = p.S;
+        const int direct = S == 1 && upper != 2;
+        e = launch_zgemm<true>(p, K, m, n, A, lda, B, ldb, direct ? C : (double2 *)ws, ldc, direct, accumulate, upper, 0, st);
+        if (e != cudaSuccess || direct) return e;
+    } else {
+        S = splitk_count(K, m, n);
+        int64_t kchunk = (K + S - 1) / S;
+        kchunk = ((kchunk + TN_BK - 1) / TN_BK) * TN_BK;
+        dim3 grid((m + TN_BM - 1) / TN_BM, (n + TN_BN - 1) / TN_BN, S);
+        k_gemm_tn<T><<<grid, 256, 0, st>>>(K, m, n, (const Cx<T> *)A, lda, (const Cx<T> *)B, ldb, (double2 *)ws, kchunk, upper);
+        e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+    }
     k_splitk_reduce<<<blocks_for((size_t)m * n), 256, 0, st>>>((const double2 *)ws, S, m, n, C, ldc, accumulate, upper);
     return cudaGetLastError();
 }
@@ -205,9 +436,14 @@ template <typename T>
 cudaError_t gemm_nn(int64_t M, int n, int k, const void *A, int64_t lda, const double2 *B, int64_t ldb, void *C,
                     int64_t ldc, int accumulate, cudaStream_t st, int tri) {
     if (M <= 0 || n <= 0) return cudaSuccess;
-    dim3 grid((unsigned)((M + NN_BM - 1) / NN_BM), (n + NN_BN - 1) / NN_BN);
-    k_gemm_nn<T><<<grid, 256, 0, st>>>(M, n, k, (const Cx<T> *)A, lda, B, ldb, (Cx<T> *)C, ldc, accumulate, tri);
-    return cudaGetLastError();
+    if constexpr (sizeof(T) == 8) {
+        return launch_zgemm<false>(zplan(k, M, n, false, tri == 2), k, M, n, A, lda, B, ldb, (double2 *)C, ldc, 1, accumulate,
+                                   0, tri, st);
+    } else {
+        dim3 grid((unsigned)((M + NN_BM - 1) / NN_BM), (n + NN_BN - 1) / NN_BN);
+        k_gemm_nn<T><<<grid, 256, 0, st>>>(M, n, k, (const Cx<T> *)A, lda, B, ldb, (Cx<T> *)C, ldc, accumulate);
+        return cudaGetLastError();
+    }
 }
 
 template cudaError_t gemm_tn<float>(int64_t, int, int, const void *, int64_t, const void *, int64_t, double2 *, int64_t,
