@@ -14,14 +14,15 @@
 //                                       real tridiagonal Tr), one grid barrier
 //                                       per column (cooperative kernel)
 //   6. lowest k eigenvalues of Tr       multisection on Sturm counts, one warp
-//                                       per eigenvalue
+//                                       per eigenvalue; the block reflectors
+//                                       of step 8 meanwhile
 //   7. eigenvectors of Tr               inverse iteration (tridiagonal LU with
 //                                       partial pivoting), re-orthogonalised
 //                                       (modified Gram-Schmidt) inside clusters
 //                                       of near-degenerate eigenvalues, one
 //                                       warp per cluster
-//   8. Z = Q Ztr                        reflectors applied in reverse order,
-//                                       one CTA per eigenvector
+//   8. Z = Q Ztr                        block reflectors (32 columns) applied
+//                                       in reverse order, 1-4 eigenvectors a CTA
 //   9. S = Linv^H Z                     FP64 complex GEMM
 // The cooperative kernels synchronise with a grid barrier of their own whose
 // waits are bounded; on expiry they record an error and run to completion.
@@ -533,47 +534,147 @@ k_tridiag(double2 *C, int n, double *d, double *e, double2 *tau, double2 *ybuf, 
     }
 }
 
-__device__ int sturm_count(const double *d, const double *e, int n, double x, double pivmin) {
-    double q = d[0] - x;
-    if (fabs(q) < pivmin) q = -pivmin;
-    int c = q < 0.0;
-    for (int i = 1; i < n; ++i) {
-        q = (d[i] - x) - e[i - 1] * e[i - 1] / q;
-        if (fabs(q) < pivmin) q = -pivmin;
-        c += q < 0.0;
+// Number of eigenvalues of a tridiagonal matrix below x from the signs of the
+// Sturm polynomials p_i = (d_i - x) p_{i-1} - e_{i-1}^2 p_{i-2} (a sign change
+// per eigenvalue; the quotients p_i / p_{i-1} are the pivots of LDL^T).  One
+// dependent multiply-add per row (8 clocks) where the pivot recurrence has a
+// division (115); n = 480, 160 values: 536 -> 164 us.  de[i] = (d_i, e_{i-1}^2) of the matrix scaled to norm 1..2,
+// with e^2 >= 2^-200 so that no two consecutive p vanish (a change of e by
+// 2^-100 of the norm); p grows at most 5-fold and shrinks at most 2^-200 per
+// two rows, so rescaling by a power of two every 8 rows stays in range.
+__device__ int sturm_count(const double2 *de, int n, double x) {
+    double pp = 1.0, p = de[0].x - x;
+    int c = (unsigned)__double2hiint(p) >> 31;
+    auto row = [&](int i) {
+        const double2 q = de[i];
+        const double pn = fma(q.x - x, p, -(q.y * pp));
+        c += (unsigned)(__double2hiint(pn) ^ __double2hiint(p)) >> 31;
+        pp = p;
+        p = pn;
+    };
+    int i = 1;
+    for (; i + 8 <= n; i += 8) {
+#pragma unroll
+        for (int u = 0; u < 8; ++u) row(i + u);
+        const int ex = (__double2hiint(fmax(fabs(p), fabs(pp))) >> 20) & 0x7ff;
+        const double f = __hiloint2double((2046 - min(max(ex, 1), 2045)) << 20, 0);
+        p *= f;
+        pp *= f;
     }
+    for (; i < n; ++i) row(i);
     return c;
+}
+
+// Block reflectors of the back-transformation: H_{j0} ... H_{j0+31} =
+// I - V T V^H with T (32 x 32, upper triangular, row-major) from the Gram
+// V^H V of the panel's Householder vectors.  128 threads; V in 32-row chunks
+// through shared memory (sm: 2 x 32 x 33 complex values).
+constexpr int WYB = 32;
+__device__ void wy_panel(const double2 *__restrict__ C, const double2 *__restrict__ tau, int n, int j0,
+                         double2 *__restrict__ T, double2 *sm) {
+    constexpr int LD = WYB + 1;
+    double2 *Vs = sm, *S = sm + WYB * LD;
+    const int tid = threadIdx.x, nv = min(WYB, n - 1 - j0);
+    const int a0 = (tid & 15) * 2, b0 = (tid >> 4) * 4;     // 2 x 4 pairs (a, b) a thread
+    double2 acc[2][4];
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int v = 0; v < 4; ++v) acc[u][v] = make_double2(0.0, 0.0);
+    for (int r0 = j0 + 1; r0 < n; r0 += WYB) {
+        for (int e = tid; e < WYB * WYB; e += 128) {
+            const int j = e / WYB, i = r0 + e % WYB;        // vector j0 + j, row i
+            double2 v = make_double2(0.0, 0.0);
+            if (j < nv && i < n && i > j0 + j) v = i == j0 + j + 1 ? make_double2(1.0, 0.0) : C[(size_t)(j0 + j) * n + i];
+            Vs[(e % WYB) * LD + j] = v;
+        }
+        __syncthreads();
+        if (b0 + 3 > a0)
+            for (int i = 0; i < WYB; ++i) {
+#pragma unroll
+                for (int u = 0; u < 2; ++u)
+#pragma unroll
+                    for (int v = 0; v < 4; ++v) {
+                        const double2 q = cmulc_d(Vs[i * LD + a0 + u], Vs[i * LD + b0 + v]);
+                        acc[u][v].x += q.x;
+                        acc[u][v].y += q.y;
+                    }
+            }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int v = 0; v < 4; ++v) S[(a0 + u) * LD + b0 + v] = acc[u][v];
+    __syncthreads();
+    // T[:, i] = -tau_i T[0:i, 0:i] (V^H v_i)[0:i], T_ii = tau_i (Vs holds T)
+    for (int i = 0; i < WYB; ++i) {
+        const double2 ti = i < nv ? tau[j0 + i] : make_double2(0.0, 0.0);
+        if (tid < WYB) {
+            double2 y = make_double2(0.0, 0.0);
+            for (int q = tid; q < i; ++q) {
+                const double2 w = cmul_d(Vs[tid * LD + q], S[q * LD + i]);
+                y.x += w.x;
+                y.y += w.y;
+            }
+            y = cmul_d(make_double2(-ti.x, -ti.y), y);
+            Vs[tid * LD + i] = tid < i ? y : tid == i ? ti : make_double2(0.0, 0.0);
+        }
+        __syncthreads();
+    }
+    for (int e = tid; e < WYB * WYB; e += 128) T[e] = Vs[(e / WYB) * LD + e % WYB];
 }
 
 // lowest k eigenvalues of the real symmetric tridiagonal (d, e), ascending.
 // Multisection: one warp per eigenvalue; each round the 32 lanes take Sturm
 // counts at 32 interior points of the current interval [a, b], which then
-// shrinks 33-fold to the sub-interval that holds eigenvalue i.
-__global__ void k_bisect(const double *__restrict__ d, const double *__restrict__ e, int n, int k, double *__restrict__ lam,
-                         double *__restrict__ nrm_out) {
+// shrinks 33-fold to the sub-interval that holds eigenvalue i.  The first nwy
+// CTAs form the block reflectors of the back-transformation meanwhile (they
+// need the Householder vectors only).  Latency-bound: n dependent
+// multiply-adds a round, about 12 rounds.
+constexpr int BIS_THREADS = 128;
+inline size_t bisect_smem(int n) { return std::max((size_t)n, (size_t)2 * WYB * (WYB + 1)) * sizeof(double2); }
+__global__ void __launch_bounds__(BIS_THREADS)
+k_bisect(const double *__restrict__ d, const double *__restrict__ e, int n, int k, double *__restrict__ lam,
+         double *__restrict__ nrm_out, const double2 *__restrict__ C, const double2 *__restrict__ tau, int nwy,
+         double2 *__restrict__ T) {
+    extern __shared__ __align__(16) unsigned char sm[];
+    double2 *de = reinterpret_cast<double2 *>(sm);
+    if ((int)blockIdx.x < nwy) {
+        wy_panel(C, tau, n, blockIdx.x * WYB, T + (size_t)blockIdx.x * WYB * WYB, de);
+        return;
+    }
     const int lane = threadIdx.x & 31;
-    const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (i >= k) return;
-    double lo = 1e300, hi = -1e300, emax2 = 0.0;
+    const int i = (blockIdx.x - nwy) * (BIS_THREADS >> 5) + (threadIdx.x >> 5);
+    double lo = 1e300, hi = -1e300;
     for (int r = lane; r < n; r += 32) {
         const double rad = (r > 0 ? fabs(e[r - 1]) : 0.0) + (r < n - 1 ? fabs(e[r]) : 0.0);
         lo = fmin(lo, d[r] - rad);
         hi = fmax(hi, d[r] + rad);
-        if (r < n - 1) emax2 = fmax(emax2, e[r] * e[r]);
     }
     for (int o = 16; o > 0; o >>= 1) {
         lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
         hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-        emax2 = fmax(emax2, __shfl_xor_sync(0xffffffffu, emax2, o));
     }
     const double nrm = fmax(fabs(lo), fabs(hi));
-    const double pivmin = fmax(2.2250738585072014e-308, 2.2250738585072014e-308 * emax2) * 4.0;
-    double a = lo - 1e-14 * nrm - 1e-300, b = hi + 1e-14 * nrm + 1e-300;
+    // exact scaling by a power of two to a norm of 1..2 (a zero or non-finite
+    // matrix stays as it is)
+    const int ex = (__double2hiint(nrm) >> 20) & 0x7ff;
+    const bool ok = ex > 0 && ex < 2046;
+    const double sc = ok ? __hiloint2double((2046 - ex) << 20, 0) : 1.0, un = ok ? __hiloint2double(ex << 20, 0) : 1.0;
+    for (int r = threadIdx.x; r < n; r += BIS_THREADS) {
+        const double es = r > 0 ? e[r - 1] * sc : 0.0;
+        de[r] = make_double2(d[r] * sc, fmax(es * es, 6.223015277861142e-61));   // 2^-200
+    }
+    __syncthreads();
+    if (i >= k) return;
+    const double nrs = nrm * sc;
+    double a = lo * sc - 1e-14 * nrs - 1e-300, b = hi * sc + 1e-14 * nrs + 1e-300;
     for (int it = 0; it < 64; ++it) {
         if (b - a <= 2.0 * 2.220446049250313e-16 * fmax(fabs(a), fabs(b))) break;
         const double h = (b - a) / 33.0;
         const double x = fmin(fmax(a + (lane + 1) * h, a), b);
-        const bool above = sturm_count(d, e, n, x, pivmin) > i;   // eigenvalue i lies below x
+        const bool above = sturm_count(de, n, x) > i;             // eigenvalue i lies below x
         const unsigned m = __ballot_sync(0xffffffffu, above);
         const int f = m ? __ffs(m) - 1 : 32;                       // first sample point above it (warp-uniform)
         const double xl = __shfl_sync(0xffffffffu, x, f > 0 ? f - 1 : 0);
@@ -584,71 +685,104 @@ __global__ void k_bisect(const double *__restrict__ d, const double *__restrict_
         b = nb;
     }
     if (lane == 0) {
-        lam[i] = 0.5 * (a + b);
+        lam[i] = 0.5 * (a + b) * un;
         if (i == 0) *nrm_out = nrm;
     }
 }
 
 // LU factorisation with partial pivoting of (Tr - lam I) (LAPACK dgttrf
-// pattern): rows i and i+1 swap when |sub| > |pivot|.  Outputs, per row:
-// rd = 1 / U[i][i], du = U[i][i+1], du2 = U[i][i+2], lm = multiplier,
-// pv = 1 where rows i, i+1 were swapped.  A zero pivot is replaced by a
-// tiny one (the shift sits on an eigenvalue to working precision).
-__device__ void tri_factor(const double *d, const double *e, int n, double lam, double *rd, double *du, double *du2,
-                           double *lm, unsigned char *pv) {
+// pattern): rows i and i+1 swap when |sub| > |pivot|.  Per row, what the
+// solve below multiplies by: rd = 1 / U[i][i], du = U[i][i+1] rd, du2 =
+// U[i][i+2] rd, lm = multiplier, pv = 1 where rows i, i+1 were swapped.  A
+// pivot below `tiny` is replaced by it (the shift sits on an eigenvalue to working
+// precision; 1e-30 of the norm, so that the solution's norm stays finite).
+// One lane runs it; rows go through registers 8 at a time so that
+// only the recurrence itself is serial.
+constexpr int TRB = 8;
+__device__ void tri_factor(const double *__restrict__ d, const double *__restrict__ e, int n, double lam, double tiny,
+                           double *__restrict__ rd, double *__restrict__ du, double *__restrict__ du2,
+                           double *__restrict__ lm, unsigned char *__restrict__ pv) {
     double di = d[0] - lam, ui = n > 1 ? e[0] : 0.0;
-    for (int i = 0; i < n - 1; ++i) {
-        const double sub = e[i];
-        const double dn = d[i + 1] - lam, un = (i + 1 < n - 1) ? e[i + 1] : 0.0;
-        if (fabs(di) >= fabs(sub)) {
-            if (di == 0.0) di = 1e-300;
-            const double f = sub / di;
-            rd[i] = 1.0 / di;
-            du[i] = ui;
-            du2[i] = 0.0;
-            lm[i] = f;
-            pv[i] = 0;
-            di = dn - f * ui;
-            ui = un;
-        } else {
-            const double f = di / sub;
-            rd[i] = 1.0 / sub;
-            du[i] = dn;
-            du2[i] = un;
-            lm[i] = f;
-            pv[i] = 1;
-            di = ui - f * dn;
-            ui = -f * un;
+    for (int i0 = 0; i0 < n - 1; i0 += TRB) {
+        double dd[TRB], ee[TRB + 1];
+#pragma unroll
+        for (int u = 0; u < TRB; ++u) {
+            dd[u] = i0 + u + 1 < n ? d[i0 + u + 1] - lam : 0.0;
+            ee[u] = i0 + u < n - 1 ? e[i0 + u] : 0.0;
+        }
+        ee[TRB] = i0 + TRB < n - 1 ? e[i0 + TRB] : 0.0;
+#pragma unroll
+        for (int u = 0; u < TRB; ++u) {
+            const int i = i0 + u;
+            if (i < n - 1) {
+                const double sub = ee[u], dn = dd[u], un = ee[u + 1];
+                const bool keep = fabs(di) >= fabs(sub);
+                if (keep && fabs(di) < tiny) di = copysign(tiny, di);
+                const double r = 1.0 / (keep ? di : sub);
+                const double f = (keep ? sub : di) * r;
+                rd[i] = r;
+                du[i] = (keep ? ui : dn) * r;
+                du2[i] = keep ? 0.0 : un * r;
+                lm[i] = f;
+                pv[i] = keep ? 0 : 1;
+                di = keep ? fma(-f, ui, dn) : fma(-f, dn, ui);
+                ui = keep ? un : -f * un;
+            }
         }
     }
-    if (di == 0.0) di = 1e-300;
+    if (fabs(di) < tiny) di = copysign(tiny, di);
     rd[n - 1] = 1.0 / di;
     du[n - 1] = 0.0;
     du2[n - 1] = 0.0;
 }
 
 // b := (Tr - lam I)^-1 b with the factorisation of tri_factor.
-__device__ void tri_solve(int n, const double *rd, const double *du, const double *du2, const double *lm,
-                          const unsigned char *pv, double *b) {
+__device__ void tri_solve(int n, const double *__restrict__ rd, const double *__restrict__ du,
+                          const double *__restrict__ du2, const double *__restrict__ lm,
+                          const unsigned char *__restrict__ pv, double *b) {
     double bi = b[0];
-    for (int i = 0; i < n - 1; ++i) {
-        const double bn = b[i + 1];
-        if (pv[i]) {
-            b[i] = bn;
-            bi = bi - lm[i] * bn;
-        } else {
-            b[i] = bi;
-            bi = bn - lm[i] * bi;
+    for (int i0 = 0; i0 < n - 1; i0 += TRB) {
+        double bn[TRB], l[TRB], o[TRB];
+        bool sw[TRB];
+#pragma unroll
+        for (int u = 0; u < TRB; ++u) {
+            const int i = min(i0 + u, n - 2);
+            bn[u] = b[i + 1];
+            l[u] = lm[i];
+            sw[u] = pv[i] != 0;
         }
+#pragma unroll
+        for (int u = 0; u < TRB; ++u)
+            if (i0 + u < n - 1) {
+                o[u] = sw[u] ? bn[u] : bi;
+                bi = sw[u] ? fma(-l[u], bn[u], bi) : fma(-l[u], bi, bn[u]);
+            }
+#pragma unroll
+        for (int u = 0; u < TRB; ++u)
+            if (i0 + u < n - 1) b[i0 + u] = o[u];
     }
-    b[n - 1] = bi;
-    double x2 = 0.0, x1 = b[n - 1] * rd[n - 1];
+    double x2 = 0.0, x1 = bi * rd[n - 1];
     b[n - 1] = x1;
-    for (int i = n - 2; i >= 0; --i) {
-        const double x = (b[i] - du[i] * x1 - du2[i] * x2) * rd[i];
-        b[i] = x;
-        x2 = x1;
-        x1 = x;
+    for (int i0 = n - 2; i0 >= 0; i0 -= TRB) {
+        double c[TRB], p[TRB], q[TRB];
+#pragma unroll
+        for (int u = 0; u < TRB; ++u) {
+            const int i = max(i0 - u, 0);
+            c[u] = b[i] * rd[i];
+            p[u] = du[i];
+            q[u] = du2[i];
+        }
+#pragma unroll
+        for (int u = 0; u < TRB; ++u)
+            if (i0 - u >= 0) {
+                const double x = fma(-p[u], x1, fma(-q[u], x2, c[u]));
+                x2 = x1;
+                x1 = x;
+                c[u] = x;
+            }
+#pragma unroll
+        for (int u = 0; u < TRB; ++u)
+            if (i0 - u >= 0) b[i0 - u] = c[u];
     }
 }
 
@@ -688,7 +822,7 @@ __global__ void k_invit(const double *__restrict__ d, const double *__restrict__
             h ^= h >> 13;
             x[r] = ((double)(h & 0xFFFFFF) / 16777216.0) - 0.5;
         }
-        if (lane == 0) tri_factor(d, e, n, li, rd, du, du2, lm, pv);
+        if (lane == 0) tri_factor(d, e, n, li, nrm > 0.0 ? 1e-30 * nrm : 1e-30, rd, du, du2, lm, pv);
         __syncwarp();
         for (int it = 0; it < INVIT_STEPS; ++it) {
             if (lane == 0) tri_solve(n, rd, du, du2, lm, pv, x);
@@ -717,37 +851,126 @@ __global__ void k_invit(const double *__restrict__ d, const double *__restrict__
 // shared memory of k_invit per warp
 inline size_t invit_smem_per_warp(int n) { return (size_t)n * (5 * sizeof(double) + 1); }
 
-// Z[:, c] = Q Ztr[:, c], Q = H_0 H_1 ... H_{n-2}: reflectors in reverse order.
-__global__ void k_backtr(const double2 *__restrict__ C, const double2 *__restrict__ tau, int n,
-                         const double *__restrict__ Zt, double2 *__restrict__ Z) {
+// Z[:, c] = Q Ztr[:, c], Q = H_0 H_1 ... H_{n-2}: 32 reflectors at a time,
+// z -= V T (V^H z), in reverse order; NV eigenvectors a CTA, held in shared
+// memory.  Per panel: the 32 dot products (4 vectors a warp), t = T s, the
+// update (rows over threads), one block barrier each, where one reflector at a
+// time took three (n = 480, 160 vectors: 655 -> 199 us).  Bound by reading V
+// (n^2 / 2 values twice a CTA, the second time mostly from L1), so NV grows
+// with k.
+template <int NV>
+__global__ void __launch_bounds__(256)
+k_backtr(const double2 *__restrict__ C, const double2 *__restrict__ T, int n, int k, const double *__restrict__ Zt,
+         double2 *__restrict__ Z) {
     extern __shared__ __align__(16) unsigned char sm[];
-    double2 *z = reinterpret_cast<double2 *>(sm);
-    double2 *red = z + n;
-    const int c = blockIdx.x;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) z[i] = make_double2(Zt[(size_t)c * n + i], 0.0);
+    double2 *z = reinterpret_cast<double2 *>(sm);           // [NV][n]
+    double2 *s = z + (size_t)NV * n, *t = s + NV * WYB;     // [NV][32] each
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int c0 = blockIdx.x * NV;
+#pragma unroll
+    for (int q = 0; q < NV; ++q)
+        for (int i = threadIdx.x; i < n; i += 256)
+            z[q * n + i] = make_double2(c0 + q < k ? Zt[(size_t)(c0 + q) * n + i] : 0.0, 0.0);
     __syncthreads();
-    for (int j = n - 2; j >= 0; --j) {
-        const double2 t = tau[j];
-        if (t.x == 0.0 && t.y == 0.0) continue;
-        const double2 *vj = C + (size_t)j * n;  // v_j[i] at row i >= j+1, v_j[j+1] = 1
-        double2 acc = make_double2(0.0, 0.0);
-        for (int i = j + 1 + threadIdx.x; i < n; i += blockDim.x) {
-            const double2 vi = (i == j + 1) ? make_double2(1.0, 0.0) : vj[i];
-            const double2 p = cmulc_d(vi, z[i]);
-            acc.x += p.x;
-            acc.y += p.y;
+    for (int p = (n - 2) / WYB; p >= 0; --p) {
+        const int j0 = p * WYB, nv = min(WYB, n - 1 - j0);
+        double2 acc[4][NV];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int q = 0; q < NV; ++q) acc[u][q] = make_double2(0.0, 0.0);
+        const int jw = j0 + warp * 4;                       // this warp's vectors jw .. jw + 3
+        if (warp * 4 < nv) {
+#pragma unroll 2
+            for (int i = jw + 1 + lane; i < n; i += 32) {
+                double2 v[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const int j = jw + u;
+                    v[u] = (j < j0 + nv && i > j + 1) ? C[(size_t)j * n + i]
+                                                      : make_double2(j < j0 + nv && i == j + 1 ? 1.0 : 0.0, 0.0);
+                }
+#pragma unroll
+                for (int q = 0; q < NV; ++q) {
+                    const double2 x = z[q * n + i];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const double2 w = cmulc_d(v[u], x);
+                        acc[u][q].x += w.x;
+                        acc[u][q].y += w.y;
+                    }
+                }
+            }
         }
-        acc = block_sum<double2>(acc, red);
-        const double2 f = cmul_d(t, acc);
-        for (int i = j + 1 + threadIdx.x; i < n; i += blockDim.x) {
-            const double2 vi = (i == j + 1) ? make_double2(1.0, 0.0) : vj[i];
-            const double2 p = cmul_d(vi, f);
-            z[i].x -= p.x;
-            z[i].y -= p.y;
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+#pragma unroll
+            for (int q = 0; q < NV; ++q) {
+                double2 a = acc[u][q];
+                for (int o = 16; o > 0; o >>= 1) {
+                    a.x += __shfl_xor_sync(0xffffffffu, a.x, o);
+                    a.y += __shfl_xor_sync(0xffffffffu, a.y, o);
+                }
+                if (lane == 0) s[q * WYB + warp * 4 + u] = a;
+            }
+        // t = T s, 8 lanes a row (the loads of T do not wait for s)
+        const int r = threadIdx.x >> 3, l8 = threadIdx.x & 7;
+        double2 tr[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) tr[u] = T[(size_t)p * WYB * WYB + r * WYB + l8 + 8 * u];
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < NV; ++q) {
+            double2 a = make_double2(0.0, 0.0);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const double2 w = cmul_d(tr[u], s[q * WYB + l8 + 8 * u]);
+                a.x += w.x;
+                a.y += w.y;
+            }
+            for (int o = 4; o > 0; o >>= 1) {
+                a.x += __shfl_xor_sync(0xffffffffu, a.x, o);
+                a.y += __shfl_xor_sync(0xffffffffu, a.y, o);
+            }
+            if (l8 == 0) t[q * WYB + r] = a;
+        }
+        __syncthreads();
+        // rows i of z; T's zero rows make t vanish beyond nv
+        for (int i = j0 + 1 + threadIdx.x; i < n; i += 256) {
+            double2 x[NV];
+#pragma unroll
+            for (int q = 0; q < NV; ++q) x[q] = z[q * n + i];
+#pragma unroll 8
+            for (int j = 0; j < nv; ++j) {
+                const double2 v = i > j0 + j + 1 ? C[(size_t)(j0 + j) * n + i]
+                                                 : make_double2(i == j0 + j + 1 ? 1.0 : 0.0, 0.0);
+#pragma unroll
+                for (int q = 0; q < NV; ++q) {
+                    const double2 w = cmul_d(v, t[q * WYB + j]);
+                    x[q].x -= w.x;
+                    x[q].y -= w.y;
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < NV; ++q) z[q * n + i] = x[q];
         }
         __syncthreads();
     }
-    for (int i = threadIdx.x; i < n; i += blockDim.x) Z[(size_t)c * n + i] = z[i];
+#pragma unroll
+    for (int q = 0; q < NV; ++q)
+        if (c0 + q < k)
+            for (int i = threadIdx.x; i < n; i += 256) Z[(size_t)(c0 + q) * n + i] = z[q * n + i];
+}
+
+template <int NV>
+cudaError_t launch_backtr(const double2 *C, const double2 *T, int n, int k, const double *Zt, double2 *Z, cudaStream_t st) {
+    const size_t smem = (size_t)NV * (n + 2 * WYB) * sizeof(double2);
+    if (smem > 48 * 1024) {
+        cudaError_t e = cudaFuncSetAttribute((const void *)k_backtr<NV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+    }
+    k_backtr<NV><<<(k + NV - 1) / NV, 256, smem, st>>>(C, T, n, k, Zt, Z);
+    return cudaGetLastError();
 }
 
 int blocks_for(size_t total) {
@@ -875,7 +1098,17 @@ cudaError_t hegv_lowest(double2 *T, double2 *G, int n, int k, double *lam_out, d
     // a non-finite T or G reaches the tridiagonal matrix: report it (the
     // Sturm counts would otherwise turn it into finite, meaningless values)
     k_check_finite<<<1, 256, 0, st>>>(d, e, n, err + 2);
-    k_bisect<<<(k + 7) / 8, 256, 0, st>>>(d, e, n, k, lam, nrm);
+    // DI (the inverse diagonal tiles, not needed any more) holds the block
+    // reflectors' T: 32 x 32 values for each 32 of the n - 1 reflectors
+    double2 *Tw = DI;
+    {
+        const size_t smem = bisect_smem(n);
+        const int nwy = S ? (n - 1 + WYB - 1) / WYB : 0, per = BIS_THREADS / 32;
+        if (smem > 48 * 1024 &&
+            (e_ = cudaFuncSetAttribute((const void *)k_bisect, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
+            return e_;
+        k_bisect<<<nwy + (k + per - 1) / per, BIS_THREADS, smem, st>>>(d, e, n, k, lam, nrm, Cm, tau, nwy, Tw);
+    }
     if ((e_ = cudaMemcpyAsync(lam_out, lam, k * sizeof(double), cudaMemcpyDeviceToDevice, st)) != cudaSuccess) return e_;
     if (S) {
         {
@@ -889,12 +1122,15 @@ cudaError_t hegv_lowest(double2 *T, double2 *G, int n, int k, double *lam_out, d
                 return e_;
             k_invit<<<(k + wpc - 1) / wpc, 32 * wpc, smem, st>>>(d, e, n, k, lam, nrm, 1e-7, Zt);
         }
-        const size_t smem = (size_t)(n + 32) * sizeof(double2);
-        if (smem > 48 * 1024 &&
-            (e_ = cudaFuncSetAttribute((const void *)k_backtr, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) !=
-                cudaSuccess)
-            return e_;
-        k_backtr<<<k, 256, smem, st>>>(Cm, tau, n, Zt, G ? Z : S);
+        // one eigenvector a CTA until there are enough for every SM several times
+        double2 *Zo = G ? Z : S;
+        if (k >= 4 * 148 && n <= 2048)
+            e_ = launch_backtr<4>(Cm, Tw, n, k, Zt, Zo, st);
+        else if (k >= 2 * 148 && n <= 4096)
+            e_ = launch_backtr<2>(Cm, Tw, n, k, Zt, Zo, st);
+        else
+            e_ = launch_backtr<1>(Cm, Tw, n, k, Zt, Zo, st);
+        if (e_ != cudaSuccess) return e_;
         if (G) {
             // S = Linv^H Z  (Linv^H sits in G)
             if ((e_ = gemm_nn<double>(n, k, n, G, n, Z, n, S, n, 0, st, 3)) != cudaSuccess) return e_;
