@@ -3,11 +3,10 @@
 // (LAPACK zhegv / zheev in the reference).
 //
 //   1. hermitise T and G from their upper triangles (Julia's Hermitian(A))
-//   2. G = L L^H                        blocked right-looking Cholesky on
-//                                       32 x 32 tiles, two grid barriers per
-//                                       32-column panel (cooperative kernel)
-//   3. Linv = L^-1                      blocked right-looking triangular
-//                                       inverse on 32 x 32 tiles
+//   2. G = L L^H                        blocked right-looking elimination of
+//   3. Linv = L^-1                      [G | I] on 32 x 32 tiles, two grid
+//                                       barriers per 32-column panel
+//                                       (cooperative kernel)
 //   4. C = Linv T Linv^H                two FP64 complex GEMMs
 //   5. C = Q Tr Q^H                     Householder tridiagonalisation (LAPACK
 //                                       zhetd2 conventions: H = I - tau v v^H,
@@ -140,234 +139,210 @@ __global__ void k_conj_transpose(const double2 *__restrict__ A, double2 *__restr
 }
 
 // ---------------------------------------------------------------- blocked
-// Cholesky and triangular inverse on 32 x 32 tiles (cooperative kernels).
+// Cholesky and triangular inverse on 32 x 32 tiles, in one elimination of the
+// augmented matrix [G | I] -> [L^H | L^-1] (cooperative kernel).
 constexpr int TB = 32;
-constexpr int TLD = TB + 1;  // shared-memory tile leading dimension (row-major)
+constexpr int TLD = TB + 1;  // leading dimension of the diagonal block (row-major)
+constexpr int KLD = TB + 2;  // tiles stored [k][row]: the 8 lanes of a 128-byte phase of a fragment
+constexpr int CLD = TB + 4;  // read (4 k x 2 rows) fall on different banks; tiles stored [column][k]
 
-// In-place Cholesky of the bs x bs lower block D (row-major, ld TLD).
-// Returns the first failing local column + 1, or 0.  A non-positive pivot
-// is replaced by a tiny one so the factorisation runs to completion.
-__device__ int chol_tile(double2 *D, int bs) {
-    int fail = 0;
-    for (int t = 0; t < bs; ++t) {
-        const double dt = D[t * TLD + t].x;
-        if (!(dt > 0.0) && fail == 0) fail = t + 1;
-        const double s = sqrt(fmax(dt, 1e-300)), inv = 1.0 / s;
-        __syncthreads();
-        for (int i = t + threadIdx.x; i < bs; i += blockDim.x)
-            D[i * TLD + t] = (i == t) ? make_double2(s, 0.0) : make_double2(D[i * TLD + t].x * inv, D[i * TLD + t].y * inv);
-        __syncthreads();
-        for (int idx = threadIdx.x; idx < bs * bs; idx += blockDim.x) {
-            const int i = idx / bs, k = idx - i * bs;
-            if (k > t && i >= k) {
-                const double2 p = cmulc_d(D[k * TLD + t], D[i * TLD + t]);  // D[i][t] conj(D[k][t])
-                D[i * TLD + k].x -= p.x;
-                D[i * TLD + k].y -= p.y;
-            }
+__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                 : "+d"(c[0]), "+d"(c[1])
+                 : "d"(a), "d"(b));
+}
+
+// Cholesky of the diagonal block at (p, p) (rows and columns past n read as
+// the unit matrix) into D (row-major, ld TLD, lower part), 1 / L_tt into rdiag.
+// Right-looking with the elements in registers (thread (tx, ty) owns rows
+// tx + 16 a, columns ty + 16 b): a step publishes one raw column, and
+// everyone subtracts raw_r conj(raw_c) / pivot; one block barrier a step.
+// Returns the first failing local column + 1, or 0; a non-positive pivot is
+// replaced by a tiny one so the factorisation runs to completion.
+__device__ int chol_tile(const double2 *A, int n, int p, double2 *D, double *rdiag, double2 (*col)[TB]) {
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    double2 v[2][2];
+#pragma unroll
+    for (int a = 0; a < 2; ++a)
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+            const int r = tx + 16 * a, c = ty + 16 * b;
+            v[a][b] = (p + r < n && p + c < n) ? __ldcg(&A[(size_t)(p + c) * n + p + r]) : make_double2(r == c ? 1.0 : 0.0, 0.0);
         }
-        __syncthreads();
-    }
+    int fail = 0;
+#pragma unroll
+    for (int b = 0; b < 2; ++b)
+        for (int tt = 0; tt < 16; ++tt) {
+            const int t = 16 * b + tt;
+            double2 *cb = col[t & 1];
+            if (ty == tt) {
+                cb[tx] = v[0][b];
+                cb[tx + 16] = v[1][b];
+            }
+            __syncthreads();   // the buffer two steps back is free: everyone passed the last barrier after reading it
+            const double dt = cb[t].x;
+            if (!(dt > 0.0) && fail == 0) fail = t + 1;
+            const double inv = 1.0 / fmax(dt, 1e-300);
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const double2 rc = cb[ty + 16 * q];
+                const double2 f = make_double2(rc.x * inv, -rc.y * inv);
+#pragma unroll
+                for (int a = 0; a < 2; ++a) {
+                    if (ty + 16 * q > t) {
+                        const double2 m = cmul_d(cb[tx + 16 * a], f);
+                        v[a][q].x -= m.x;
+                        v[a][q].y -= m.y;
+                    }
+                }
+            }
+            // column t stays raw in its owners' registers; its scale 1 / sqrt(pivot)
+            if (threadIdx.x == t) rdiag[t] = 1.0 / sqrt(fmax(dt, 1e-300));
+        }
+    __syncthreads();
+#pragma unroll
+    for (int a = 0; a < 2; ++a)
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+            const int r = tx + 16 * a, c = ty + 16 * b;
+            D[r * TLD + c] = make_double2(v[a][b].x * rdiag[c], v[a][b].y * rdiag[c]);
+        }
     return fail;
 }
 
-// X = L^-1 for the bs x bs lower block L (both row-major, ld TLD): thread c
-// solves column c by forward substitution.
-__device__ void trinv_tile(const double2 *L, double2 *X, int bs) {
-    for (int idx = threadIdx.x; idx < TB * TLD; idx += blockDim.x) X[idx] = make_double2(0.0, 0.0);
-    __syncthreads();
-    const int c = threadIdx.x;
-    if (c < bs) {
-        const double2 lcc = L[c * TLD + c];
-        X[c * TLD + c] = make_double2(1.0 / lcc.x, 0.0);
-        for (int r = c + 1; r < bs; ++r) {
-            double2 s = make_double2(0.0, 0.0);
-            for (int q = c; q < r; ++q) {
-                const double2 p = cmul_d(L[r * TLD + q], X[q * TLD + c]);
-                s.x += p.x;
-                s.y += p.y;
-            }
-            const double il = -1.0 / L[r * TLD + r].x;
-            X[r * TLD + c] = make_double2(s.x * il, s.y * il);
-        }
-    }
-    __syncthreads();
-}
-
-// Tile (r0, c0) of the column-major n x n matrix A into T (row-major, ld
-// TLD); entries outside the matrix read as zero.
-__device__ void load_tile(const double2 *A, int n, int r0, int c0, double2 *T) {
-#pragma unroll
-    for (int idx = threadIdx.x; idx < TB * TB; idx += COOP_THREADS) {
-        const int c = idx / TB, r = idx - c * TB;
-        const int gr = r0 + r, gc = c0 + c;
-        T[r * TLD + c] = (gr < n && gc < n) ? __ldcg(&A[(size_t)gc * n + gr]) : make_double2(0.0, 0.0);
-    }
-}
-__device__ void store_tile(double2 *A, int n, int r0, int c0, const double2 *T) {
-    for (int idx = threadIdx.x; idx < TB * TB; idx += blockDim.x) {
-        const int c = idx / TB, r = idx - c * TB;
-        const int gr = r0 + r, gc = c0 + c;
-        if (gr < n && gc < n) A[(size_t)gc * n + gr] = T[r * TLD + c];
-    }
-}
-
-// Cholesky G = L L^H, lower, in place, right-looking over 32-column panels:
-//   phase 1 (every CTA): factor the diagonal block L11; the panel rows
-//           below it, L21 = A21 L11^-H, by forward substitution, one warp
-//           per row;
+// G = L L^H and X = L^-1 together, right-looking over 32-column panels:
+//   phase 1 (one warp per row or column, after every CTA has factored the
+//           diagonal block L11 for itself): the panel rows L21 = A21 L11^-H
+//           and the block row X_p = L11^-1 X_p, by substitution;
 //   barrier;
-//   phase 2: trailing update A22 -= L21 L21^H on lower 32 x 32 tiles
-//           (cyclic over CTAs); CTA 0 stores L11;
+//   phase 2: A_IJ -= L_I L_J^H on the lower trailing tiles and
+//           X_IJ -= L_I X_pJ below the block row (cyclic over CTAs), on the
+//           FP64 tensor cores;
 //   barrier.
-// The strict upper triangle is left as it was.  info = first failing
-// column (1-based) or 0.
-__global__ void __launch_bounds__(COOP_THREADS) k_chol(double2 *A, int n, unsigned *ctr, int *err, int *info) {
+// G's lower triangle is overwritten, its upper triangle left; X is written in
+// full (zero above the diagonal).  info = first failing column (1-based) or 0.
+// Latency-bound (15 panels at n = 480): 306 us at n = 480 and 117 us at n = 160;
+// two kernels, Cholesky and inverse, with three block barriers a column in the
+// diagonal block, took 549 + 307 and 181 + 109 us.
+constexpr size_t CHOL_SMEM = (size_t)(TB * TLD + 2 * TB * CLD) * sizeof(double2);
+__global__ void __launch_bounds__(COOP_THREADS) k_chol_inv(double2 *A, double2 *X, int n, unsigned *ctr, int *err, int *info) {
     extern __shared__ __align__(16) unsigned char sm[];
     double2 *D = reinterpret_cast<double2 *>(sm);  // diagonal block
-    double2 *Xi = D + TB * TLD;                     // 1 / diagonal of L11
-    double2 *Tr = Xi + TB * TLD;                    // rows tile
-    double2 *Tc = Tr + TB * TLD;                    // columns tile
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    double2 *Ta = D + TB * TLD;                     // L_I, [k][row]
+    double2 *Tb = Ta + TB * CLD;                    // L_J, [k][row], or X_pJ, [column][k]
+    __shared__ double rdiag[TB];
+    __shared__ double2 col[2][TB];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = COOP_THREADS >> 5;
     unsigned tgt = 0;
     for (int p = 0; p < n; p += TB) {
-        const int bs = min(TB, n - p);
-        load_tile(A, n, p, p, D);
-        __syncthreads();
-        const int f = chol_tile(D, bs);
+        const int bs = min(TB, n - p), q0 = p + bs, P = p / TB;
+        // the first row or column of this warp: loaded before the factorisation
+        auto load = [&](int i) {
+            double2 z = make_double2(0.0, 0.0);
+            if (lane >= bs) return z;
+            if (i >= q0) return i < n ? __ldcg(&A[(size_t)(p + lane) * n + i]) : z;                 // row i of A21
+            if (i >= p) return make_double2(i - p == lane ? 1.0 : 0.0, 0.0);                        // X_pp = I
+            return __ldcg(&X[(size_t)i * n + p + lane]);                                             // column i of X_p
+        };
+        const int i0 = blockIdx.x * nw + warp, step = gridDim.x * nw;
+        double2 acc = i0 < n ? load(i0) : make_double2(0.0, 0.0);
+        const int f = chol_tile(A, n, p, D, rdiag, col);
         if (f && blockIdx.x == 0 && threadIdx.x == 0) atomicCAS(info, 0, p + f);
-        if (threadIdx.x < TB) Xi[threadIdx.x] = make_double2(threadIdx.x < bs ? 1.0 / D[threadIdx.x * TLD + threadIdx.x].x : 0.0, 0.0);
         __syncthreads();
-        // L21 rows by forward substitution, one warp per row i, lane t holding
-        // column t:  l[t] = (a[t] - sum_{s<t} l[s] conj(L11[t][s])) / L11[t][t]
-        for (int i = p + bs + blockIdx.x * nw + warp; i < n; i += gridDim.x * nw) {
-            double2 acc = lane < bs ? __ldcg(&A[(size_t)(p + lane) * n + i]) : make_double2(0.0, 0.0);
+        // l[t] = (a[t] - sum_{s<t} l[s] L11[t][s]^(*)) / L11[t][t], lane t holding
+        // entry t: conjugated for the rows of L21, plain for the columns of X
+        for (int i = i0; i < n; i += step) {
+            if (i != i0) acc = load(i);
+            const double cj = i >= q0 ? -1.0 : 1.0;
             double2 l = make_double2(0.0, 0.0);
-            for (int s = 0; s < bs; ++s) {
-                const double is = Xi[s].x;
+#pragma unroll 8
+            for (int s = 0; s < TB; ++s) {
+                const double is = rdiag[s];
                 const double2 ls = make_double2(__shfl_sync(0xffffffffu, acc.x, s) * is, __shfl_sync(0xffffffffu, acc.y, s) * is);
                 if (lane == s) l = ls;
                 if (lane > s) {
-                    const double2 q = cmulc_d(D[lane * TLD + s], ls);  // ls conj(L11[lane][s])
+                    double2 m = D[lane * TLD + s];
+                    m.y *= cj;
+                    const double2 q = cmul_d(m, ls);
                     acc.x -= q.x;
                     acc.y -= q.y;
                 }
             }
-            if (lane < bs) A[(size_t)(p + lane) * n + i] = l;
-        }
-        gsync(ctr, tgt, err);
-        if (blockIdx.x == 0) {
-            for (int idx = threadIdx.x; idx < bs * bs; idx += blockDim.x) {
-                const int c = idx / bs, r = idx - c * bs;
-                if (r >= c) A[(size_t)(p + c) * n + p + r] = D[r * TLD + c];
+            if (lane < bs) {
+                if (i >= q0)
+                    A[(size_t)(p + lane) * n + i] = l;
+                else
+                    X[(size_t)i * n + p + lane] = l;
             }
         }
-        const int q0 = p + bs;
-        if (q0 < n) {
-            const int nt = (n - q0 + TB - 1) / TB;
-            const int ntiles = nt * (nt + 1) / 2;
-            for (int tt = blockIdx.x; tt < ntiles; tt += gridDim.x) {
-                int I = 0, rem = tt;
+        // zeros above X's block diagonal (nobody reads them here)
+        for (int e = blockIdx.x * COOP_THREADS + threadIdx.x; e < p * bs; e += gridDim.x * COOP_THREADS)
+            X[(size_t)(p + e / p) * n + e % p] = make_double2(0.0, 0.0);
+        gsync(ctr, tgt, err);
+        if (q0 >= n) break;
+        const int nt = (n - q0 + TB - 1) / TB, ng = nt * (nt + 1) / 2, ntile = ng + nt * (P + 1);
+        for (int tt = blockIdx.x; tt < ntile; tt += gridDim.x) {
+            int I, J;
+            const bool isx = tt >= ng;
+            if (isx) {
+                I = (tt - ng) % nt;
+                J = (tt - ng) / nt;
+            } else {
+                I = 0;
+                int rem = tt;
                 while (rem > I) {
                     rem -= I + 1;
                     ++I;
                 }
-                const int J = rem;
-                const int r0 = q0 + I * TB, c0 = q0 + J * TB;
-                // Tr[r][t] = L21[r0 + r, t], Tc[c][t] = L21[c0 + c, t]
+                J = rem;
+            }
+            const int r0 = q0 + I * TB, c0 = isx ? J * TB : q0 + J * TB;
+            double2 *M = isx ? X : A;
+            // this lane's entries of the target: rows rr, columns cc .. cc + 1 of two 8 x 8 blocks
+            const int g = lane >> 2, t4 = lane & 3, rr = r0 + (warp & 3) * 8 + g;
+            double2 old[2][2];
 #pragma unroll
-                for (int idx = threadIdx.x; idx < TB * TB; idx += COOP_THREADS) {
-                    const int t = idx / TB, r = idx - t * TB;
-                    Tr[r * TLD + t] = (t < bs && r0 + r < n) ? __ldcg(&A[(size_t)(p + t) * n + r0 + r]) : make_double2(0.0, 0.0);
-                    Tc[r * TLD + t] = (t < bs && c0 + r < n) ? __ldcg(&A[(size_t)(p + t) * n + c0 + r]) : make_double2(0.0, 0.0);
+            for (int b = 0; b < 2; ++b)
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    const int cc = c0 + (warp >> 2) * 16 + 8 * b + 2 * t4 + q;
+                    // X's block column p starts from zero
+                    old[b][q] = rr < n && cc < n && !(isx && J == P) ? __ldcg(&M[(size_t)cc * n + rr]) : make_double2(0.0, 0.0);
                 }
-                __syncthreads();
-                const int r = threadIdx.x & (TB - 1);
-                for (int c = threadIdx.x / TB; c < TB; c += blockDim.x / TB) {
-                    const int gr = r0 + r, gc = c0 + c;
-                    if (gr < n && gc < n && gr >= gc) {
-                        double2 s = make_double2(0.0, 0.0);
-                        for (int t = 0; t < bs; ++t) {
-                            const double2 q = cmulc_d(Tc[c * TLD + t], Tr[r * TLD + t]);
-                            s.x += q.x;
-                            s.y += q.y;
-                        }
-                        double2 *a = &A[(size_t)gc * n + gr];
-                        const double2 v = __ldcg(a);
-                        *a = make_double2(v.x - s.x, v.y - s.y);
-                    }
-                }
-                __syncthreads();
-            }
-        }
-        gsync(ctr, tgt, err);
-    }
-}
-
-// X = L^-1 (L lower, column-major; X full n x n, lower result), right-looking
-// over 32 x 32 tiles with X initialised to I:
-//   phase 0: the diagonal block inverses DI[K] = L_KK^-1 (cyclic), X = I;
-//   for each block row K:  X_KJ = DI[K] X_KJ for J <= K;  barrier;
-//                          X_IJ -= L_IK X_KJ for I > K >= J;  barrier.
-__global__ void __launch_bounds__(COOP_THREADS)
-k_trinv(const double2 *__restrict__ L, double2 *__restrict__ X, double2 *__restrict__ DI, int n, unsigned *ctr, int *err) {
-    extern __shared__ __align__(16) unsigned char sm[];
-    double2 *Ta = reinterpret_cast<double2 *>(sm);
-    double2 *Tb = Ta + TB * TLD;
-    double2 *Tx = Tb + TB * TLD;
-    unsigned tgt = 0;
-    const int nbk = (n + TB - 1) / TB;
-    for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < (size_t)n * n; t += (size_t)gridDim.x * blockDim.x) {
-        const int j = (int)(t / n), i = (int)(t - (size_t)j * n);
-        X[t] = make_double2(i == j ? 1.0 : 0.0, 0.0);
-    }
-    for (int K = blockIdx.x; K < nbk; K += gridDim.x) {
-        load_tile(L, n, K * TB, K * TB, Ta);
-        __syncthreads();
-        trinv_tile(Ta, Tb, min(TB, n - K * TB));
-        for (int idx = threadIdx.x; idx < TB * TB; idx += blockDim.x) DI[(size_t)K * TB * TB + idx] = Tb[(idx / TB) * TLD + idx % TB];
-        __syncthreads();
-    }
-    gsync(ctr, tgt, err);
-    const int r = threadIdx.x & (TB - 1);
-    for (int K = 0; K < nbk; ++K) {
-        // X_KJ = DI[K] X_KJ
-        for (int J = blockIdx.x; J <= K; J += gridDim.x) {
-            for (int idx = threadIdx.x; idx < TB * TB; idx += blockDim.x) Ta[(idx / TB) * TLD + idx % TB] = DI[(size_t)K * TB * TB + idx];
-            load_tile(X, n, K * TB, J * TB, Tx);
-            __syncthreads();
-            for (int c = threadIdx.x / TB; c < TB; c += blockDim.x / TB) {
-                double2 s = make_double2(0.0, 0.0);
-                for (int q = 0; q <= r; ++q) {
-                    const double2 p = cmul_d(Ta[r * TLD + q], Tx[q * TLD + c]);
-                    s.x += p.x;
-                    s.y += p.y;
-                }
-                Tb[r * TLD + c] = s;
+#pragma unroll
+            for (int e = threadIdx.x; e < TB * TB; e += COOP_THREADS) {
+                const int hi = e / TB, lo = e % TB;
+                Ta[hi * KLD + lo] = hi < bs && r0 + lo < n ? __ldcg(&A[(size_t)(p + hi) * n + r0 + lo]) : make_double2(0.0, 0.0);
+                if (isx)
+                    Tb[hi * CLD + lo] = lo < bs ? __ldcg(&X[(size_t)(c0 + hi) * n + p + lo]) : make_double2(0.0, 0.0);
+                else
+                    Tb[hi * KLD + lo] = hi < bs && c0 + lo < n ? __ldcg(&A[(size_t)(p + hi) * n + c0 + lo]) : make_double2(0.0, 0.0);
             }
             __syncthreads();
-            store_tile(X, n, K * TB, J * TB, Tb);
-            __syncthreads();
-        }
-        gsync(ctr, tgt, err);
-        // X_IJ -= L_IK X_KJ
-        const int ni = nbk - K - 1, nj = K + 1;
-        for (int tt = blockIdx.x; tt < ni * nj; tt += gridDim.x) {
-            const int I = K + 1 + tt / nj, J = tt % nj;
-            load_tile(L, n, I * TB, K * TB, Ta);
-            load_tile(X, n, K * TB, J * TB, Tx);
-            load_tile(X, n, I * TB, J * TB, Tb);
-            __syncthreads();
-            for (int c = threadIdx.x / TB; c < TB; c += blockDim.x / TB) {
-                double2 s = Tb[r * TLD + c];
-                for (int q = 0; q < TB; ++q) {
-                    const double2 p = cmul_d(Ta[r * TLD + q], Tx[q * TLD + c]);
-                    s.x -= p.x;
-                    s.y -= p.y;
+            double re[2][2] = {{0.0, 0.0}, {0.0, 0.0}}, im[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+            const int ra = (warp & 3) * 8 + g;
+#pragma unroll
+            for (int kk = 0; kk < TB; kk += 4) {
+                const double2 a = Ta[(kk + t4) * KLD + ra];
+#pragma unroll
+                for (int b = 0; b < 2; ++b) {
+                    const int cb = (warp >> 2) * 16 + 8 * b + g;
+                    double2 m = isx ? Tb[cb * CLD + kk + t4] : Tb[(kk + t4) * KLD + cb];
+                    if (!isx) m.y = -m.y;
+                    dmma(re[b], a.x, m.x);
+                    dmma(im[b], a.x, m.y);
+                    dmma(re[b], -a.y, m.y);
+                    dmma(im[b], a.y, m.x);
                 }
-                Tb[r * TLD + c] = s;
             }
-            __syncthreads();
-            store_tile(X, n, I * TB, J * TB, Tb);
+#pragma unroll
+            for (int b = 0; b < 2; ++b)
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    const int cc = c0 + (warp >> 2) * 16 + 8 * b + 2 * t4 + q;
+                    if (rr < n && cc < n && (isx || rr >= cc))
+                        M[(size_t)cc * n + rr] = make_double2(old[b][q].x - re[b][q], old[b][q].y - im[b][q]);
+                }
             __syncthreads();
         }
         gsync(ctr, tgt, err);
@@ -1004,35 +979,23 @@ size_t eig_work_bytes(int n, int k) {
            + (size_t)n * sizeof(double2)              // tau
            + (size_t)n * k * sizeof(double)           // Ztr
            + (size_t)n * k * sizeof(double2)          // Z
-           + (size_t)((n + TB - 1) / TB) * TB * TB * sizeof(double2)   // inverse diagonal tiles
+           + (size_t)((n + WYB - 1) / WYB) * WYB * WYB * sizeof(double2)   // block reflectors
            + 16 * 256;                                // barrier, status, norm + 256-byte rounding of 13 pieces
 }
 
-// L = chol(G) in place (lower), Linv = L^-1.  ctr: barrier counter, err:
-// [0] barrier expiry, [1] first failing Cholesky column (1-based).
-cudaError_t chol_and_inverse(double2 *G, int n, double2 *Linv, double2 *DI, unsigned *ctr, int *err, cudaStream_t st) {
+// Linv = L^-1 with G = L L^H (G's lower triangle is overwritten).  ctr:
+// barrier counter, err: [0] barrier expiry, [1] first failing Cholesky column
+// (1-based).
+cudaError_t chol_and_inverse(double2 *G, int n, double2 *Linv, unsigned *ctr, int *err, cudaStream_t st) {
     cudaError_t e_;
     const int nt = (n + TB - 1) / TB;
-    {
-        const size_t smem = 4 * (size_t)TB * TLD * sizeof(double2);
-        int nblk = 0;
-        if ((e_ = coop_blocks((const void *)k_chol, smem, &nblk)) != cudaSuccess) return e_;
-        nblk = std::max(1, std::min(nblk, nt * (nt + 1) / 2));
-        if ((e_ = cudaMemsetAsync(ctr, 0, sizeof(unsigned), st)) != cudaSuccess) return e_;
-        int *info = err + 1;
-        void *args[] = {(void *)&G, (void *)&n, (void *)&ctr, (void *)&err, (void *)&info};
-        if ((e_ = cudaLaunchCooperativeKernel((const void *)k_chol, nblk, COOP_THREADS, args, smem, st)) != cudaSuccess) return e_;
-    }
-    {
-        const size_t smem = 3 * (size_t)TB * TLD * sizeof(double2);
-        int nblk = 0;
-        if ((e_ = coop_blocks((const void *)k_trinv, smem, &nblk)) != cudaSuccess) return e_;
-        nblk = std::max(1, std::min(nblk, std::max(nt, (nt * nt + 3) / 4)));
-        if ((e_ = cudaMemsetAsync(ctr, 0, sizeof(unsigned), st)) != cudaSuccess) return e_;
-        void *args[] = {(void *)&G, (void *)&Linv, (void *)&DI, (void *)&n, (void *)&ctr, (void *)&err};
-        if ((e_ = cudaLaunchCooperativeKernel((const void *)k_trinv, nblk, COOP_THREADS, args, smem, st)) != cudaSuccess) return e_;
-    }
-    return cudaSuccess;
+    int nblk = 0;
+    if ((e_ = coop_blocks((const void *)k_chol_inv, CHOL_SMEM, &nblk)) != cudaSuccess) return e_;
+    nblk = std::max(1, std::min(nblk, nt * (nt + 1) / 2));
+    if ((e_ = cudaMemsetAsync(ctr, 0, sizeof(unsigned), st)) != cudaSuccess) return e_;
+    int *info = err + 1;
+    void *args[] = {(void *)&G, (void *)&Linv, (void *)&n, (void *)&ctr, (void *)&err, (void *)&info};
+    return cudaLaunchCooperativeKernel((const void *)k_chol_inv, nblk, COOP_THREADS, args, CHOL_SMEM, st);
 }
 
 // flag[0] = 1 if any diagonal or off-diagonal entry of the tridiagonal
@@ -1062,7 +1025,7 @@ cudaError_t hegv_lowest(double2 *T, double2 *G, int n, int k, double *lam_out, d
     double2 *tau = (double2 *)take(n * sizeof(double2));
     double *Zt = (double *)take((size_t)n * k * sizeof(double));
     double2 *Z = (double2 *)take((size_t)n * k * sizeof(double2));
-    double2 *DI = (double2 *)take((size_t)((n + TB - 1) / TB) * TB * TB * sizeof(double2));
+    double2 *Tw = (double2 *)take((size_t)((n + WYB - 1) / WYB) * WYB * WYB * sizeof(double2));   // block reflectors' T
     GridBar *gb = (GridBar *)take(sizeof(GridBar));
     int *err = (int *)take(sizeof(int) * 4);
     double *nrm = (double *)take(sizeof(double));
@@ -1075,7 +1038,7 @@ cudaError_t hegv_lowest(double2 *T, double2 *G, int n, int k, double *lam_out, d
     double2 *Cm = T;
     if (G) {
         k_herm_upper<<<nb, 256, 0, st>>>(G, n);
-        if ((e_ = chol_and_inverse(G, n, Linv, DI, ctr, err, st)) != cudaSuccess) return e_;
+        if ((e_ = chol_and_inverse(G, n, Linv, ctr, err, st)) != cudaSuccess) return e_;
         // C = Linv T Linv^H: Linv lower triangular, only C's upper triangle
         // is read (n = 1440: the two full products took 3.06 ms)
         if ((e_ = gemm_nn<double>(n, n, n, Linv, n, T, n, M1, n, 0, st, 1)) != cudaSuccess) return e_;
@@ -1098,9 +1061,6 @@ cudaError_t hegv_lowest(double2 *T, double2 *G, int n, int k, double *lam_out, d
     // a non-finite T or G reaches the tridiagonal matrix: report it (the
     // Sturm counts would otherwise turn it into finite, meaningless values)
     k_check_finite<<<1, 256, 0, st>>>(d, e, n, err + 2);
-    // DI (the inverse diagonal tiles, not needed any more) holds the block
-    // reflectors' T: 32 x 32 values for each 32 of the n - 1 reflectors
-    double2 *Tw = DI;
     {
         const size_t smem = bisect_smem(n);
         const int nwy = S ? (n - 1 + WYB - 1) / WYB : 0, per = BIS_THREADS / 32;
@@ -1146,8 +1106,6 @@ cudaError_t chol_inverse_upper(double2 *C, int n, double2 *Rinv, void *work, int
     unsigned char *p = (unsigned char *)work;
     double2 *Linv = (double2 *)p;
     p += (((size_t)n * n * sizeof(double2)) + 255) & ~(size_t)255;
-    double2 *DI = (double2 *)p;
-    p += (((size_t)((n + TB - 1) / TB) * TB * TB * sizeof(double2)) + 255) & ~(size_t)255;
     unsigned *ctr = (unsigned *)p;
     p += 256;
     int *err = (int *)p;
@@ -1155,7 +1113,7 @@ cudaError_t chol_inverse_upper(double2 *C, int n, double2 *Rinv, void *work, int
     if ((e_ = cudaMemsetAsync(err, 0, sizeof(int) * 4, st)) != cudaSuccess) return e_;
     const int nb = blocks_for((size_t)n * n);
     k_herm_upper<<<nb, 256, 0, st>>>(C, n);
-    if ((e_ = chol_and_inverse(C, n, Linv, DI, ctr, err, st)) != cudaSuccess) return e_;
+    if ((e_ = chol_and_inverse(C, n, Linv, ctr, err, st)) != cudaSuccess) return e_;
     k_conj_transpose<<<nb, 256, 0, st>>>(Linv, Rinv, n);
     if ((e_ = cudaGetLastError()) != cudaSuccess) return e_;
     return cudaMemcpyAsync(d_status, err, 2 * sizeof(int), cudaMemcpyDeviceToDevice, st);
