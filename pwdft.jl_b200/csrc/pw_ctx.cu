@@ -328,6 +328,7 @@ FftLaunch make_launch_kd(const pw_ctx *c, const KData &kd) {
         const int cmax = std::max(1, (int)((190 * 1024 / es - c->N3) / c->N3) - 16);
         L.Cg = std::min(c->z_cols, cmax);
     }
+    L.bpc_set = c->plane_bpc;
     L.bpc = c->plane_bpc > 0 ? c->plane_bpc : (c->N1 == 75 ? 3 : 1);
     // plane passes: a 100 KB budget (two CTAs per SM) when it holds at
     // least 16 full x lines, otherwise up to 220 KB

@@ -117,8 +117,12 @@ template <typename T, int R1, int R2> struct PfaDft {
         }
     }
 };
+template <typename T> struct Dft<T, 10> { static __host__ __device__ __forceinline__ void run(Cx<T> *v, T s, const Cx<T> *tw, int st) { PfaDft<T, 2, 5>::run(v, s, tw, st); } };
+template <typename T> struct Dft<T, 12> { static __host__ __device__ __forceinline__ void run(Cx<T> *v, T s, const Cx<T> *tw, int st) { PfaDft<T, 3, 4>::run(v, s, tw, st); } };
+template <typename T> struct Dft<T, 16> { static __host__ __device__ __forceinline__ void run(Cx<T> *v, T s, const Cx<T> *tw, int st) { CompDft<T, 4, 4>::run(v, s, tw, st); } };
 template <typename T> struct Dft<T, 9> { static __host__ __device__ __forceinline__ void run(Cx<T> *v, T s, const Cx<T> *tw, int st) { CompDft<T, 3, 3>::run(v, s, tw, st); } };
 template <typename T> struct Dft<T, 15> { static __host__ __device__ __forceinline__ void run(Cx<T> *v, T s, const Cx<T> *tw, int st) { PfaDft<T, 3, 5>::run(v, s, tw, st); } };
+template <typename T> struct Dft<T, 18> { static __host__ __device__ __forceinline__ void run(Cx<T> *v, T s, const Cx<T> *tw, int st) { PfaDft<T, 2, 9>::run(v, s, tw, st); } };
 template <typename T> struct Dft<T, 24> { static __host__ __device__ __forceinline__ void run(Cx<T> *v, T s, const Cx<T> *tw, int st) { CompDft<T, 8, 3>::run(v, s, tw, st); } };
 template <typename T> struct Dft<T, 25> { static __host__ __device__ __forceinline__ void run(Cx<T> *v, T s, const Cx<T> *tw, int st) { CompDft<T, 5, 5>::run(v, s, tw, st); } };
 template <typename T> struct Dft<T, 27> { static __host__ __device__ __forceinline__ void run(Cx<T> *v, T s, const Cx<T> *tw, int st) { CompDft<T, 9, 3>::run(v, s, tw, st); } };
@@ -130,6 +134,36 @@ template <> struct FPlan<75> { static constexpr int nst = 2; static __host__ __d
 // 120 = 15 * 8: 91-110 registers in the z and plane kernels (24 * 5 needed 128 and spilled
 // 72-432 bytes); measured Si216 FFT round trip 7.95 -> 6.52 ms
 template <> struct FPlan<120> { static constexpr int nst = 2; static __host__ __device__ constexpr int r(int s) { return s == 0 ? 15 : 8; } };
+
+// The other line lengths of common cutoffs: R0 R1 with R1 <= R0 (a warp's
+// first-stage butterflies of its 32 / R1 lines then fill one round) and R0 odd
+// where there is a choice (its outputs, R0 apart, fall on different banks;
+// the even ones are padded, see fp_pad).
+#define PW_FPLAN2(N, R0, R1) \
+    template <> struct FPlan<N> { static constexpr int nst = 2; static __host__ __device__ constexpr int r(int s) { return s == 0 ? R0 : R1; } };
+PW_FPLAN2(20, 5, 4)
+PW_FPLAN2(24, 8, 3)
+PW_FPLAN2(25, 5, 5)
+PW_FPLAN2(30, 15, 2)
+PW_FPLAN2(32, 8, 4)
+PW_FPLAN2(36, 9, 4)
+PW_FPLAN2(40, 8, 5)
+PW_FPLAN2(45, 9, 5)
+PW_FPLAN2(48, 12, 4)
+PW_FPLAN2(50, 10, 5)
+PW_FPLAN2(54, 18, 3)
+PW_FPLAN2(60, 15, 4)
+PW_FPLAN2(64, 8, 8)
+PW_FPLAN2(72, 9, 8)
+PW_FPLAN2(80, 16, 5)
+PW_FPLAN2(81, 27, 3)
+PW_FPLAN2(90, 18, 5)
+PW_FPLAN2(96, 12, 8)
+PW_FPLAN2(100, 25, 4)
+PW_FPLAN2(108, 27, 4)
+PW_FPLAN2(125, 25, 5)
+PW_FPLAN2(128, 16, 8)
+#undef PW_FPLAN2
 
 template <int N> __host__ __device__ constexpr int fp_ns(int s) {
     int p = 1;
@@ -174,20 +208,29 @@ template <int N, int S> __host__ __device__ constexpr int tw_step() {
 }
 // twiddle of element r of stage-S butterfly jm (jm < N_S, the stage's span)
 // Padded element positions of a line held in shared memory: pos(x) = x +
-// (x / R0) * fp_pad, line stride fp_xs.  A plan whose first-stage outputs put
-// several lanes of a half-warp on one bank can pad here (the earlier
-// 120 = 24 * 5 plan needed one spare word per 24 elements and stride 125);
-// the current plans are unpadded.
-template <int N> __host__ __device__ constexpr int fp_pad() { return 0; }
+// (x / R0) * fp_pad, line stride fp_xs.  Plans with an even R0 would put the
+// first stage's outputs (R0 elements apart across lanes) on few banks, so they
+// take one spare element per R0; odd ones are unpadded.
+template <int N> __host__ __device__ constexpr int fp_pad() { return FPlan<N>::nst == 2 && FPlan<N>::r(0) % 2 == 0 ? 1 : 0; }
 template <int N> __host__ __device__ constexpr int fp_pos(int x) {
     if constexpr (fp_pad<N>() == 0)
         return x;
     else
         return x + (x / FPlan<N>::r(0)) * fp_pad<N>();
 }
-template <int N> __host__ __device__ constexpr int fp_xs() { return fp_pad<N>() == 0 ? N : N + N / FPlan<N>::r(0) * fp_pad<N>() + 1; }
-static_assert(fp_xs<120>() >= fp_pos<120>(119) + 1, "padded line fits its stride");
+// Line stride = R1 modulo 16: the 16 / R1 lines of a half-warp then start on
+// different banks in the first stage (75 = 11 modulo 16 does as well).
+template <int N> __host__ __device__ constexpr int fp_xs() {
+    if constexpr (FPlan<N>::nst == 1 || N == 75) {
+        return N;
+    } else {
+        constexpr int base = N + N / FPlan<N>::r(0) * fp_pad<N>(), r1 = FPlan<N>::r(1);
+        return base + ((r1 - base) % 16 + 16) % 16;
+    }
+}
+static_assert(fp_xs<120>() == 120 && fp_pad<120>() == 0, "the 120-point plan is unpadded");
 
+// twiddle of element r of stage-S butterfly jm (jm < N_S, the stage's span)
 template <int N, int S> __device__ __forceinline__ int tw_at(int r, int jm) {
     if constexpr (FPlan<N>::nst == 2 && S == 1) {
         constexpr int R0 = FPlan<N>::r(0);
@@ -248,7 +291,8 @@ __device__ __forceinline__ void apply_tw(Cx<T> (&v)[R], const Cx<T> *tw, int jm,
     for (int r = 1; r < R; ++r) v[r] = cmul(v[r], w[r]);
 }
 
-// PAD: elements at fp_pos(x) (es must be 1)
+// PAD: elements at fp_pos(x) (es must be 1, two-stage plans): stage 0 writes
+// block j of R0 elements, stage 1 touches element j < R0 of block r
 template <typename T, int N, int S, bool JFAST, bool PAD>
 __device__ __forceinline__ void fstage(Cx<T> *buf, int l0, int nl, int es, int ls, const Cx<T> *tw, int sign, int lane) {
     constexpr int R = FPlan<N>::r(S);
@@ -280,7 +324,8 @@ __device__ __forceinline__ void fstage(Cx<T> *buf, int l0, int nl, int es, int l
             const int jm = j % NS;
             const Cx<T> *p = buf + line * ls + j * es;
 #pragma unroll
-            for (int r = 0; r < R; ++r) v[t][r] = PAD ? buf[line * ls + fp_pos<N>(j + r * NBF)] : p[r * NBF * es];
+            for (int r = 0; r < R; ++r)
+                v[t][r] = PAD ? buf[line * ls + (S == 1 ? j + r * (NBF + fp_pad<N>()) : fp_pos<N>(j + r * NBF))] : p[r * NBF * es];
             if constexpr (NS > 1) apply_tw<T, N, S, R>(v[t], tw, jm, sign);
             Dft<T, R>::run(v[t], sg, tw, tw_step<N, S>());
         }
@@ -296,7 +341,7 @@ __device__ __forceinline__ void fstage(Cx<T> *buf, int l0, int nl, int es, int l
 #pragma unroll
             for (int r = 0; r < R; ++r) {
                 if (PAD)
-                    buf[line * ls + fp_pos<N>(x0 + r * NS)] = v[t][r];
+                    buf[line * ls + (S == 1 ? x0 + r * (NS + fp_pad<N>()) : x0 + j * fp_pad<N>() + r)] = v[t][r];
                 else
                     q[r * NS * es] = v[t][r];
             }
@@ -368,8 +413,9 @@ __device__ __forceinline__ void fstage_io(int nl, const Cx<T> *tw, int sign, int
 template <typename T, int N, class LD0, class STL>
 __device__ __forceinline__ void group_fft(Cx<T> *buf, int nl, const Cx<T> *tw, int sign, int lane, LD0 &ld0, STL &stl) {
     constexpr int XS = fp_xs<N>();
-    auto bld = [&](int line, int x, int) { return buf[line * XS + fp_pos<N>(x)]; };
-    auto bst = [&](int line, int x, int, Cx<T> v) { buf[line * XS + fp_pos<N>(x)] = v; };
+    // stage 0 writes element r of block (x - r) / R0, stage 1 reads element x - r R0 of block r
+    auto bld = [&](int line, int x, int r) { return buf[line * XS + x + r * fp_pad<N>()]; };
+    auto bst = [&](int line, int x, int r, Cx<T> v) { buf[line * XS + fp_pos<N>(x - r) + r] = v; };
     constexpr int NST = FPlan<N>::nst;
     static_assert(NST == 1 || NST == 2, "fused plans have one or two stages");
     if constexpr (NST == 1) {
@@ -411,7 +457,7 @@ __device__ __forceinline__ void group_fft_vpair(Cx<T> *buf, int nl, const Cx<T> 
         constexpr int R0 = FPlan<N>::r(0), R1 = FPlan<N>::r(1);
         constexpr int G = fp_group<N>();
         constexpr int XS = fp_xs<N>(), RP = R0 + fp_pad<N>();   // fp_pos(j + R0 r) = j + RP r for j < R0
-        auto bst = [&](int line, int x, int, Cx<T> v) { buf[line * XS + fp_pos<N>(x)] = v; };
+        auto bst = [&](int line, int x, int r, Cx<T> v) { buf[line * XS + fp_pos<N>(x - r) + r] = v; };
         fstage_io<T, N, 0>(nl, tw, 1, lane, ld0, bst);   // inverse stage 0 into buf
         using L1 = LaneMap<R0, G>;                         // stage-1 butterflies: R0 per line
         Cx<T> v[L1::ROUNDS][R1];

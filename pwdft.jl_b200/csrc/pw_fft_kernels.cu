@@ -690,9 +690,8 @@ __device__ __forceinline__ void plane_vloc_x_band(const KPlan &kp, const Cx<T> *
         const int g0 = (q % NGRP) * G;
         Cx<T> *Sb = S + (q / NGRP) * SP;
         const int nl = min(G, N2 - g0);
-        // rows g0 .. g0 + G - 1 lie in one padding block (G divides R0)
-        static_assert(pwf::fp_pad<N2>() == 0 || pwf::FPlan<N2>::r(0) % G == 0, "row groups inside a padding block");
-        const int yp = pwf::fp_pos<N2>(g0);
+        static_assert(pwf::fp_pad<N2>() == 0, "unpadded plans");
+        const int yp = g0;
         auto ld_s = [&](int line, int x, int r) {
             const int ia = iax_at(x, r);
             return ia >= 0 ? Sb[ia * LD + yp + line] : cmake((T)0, (T)0);
@@ -1124,9 +1123,15 @@ static cudaError_t set_smem(const void *fn, size_t bytes) {
     return cudaSuccess;
 }
 
-// Line lengths with compile-time kernels (every dimension of the grids of
-// the Si2/Al4 (27), Si64 (75) and Si216 (120) systems).
+// Line lengths of the cube-grid plane and batched kernels (the grids of the
+// Si2/Al4 (27), Si64 (75) and Si216 (120) systems).
 #define FIXED_SIZES(X) X(27) X(75) X(120)
+// and of the compile-time z passes: every length with a fused plan (op_H of 8
+// atoms on a 40-point cube: inverse and forward z pass 26.6 us with run-time
+// plans); other lengths take k_zinv / k_zfwd
+#define Z_SIZES(X)                                                                                                   \
+    X(20) X(24) X(25) X(27) X(30) X(32) X(36) X(40) X(45) X(48) X(50) X(54) X(60) X(64) X(72) X(75) X(80) X(81) X(90) \
+    X(96) X(100) X(108) X(120) X(125) X(128)
 
 template <typename T>
 cudaError_t launch_zinv(const FftLaunch &L, const void *psi, int64_t ld, int nb, void *A, cudaStream_t st) {
@@ -1143,7 +1148,7 @@ cudaError_t launch_zinv(const FftLaunch &L, const void *psi, int64_t ld, int nb,
         kf_zinv<T, NN><<<grid, FFT_THREADS, zsm, st>>>(kp, (const Cx<T> *)L.twz, (const Cx<T> *)psi, ld, (Cx<T> *)A, Cg); \
         return cudaGetLastError();                                                                                   \
     }
-        FIXED_SIZES(PW_CASE)
+        Z_SIZES(PW_CASE)
 #undef PW_CASE
     }
     cudaError_t e = set_smem<T>((const void *)k_zinv<T>, smem);
@@ -1170,7 +1175,7 @@ cudaError_t launch_zfwd(const FftLaunch &L, const void *A, const void *psi, void
                                                         (Cx<T> *)Hpsi, ld, Cg, flags);                               \
         return cudaGetLastError();                                                                                   \
     }
-        FIXED_SIZES(PW_CASE)
+        Z_SIZES(PW_CASE)
 #undef PW_CASE
     }
     cudaError_t e = set_smem<T>((const void *)k_zfwd<T>, smem);
@@ -1400,12 +1405,18 @@ cudaError_t launch_plane_vloc(const FftLaunch &L, const void *Vr, void *A, int n
                                           : launch_plane_vloc64_x<120>(L, Vr, A, nb, st);
         if (e != cudaErrorNotSupported) return e;
     }
+    // (not 27 x 27: one lane a line leaves seven of eight warps idle there, the
+    // plane-wide FP64 kernel below takes 66 us an op_H of 8 bands, this one 82)
+    if (!(kp.N1 == 27 && kp.N2 == 27)) {
+        const cudaError_t e = launch_any_plane_vloc<T>(L, Vr, A, nb, st);
+        if (e != cudaErrorNotSupported) return e;
+    }
     PlaneSmem ps{kp.N1, kp.N2, kp.Nxa, L.Jc};
     size_t smem = ps.elems() * sizeof(Cx<T>);
-    if (kp.N1 == kp.N2) {
+    if constexpr (sizeof(T) == 8) {   // 27 x 27, and planes that do not fit the x-fused kernels
         dim3 grid(kp.N3, nb);
 #define PW_CASE(NN)                                                                                                  \
-    if (kp.N1 == NN) {                                                                                               \
+    if (kp.N1 == NN && kp.N2 == NN) {                                                                                \
         cudaError_t e = set_smem<T>((const void *)kf_plane_vloc<T, NN, NN>, smem);                                   \
         if (e != cudaSuccess) return e;                                                                              \
         kf_plane_vloc<T, NN, NN><<<grid, FFT_THREADS, smem, st>>>(kp, (const Cx<T> *)L.twx, (const Cx<T> *)L.twy,    \
@@ -1439,12 +1450,16 @@ cudaError_t launch_plane_rho(const FftLaunch &L, const void *A, int nb, int G, i
                                           : launch_plane_rho64_x<120>(L, A, nb, G, Bg, w, rho_part, st);
         if (e != cudaErrorNotSupported) return e;
     }
+    if (!(kp.N1 == 27 && kp.N2 == 27)) {
+        const cudaError_t e = launch_any_plane_rho<T>(L, A, nb, G, Bg, w, rho_part, st);
+        if (e != cudaErrorNotSupported) return e;
+    }
     PlaneSmem ps{kp.N1, kp.N2, kp.Nxa, L.Jc};
     size_t smem = ps.elems() * sizeof(Cx<T>);
-    if (kp.N1 == kp.N2) {
+    if constexpr (sizeof(T) == 8) {
         dim3 grid(kp.N3, G);
 #define PW_CASE(NN)                                                                                                  \
-    if (kp.N1 == NN) {                                                                                               \
+    if (kp.N1 == NN && kp.N2 == NN) {                                                                                \
         cudaError_t e = set_smem<T>((const void *)kf_plane_rho<T, NN, NN>, smem);                                    \
         if (e != cudaSuccess) return e;                                                                              \
         kf_plane_rho<T, NN, NN><<<grid, FFT_THREADS, smem, st>>>(kp, (const Cx<T> *)L.twx, (const Cx<T> *)L.twy,     \

@@ -36,6 +36,7 @@ struct FftLaunch {
     int Cg;                       // columns per CTA in the z passes
     int Jc;                       // y lines per x chunk in the plane passes
     int bpc = 1;                  // bands of one z-plane per CTA in the FP32 plane pass (1..3)
+    int bpc_set = 0;              // bpc if the caller set it (pw_tuning.plane_bands), else 0
 };
 
 template <typename T> cudaError_t launch_zinv(const FftLaunch &, const void *psi, int64_t ld, int nb, void *A, cudaStream_t);
@@ -43,6 +44,19 @@ template <typename T>
 cudaError_t launch_zfwd(const FftLaunch &, const void *A, const void *psi, void *Hpsi, int64_t ld, int nb, int flags,
                         cudaStream_t);
 template <typename T> cudaError_t launch_plane_vloc(const FftLaunch &, const void *Vr, void *A, int nb, cudaStream_t);
+// The plane passes for any pair of line lengths with a fused plan;
+// cudaErrorNotSupported for other lengths or when a plane does not fit in
+// shared memory.
+template <typename T> cudaError_t launch_any_plane_vloc(const FftLaunch &, const void *Vr, void *A, int nb, cudaStream_t);
+template <typename T>
+cudaError_t launch_any_plane_rho(const FftLaunch &, const void *A, int nb, int G, int Bg, const double *w, void *rho_part,
+                                 cudaStream_t);
+template <> cudaError_t launch_any_plane_vloc<float>(const FftLaunch &, const void *, void *, int, cudaStream_t);
+template <> cudaError_t launch_any_plane_vloc<double>(const FftLaunch &, const void *, void *, int, cudaStream_t);
+template <>
+cudaError_t launch_any_plane_rho<float>(const FftLaunch &, const void *, int, int, int, const double *, void *, cudaStream_t);
+template <>
+cudaError_t launch_any_plane_rho<double>(const FftLaunch &, const void *, int, int, int, const double *, void *, cudaStream_t);
 // One projector column of betaNL (PsPotNL.jl:147-195 order): its atom,
 // angular momentum l, m in [-l, l], radial index i (1-based), r_l and the
 // normalisation of eval_proj_G.
