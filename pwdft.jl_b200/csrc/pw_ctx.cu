@@ -398,17 +398,13 @@ int umma_tn(pw_ctx *c, int64_t K, int m, int n, const void *Z, int64_t ldz, cons
 }
 
 // C (M x n, complex64) (+)= A (M x k, complex64) U (k x n, complex128) on tensor cores.
-int umma_nn(pw_ctx *c, int64_t M, int n, int k, const void *A, int64_t lda, const UmmaOperand *Aprep, const double2 *U,
-            int64_t ldu, void *C, int64_t ldc, int acc) {
+int umma_nn(pw_ctx *c, int64_t M, int n, int k, const void *A, int64_t lda, const double2 *U, int64_t ldu, void *C,
+            int64_t ldc, int acc) {
     UmmaOperand Ao, B;
     int s;
-    if (Aprep) {
-        Ao = *Aprep;
-    } else {
-        if ((s = umma_scratch(c, c->um_a_hi, c->um_a_lo, 2 * M, k, Ao))) return s;
-        CK(c, umma_prep_nn_a<float2>(A, lda, M, k, Ao, c->stream));
-        c->launches += 2;
-    }
+    if ((s = umma_scratch(c, c->um_a_hi, c->um_a_lo, 2 * M, k, Ao))) return s;
+    CK(c, umma_prep_nn_a<float2>(A, lda, M, k, Ao, c->stream));
+    c->launches += 2;
     if ((s = umma_scratch(c, c->um_b_hi, c->um_b_lo, n, k, B))) return s;
     CK(c, umma_prep_tn_b<double2>(U, ldu, k, n, B, c->stream));
     if ((s = ensure(c, c->um_ws, umma_ws_bytes(Ao.rows, n, Ao.Kp, c->gemm_splits)))) return s;
@@ -426,12 +422,14 @@ int apply_T(pw_ctx *c, int ik, int ispin, const void *psi, void *Hpsi, int64_t l
     const size_t es = 2 * sizeof(T);
     cudaStream_t st = c->stream;
     const void *beta = sizeof(T) == 8 ? (const void *)kd.d_beta64 : (const void *)kd.d_beta32;
+    UmmaOperand P2op;
     if (o & PW_OP_VNL) {
         if (c->nbeta <= 0 || !beta || !c->have_D)
             return fail(c, PW_ERR_STATE, "op_V_Ps_nloc requested but the projectors of k-point %d are not set", ik);
         int s;
+        // P2 = D betaNL' psi (on the tensor-core path straight as the operand of
+        // betaNL P2 in um_b_hi/lo), the split sums of betaNL' psi read once
         const size_t pb = (size_t)c->nbeta * nb * sizeof(double2);
-        if ((s = ensure(c, c->P, pb)) || (s = ensure(c, c->P2, pb))) return s;
         if (sizeof(T) == 4 && c->use_umma) {
             // betaNL' psi cancels heavily (|beta' psi| << |beta||psi|): three
             // BF16 pieces keep its error at FP32 level; two bias <psi|V_NL|psi>
@@ -439,15 +437,25 @@ int apply_T(pw_ctx *c, int ik, int ispin, const void *psi, void *Hpsi, int64_t l
             if ((s = umma_scratch(c, c->um_b_hi, c->um_b_lo, nb, kd.Ngw, B, &c->um_b_lo2))) return s;
             CK(c, umma_prep_tn_b<float2>(psi, ld, kd.Ngw, nb, B, st));
             if ((s = ensure(c, c->um_ws, umma_ws_bytes(kd.beta_tn.rows, nb, kd.beta_tn.Kp)))) return s;
-            CK(c, umma_gemm<double2>(kd.beta_tn, B, c->nbeta, nb, c->P.p, c->nbeta, 0, (float *)c->um_ws.p, c->d_err, st));
-            c->launches += 2 + (umma_splits(kd.beta_tn.rows, nb, kd.beta_tn.Kp) > 1 ? 1 : 0);
+            CK(c, umma_gemm<double2>(kd.beta_tn, B, c->nbeta, nb, nullptr, 0, 0, (float *)c->um_ws.p, c->d_err, st));
+            if ((s = umma_scratch(c, c->um_b_hi, c->um_b_lo, nb, c->nbeta, P2op))) return s;
+            CK(c, umma_dcsr_prep((const float *)c->um_ws.p, umma_splits(kd.beta_tn.rows, nb, kd.beta_tn.Kp), c->nbeta, nb,
+                                 c->d_Drow, c->d_Dcol, c->d_Dval, P2op, st));
+            c->launches += 3;
         } else {
+            if ((s = ensure(c, c->P2, pb))) return s;
             if ((s = ensure(c, c->gemm_ws, gemm_tn_ws_bytes((int)sizeof(T), kd.Ngw, c->nbeta, nb)))) return s;
-            CK(c, (gemm_tn<T>(kd.Ngw, c->nbeta, nb, beta, kd.Ngw, psi, ld, (double2 *)c->P.p, c->nbeta, 0, c->gemm_ws.p, st)));
-            c->launches += 2;
+            if (sizeof(T) == 8) {
+                CK(c, project_dcsr(kd.Ngw, c->nbeta, nb, kd.d_beta64, (const double2 *)psi, ld, c->d_Drow, c->d_Dcol, c->d_Dval,
+                                   (double2 *)c->P2.p, c->gemm_ws.p, st));
+                c->launches += 2;
+            } else {
+                if ((s = ensure(c, c->P, pb))) return s;
+                CK(c, (gemm_tn<T>(kd.Ngw, c->nbeta, nb, beta, kd.Ngw, psi, ld, (double2 *)c->P.p, c->nbeta, 0, c->gemm_ws.p, st)));
+                CK(c, apply_dcsr(c->nbeta, nb, c->d_Drow, c->d_Dcol, c->d_Dval, (const double2 *)c->P.p, (double2 *)c->P2.p, st));
+                c->launches += 3;
+            }
         }
-        CK(c, apply_dcsr(c->nbeta, nb, c->d_Drow, c->d_Dcol, c->d_Dval, (const double2 *)c->P.p, (double2 *)c->P2.p, st));
-        c->launches += 1;
     }
     if (o & PW_OP_VLOC) {
         if (c->vloc_nspin <= 0) return fail(c, PW_ERR_STATE, "op_V_loc requested before pw_set_vloc");
@@ -478,9 +486,10 @@ int apply_T(pw_ctx *c, int ik, int ispin, const void *psi, void *Hpsi, int64_t l
     if (o & PW_OP_VNL) {
         if (sizeof(T) == 4 && c->use_umma) {
             int s;
-            if ((s = umma_nn(c, kd.Ngw, nb, c->nbeta, nullptr, 0, &kd.beta_nn, (const double2 *)c->P2.p, c->nbeta, Hpsi,
-                             ld, 1)))
-                return s;
+            if ((s = ensure(c, c->um_ws, umma_ws_bytes(kd.beta_nn.rows, nb, kd.beta_nn.Kp, c->gemm_splits)))) return s;
+            CK(c, umma_gemm<float2>(kd.beta_nn, P2op, kd.Ngw, nb, Hpsi, ld, 1, (float *)c->um_ws.p, c->d_err, st, 0, 0,
+                                    c->gemm_splits));
+            c->launches += 2;
         } else {
             CK(c, gemm_nn<T>(kd.Ngw, nb, c->nbeta, beta, kd.Ngw, (const double2 *)c->P2.p, c->nbeta, Hpsi, ld, 1, st));
             c->launches += 1;
@@ -1139,7 +1148,7 @@ extern "C" int pw_rotate(pw_ctx *c, int dtype, int64_t M, int n, int k, const vo
     if (A == C) return fail(c, PW_ERR_ARG, "A and C must not alias");
     CK(c, cudaSetDevice(c->device));
     if (dtype == PW_C64 && c->use_umma)
-        return umma_nn(c, M, n, k, A, lda, nullptr, (const double2 *)U, ldu, C, ldc, accumulate);
+        return umma_nn(c, M, n, k, A, lda, (const double2 *)U, ldu, C, ldc, accumulate);
     if (dtype == PW_C128)
         CK(c, gemm_nn<double>(M, n, k, A, lda, (const double2 *)U, ldu, C, ldc, accumulate, c->stream));
     else

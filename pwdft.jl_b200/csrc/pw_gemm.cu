@@ -368,6 +368,26 @@ __global__ void k_dcsr(int nbeta, int nb, const int *__restrict__ rowptr, const 
     }
 }
 
+// P2[b][i] = sum_j D[i][j] sum_z W[z][b][j]: the split-K sum of P = betaNL' psi and
+// D P in one pass (P itself is not needed by op_V_Ps_nloc).
+__global__ void k_dcsr_splits(int nbeta, int nb, const int *__restrict__ rowptr, const int *__restrict__ col,
+                              const double *__restrict__ val, const double2 *__restrict__ W, int S, double2 *__restrict__ P2) {
+    const size_t total = (size_t)nbeta * nb;
+    for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
+        const int b = (int)(t / nbeta), i = (int)(t - (size_t)b * nbeta);
+        double2 s = make_double2(0.0, 0.0);
+        for (int e = rowptr[i]; e < rowptr[i + 1]; ++e) {
+            const double2 *w = W + (size_t)b * nbeta + col[e];
+            double2 p = make_double2(0.0, 0.0);
+#pragma unroll 4
+            for (int z = 0; z < S; ++z) p = cadd(p, w[(size_t)z * total]);
+            s.x += val[e] * p.x;
+            s.y += val[e] * p.y;
+        }
+        P2[t] = s;
+    }
+}
+
 __global__ void k_c128_to_c64(const double2 *in, float2 *out, size_t n) {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
         out[i] = make_float2((float)in[i].x, (float)in[i].y);
@@ -455,6 +475,14 @@ template cudaError_t gemm_nn<float>(int64_t, int, int, const void *, int64_t, co
 template cudaError_t gemm_nn<double>(int64_t, int, int, const void *, int64_t, const double2 *, int64_t, void *, int64_t,
                                      int, cudaStream_t, int);
 
+cudaError_t project_dcsr(int64_t K, int nbeta, int nb, const double2 *beta, const double2 *psi, int64_t ldp, const int *rowptr,
+                         const int *col, const double *val, double2 *P2, void *ws, cudaStream_t st) {
+    const ZPlan p = zplan(K, nbeta, nb, true, 0);
+    cudaError_t e = launch_zgemm<true>(p, K, nbeta, nb, beta, K, psi, ldp, (double2 *)ws, 0, 0, 0, 0, 0, st);
+    if (e != cudaSuccess) return e;
+    k_dcsr_splits<<<blocks_for((size_t)nbeta * nb), 256, 0, st>>>(nbeta, nb, rowptr, col, val, (const double2 *)ws, p.S, P2);
+    return cudaGetLastError();
+}
 cudaError_t apply_dcsr(int nbeta, int nb, const int *rowptr, const int *col, const double *val, const double2 *P,
                        double2 *P2, cudaStream_t st) {
     k_dcsr<<<blocks_for((size_t)nbeta * nb), 256, 0, st>>>(nbeta, nb, rowptr, col, val, P, P2);

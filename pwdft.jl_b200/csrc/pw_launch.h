@@ -104,6 +104,10 @@ cudaError_t gemm_tn(int64_t K, int m, int n, const void *A, int64_t lda, const v
 template <typename T>
 cudaError_t gemm_nn(int64_t M, int n, int k, const void *A, int64_t lda, const double2 *B, int64_t ldb, void *C,
                     int64_t ldc, int accumulate, cudaStream_t, int tri = 0);
+// P2 = D (beta^H psi) in FP64 (beta K x nbeta with ld K; CSR D; P2 nbeta x nb,
+// ld = nbeta); ws as gemm_tn's (gemm_tn_ws_bytes(8, K, nbeta, nb))
+cudaError_t project_dcsr(int64_t K, int nbeta, int nb, const double2 *beta, const double2 *psi, int64_t ldp, const int *rowptr,
+                         const int *col, const double *val, double2 *P2, void *ws, cudaStream_t);
 // P2[i][b] = sum_j D[i][j] P[j][b]  (CSR D; P, P2 are nbeta x nb, ld = nbeta)
 cudaError_t apply_dcsr(int nbeta, int nb, const int *rowptr, const int *col, const double *val, const double2 *P,
                        double2 *P2, cudaStream_t);

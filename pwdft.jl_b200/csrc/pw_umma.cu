@@ -489,6 +489,39 @@ __global__ void k_finalize(const float *__restrict__ W, int S, int m, int n, CT 
     }
 }
 
+// B' of D P (the operand of betaNL (D P)) straight from the split sums W of
+// P = betaNL' psi: row b = [Re, Im] of sum_j D[i][j] sum_z W[z][b][j] along i,
+// two BF16 pieces, zero past nbeta.  One pass where finalize, D P and the
+// operand's own prep pass were three launches (about 4 us each).
+__global__ void k_dcsr_prep(const float2 *__restrict__ W, int S, int nbeta, int nb, const int *__restrict__ rowptr,
+                            const int *__restrict__ col, const double *__restrict__ val, int Kp,
+                            __nv_bfloat162 *__restrict__ hi, __nv_bfloat162 *__restrict__ lo) {
+    const int kp2 = Kp / 2;
+    const size_t total = (size_t)kp2 * nb, wz = (size_t)nbeta * nb;
+    for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
+        const int b = (int)(t / kp2), i = (int)(t - (size_t)b * kp2);
+        double re = 0.0, im = 0.0;
+        if (i < nbeta)
+            for (int e = rowptr[i]; e < rowptr[i + 1]; ++e) {
+                const float2 *w = W + (size_t)b * nbeta + col[e];
+                double pr = 0.0, pi = 0.0;
+#pragma unroll 4
+                for (int z = 0; z < S; ++z) {
+                    const float2 v = w[z * wz];
+                    pr += (double)v.x;
+                    pi += (double)v.y;
+                }
+                re += val[e] * pr;
+                im += val[e] * pi;
+            }
+        __nv_bfloat16 a[2], c[2];
+        splitn<2>((float)re, a);
+        splitn<2>((float)im, c);
+        hi[t] = __nv_bfloat162(a[0], c[0]);
+        lo[t] = __nv_bfloat162(a[1], c[1]);
+    }
+}
+
 // ------------------------------------------------------------- host side
 PFN_cuTensorMapEncodeTiled_v12000 g_encode = nullptr;
 
@@ -631,6 +664,15 @@ static cudaError_t launch_umma(const CUtensorMap *mA, const CUtensorMap *mB, dim
     return cudaGetLastError();
 }
 
+cudaError_t umma_dcsr_prep(const float *ws, int S, int nbeta, int nb, const int *rowptr, const int *col, const double *val,
+                           UmmaOperand &op, cudaStream_t st) {
+    op.rows = nb;
+    op.Kp = umma_kpad(nbeta);
+    k_dcsr_prep<<<blocks_for((size_t)op.Kp / 2 * nb), 256, 0, st>>>((const float2 *)ws, S, nbeta, nb, rowptr, col, val, op.Kp,
+                                                                   (__nv_bfloat162 *)op.hi, (__nv_bfloat162 *)op.lo);
+    return cudaGetLastError();
+}
+
 template <typename CT>
 cudaError_t umma_gemm(const UmmaOperand &A, const UmmaOperand &B, int m, int n, void *C, int64_t ldc, int accumulate,
                       float *ws, int *err, cudaStream_t st, int upper, int lolo, int splits) {
@@ -662,7 +704,7 @@ cudaError_t umma_gemm(const UmmaOperand &A, const UmmaOperand &B, int m, int n, 
     else
         e = bn == 160 ? launch_umma<2, 160>(mA, mB, grid, (int)A.rows, n, KB, kb_per, ws, err, upper, lolo, Cd, ldc, cd, accumulate, st)
                       : launch_umma<2, 128>(mA, mB, grid, (int)A.rows, n, KB, kb_per, ws, err, upper, lolo, Cd, ldc, cd, accumulate, st);
-    if (e != cudaSuccess || Cd) return e;
+    if (e != cudaSuccess || Cd || !C) return e;
     k_finalize<CT><<<blocks_for((size_t)m * n), 256, 0, st>>>(ws, S, m, n, (CT *)C, ldc, accumulate, upper);
     return cudaGetLastError();
 }

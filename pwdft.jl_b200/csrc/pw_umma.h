@@ -37,7 +37,13 @@ template <typename CT> cudaError_t umma_prep_tn_a(const void *Z, int64_t ld, int
 template <typename CT> cudaError_t umma_prep_tn_b(const void *W, int64_t ld, int64_t K, int n, UmmaOperand &, cudaStream_t);
 template <typename CT> cudaError_t umma_prep_nn_a(const void *A, int64_t lda, int64_t M, int k, UmmaOperand &, cudaStream_t);
 
+// B' operand of D P from the S split sums that umma_gemm with C == nullptr left
+// in ws (P = betaNL' psi, nbeta x nb; D as CSR)
+cudaError_t umma_dcsr_prep(const float *ws, int S, int nbeta, int nb, const int *rowptr, const int *col, const double *val,
+                           UmmaOperand &, cudaStream_t);
+
 // C (m x n complex of type CT, ldc) (+)= result; A.rows == 2m, B.rows == n.
+// C == nullptr: the split sums stay in ws ([split][n][2m] floats).
 // err: device int set non-zero if a bounded wait in the kernel expired.
 template <typename CT>
 // upper != 0: C is Hermitian and only C[i][j], i <= j, is formed and written.
