@@ -464,7 +464,9 @@ __global__ void k_zero_pad(__nv_bfloat16 *hi, __nv_bfloat16 *lo, int64_t rows, i
     }
 }
 
-// C (m x n complex, ldc) (+)= sum_z W[z]  with W[z][j][2i + {0,1}] = {Re, Im}
+// C (m x n complex, ldc) (+)= sum_z W[z]  with W[z][j][2i + {0,1}] = {Re, Im}.
+// upper: 1 = only i <= j is formed and written, 2 = only i <= j was formed
+// (Z^H Z) and the other triangle gets its conjugate.
 template <typename CT>
 __global__ void k_finalize(const float *__restrict__ W, int S, int m, int n, CT *__restrict__ C, int64_t ldc, int accumulate,
                            int upper) {
@@ -479,13 +481,12 @@ __global__ void k_finalize(const float *__restrict__ W, int S, int m, int n, CT 
             re += (double)w[0];
             im += (double)w[1];
         }
-        CT *p = C + j * ldc + i;
-        if (accumulate) {
-            re += (double)p->x;
-            im += (double)p->y;
-        }
-        p->x = re;
-        p->y = im;
+        auto put = [&](CT *p, double y) {
+            p->x = accumulate ? re + (double)p->x : re;
+            p->y = accumulate ? y + (double)p->y : y;
+        };
+        put(C + j * ldc + i, im);
+        if (upper == 2 && i < j) put(C + i * ldc + j, -im);
     }
 }
 
@@ -696,7 +697,7 @@ cudaError_t umma_gemm(const UmmaOperand &A, const UmmaOperand &B, int m, int n, 
     // one split and no accumulation: the epilogue writes C itself, no
     // workspace pass (accumulating, its read-modify-write of C measured
     // slower than the workspace + finalize pass: Si64 op_H 0.78 -> 0.95 ms)
-    void *Cd = (S == 1 && !accumulate) ? C : nullptr;
+    void *Cd = (S == 1 && !accumulate && upper != 2) ? C : nullptr;
     const int cd = sizeof(CT) == 16 ? 1 : 0;
     if (ns == 3)
         e = bn == 160 ? launch_umma<3, 160>(mA, mB, grid, (int)A.rows, n, KB, kb_per, ws, err, upper, 0, Cd, ldc, cd, accumulate, st)
