@@ -902,6 +902,7 @@ int apply_multi_T(pw_ctx *c, int nk, const int *iks, int ispin, void *const *psi
     if (vnl && c->nbeta > 2048) return fail(c, PW_ERR_UNSUPPORTED, "the batched op_V_Ps_nloc takes at most 2048 projectors");
     std::vector<MkK> tab(nk);
     std::vector<int> band_k;
+    std::vector<int2> groups;   // (k-point entry, first band) of each 16 bands: the nonlocal part's CTAs
     size_t aoff = 0;
     int maxcol = 0, maxnb = 0, kx = iks[0];
     for (int i = 0; i < nk; ++i) {
@@ -919,6 +920,7 @@ int apply_multi_T(pw_ctx *c, int nk, const int *iks, int ispin, void *const *psi
         K.nb = nb[i];
         aoff += (size_t)nb[i] * c->N3 * kd.Ncol;
         band_k.insert(band_k.end(), nb[i], i);
+        for (int b = 0; b < nb[i]; b += 16) groups.push_back(make_int2(i, b));
         maxcol = std::max(maxcol, kd.Ncol);
         maxnb = std::max(maxnb, nb[i]);
         if (kd.Nxa > c->k[kx].Nxa) kx = iks[i];
@@ -930,7 +932,8 @@ int apply_multi_T(pw_ctx *c, int nk, const int *iks, int ispin, void *const *psi
     const size_t tab_bytes = (size_t)nk * sizeof(MkK), bk_bytes = (size_t)nbands * sizeof(int);
     const size_t bk_off = (tab_bytes + 255) / 256 * 256;
     const size_t ctr_off = (bk_off + bk_bytes + 255) / 256 * 256;   // grid-barrier counter of the persistent launch
-    if ((s = ensure(c, c->mk_tab, ctr_off + 256))) return s;
+    const size_t gr_off = ctr_off + 256, gr_bytes = groups.size() * sizeof(int2);
+    if ((s = ensure(c, c->mk_tab, gr_off + gr_bytes))) return s;
     const void *V = sizeof(T) == 8 ? (const void *)(c->d_V64 + (size_t)ispin * c->N)
                                    : (const void *)(c->d_V32 + (size_t)ispin * c->N);
     const int flags = ((o & PW_OP_K) ? 2 : 0) | ((ops & PW_ACCUMULATE) ? 4 : 0);
@@ -938,6 +941,7 @@ int apply_multi_T(pw_ctx *c, int nk, const int *iks, int ispin, void *const *psi
     const MkK *d_tab = (const MkK *)c->mk_tab.p;
     const int *d_bk = (const int *)((const char *)c->mk_tab.p + bk_off);
     unsigned *d_ctr = (unsigned *)((char *)c->mk_tab.p + ctr_off);
+    const int2 *d_gr = (const int2 *)((const char *)c->mk_tab.p + gr_off);
     // graph replay: same blocks, k-points, flags and buffers as the captured call
     uint64_t key = 1469598103934665603ull;
     key = fnv(key, tab.data(), tab_bytes);
@@ -955,6 +959,7 @@ int apply_multi_T(pw_ctx *c, int nk, const int *iks, int ispin, void *const *psi
     }
     CK(c, cudaMemcpyAsync(c->mk_tab.p, tab.data(), tab_bytes, cudaMemcpyHostToDevice, c->stream));
     CK(c, cudaMemcpyAsync((char *)c->mk_tab.p + bk_off, band_k.data(), bk_bytes, cudaMemcpyHostToDevice, c->stream));
+    CK(c, cudaMemcpyAsync((char *)c->mk_tab.p + gr_off, groups.data(), gr_bytes, cudaMemcpyHostToDevice, c->stream));
     // one persistent cooperative launch for every stage (the per-stage
     // launches when it does not fit or a stream capture refuses it)
     bool persistent = (ops & PW_PERSISTENT) != 0;
@@ -973,7 +978,7 @@ int apply_multi_T(pw_ctx *c, int nk, const int *iks, int ispin, void *const *psi
         }
         nlaunch = vnl ? 4 : 3;
         return launch_multik<T>(L, d_tab, d_bk, nk, nbands, maxnb, maxcol, V, c->A.p, flags, c->d_Drow, c->d_Dcol,
-                                c->d_Dval, vnl ? c->nbeta : 0, st);
+                                c->d_Dval, vnl ? c->nbeta : 0, d_gr, (int)groups.size(), st);
     };
     CK(c, run(c->stream));
     c->launches += nlaunch;
