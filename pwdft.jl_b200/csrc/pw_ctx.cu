@@ -501,6 +501,28 @@ int apply_T(pw_ctx *c, int ik, int ispin, const void *psi, void *Hpsi, int64_t l
     return PW_OK;
 }
 
+// Band groups of the density pass: each of the N3 G CTAs takes one z-plane of
+// ceil(cnt / G) bands, two (FP32) or one (FP64) to an SM, so the time goes with
+// waves x bands per group, plus about 0.3 of a band for a CTA's set-up and
+// plane and 0.1 a group for the reduction.  (75-point grid, 41 FP64 bands: 7
+// groups run 4 x 6 bands deep, 4 groups, "enough CTAs to fill the GPU twice",
+// 3 x 11, their third wave nearly empty: 128 bands 882 -> 812 us.)
+template <typename T>
+int rho_groups(const pw_ctx *c, int cnt) {
+    const int slots = sizeof(T) == 4 ? 2 * 148 : 148;
+    int best = 1;
+    double tbest = 1e300;
+    for (int G = 1; G <= std::min(cnt, 16); ++G) {
+        const int waves = (c->N3 * G + slots - 1) / slots, Bg = (cnt + G - 1) / G;
+        const double t = waves * (Bg + 0.3) + 0.1 * G;
+        if (t < tbest) {
+            tbest = t;
+            best = G;
+        }
+    }
+    return best;
+}
+
 template <typename T>
 int rhoe_T(pw_ctx *c, int ik, const void *psi, int64_t ld, int nb, const double *w_host, double *rhoe, int accumulate) {
     const KData &kd = c->k[ik];
@@ -510,8 +532,8 @@ int rhoe_T(pw_ctx *c, int ik, const void *psi, int64_t ld, int nb, const double 
     const int nbc = band_chunk(c, ik, es, nb);
     int s;
     if ((s = ensure(c, c->A, (size_t)nbc * c->N3 * kd.Ncol * es))) return s;
-    // band groups: enough CTAs (N3 * G) to fill the GPU twice
-    int G = std::max(1, std::min(nbc, (2 * 148 + c->N3 - 1) / c->N3));
+    int G = 1;
+    for (int b0 = 0; b0 < nb; b0 += nbc) G = std::max(G, rho_groups<T>(c, std::min(nbc, nb - b0)));
     if ((s = ensure(c, c->rho_part, (size_t)G * c->N * sizeof(T)))) return s;
     if ((s = ensure(c, c->w, (size_t)nb * sizeof(double)))) return s;
     std::vector<double> wv(w_host, w_host + nb);
@@ -519,7 +541,7 @@ int rhoe_T(pw_ctx *c, int ik, const void *psi, int64_t ld, int nb, const double 
     CK(c, cudaMemcpyAsync(c->w.p, wv.data(), nb * sizeof(double), cudaMemcpyHostToDevice, st));
     for (int b0 = 0; b0 < nb; b0 += nbc) {
         const int cnt = std::min(nbc, nb - b0);
-        const int Gc = std::min(G, cnt);
+        const int Gc = rho_groups<T>(c, cnt);
         const int Bg = (cnt + Gc - 1) / Gc;
         const int Gu = (cnt + Bg - 1) / Bg;
         const char *pin = (const char *)psi + (size_t)b0 * ld * es;
