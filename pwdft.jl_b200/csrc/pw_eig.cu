@@ -10,8 +10,10 @@
 //   4. C = Linv T Linv^H                two FP64 complex GEMMs
 //   5. C = Q Tr Q^H                     Householder tridiagonalisation (LAPACK
 //                                       zhetd2 conventions: H = I - tau v v^H,
-//                                       real tridiagonal Tr), one grid barrier
-//                                       per column (cooperative kernel)
+//                                       real tridiagonal Tr): columns in
+//                                       registers up to n = 1024, above that
+//                                       in L2 with one grid barrier per
+//                                       column (cooperative kernels)
 //   6. lowest k eigenvalues of Tr       multisection on Sturm counts, one warp
 //                                       per eigenvalue; the block reflectors
 //                                       of step 8 meanwhile
@@ -509,6 +511,241 @@ k_tridiag(double2 *C, int n, double *d, double *e, double2 *tau, double2 *ybuf, 
     }
 }
 
+// The same tridiagonalisation for n <= 1024 with the trailing matrix in
+// registers (CPW columns a warp, row lane + 32 u in register u) and no grid
+// barrier.  What the CTAs exchange per column, for each column i > j its y_i =
+// (column i)^H v_j and its entry of row j + 1 (the conjugate of column j + 1, by
+// symmetry), is written once to its own place (ybuf, filled with all-ones words
+// before the launch), and every CTA reads it as soon as the words it polls are
+// there: the data is its own flag, and a column costs one store-to-load trip
+// through L2 instead of a fence, an atomic, a poll and then the loads.  A CTA's
+// values lie together and leave in one store: with eight SMs writing to a line
+// that others poll, a column took 1.5 to 3 us more.  Each thread keeps its EPT
+// elements of v_j in registers through the redundant step (y, the next column
+// and its Householder vector), which takes three block barriers.  A word that
+// stays all-ones past the poll limit sets *err, after which nobody waits long
+// any more.  Latency-bound: n = 160 / 480 / 900 take 0.54 / 1.95 / 4.72 ms, the
+// grid-barrier kernel 0.78 / 2.71 / 6.21 ms.
+__device__ __forceinline__ bool unset(double2 v) {
+    return __double_as_longlong(v.x) == -1ll || __double_as_longlong(v.y) == -1ll;
+}
+__device__ __forceinline__ double2 ld_relaxed(const double2 *p) {
+    double2 v;
+    asm volatile("ld.relaxed.gpu.global.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_relaxed(double2 *p, double2 v) {
+    // a NaN that carries the all-ones pattern would read as "not there yet"
+    if (__double_as_longlong(v.x) == -1ll) v.x = __longlong_as_double(0x7ff8000000000000ll);
+    if (__double_as_longlong(v.y) == -1ll) v.y = __longlong_as_double(0x7ff8000000000000ll);
+    asm volatile("st.relaxed.gpu.global.v2.f64 [%0], {%1, %2};" ::"l"(p), "d"(v.x), "d"(v.y) : "memory");
+}
+
+// Warp sum of a complex value: the real part in lanes 0..15, the imaginary
+// part in lanes 16..31.
+__device__ __forceinline__ double half_sums(double2 v, int lane) {
+    const double o = __shfl_xor_sync(0xffffffffu, lane < 16 ? v.y : v.x, 16);
+    double s = (lane < 16 ? v.x : v.y) + o;
+#pragma unroll
+    for (int m = 8; m > 0; m >>= 1) s += __shfl_xor_sync(0xffffffffu, s, m);
+    return s;
+}
+
+template <int NR, int W, int CPW>
+__global__ void __launch_bounds__(32 * W)
+k_tridiag_r(double2 *C, int n, double *d, double *e, double2 *tau, double2 *ybuf, int *err) {
+    constexpr int TH = 32 * W, EPT = 32 * NR / TH, NN = 32 * NR;
+    static_assert(EPT * TH == NN, "every row has a thread");
+    extern __shared__ __align__(16) unsigned char sm[];
+    double2 *vc = reinterpret_cast<double2 *>(sm), *vp = vc + NN, *wp = vp + NN;   // v_j, v_{j-1}, w_{j-1}
+    constexpr int SL = W * CPW;                      // columns of a CTA
+    __shared__ double2 ysm[2 * SL];                  // (y, row j+1 of the column) pairs
+    __shared__ double2 red[2][W + 1];               // block sums, and one broadcast value each
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const bool mute = (int)blockIdx.x == g_gsync_withhold;
+    const long long lim = g_gsync_limit;
+    // this warp's columns (rows >= its index matter)
+    int ci[CPW];
+    double2 a[CPW][NR];
+#pragma unroll
+    for (int c = 0; c < CPW; ++c) {
+        ci[c] = 1 + blockIdx.x + gridDim.x * (warp + W * c);
+#pragma unroll
+        for (int u = 0; u < NR; ++u) {
+            const int r = lane + 32 * u;
+            a[c][u] = ci[c] < n && r < n ? __ldcg(&C[(size_t)ci[c] * n + r]) : make_double2(0.0, 0.0);
+        }
+    }
+    const int ldy = gridDim.x * SL;
+    double2 x[EPT], v[EPT];                         // this thread's elements of column j+1 and of v_j
+    auto row = [&](int u) { return tid + TH * u; };
+#pragma unroll
+    for (int u = 0; u < EPT; ++u) x[u] = row(u) < n ? __ldcg(&C[row(u)]) : make_double2(0.0, 0.0);
+    // y of column i sits with its CTA's other columns: one writer a line
+    int pos[EPT];
+#pragma unroll
+    for (int u = 0; u < EPT; ++u) {
+        const int i = max(row(u) - 1, 0);
+        pos[u] = (i % gridDim.x) * SL + i / gridDim.x;
+    }
+    double2 tj = make_double2(0.0, 0.0);
+
+    // Householder vector of x = column j (rows > j) into v, vc; returns tau
+    auto householder = [&](int j) {
+        double s2 = 0.0;
+#pragma unroll
+        for (int u = 0; u < EPT; ++u) {
+            if (row(u) > j + 1) s2 += x[u].x * x[u].x + x[u].y * x[u].y;
+            if (row(u) == j + 1) red[1][W] = x[u];
+        }
+        for (int o = 16; o > 0; o >>= 1) s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+        if (lane == 0) red[1][warp].x = s2;
+        __syncthreads();
+        s2 = 0.0;
+#pragma unroll
+        for (int w = 0; w < W; ++w) s2 += red[1][w].x;
+        const double2 alpha = red[1][W];
+        double2 t = make_double2(0.0, 0.0), scal = t;
+        double beta = alpha.x;
+        if (s2 != 0.0 || alpha.y != 0.0) {
+            beta = -copysign(sqrt(alpha.x * alpha.x + alpha.y * alpha.y + s2), alpha.x);
+            const double ib = 1.0 / beta;
+            t = make_double2((beta - alpha.x) * ib, -alpha.y * ib);
+            const double ar = alpha.x - beta, ai = alpha.y, den = 1.0 / (ar * ar + ai * ai);
+            scal = make_double2(ar * den, -ai * den);
+        }
+#pragma unroll
+        for (int u = 0; u < EPT; ++u) {
+            v[u] = row(u) <= j ? make_double2(0.0, 0.0) : row(u) == j + 1 ? make_double2(1.0, 0.0) : cmul_d(x[u], scal);
+            vc[row(u)] = v[u];
+        }
+        if (blockIdx.x == 0 && tid == 0) {
+            e[j] = beta;
+            tau[j] = t;
+        }
+        __syncthreads();
+        return t;
+    };
+
+    if (blockIdx.x == 0 && tid == 0) d[0] = x[0].x;
+    if (n >= 2) tj = householder(0);
+    for (int j = 0; j < n - 1; ++j) {
+        const int c1 = j + 1;
+        double2 *yb = ybuf + (size_t)j * ldy * 2;
+        // ---- the warp's column: rank-2 update with (v_{j-1}, w_{j-1}), then y = column^H v_j
+        {
+            double2 cw[CPW], cv[CPW], acc[CPW], pick[CPW];
+            bool any = false;
+#pragma unroll
+            for (int c = 0; c < CPW; ++c) {
+                const bool on = ci[c] > j && ci[c] < n;
+                any |= on;
+                cw[c] = cv[c] = acc[c] = pick[c] = make_double2(0.0, 0.0);
+                if (on && j > 0) {
+                    cw[c] = make_double2(wp[ci[c]].x, -wp[ci[c]].y);
+                    cv[c] = make_double2(vp[ci[c]].x, -vp[ci[c]].y);
+                }
+            }
+            if (any) {
+#pragma unroll
+                for (int u = 0; u < NR; ++u) {
+                    const int r = lane + 32 * u;
+                    if (32 * u + 31 > j && 32 * u < n) {
+                        const double2 pv = vp[r], pw = wp[r], pc = vc[r];
+#pragma unroll
+                        for (int c = 0; c < CPW; ++c) {
+                            if (j > 0) {
+                                double2 &t = a[c][u];
+                                t.x = fma(-pv.x, cw[c].x, fma(pv.y, cw[c].y, fma(-pw.x, cv[c].x, fma(pw.y, cv[c].y, t.x))));
+                                t.y = fma(-pv.x, cw[c].y, fma(-pv.y, cw[c].x, fma(-pw.x, cv[c].y, fma(-pw.y, cv[c].x, t.y))));
+                            }
+                            if (u == (c1 >> 5)) pick[c] = a[c][u];
+                            if (r > j) {
+                                acc[c].x = fma(a[c][u].x, pc.x, fma(a[c][u].y, pc.y, acc[c].x));
+                                acc[c].y = fma(a[c][u].x, pc.y, fma(-a[c][u].y, pc.x, acc[c].y));
+                            }
+                        }
+                    }
+                }
+#pragma unroll
+                for (int c = 0; c < CPW; ++c) {
+                    const double h = half_sums(acc[c], lane);
+                    if ((lane & 15) == 0) (lane ? ysm[2 * (warp + W * c)].y : ysm[2 * (warp + W * c)].x) = h;
+                    if (lane == (c1 & 31)) ysm[2 * (warp + W * c) + 1] = make_double2(pick[c].x, -pick[c].y);
+                }
+            }
+        }
+        __syncthreads();
+        if (tid < 2 * SL) {
+            const int i = 1 + blockIdx.x + gridDim.x * (tid >> 1);
+            if (i > j && i < n && !mute) st_relaxed(&yb[2 * blockIdx.x * SL + tid], ysm[tid]);
+        }
+        // ---- every CTA: y and the raw column j+1, as they arrive
+        double2 y[EPT];
+#pragma unroll
+        for (int u = 0; u < EPT; ++u) {
+            const bool in = row(u) > j && row(u) < n;
+            y[u] = in ? ld_relaxed(&yb[2 * pos[u]]) : make_double2(0.0, 0.0);
+            x[u] = in ? ld_relaxed(&yb[2 * pos[u] + 1]) : make_double2(0.0, 0.0);
+        }
+        for (long long it = 0;; ++it) {
+            bool wait = false;
+#pragma unroll
+            for (int u = 0; u < EPT; ++u) {
+                if (unset(y[u])) {
+                    y[u] = ld_relaxed(&yb[2 * pos[u]]);
+                    wait = true;
+                }
+                if (unset(x[u])) {
+                    x[u] = ld_relaxed(&yb[2 * pos[u] + 1]);
+                    wait = true;
+                }
+            }
+            if (!wait) break;
+            if (it > lim) {
+                atomicExch(err, 1);
+                break;
+            }
+            if ((it & 63) == 63 && *(volatile int *)err) break;
+        }
+        // v_j to its place in C (all of column j has been read: every CTA has published this step)
+        if ((j % gridDim.x) == blockIdx.x) {
+#pragma unroll
+            for (int u = 0; u < EPT; ++u)
+                if (row(u) > c1 && row(u) < n) C[(size_t)j * n + row(u)] = v[u];
+        }
+        // w_j = tau y + alpha v_j, alpha = -tau/2 (tau y)^H v_j
+        double2 yv = make_double2(0.0, 0.0);
+#pragma unroll
+        for (int u = 0; u < EPT; ++u) {
+            y[u] = cmul_d(tj, y[u]);
+            const double2 q = cmulc_d(y[u], v[u]);
+            yv.x += q.x;
+            yv.y += q.y;
+            if (row(u) == c1) red[0][W] = y[u];
+        }
+        const double h = half_sums(yv, lane);
+        if ((lane & 15) == 0) (lane ? red[0][warp].y : red[0][warp].x) = h;
+        __syncthreads();   // also: every warp is done with vp, wp of this column's update
+        yv = make_double2(0.0, 0.0);
+#pragma unroll
+        for (int w = 0; w < W; ++w) yv = cadd(yv, red[0][w]);
+        const double2 al = cmul_d(make_double2(-0.5 * tj.x, -0.5 * tj.y), yv);
+        // column j+1 given the step-j update: x -= v conj(w_{j+1}) + w (v_{j+1} = 1)
+        const double2 wc = cadd(red[0][W], al), cw = make_double2(wc.x, -wc.y);
+#pragma unroll
+        for (int u = 0; u < EPT; ++u) {
+            const double2 w = cadd(y[u], cmul_d(al, v[u])), p = cmul_d(v[u], cw);
+            vp[row(u)] = v[u];
+            wp[row(u)] = w;
+            x[u].x -= p.x + w.x;
+            x[u].y -= p.y + w.y;
+            if (row(u) == c1 && blockIdx.x == 0) d[c1] = x[u].x;
+        }
+        if (c1 < n - 1) tj = householder(c1);
+    }
+}
+
 // Number of eigenvalues of a tridiagonal matrix below x from the signs of the
 // Sturm polynomials p_i = (d_i - x) p_{i-1} - e_{i-1}^2 p_{i-2} (a sign change
 // per eigenvalue; the quotients p_i / p_{i-1} are the pivots of LDL^T).  One
@@ -973,7 +1210,7 @@ using namespace eig;
 
 size_t eig_work_bytes(int n, int k) {
     const size_t nn = (size_t)n * n * sizeof(double2);
-    return 2 * nn                                     // L^-1, scratch n x n
+    return 2 * nn + (size_t)32 * n * sizeof(double2)  // L^-1, scratch n x n (or the tridiagonalisation's exchange)
            + (size_t)2 * n * sizeof(double2)          // y (two buffers)
            + (size_t)(3 * n) * sizeof(double)         // d, e, lam
            + (size_t)n * sizeof(double2)              // tau
@@ -1016,8 +1253,10 @@ cudaError_t hegv_lowest(double2 *T, double2 *G, int n, int k, double *lam_out, d
         return (void *)q;
     };
     const size_t nn = (size_t)n * n;
-    double2 *Linv = (double2 *)take(nn * sizeof(double2));
-    double2 *M1 = (double2 *)take(nn * sizeof(double2));
+    // L^-1 and a scratch matrix, and after them the exchange buffer of the
+    // register tridiagonalisation (n rows of pairs for at most n + 16 columns)
+    double2 *ybuf = (double2 *)take((2 * nn + 32 * (size_t)n) * sizeof(double2));
+    double2 *Linv = ybuf, *M1 = ybuf + nn;
     double2 *xg = (double2 *)take(2 * (size_t)n * sizeof(double2));
     double *d = (double *)take(n * sizeof(double));
     double *e = (double *)take(n * sizeof(double));
@@ -1046,7 +1285,22 @@ cudaError_t hegv_lowest(double2 *T, double2 *G, int n, int k, double *lam_out, d
         if ((e_ = gemm_nn<double>(n, n, n, M1, n, G, n, T, n, 0, st, 2)) != cudaSuccess) return e_;
         k_herm_upper<<<nb, 256, 0, st>>>(T, n);
     }
-    {
+    if (n <= 1024) {
+        // register-resident columns: few CTAs keep the exchange short, few
+        // columns a CTA the update (n = 160, us a column: 20 CTAs of 8 columns
+        // 3.4, 10 of 16 3.6; n = 480: 120 of 4 4.1, 60 of 8 4.5, 30 of 16 5.4)
+        const void *fn = n <= 256 ? (const void *)k_tridiag_r<8, 8, 1>
+                                  : n <= 512 ? (const void *)k_tridiag_r<16, 4, 1> : (const void *)k_tridiag_r<32, 8, 1>;
+        const int W = n <= 256 || n > 512 ? 8 : 4, sl = W;
+        const int nblk = std::max(1, (n - 1 + sl - 1) / sl);
+        if ((e_ = cudaMemsetAsync(ybuf, 0xff, (size_t)n * 2 * nblk * sl * sizeof(double2), st)) != cudaSuccess) return e_;
+        const size_t smem = 3 * (size_t)(n <= 256 ? 256 : n <= 512 ? 512 : 1024) * sizeof(double2);
+        if (smem > 48 * 1024 - 4096 &&
+            (e_ = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
+            return e_;
+        void *args[] = {(void *)&Cm, (void *)&n, (void *)&d, (void *)&e, (void *)&tau, (void *)&ybuf, (void *)&err};
+        if ((e_ = cudaLaunchCooperativeKernel(fn, nblk, 32 * W, args, smem, st)) != cudaSuccess) return e_;
+    } else {
         const size_t smem = (size_t)(3 * n + 32) * sizeof(double2);
         int nblk = 0;
         if ((e_ = coop_blocks((const void *)k_tridiag, smem, &nblk)) != cudaSuccess) return e_;
