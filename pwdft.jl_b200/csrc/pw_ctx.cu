@@ -380,23 +380,20 @@ int umma_tn(pw_ctx *c, int64_t K, int m, int n, const void *Z, int64_t ldz, cons
     UmmaOperand A, B;
     int s;
     const int same = (Z == Wm && ldz == ldw && m == n);   // Z^H Z: add the lo*lo product
-    if ((s = umma_scratch(c, c->um_a_hi, c->um_a_lo, 2 * (int64_t)m, K, A))) return s;
-    CK(c, umma_prep_tn_a<float2>(Z, ldz, K, m, A, c->stream));
+    if ((s = umma_scratch(c, c->um_a_hi, c->um_a_lo, m, K, A))) return s;
+    CK(c, umma_prep_tn<float2>(Z, ldz, K, m, A, c->stream));
     if (same) {
-        // the B' rows [Re z_j, Im z_j] of Z^H Z are the even rows of A'
         B = A;
-        B.rows = n;
-        B.rstride = 2;
         // one triangle of tiles is formed, the other filled with its conjugate
         // (Q'Q of 1440 columns over 80,797: half of 115 of 207 tiles saved)
         if (!upper) upper = 2;
     } else {
         if ((s = umma_scratch(c, c->um_b_hi, c->um_b_lo, n, K, B))) return s;
-        CK(c, umma_prep_tn_b<float2>(Wm, ldw, K, n, B, c->stream));
+        CK(c, umma_prep_tn<float2>(Wm, ldw, K, n, B, c->stream));
     }
     if ((s = ensure(c, c->um_ws, umma_ws_bytes(A.rows, n, A.Kp, c->gemm_splits, upper)))) return s;
     CK(c, umma_gemm<CT>(A, B, m, n, C, ldc, acc, (float *)c->um_ws.p, c->d_err, c->stream, upper, same, c->gemm_splits));
-    c->launches += (same ? 2 : 3) + (acc || upper == 2 || umma_splits(A.rows, n, A.Kp, c->gemm_splits, upper) > 1 ? 1 : 0);
+    c->launches += (same ? 2 : 3) + (upper == 2 || umma_splits(A.rows, n, A.Kp, c->gemm_splits, upper) > 1 ? 1 : 0);
     return PW_OK;
 }
 
@@ -405,15 +402,15 @@ int umma_nn(pw_ctx *c, int64_t M, int n, int k, const void *A, int64_t lda, cons
             int64_t ldc, int acc) {
     UmmaOperand Ao, B;
     int s;
-    if ((s = umma_scratch(c, c->um_a_hi, c->um_a_lo, 2 * M, k, Ao))) return s;
+    if ((s = umma_scratch(c, c->um_a_hi, c->um_a_lo, M, k, Ao))) return s;
     CK(c, umma_prep_nn_a<float2>(A, lda, M, k, Ao, c->stream));
-    c->launches += 2;
+    c->launches += 1;
     if ((s = umma_scratch(c, c->um_b_hi, c->um_b_lo, n, k, B))) return s;
-    CK(c, umma_prep_tn_b<double2>(U, ldu, k, n, B, c->stream));
+    CK(c, umma_prep_tn<double2>(U, ldu, k, n, B, c->stream));
     if ((s = ensure(c, c->um_ws, umma_ws_bytes(Ao.rows, n, Ao.Kp, c->gemm_splits)))) return s;
     CK(c, umma_gemm<float2>(Ao, B, (int)M, n, C, ldc, acc, (float *)c->um_ws.p, c->d_err, c->stream, 0, 0,
                             c->gemm_splits));
-    c->launches += 2 + (acc || umma_splits(Ao.rows, n, Ao.Kp, c->gemm_splits) > 1 ? 1 : 0);
+    c->launches += 2 + (umma_splits(Ao.rows, n, Ao.Kp, c->gemm_splits) > 1 ? 1 : 0);
     return PW_OK;
 }
 
@@ -438,7 +435,7 @@ int apply_T(pw_ctx *c, int ik, int ispin, const void *psi, void *Hpsi, int64_t l
             // BF16 pieces keep its error at FP32 level; two bias <psi|V_NL|psi>
             UmmaOperand B;
             if ((s = umma_scratch(c, c->um_b_hi, c->um_b_lo, nb, kd.Ngw, B, &c->um_b_lo2))) return s;
-            CK(c, umma_prep_tn_b<float2>(psi, ld, kd.Ngw, nb, B, st));
+            CK(c, umma_prep_tn<float2>(psi, ld, kd.Ngw, nb, B, st));
             if ((s = ensure(c, c->um_ws, umma_ws_bytes(kd.beta_tn.rows, nb, kd.beta_tn.Kp)))) return s;
             CK(c, umma_gemm<double2>(kd.beta_tn, B, c->nbeta, nb, nullptr, 0, 0, (float *)c->um_ws.p, c->d_err, st));
             if ((s = umma_scratch(c, c->um_b_hi, c->um_b_lo, nb, c->nbeta, P2op))) return s;
@@ -789,7 +786,7 @@ int set_beta(pw_ctx *c, int ik, int nbeta, Fill fill) {
     if (c->use_umma) {
         // split-BF16 copies of betaNL for both tensor-core products, built once
         for (UmmaOperand *op : {&kd.beta_tn, &kd.beta_nn}) {
-            const int64_t rows = (op == &kd.beta_tn) ? 2 * (int64_t)nbeta : 2 * (int64_t)kd.Ngw;
+            const int64_t rows = (op == &kd.beta_tn) ? (int64_t)nbeta : (int64_t)kd.Ngw;
             const int64_t K = (op == &kd.beta_tn) ? kd.Ngw : nbeta;
             if (!op->hi) {
                 const size_t half = umma_operand_bytes(rows, K) / 2;
@@ -799,7 +796,7 @@ int set_beta(pw_ctx *c, int ik, int nbeta, Fill fill) {
                 if (op == &kd.beta_tn && (s = dalloc(c, (unsigned char **)&op->lo2, half))) return s;
             }
         }
-        CK(c, umma_prep_tn_a<float2>(kd.d_beta32, kd.Ngw, kd.Ngw, nbeta, kd.beta_tn, c->stream));
+        CK(c, umma_prep_tn<float2>(kd.d_beta32, kd.Ngw, kd.Ngw, nbeta, kd.beta_tn, c->stream));
         CK(c, umma_prep_nn_a<float2>(kd.d_beta32, kd.Ngw, kd.Ngw, nbeta, kd.beta_nn, c->stream));
     }
     CK(c, cudaStreamSynchronize(c->stream));
@@ -1341,7 +1338,7 @@ int pwk_beta_dot(pw_ctx *c, int ik, int dtype, const void *psi, int64_t ld, int 
     if (dtype == PW_C64 && c->use_umma) {
         UmmaOperand B;
         if ((s = umma_scratch(c, c->um_b_hi, c->um_b_lo, nb, kd.Ngw, B, &c->um_b_lo2))) return s;
-        CK(c, umma_prep_tn_b<float2>(psi, ld, kd.Ngw, nb, B, st));
+        CK(c, umma_prep_tn<float2>(psi, ld, kd.Ngw, nb, B, st));
         if ((s = ensure(c, c->um_ws, umma_ws_bytes(kd.beta_tn.rows, nb, kd.beta_tn.Kp)))) return s;
         CK(c, umma_gemm<double2>(kd.beta_tn, B, c->nbeta, nb, out, c->nbeta, 0, (float *)c->um_ws.p, c->d_err, st));
         c->launches += 2 + (umma_splits(kd.beta_tn.rows, nb, kd.beta_tn.Kp) > 1 ? 1 : 0);

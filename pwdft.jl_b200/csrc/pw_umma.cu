@@ -8,28 +8,36 @@
 //   X'HX, Q'HQ, Q'Q    (diag_LOBPCG.jl:85,183-184)   Z = Q,       W = HQ / Q
 //   A*U                (diag_LOBPCG.jl:188-194,
 //                       op_V_Ps_nloc.jl:59-76)       Z = A^H,     W = U
-// and embedded as one real GEMM  D (2m x n) = A' B'^T  over K' = 2K with
-//   A' row 2i   = [Re z_i, Im z_i] interleaved along K   (z_i = column i of Z)
-//   A' row 2i+1 = [-Im z_i, Re z_i]                       (= i z_i)
-//   B' row j    = [Re w_j, Im w_j]
-// so that D[2i, j] = Re C(i, j) and D[2i+1, j] = Im C(i, j): D stored column-
-// major IS the interleaved complex C.
+// and formed as two real products over the real and imaginary parts,
+//   Re C = Zr' Wr + Zi' Wi,   Im C = Zr' Wi - Zi' Wr.
+// An operand row (one column of Z or W) holds its values along K in blocks of
+// 32: 32 real parts, then 32 imaginary parts, one 128-byte swizzle row of BF16
+// a block.  A k-block of Z and W in shared memory then serves both
+// accumulators: Re C takes the parts as they lie, Im C pairs each half with
+// the other half of W (the Zi half with a negated A operand), so each byte
+// loaded feeds two products.  (Rows [Re, Im] and [-Im, Re] of one real GEMM of
+// twice the rows, the form before this, load and store every Z value twice:
+// betaNL P of 216 atoms and 480 bands ran at 75 loaded bytes a clock and SM,
+// 0.91 of 1.38 PFLOP/s; this form loads 43.)  Measured: Q'HQ, Q'Q and Q U of
+// 480 bands over 80,797 plane waves 11.0 -> 9.6 ms, op_H of 64 atoms (160 bands)
+// 720 -> 694 us, of 216 atoms (480 bands) 8.86 -> 8.55 ms.
 //
 // Precision: split BF16 x 3.  Each FP32 operand x = hi + lo with
-// hi = bf16(x), lo = bf16(x - hi); A'B'^T ~ hi*hi + hi*lo + lo*hi, all three
+// hi = bf16(x), lo = bf16(x - hi); Z'W ~ hi*hi + hi*lo + lo*hi, all three
 // accumulated in the same FP32 TMEM accumulator (relative error ~2^-17 per
 // product, then FP32 accumulation).  The "prep" kernels below write the
-// K-major BF16 hi/lo operands (transposing where Z = A^H) so that the MMA
-// kernel only ever sees K-major A and B.
+// K-major BF16 pieces (transposing where Z = A^H) so that the MMA kernel only
+// ever sees K-major operands.
 //
-// MMA kernel: 128 x 128 output tile per CTA, BK = 64 (one 128-byte swizzle
-// row of BF16), 3-stage TMA -> MMA pipeline on mbarriers, split-K over
-// gridDim.z into an FP32 workspace, then a finalize kernel that sums the
-// splits and writes the complex result (FP32 or FP64, overwrite or add).
+// MMA kernel: 128 x BN complex output tile per CTA, k-blocks of 32 complex
+// values, 2-3 stage TMA -> MMA pipeline on mbarriers, split-K over gridDim.z
+// into an FP32 workspace, then a finalize kernel that sums the splits and
+// writes the complex result (FP32 or FP64, overwrite or add); a single split
+// goes through shared memory straight into C.
 // Warp roles: warp 0 = TMA producer, warp 1 = TMEM owner + MMA issuer,
-// warps 2..5 = epilogue (TMEM -> registers -> global).  Every mbarrier wait
-// is bounded; on expiry the CTA records an error code and returns after
-// releasing its TMEM.
+// warps 2..5 = epilogue of Re C, warps 6..9 of Im C (TMEM -> registers ->
+// global).  Every mbarrier wait is bounded; on expiry the CTA records an error
+// code and returns after releasing its TMEM.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cudaTypedefs.h>
@@ -40,44 +48,39 @@
 namespace pwk {
 namespace umma {
 
-constexpr int BM = 128, BK = 64;
+constexpr int BM = 128, BK = 64;            // complex rows of a tile; BF16 values of a k-block row (32 Re, 32 Im)
 constexpr int TILE_A_BYTES = BM * BK * 2;   // 16 KB per A operand tile
-constexpr int THREADS = 192;
+constexpr int THREADS = 320;
 constexpr long long WAIT_LIMIT = 1ll << 26;
 constexpr int MAX_STAGES = 3;
-// k-blocks accumulated in one TMEM tile before the epilogue drains it (each
-// tile is one accumulation chain of the tensor core's truncating FP32 adds;
-// measured: 2 to 8 k-blocks per chain gain at most 6 % on the Si216 Gram and
-// bias its diagonal by -6e-7 to -3e-6, one k-block by -1e-7)
-#ifndef PW_UMMA_CHAIN
-#define PW_UMMA_CHAIN 1
-#endif
-constexpr int CHAIN = PW_UMMA_CHAIN;
 
 // NS = number of BF16 pieces per FP32 value: 2 (hi, lo: 3 products, ~2^-17)
 // or 3 (hi, mid, lo: 6 products, ~2^-24, for products with heavy
 // cancellation such as betaNL' psi).  BN = output tile width (complex
-// columns): 128, or 160 when it pads n less (n = 160, 480, 1440 bands: one
-// MMA of N = 160 instead of two of N = 128 with 96 columns of padding, and
-// the A tiles read once per 160 columns).  Stages: as many as fit in 227 KB.
+// columns).  Stages: as many as fit in 225 KB.
 template <int NS, int BN> struct Cfg {
-    static_assert(BN % 32 == 0 && BN >= 32 && BN <= 256, "tcgen05 N for M = 128, whole 32-column TMEM loads");
+    static_assert(BN % 16 == 0 && BN >= 16 && BN <= 128, "tcgen05 N for M = 128; four accumulators in 512 TMEM columns");
     static constexpr int TILE_B_BYTES = BN * BK * 2;
     static constexpr int STAGE_BYTES = NS * (TILE_A_BYTES + TILE_B_BYTES);
     static constexpr int STAGES = (225 * 1024) / STAGE_BYTES < MAX_STAGES ? (225 * 1024) / STAGE_BYTES : MAX_STAGES;
     static_assert(STAGES >= 2, "at least a double-buffered pipeline");
-    // two accumulator tiles (double buffer), allocation a power of two >= 32
-    static constexpr uint32_t TMEM_COLS = 2 * BN <= 256 ? 256u : 512u;
-    // kind::f16, A = B = BF16, D = F32, both K-major, M = 128, N = BN
+    // the epilogue's copy of the tile (BN columns of BM + 1 complex values) reuses the stages
+    static_assert((size_t)BN * (BM + 1) * 8 <= (size_t)STAGES * STAGE_BYTES, "output tile fits the stages");
+    // Re and Im accumulators, double-buffered, each from a multiple of 32
+    // columns on; allocation a power of two >= 32
+    static constexpr int ACC = (BN + 31) / 32 * 32;
+    static constexpr uint32_t TMEM_COLS = 4 * ACC <= 128 ? 128u : 4 * ACC <= 256 ? 256u : 512u;
+    // kind::f16, A = B = BF16, D = F32, both K-major, M = 128, N = BN; NEG: A negated
     static constexpr uint32_t IDESC =
         (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+    static constexpr uint32_t NEG = 1u << 13;
 };
 
 struct __align__(8) Bars {
     uint64_t full[MAX_STAGES];
     uint64_t empty[MAX_STAGES];
-    uint64_t tfull[2];    // accumulator tile b holds a finished k-block
-    uint64_t tempty[2];   // the epilogue has drained accumulator tile b
+    uint64_t tfull[2];    // accumulator pair b holds a finished k-block
+    uint64_t tempty[2];   // the epilogue has drained accumulator pair b
     uint32_t tmem_base;
     int failed;
 };
@@ -134,50 +137,44 @@ __device__ __forceinline__ void mma_commit(uint64_t *bar) {
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float *v) {
-    uint32_t r[32];
+// 16 consecutive TMEM columns of this thread's lane (wait before use)
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
     asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,"
-        "%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-          "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-          "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
         : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
+__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
-// D (Mp x Np) = sum over the split's k-blocks of the piece products
-//   NS = 2:  A0 B0^T + A0 B1^T + A1 B0^T
-//   NS = 3:  A0 B0^T + A0 B1^T + A1 B0^T + A0 B2^T + A1 B1^T + A2 B0^T
-// written to W[z][n][m] (fp32, column-major, ld = Mp), or, with a single
-// split (gridDim.z == 1) and C given, straight into the complex result C
-// (element (i, j) at C[j ldc + i], rows 2i and 2i + 1 of D its real and
-// imaginary parts; cdouble: C is complex128; accumulate: C += D; upper: only
+// C (m x n complex) = sum over the split's k-blocks of the piece products
+//   NS = 2:  A0 B0 + A0 B1 + A1 B0
+//   NS = 3:  A0 B0 + A0 B1 + A1 B0 + A0 B2 + A1 B1 + A2 B0
+// written to W[z][n][m] (float2, column-major, ld = m), or, with a single
+// split (gridDim.z == 1) and C given, into the result C (element (i, j) at
+// C[j ldc + i]; cdouble: C is complex128; accumulate: C += D; upper: only
 // i <= j written).
 template <int NS, int BN>
 __global__ void __launch_bounds__(THREADS, 1)
 k_umma_gemm(const __grid_constant__ CUtensorMap tA0, const __grid_constant__ CUtensorMap tA1,
             const __grid_constant__ CUtensorMap tA2, const __grid_constant__ CUtensorMap tB0,
-            const __grid_constant__ CUtensorMap tB1, const __grid_constant__ CUtensorMap tB2, int Mp, int Np, int KB,
-            int kb_per, float *__restrict__ W, int *__restrict__ err, int upper, int lolo, void *__restrict__ C,
+            const __grid_constant__ CUtensorMap tB1, const __grid_constant__ CUtensorMap tB2, int M, int N, int KB,
+            int kb_per, float2 *__restrict__ W, int *__restrict__ err, int upper, int lolo, void *__restrict__ C,
             int64_t ldc, int cdouble, int accumulate) {
     using CF = Cfg<NS, BN>;
     constexpr int STAGES = CF::STAGES;
     constexpr int STAGE_BYTES = CF::STAGE_BYTES;
     constexpr int TB = CF::TILE_B_BYTES;
     constexpr int TA = TILE_A_BYTES;
+    const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
     // upper: C = Z^H W is Hermitian and only its upper triangle is read; a
-    // tile whose complex rows (m0/2 ..) all lie below its columns is skipped
-    // before any barrier or TMEM allocation
-    if (upper && (int)(blockIdx.x * BM) / 2 > (int)(blockIdx.y * BN) + BN - 1) return;
+    // tile whose rows all lie below its columns is skipped before any barrier
+    // or TMEM allocation
+    if (upper && m0 > n0 + BN - 1) return;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char *smem = (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     Bars *bars = reinterpret_cast<Bars *>(smem + (size_t)STAGES * STAGE_BYTES);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
     const int kb0 = blockIdx.z * kb_per;
     const int kb1 = min(KB, kb0 + kb_per);
     const int nkb = max(0, kb1 - kb0);
@@ -189,7 +186,7 @@ k_umma_gemm(const __grid_constant__ CUtensorMap tA0, const __grid_constant__ CUt
         }
         for (int b = 0; b < 2; ++b) {
             mbar_init(&bars->tfull[b], 1);
-            mbar_init(&bars->tempty[b], 4);   // one arrival per epilogue warp
+            mbar_init(&bars->tempty[b], 8);   // one arrival per epilogue warp
         }
         bars->failed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -202,7 +199,7 @@ k_umma_gemm(const __grid_constant__ CUtensorMap tA0, const __grid_constant__ CUt
     fence_before();
     __syncthreads();
     fence_after();
-    const uint32_t tmem = bars->tmem_base;
+    const uint32_t tmem = bars->tmem_base;   // columns: [pair 0: Re, Im][pair 1: Re, Im], ACC each
 
     if (warp == 0 && lane == 0) {
         // ---------------- TMA producer
@@ -230,63 +227,74 @@ k_umma_gemm(const __grid_constant__ CUtensorMap tA0, const __grid_constant__ CUt
             if (!mbar_wait(&bars->full[s], (uint32_t)((i / STAGES) & 1))) bars->failed = 1;
         }
     } else if (warp == 1 && lane == 0) {
-        // ---------------- MMA issuer: every CHAIN k-blocks accumulate into a
-        // fresh TMEM tile (b = chain & 1), within a k-block the correction
-        // products first and the main product last, so that the tensor
-        // core's truncating FP32 accumulation touches each value only a few
-        // times; the epilogue sums the tiles with round-to-nearest adds
+        // ---------------- MMA issuer: every k-block accumulates into a fresh
+        // pair of TMEM tiles, the correction products first and the main
+        // product last, so that the tensor core's truncating FP32 accumulation
+        // touches each value only a few times; the epilogue sums the tiles
+        // with round-to-nearest adds (chains of 2 to 8 k-blocks gain at most
+        // 6 % and bias the Gram diagonal by -6e-7 to -3e-6, one by -1e-7)
         for (int i = 0; i < nkb; ++i) {
             const int s = i % STAGES;
             const uint32_t ph = (uint32_t)((i / STAGES) & 1);
-            const int ch = i / CHAIN;
-            const bool first = i % CHAIN == 0;
-            const int b = ch & 1;
-            const uint32_t tu = (uint32_t)((ch >> 1) & 1);
-            if ((first && !mbar_wait(&bars->tempty[b], tu ^ 1)) || !mbar_wait(&bars->full[s], ph)) {
+            const int b = i & 1;
+            const uint32_t tu = (uint32_t)((i >> 1) & 1);
+            if (!mbar_wait(&bars->tempty[b], tu ^ 1) || !mbar_wait(&bars->full[s], ph)) {
                 bars->failed = 1;
                 break;
             }
             fence_after();
             const uint32_t base = su32(smem + (size_t)s * STAGE_BYTES);
-            const uint32_t d = tmem + (uint32_t)(b * BN);
-            constexpr uint32_t ID = CF::IDESC;
 #pragma unroll
-            for (int kk = 0; kk < BK / 16; ++kk) {
-                const uint32_t off = kk * 32;
-                const uint64_t a0 = sdesc(base + off), a1 = sdesc(base + TA + off);
-                const uint64_t b0 = sdesc(base + NS * TA + off), b1 = sdesc(base + NS * TA + TB + off);
-                const bool fresh = first && kk == 0;
-                // lolo (two pieces, A and B the same block): the lo*lo term
-                // too, whose omission would bias every |z|^2 on the diagonal low
-                if (NS == 2 && lolo) mma_bf16(d, a1, b1, ID, fresh ? 0u : 1u);
-                mma_bf16(d, a0, b1, ID, (!fresh || (NS == 2 && lolo)) ? 1u : 0u);
-                mma_bf16(d, a1, b0, ID, 1u);
-                if constexpr (NS == 3) {
-                    const uint64_t a2 = sdesc(base + 2 * TA + off), b2 = sdesc(base + NS * TA + 2 * TB + off);
-                    mma_bf16(d, a0, b2, ID, 1u);
-                    mma_bf16(d, a1, b1, ID, 1u);
-                    mma_bf16(d, a2, b0, ID, 1u);
+            for (int part = 0; part < 2; ++part) {
+                const uint32_t d = tmem + (uint32_t)((2 * b + part) * CF::ACC);
+                // 16-value step kk of A (0, 1: Re, 2, 3: Im) against kk of B for
+                // Re C, against the other half for Im C (Zi Wr negated)
+                auto da = [&](int q, int kk) { return sdesc(base + q * TA + kk * 32); };
+                auto db = [&](int q, int kk) { return sdesc(base + NS * TA + q * TB + (part ? kk ^ 2 : kk) * 32); };
+#pragma unroll
+                for (int kk = 0; kk < BK / 16; ++kk) {
+                    const uint32_t ID = CF::IDESC | (part && kk >= 2 ? CF::NEG : 0u);
+                    // lolo (two pieces, A and B the same block): the lo*lo term
+                    // too, whose omission would bias every |z|^2 on the diagonal low
+                    if (NS == 2 && lolo) mma_bf16(d, da(1, kk), db(1, kk), ID, kk > 0 ? 1u : 0u);
+                    mma_bf16(d, da(0, kk), db(1, kk), ID, (kk > 0 || (NS == 2 && lolo)) ? 1u : 0u);
+                    mma_bf16(d, da(1, kk), db(0, kk), ID, 1u);
+                    if constexpr (NS == 3) {
+                        mma_bf16(d, da(0, kk), db(2, kk), ID, 1u);
+                        mma_bf16(d, da(1, kk), db(1, kk), ID, 1u);
+                        mma_bf16(d, da(2, kk), db(0, kk), ID, 1u);
+                    }
                 }
-            }
 #pragma unroll
-            for (int kk = 0; kk < BK / 16; ++kk) {
-                const uint32_t off = kk * 32;
-                mma_bf16(d, sdesc(base + off), sdesc(base + NS * TA + off), ID, 1u);
+                for (int kk = 0; kk < BK / 16; ++kk)
+                    mma_bf16(d, da(0, kk), db(0, kk), CF::IDESC | (part && kk >= 2 ? CF::NEG : 0u), 1u);
             }
             mma_commit(&bars->empty[s]);
-            if (i % CHAIN == CHAIN - 1 || i == nkb - 1) mma_commit(&bars->tfull[b]);
+            mma_commit(&bars->tfull[b]);
         }
     } else if (warp >= 2) {
-        // ---------------- epilogue: TMEM lanes [32q, 32q+32) -> rows m0 + 32q + lane,
-        // the chain tiles summed in registers
-        const int q = warp & 3;
-        const int m = m0 + 32 * q + lane;
+        // ---------------- epilogue: warps 2..5 Re C, 6..9 Im C; TMEM lanes
+        // [32q, 32q+32) (q = warp mod 4) -> rows m0 + 32q + lane, the k-blocks'
+        // tiles summed in registers
+        const int q = warp & 3, part = warp >= 6 ? 1 : 0;
+        const int ml = 32 * q + lane;
+        // the values to add to, on their way to L2 while the products run (the
+        // epilogue has no other CTA on its SM to hide behind: betaNL P of 216
+        // atoms took 1.51 ms with plain loads at the end)
+        const bool direct = gridDim.z == 1 && C;
+        if (direct && accumulate) {
+            const int es = cdouble ? 16 : 8, rows = 128 / es, lines = BM / rows;
+            for (int e = threadIdx.x - 64; e < BN * lines; e += 256) {
+                const int n = n0 + e / lines, i = m0 + (e % lines) * rows;
+                if (n < N && i < M)
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"((const char *)C + ((size_t)n * ldc + i) * es));
+            }
+        }
         float acc[BN];
 #pragma unroll
         for (int t = 0; t < BN; ++t) acc[t] = 0.f;
         bool ok = true;
-        const int nch = (nkb + CHAIN - 1) / CHAIN;
-        for (int i = 0; i < nch; ++i) {
+        for (int i = 0; i < nkb; ++i) {
             const int b = i & 1;
             const uint32_t tu = (uint32_t)((i >> 1) & 1);
             if (!mbar_wait(&bars->tfull[b], tu)) {
@@ -294,51 +302,66 @@ k_umma_gemm(const __grid_constant__ CUtensorMap tA0, const __grid_constant__ CUt
                 break;
             }
             fence_after();
+            const uint32_t ta = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)((2 * b + part) * CF::ACC);
+            // two 16-column loads in flight
 #pragma unroll
-            for (int c = 0; c < BN / 32; ++c) {
-                float v[32];
-                tmem_ld32(tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(b * BN + 32 * c), v);
+            for (int c = 0; c < BN / 16; c += 2) {
+                uint32_t r0[16], r1[16];
+                tmem_ld16(ta + 16 * c, r0);
+                if (c + 1 < BN / 16) tmem_ld16(ta + 16 * (c + 1), r1);
+                tmem_wait_ld();
 #pragma unroll
-                for (int t = 0; t < 32; ++t) acc[32 * c + t] += v[t];
+                for (int t = 0; t < 16; ++t) acc[16 * c + t] += __uint_as_float(r0[t]);
+                if (c + 1 < BN / 16) {
+#pragma unroll
+                    for (int t = 0; t < 16; ++t) acc[16 * (c + 1) + t] += __uint_as_float(r1[t]);
+                }
             }
             fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&bars->tempty[b]);
         }
         if (!ok) atomicExch(err, 2);
-        if (m < Mp) {
-            if (gridDim.z == 1 && C) {
-                // lanes hold consecutive rows of D = alternating Re / Im of
-                // consecutive complex rows: coalesced component stores
-                const int i = m >> 1, part = m & 1;
-                if (cdouble) {
-                    double *Cd = (double *)C;
+        // the tile through shared memory (every MMA has completed: the stages
+        // are free), so that complex values leave in runs along the rows
+        float *T = reinterpret_cast<float *>(smem);
 #pragma unroll
-                    for (int t = 0; t < BN; ++t) {
-                        const int n = n0 + t;
-                        if (n < Np && !(upper && i > n)) {
-                            double *p = Cd + 2 * ((size_t)n * ldc + i) + part;
-                            *p = accumulate ? *p + (double)acc[t] : (double)acc[t];
-                        }
-                    }
-                } else {
-                    float *Cf = (float *)C;
+        for (int t = 0; t < BN; ++t) T[2 * (t * (BM + 1) + ml) + part] = acc[t];
+        asm volatile("bar.sync 1, 256;" ::: "memory");   // the eight epilogue warps
+        const float2 *T2 = reinterpret_cast<const float2 *>(smem);
+        float2 *Wz = W + (size_t)blockIdx.z * M * (size_t)N;
+        // eight values a thread and round, the old ones loaded together
+        static_assert(BN * BM % (256 * 8) == 0, "whole rounds");
+#pragma unroll 1
+        for (int e0 = threadIdx.x - 64; e0 < BN * BM; e0 += 256 * 8) {
+            float2 v[8], o[8];
+            double2 od[8];
+            size_t at[8];
+            bool in[8];
 #pragma unroll
-                    for (int t = 0; t < BN; ++t) {
-                        const int n = n0 + t;
-                        if (n < Np && !(upper && i > n)) {
-                            float *p = Cf + 2 * ((size_t)n * ldc + i) + part;
-                            *p = accumulate ? *p + acc[t] : acc[t];
-                        }
-                    }
+            for (int u = 0; u < 8; ++u) {
+                const int e = e0 + 256 * u, i = m0 + e % BM, n = n0 + e / BM;
+                v[u] = T2[(e / BM) * (BM + 1) + e % BM];
+                in[u] = i < M && n < N && !(direct && upper && i > n);
+                at[u] = (size_t)n * (direct ? ldc : (int64_t)M) + i;
+                o[u] = make_float2(0.f, 0.f);
+                od[u] = make_double2(0.0, 0.0);
+                if (direct && accumulate && in[u]) {
+                    if (cdouble)
+                        od[u] = ((const double2 *)C)[at[u]];
+                    else
+                        o[u] = ((const float2 *)C)[at[u]];
                 }
-            } else {
-                float *Wz = W + (size_t)blockIdx.z * Mp * (size_t)Np;
+            }
 #pragma unroll
-                for (int t = 0; t < BN; ++t) {
-                    const int n = n0 + t;
-                    if (n < Np) Wz[(size_t)n * Mp + m] = acc[t];
-                }
+            for (int u = 0; u < 8; ++u) {
+                if (!in[u]) continue;
+                if (!direct)
+                    Wz[at[u]] = v[u];
+                else if (cdouble)
+                    ((double2 *)C)[at[u]] = make_double2(od[u].x + (double)v[u].x, od[u].y + (double)v[u].y);
+                else
+                    ((float2 *)C)[at[u]] = make_float2(o[u].x + v[u].x, o[u].y + v[u].y);
             }
         }
     }
@@ -364,63 +387,47 @@ template <int NS> __device__ __forceinline__ void splitn(float x, __nv_bfloat16 
     if constexpr (NS == 3) p[2] = __float2bfloat16_rn(r - __bfloat162float(p[1]));
 }
 
-// A' from Z (K x m, complex, column-major, ld): rows 2i, 2i+1 of length Kp,
-// one array per BF16 piece (pc[0..NS-1]).
+// position of the real part of value k in an operand row (its imaginary part
+// 32 further on)
+__host__ __device__ constexpr int64_t kpos(int64_t k) { return (k >> 5) * 64 + (k & 31); }
+
+// Operand rows from the columns of Z (K x m, complex, column-major, ld), one
+// array of m rows per BF16 piece (pc[0..NS-1]); two values a thread.
 template <typename CT, int NS>
-__global__ void k_prep_tn_a(const CT *__restrict__ Z, int64_t ld, int64_t K, int m, int Kp, __nv_bfloat16 *__restrict__ p0,
-                            __nv_bfloat16 *__restrict__ p1, __nv_bfloat16 *__restrict__ p2) {
-    const int i = blockIdx.y;
-    const CT *z = Z + (size_t)i * ld;
+__global__ void k_prep_tn(const CT *__restrict__ Z, int64_t ld, int64_t K, int m, int Kp, __nv_bfloat16 *__restrict__ p0,
+                          __nv_bfloat16 *__restrict__ p1, __nv_bfloat16 *__restrict__ p2) {
     __nv_bfloat16 *pc[3] = {p0, p1, p2};
-    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < Kp / 2; k += (int64_t)gridDim.x * blockDim.x) {
-        float re = 0.f, im = 0.f;
-        if (k < K) {
-            re = (float)z[k].x;
-            im = (float)z[k].y;
-        }
-        __nv_bfloat16 a[3], c[3];
-        splitn<NS>(re, a);
-        splitn<NS>(im, c);
+    for (int i = blockIdx.y; i < m; i += gridDim.y) {
+        const CT *z = Z + (size_t)i * ld;
+        for (int64_t k = 2 * (blockIdx.x * (int64_t)blockDim.x + threadIdx.x); k < Kp / 2;
+             k += 2 * (int64_t)gridDim.x * blockDim.x) {
+            float re[2], im[2];
 #pragma unroll
-        for (int q = 0; q < NS; ++q) {
-            __nv_bfloat16 *r0 = pc[q] + (size_t)(2 * i) * Kp, *r1 = r0 + Kp;
-            r0[2 * k] = a[q];
-            r0[2 * k + 1] = c[q];
-            r1[2 * k] = __hneg(c[q]);  // i z = (-im, re)
-            r1[2 * k + 1] = a[q];
+            for (int u = 0; u < 2; ++u) {
+                const bool in = k + u < K;
+                re[u] = in ? (float)z[k + u].x : 0.f;
+                im[u] = in ? (float)z[k + u].y : 0.f;
+            }
+            __nv_bfloat16 a[2][3], c[2][3];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                splitn<NS>(re[u], a[u]);
+                splitn<NS>(im[u], c[u]);
+            }
+            const size_t o = (size_t)i * Kp + kpos(k);
+#pragma unroll
+            for (int q = 0; q < NS; ++q) {
+                *reinterpret_cast<__nv_bfloat162 *>(pc[q] + o) = __nv_bfloat162(a[0][q], a[1][q]);
+                *reinterpret_cast<__nv_bfloat162 *>(pc[q] + o + 32) = __nv_bfloat162(c[0][q], c[1][q]);
+            }
         }
     }
 }
 
-// B' from W (K x n, complex, column-major, ld): row j = [Re w_j, Im w_j].
-template <typename CT, int NS>
-__global__ void k_prep_tn_b(const CT *__restrict__ Wm, int64_t ld, int64_t K, int n, int Kp, __nv_bfloat16 *__restrict__ p0,
-                            __nv_bfloat16 *__restrict__ p1, __nv_bfloat16 *__restrict__ p2) {
-    const int j = blockIdx.y;
-    const CT *w = Wm + (size_t)j * ld;
-    __nv_bfloat16 *pc[3] = {p0, p1, p2};
-    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < Kp / 2; k += (int64_t)gridDim.x * blockDim.x) {
-        float re = 0.f, im = 0.f;
-        if (k < K) {
-            re = (float)w[k].x;
-            im = (float)w[k].y;
-        }
-        __nv_bfloat16 a[3], c[3];
-        splitn<NS>(re, a);
-        splitn<NS>(im, c);
-#pragma unroll
-        for (int q = 0; q < NS; ++q) {
-            __nv_bfloat16 *r = pc[q] + (size_t)j * Kp;
-            r[2 * k] = a[q];
-            r[2 * k + 1] = c[q];
-        }
-    }
-}
-
-// A' for Z = A^H, A (M x k complex, column-major, lda): row 2g = [Re, Im] of
-// conj(A[g, :]) = [Ar, -Ai]; row 2g+1 = i conj(A[g, :]) = [Ai, Ar].  The
-// 32 x 32 tile is transposed through shared memory so both the read of A
-// (along g) and the write of A' (along l) are coalesced.
+// Operand rows for Z = A^H, A (M x k complex, column-major, lda): row g = [Re,
+// Im] of conj(A[g, :]) = [Ar, -Ai], zero past k.  A 32 x 32 tile is transposed
+// through shared memory: A is read along g, and a warp writes the 128-byte
+// block of one row.
 template <typename CT>
 __global__ void k_prep_nn_a(const CT *__restrict__ A, int64_t lda, int64_t M, int k, int Kp, __nv_bfloat16 *__restrict__ hi,
                             __nv_bfloat16 *__restrict__ lo) {
@@ -436,50 +443,37 @@ __global__ void k_prep_nn_a(const CT *__restrict__ A, int64_t lda, int64_t M, in
         tile[r][tx] = v;  // tile[l][g]
     }
     __syncthreads();
+    // lanes 0..15: real parts of l0 + 2 lane, + 1; lanes 16..31: minus the imaginary parts
+    const int l2 = 2 * (tx & 15);
     for (int r = ty; r < 32; r += 8) {
         const int64_t g = g0 + r;
-        const int l = l0 + tx;
-        if (g >= M || 2 * l >= Kp) continue;
-        const float2 v = tile[tx][r];
+        if (g >= M) continue;
+        const float2 u = tile[l2][r], v = tile[l2 + 1][r];
         __nv_bfloat16 a, b, c, d;
-        split2(v.x, a, b);
-        split2(v.y, c, d);
-        __nv_bfloat16 *h0 = hi + (size_t)(2 * g) * Kp, *h1 = h0 + Kp;
-        __nv_bfloat16 *q0 = lo + (size_t)(2 * g) * Kp, *q1 = q0 + Kp;
-        h0[2 * l] = a; q0[2 * l] = b;                 // Re conj = Ar
-        h0[2 * l + 1] = __hneg(c); q0[2 * l + 1] = __hneg(d);   // Im conj = -Ai
-        h1[2 * l] = c; q1[2 * l] = d;                 // Re(i conj) = Ai
-        h1[2 * l + 1] = a; q1[2 * l + 1] = b;         // Im(i conj) = Ar
+        split2(tx < 16 ? u.x : -u.y, a, b);
+        split2(tx < 16 ? v.x : -v.y, c, d);
+        const size_t o = (size_t)g * Kp + (size_t)l0 * 2 + 2 * tx;
+        *reinterpret_cast<__nv_bfloat162 *>(hi + o) = __nv_bfloat162(a, c);
+        *reinterpret_cast<__nv_bfloat162 *>(lo + o) = __nv_bfloat162(b, d);
     }
 }
 
-// zero the K padding columns [2k, Kp) of every row written by k_prep_nn_a
-__global__ void k_zero_pad(__nv_bfloat16 *hi, __nv_bfloat16 *lo, int64_t rows, int Kp, int kfrom) {
-    const int w = Kp - kfrom;
-    const size_t total = (size_t)rows * w;
-    for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
-        const size_t r = t / w, c = kfrom + t % w;
-        hi[r * Kp + c] = __float2bfloat16_rn(0.f);
-        lo[r * Kp + c] = __float2bfloat16_rn(0.f);
-    }
-}
-
-// C (m x n complex, ldc) (+)= sum_z W[z]  with W[z][j][2i + {0,1}] = {Re, Im}.
-// upper: 1 = only i <= j is formed and written, 2 = only i <= j was formed
-// (Z^H Z) and the other triangle gets its conjugate.
+// C (m x n complex, ldc) (+)= sum_z W[z][j][i].  upper: 1 = only i <= j is
+// formed and written, 2 = only i <= j was formed (Z^H Z) and the other
+// triangle gets its conjugate.
 template <typename CT>
-__global__ void k_finalize(const float *__restrict__ W, int S, int m, int n, CT *__restrict__ C, int64_t ldc, int accumulate,
+__global__ void k_finalize(const float2 *__restrict__ W, int S, int m, int n, CT *__restrict__ C, int64_t ldc, int accumulate,
                            int upper) {
     const size_t total = (size_t)m * n;
-    const size_t Mp = 2 * (size_t)m;
     for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
         const size_t j = t / m, i = t - j * m;
         if (upper && i > j) continue;
         double re = 0.0, im = 0.0;
+#pragma unroll 4
         for (int z = 0; z < S; ++z) {
-            const float *w = W + (size_t)z * Mp * n + j * Mp + 2 * i;
-            re += (double)w[0];
-            im += (double)w[1];
+            const float2 w = W[(size_t)z * total + t];
+            re += (double)w.x;
+            im += (double)w.y;
         }
         auto put = [&](CT *p, double y) {
             p->x = accumulate ? re + (double)p->x : re;
@@ -490,13 +484,13 @@ __global__ void k_finalize(const float *__restrict__ W, int S, int m, int n, CT 
     }
 }
 
-// B' of D P (the operand of betaNL (D P)) straight from the split sums W of
+// The operand of betaNL (D P) straight from the split sums W of
 // P = betaNL' psi: row b = [Re, Im] of sum_j D[i][j] sum_z W[z][b][j] along i,
 // two BF16 pieces, zero past nbeta.  One pass where finalize, D P and the
 // operand's own prep pass were three launches (about 4 us each).
 __global__ void k_dcsr_prep(const float2 *__restrict__ W, int S, int nbeta, int nb, const int *__restrict__ rowptr,
                             const int *__restrict__ col, const double *__restrict__ val, int Kp,
-                            __nv_bfloat162 *__restrict__ hi, __nv_bfloat162 *__restrict__ lo) {
+                            __nv_bfloat16 *__restrict__ hi, __nv_bfloat16 *__restrict__ lo) {
     const int kp2 = Kp / 2;
     const size_t total = (size_t)kp2 * nb, wz = (size_t)nbeta * nb;
     for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
@@ -518,8 +512,11 @@ __global__ void k_dcsr_prep(const float2 *__restrict__ W, int S, int nbeta, int 
         __nv_bfloat16 a[2], c[2];
         splitn<2>((float)re, a);
         splitn<2>((float)im, c);
-        hi[t] = __nv_bfloat162(a[0], c[0]);
-        lo[t] = __nv_bfloat162(a[1], c[1]);
+        const size_t o = (size_t)b * Kp + kpos(i);
+        hi[o] = a[0];
+        hi[o + 32] = c[0];
+        lo[o] = a[1];
+        lo[o + 32] = c[1];
     }
 }
 
@@ -537,10 +534,10 @@ cudaError_t get_encoder() {
     return cudaSuccess;
 }
 
-// rows of Kp BF16 values, row r at base + r * rstride * Kp
-cudaError_t make_map(CUtensorMap *map, const void *base, int64_t rows, int Kp, int box_rows, int rstride) {
+// rows of Kp BF16 values
+cudaError_t make_map(CUtensorMap *map, const void *base, int64_t rows, int Kp, int box_rows) {
     cuuint64_t dims[2] = {(cuuint64_t)Kp, (cuuint64_t)rows};
-    cuuint64_t strides[1] = {(cuuint64_t)Kp * 2 * (cuuint64_t)rstride};
+    cuuint64_t strides[1] = {(cuuint64_t)Kp * 2};
     cuuint32_t box[2] = {(cuuint32_t)BK, (cuuint32_t)box_rows};
     cuuint32_t es[2] = {1, 1};
     CUresult r = g_encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(base), dims, strides, box, es,
@@ -564,70 +561,62 @@ int umma_kpad(int64_t K) { return (int)(((2 * K + BK - 1) / BK) * BK); }
 size_t umma_operand_bytes(int64_t rows, int64_t K) { return (size_t)rows * umma_kpad(K) * 2 * 2; }
 
 template <typename CT>
-cudaError_t umma_prep_tn_a(const void *Z, int64_t ld, int64_t K, int m, UmmaOperand &op, cudaStream_t st) {
-    op.rows = 2 * (int64_t)m;
+cudaError_t umma_prep_tn(const void *Z, int64_t ld, int64_t K, int m, UmmaOperand &op, cudaStream_t st) {
+    op.rows = m;
     op.Kp = umma_kpad(K);
-    dim3 grid((unsigned)std::min<int64_t>((op.Kp / 2 + 255) / 256, 64), m);
+    dim3 grid((unsigned)std::min<int64_t>((op.Kp / 4 + 255) / 256, 64), (unsigned)std::min(m, 65535));
     if (op.lo2)
-        k_prep_tn_a<CT, 3><<<grid, 256, 0, st>>>((const CT *)Z, ld, K, m, op.Kp, op.hi, op.lo, op.lo2);
+        k_prep_tn<CT, 3><<<grid, 256, 0, st>>>((const CT *)Z, ld, K, m, op.Kp, op.hi, op.lo, op.lo2);
     else
-        k_prep_tn_a<CT, 2><<<grid, 256, 0, st>>>((const CT *)Z, ld, K, m, op.Kp, op.hi, op.lo, nullptr);
-    return cudaGetLastError();
-}
-
-template <typename CT>
-cudaError_t umma_prep_tn_b(const void *Wm, int64_t ld, int64_t K, int n, UmmaOperand &op, cudaStream_t st) {
-    op.rows = n;
-    op.Kp = umma_kpad(K);
-    dim3 grid((unsigned)std::min<int64_t>((op.Kp / 2 + 255) / 256, 64), n);
-    if (op.lo2)
-        k_prep_tn_b<CT, 3><<<grid, 256, 0, st>>>((const CT *)Wm, ld, K, n, op.Kp, op.hi, op.lo, op.lo2);
-    else
-        k_prep_tn_b<CT, 2><<<grid, 256, 0, st>>>((const CT *)Wm, ld, K, n, op.Kp, op.hi, op.lo, nullptr);
+        k_prep_tn<CT, 2><<<grid, 256, 0, st>>>((const CT *)Z, ld, K, m, op.Kp, op.hi, op.lo, nullptr);
     return cudaGetLastError();
 }
 
 template <typename CT>
 cudaError_t umma_prep_nn_a(const void *A, int64_t lda, int64_t M, int k, UmmaOperand &op, cudaStream_t st) {
-    op.rows = 2 * M;
+    op.rows = M;
     op.Kp = umma_kpad(k);
     dim3 grid((unsigned)((M + 31) / 32), (k + 31) / 32);
     k_prep_nn_a<CT><<<grid, 256, 0, st>>>((const CT *)A, lda, M, k, op.Kp, op.hi, op.lo);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    if (op.Kp > 2 * k) {
-        k_zero_pad<<<blocks_for((size_t)op.rows * (op.Kp - 2 * k)), 256, 0, st>>>(op.hi, op.lo, op.rows, op.Kp, 2 * k);
-        e = cudaGetLastError();
-    }
-    return e;
+    return cudaGetLastError();
 }
 
-// Output tile width for n complex columns: 160 when it pads n less than 128
-// does (n = 160, 320, 480, 1440), else 128.
+// Output tile width for n complex columns: the one with the least padded
+// width, a column of a tile narrower than 128 counted dearer because the MMA
+// then waits for its operands (A's 128 rows and B's BN rows come from shared
+// memory at 128 bytes a clock: (128 + BN) / (2 BN) clocks a column).
 static int pick_bn(int n) {
-    const int p128 = (n + 127) / 128 * 128, p160 = (n + 159) / 160 * 160;
-    return p160 < p128 ? 160 : 128;
+    int best = 128;
+    double tbest = 1e300;
+    for (int bn : {128, 96, 80, 64, 32}) {
+        const double t = (double)((n + bn - 1) / bn) * std::max(1.0 * bn, 0.5 * (128 + bn));
+        if (t < tbest * (1.0 - 1e-9)) {
+            tbest = t;
+            best = bn;
+        }
+    }
+    return best;
 }
 
 // Split-K count.  One CTA fits on an SM (222 KB of shared memory); the
 // count minimises a model of the run time in k-block units: waves of the
 // active tiles (those on or above the diagonal for a Hermitian product) x
-// splits over 148 SMs, times the k-blocks per split plus ~8 for a CTA's
+// splits over 148 SMs, times the k-blocks per split plus ~5 for a CTA's
 // pipeline fill and epilogue, plus the split-K workspace pass.  (Measured:
 // the Si64 betaNL' psi at 5 tiles x 60 splits ran as 2 waves plus 4 CTAs;
 // the Si216 Gram, 115 active tiles, was slower unsplit than at 2 splits.)
-// Accuracy does not depend on it: every CHAIN k-blocks are their own
+// Accuracy does not depend on it: every k-block is its own
 // accumulation chain in TMEM.
-int umma_splits(int64_t Mp, int Np, int Kp, int splits, int upper) {
+int umma_splits(int64_t M, int N, int Kp, int splits, int upper) {
     const int KB = Kp / BK;
     if (splits > 0) return std::max(1, std::min(splits, KB));
-    const int bn = pick_bn(Np);
-    const int mt = (int)((Mp + BM - 1) / BM), nt = (Np + bn - 1) / bn;
+    const int bn = pick_bn(N);
+    const int mt = (int)((M + BM - 1) / BM), nt = (N + bn - 1) / bn;
     int active = mt * nt;
     if (upper) {
         active = 0;
         for (int by = 0; by < nt; ++by)
-            for (int bx = 0; bx < mt; ++bx) active += (bx * BM) / 2 > by * bn + bn - 1 ? 0 : 1;
+            for (int bx = 0; bx < mt; ++bx) active += bx * BM > by * bn + bn - 1 ? 0 : 1;
     }
     active = std::max(1, active);
     const int smax = std::max(1, std::min(64, KB / 4));
@@ -635,7 +624,7 @@ int umma_splits(int64_t Mp, int Np, int Kp, int splits, int upper) {
     double tbest = 1e300;
     for (int S = 1; S <= smax; ++S) {
         const double waves = (double)((active * S + 147) / 148);
-        const double t = waves * ((double)(KB + S - 1) / S + 8.0) + (S > 1 ? (double)S * Mp * Np / 1.6e6 : 0.0);
+        const double t = waves * ((double)(KB + S - 1) / S + 5.0) + (S > 1 ? (double)S * M * N / 1.3e6 : 0.0);
         if (t < tbest * (1.0 - 1e-9)) {
             tbest = t;
             best = S;
@@ -644,23 +633,19 @@ int umma_splits(int64_t Mp, int Np, int Kp, int splits, int upper) {
     return best;
 }
 
-size_t umma_ws_bytes(int64_t Mp, int Np, int Kp, int splits, int upper) {
-    return (size_t)umma_splits(Mp, Np, Kp, splits, upper) * Mp * Np * sizeof(float);
+size_t umma_ws_bytes(int64_t M, int N, int Kp, int splits, int upper) {
+    return (size_t)umma_splits(M, N, Kp, splits, upper) * M * N * sizeof(float2);
 }
 
 template <int NS, int BN>
-static cudaError_t launch_umma(const CUtensorMap *mA, const CUtensorMap *mB, dim3 grid, int Mp, int n, int KB, int kb_per,
+static cudaError_t launch_umma(const CUtensorMap *mA, const CUtensorMap *mB, dim3 grid, int M, int n, int KB, int kb_per,
                                float *ws, int *err, int upper, int lolo, void *C, int64_t ldc, int cdouble, int accumulate,
                                cudaStream_t st) {
-    static bool attr_set = false;
-    if (!attr_set) {
-        cudaError_t e = cudaFuncSetAttribute(k_umma_gemm<NS, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)smem_bytes<NS, BN>());
-        if (e != cudaSuccess) return e;
-        attr_set = true;
-    }
-    k_umma_gemm<NS, BN><<<grid, THREADS, smem_bytes<NS, BN>(), st>>>(mA[0], mA[1], mA[2], mB[0], mB[1], mB[2], Mp, n, KB,
-                                                                      kb_per, ws, err, upper, lolo, C, ldc, cdouble,
+    cudaError_t e = cudaFuncSetAttribute(k_umma_gemm<NS, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)smem_bytes<NS, BN>());
+    if (e != cudaSuccess) return e;
+    k_umma_gemm<NS, BN><<<grid, THREADS, smem_bytes<NS, BN>(), st>>>(mA[0], mA[1], mA[2], mB[0], mB[1], mB[2], M, n, KB,
+                                                                      kb_per, (float2 *)ws, err, upper, lolo, C, ldc, cdouble,
                                                                       accumulate);
     return cudaGetLastError();
 }
@@ -669,8 +654,8 @@ cudaError_t umma_dcsr_prep(const float *ws, int S, int nbeta, int nb, const int 
                            UmmaOperand &op, cudaStream_t st) {
     op.rows = nb;
     op.Kp = umma_kpad(nbeta);
-    k_dcsr_prep<<<blocks_for((size_t)op.Kp / 2 * nb), 256, 0, st>>>((const float2 *)ws, S, nbeta, nb, rowptr, col, val, op.Kp,
-                                                                   (__nv_bfloat162 *)op.hi, (__nv_bfloat162 *)op.lo);
+    k_dcsr_prep<<<blocks_for((size_t)op.Kp / 2 * nb), 256, 0, st>>>((const float2 *)ws, S, nbeta, nb, rowptr, col, val, op.Kp, op.hi,
+                                                                   op.lo);
     return cudaGetLastError();
 }
 
@@ -679,7 +664,7 @@ cudaError_t umma_gemm(const UmmaOperand &A, const UmmaOperand &B, int m, int n, 
                       float *ws, int *err, cudaStream_t st, int upper, int lolo, int splits) {
     cudaError_t e = get_encoder();
     if (e != cudaSuccess) return e;
-    if (A.Kp != B.Kp || A.rows != 2 * (int64_t)m || B.rows != n) return cudaErrorInvalidValue;
+    if (A.Kp != B.Kp || A.rows != m || B.rows != n) return cudaErrorInvalidValue;
     // three BF16 pieces only when both operands carry them
     const int ns = (A.lo2 && B.lo2) ? 3 : 2;
     const int bn = pick_bn(n);
@@ -687,32 +672,34 @@ cudaError_t umma_gemm(const UmmaOperand &A, const UmmaOperand &B, int m, int n, 
     const __nv_bfloat16 *pa[3] = {A.hi, A.lo, ns == 3 ? A.lo2 : A.lo};
     const __nv_bfloat16 *pb[3] = {B.hi, B.lo, ns == 3 ? B.lo2 : B.lo};
     for (int q = 0; q < 3; ++q) {
-        if ((e = make_map(&mA[q], pa[q], A.rows, A.Kp, BM, A.rstride)) != cudaSuccess) return e;
-        if ((e = make_map(&mB[q], pb[q], B.rows, B.Kp, bn, B.rstride)) != cudaSuccess) return e;
+        if ((e = make_map(&mA[q], pa[q], A.rows, A.Kp, BM)) != cudaSuccess) return e;
+        if ((e = make_map(&mB[q], pb[q], B.rows, B.Kp, bn)) != cudaSuccess) return e;
     }
     const int KB = A.Kp / BK;
     const int S = umma_splits(A.rows, n, A.Kp, splits, upper);
     const int kb_per = (KB + S - 1) / S;
     dim3 grid((unsigned)((A.rows + BM - 1) / BM), (n + bn - 1) / bn, S);
-    // one split and no accumulation: the epilogue writes C itself, no
-    // workspace pass (accumulating, its read-modify-write of C measured
-    // slower than the workspace + finalize pass: Si64 op_H 0.78 -> 0.95 ms)
-    void *Cd = (S == 1 && !accumulate && upper != 2) ? C : nullptr;
+    // one split: the epilogue writes or adds into C itself, no workspace pass
+    void *Cd = (S == 1 && upper != 2) ? C : nullptr;
     const int cd = sizeof(CT) == 16 ? 1 : 0;
-    if (ns == 3)
-        e = bn == 160 ? launch_umma<3, 160>(mA, mB, grid, (int)A.rows, n, KB, kb_per, ws, err, upper, 0, Cd, ldc, cd, accumulate, st)
-                      : launch_umma<3, 128>(mA, mB, grid, (int)A.rows, n, KB, kb_per, ws, err, upper, 0, Cd, ldc, cd, accumulate, st);
-    else
-        e = bn == 160 ? launch_umma<2, 160>(mA, mB, grid, (int)A.rows, n, KB, kb_per, ws, err, upper, lolo, Cd, ldc, cd, accumulate, st)
-                      : launch_umma<2, 128>(mA, mB, grid, (int)A.rows, n, KB, kb_per, ws, err, upper, lolo, Cd, ldc, cd, accumulate, st);
+    e = cudaErrorInvalidValue;
+#define PW_U(BN)                                                                                                     \
+    if (bn == BN)                                                                                                    \
+        e = ns == 3 ? launch_umma<3, BN>(mA, mB, grid, m, n, KB, kb_per, ws, err, upper, 0, Cd, ldc, cd, accumulate, st) \
+                    : launch_umma<2, BN>(mA, mB, grid, m, n, KB, kb_per, ws, err, upper, lolo, Cd, ldc, cd, accumulate, st);
+    PW_U(128)
+    PW_U(96)
+    PW_U(80)
+    PW_U(64)
+    PW_U(32)
+#undef PW_U
     if (e != cudaSuccess || Cd || !C) return e;
-    k_finalize<CT><<<blocks_for((size_t)m * n), 256, 0, st>>>(ws, S, m, n, (CT *)C, ldc, accumulate, upper);
+    k_finalize<CT><<<blocks_for((size_t)m * n), 256, 0, st>>>((const float2 *)ws, S, m, n, (CT *)C, ldc, accumulate, upper);
     return cudaGetLastError();
 }
 
-template cudaError_t umma_prep_tn_a<float2>(const void *, int64_t, int64_t, int, UmmaOperand &, cudaStream_t);
-template cudaError_t umma_prep_tn_b<float2>(const void *, int64_t, int64_t, int, UmmaOperand &, cudaStream_t);
-template cudaError_t umma_prep_tn_b<double2>(const void *, int64_t, int64_t, int, UmmaOperand &, cudaStream_t);
+template cudaError_t umma_prep_tn<float2>(const void *, int64_t, int64_t, int, UmmaOperand &, cudaStream_t);
+template cudaError_t umma_prep_tn<double2>(const void *, int64_t, int64_t, int, UmmaOperand &, cudaStream_t);
 template cudaError_t umma_prep_nn_a<float2>(const void *, int64_t, int64_t, int, UmmaOperand &, cudaStream_t);
 template cudaError_t umma_gemm<float2>(const UmmaOperand &, const UmmaOperand &, int, int, void *, int64_t, int, float *,
                                        int *, cudaStream_t, int, int, int);
