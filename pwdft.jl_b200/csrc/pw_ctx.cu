@@ -323,6 +323,7 @@ FftLaunch make_launch_kd(const pw_ctx *c, const KData &kd) {
     // z passes: ~48 KB of shared memory per CTA
     int Cg = (int)((48 * 1024 / es - c->N3) / c->N3);
     L.Cg = std::max(1, std::min(64, Cg));
+    L.Cg_set = c->z_cols;
     if (c->z_cols > 0) {
         // at most ~190 KB of shared memory per z-pass CTA
         const int cmax = std::max(1, (int)((190 * 1024 / es - c->N3) / c->N3) - 16);
@@ -444,7 +445,9 @@ int apply_T(pw_ctx *c, int ik, int ispin, const void *psi, void *Hpsi, int64_t l
             c->launches += 3;
         } else {
             if ((s = ensure(c, c->P2, pb))) return s;
-            if ((s = ensure(c, c->gemm_ws, gemm_tn_ws_bytes((int)sizeof(T), kd.Ngw, c->nbeta, nb)))) return s;
+            if ((s = ensure(c, c->gemm_ws, sizeof(T) == 8 ? project_ws_bytes(kd.Ngw, c->nbeta, nb)
+                                                          : gemm_tn_ws_bytes((int)sizeof(T), kd.Ngw, c->nbeta, nb))))
+                return s;
             if (sizeof(T) == 8) {
                 CK(c, project_dcsr(kd.Ngw, c->nbeta, nb, kd.d_beta64, (const double2 *)psi, ld, c->d_Drow, c->d_Dcol, c->d_Dval,
                                    (double2 *)c->P2.p, c->gemm_ws.p, st));

@@ -213,8 +213,9 @@ k_zgemm(int64_t K, int64_t m, int n, const double2 *__restrict__ A, int64_t lda,
 
 // Tile and split-K count of a product: the candidate with the shortest
 // modelled time in clocks.  A CTA's tile costs 16 WM WN clocks of its SM's
-// FP64 pipe per k, plus about 32 k for filling the ring and storing; the SM
-// with the most CTAs decides; a split adds the partial sums' trip through L2
+// FP64 pipe per k, but not less than 45 (the ring waits for L2: 350 clocks a step
+// of 8), plus about 32 k for filling the ring and storing; the SM with the
+// most CTAs decides; a split adds the partial sums' trip through L2
 // (about 2400 bytes a clock) and the reduction's launch (4000 clocks).
 // (480 x 480 over K = 23,871: 48 x 80 tiles, 0 % padding, against 14 % with
 // 64 x 64.)  Splitting stops at four CTAs an SM, which also bounds the workspace
@@ -223,7 +224,8 @@ struct ZPlan {
     int wm, wn, S;
     int64_t kchunk;
 };
-ZPlan zplan(int64_t K, int64_t m, int n, bool tn, int upper) {
+// fused: the caller's next pass sums the splits.
+ZPlan zplan(int64_t K, int64_t m, int n, bool tn, int upper, bool fused = false) {
     ZPlan best{2, 2, 1, K};
     double tbest = 1e300;
     for (int wm = 2; wm <= 4; ++wm)
@@ -242,8 +244,8 @@ ZPlan zplan(int64_t K, int64_t m, int n, bool tn, int upper) {
                 if (w > 0 && (S < 2 || (int64_t)S * 64 > K)) continue;
                 const double kc = (double)((K + S - 1) / S);
                 const double per = std::ceil(tiles * S / 148.0);
-                double t = per * 16.0 * wm * wn * (kc + 32.0) * (per < 1.5 ? 1.15 : 1.0);
-                if (S > 1) t += 4000.0 + (double)S * m * n * 32.0 / 2400.0;
+                double t = std::max(per * 16.0 * wm * wn * (per < 1.5 ? 1.15 : 1.0), 45.0) * (kc + 32.0);
+                if (S > 1) t += (fused ? 0.0 : 4000.0) + (double)S * m * n * 32.0 / 2400.0;
                 if (t < tbest * (1.0 - 1e-9)) {
                     tbest = t;
                     best = ZPlan{wm, wn, S, K};
@@ -370,21 +372,32 @@ __global__ void k_dcsr(int nbeta, int nb, const int *__restrict__ rowptr, const 
 
 // P2[b][i] = sum_j D[i][j] sum_z W[z][b][j]: the split-K sum of P = betaNL' psi and
 // D P in one pass (P itself is not needed by op_V_Ps_nloc).
+// Eight lanes share an element's splits (one thread summing 23 of them for 20 x 40
+// values took 11 us).
 __global__ void k_dcsr_splits(int nbeta, int nb, const int *__restrict__ rowptr, const int *__restrict__ col,
                               const double *__restrict__ val, const double2 *__restrict__ W, int S, double2 *__restrict__ P2) {
     const size_t total = (size_t)nbeta * nb;
-    for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
-        const int b = (int)(t / nbeta), i = (int)(t - (size_t)b * nbeta);
+    const int l8 = threadIdx.x & 7;
+    for (size_t t0 = (blockIdx.x * (size_t)blockDim.x + (threadIdx.x & ~31)) >> 3; t0 < total;
+         t0 += ((size_t)gridDim.x * blockDim.x) >> 3) {
+        const size_t t = t0 + ((threadIdx.x & 31) >> 3);
         double2 s = make_double2(0.0, 0.0);
-        for (int e = rowptr[i]; e < rowptr[i + 1]; ++e) {
-            const double2 *w = W + (size_t)b * nbeta + col[e];
-            double2 p = make_double2(0.0, 0.0);
+        if (t < total) {
+            const int b = (int)(t / nbeta), i = (int)(t - (size_t)b * nbeta);
+            for (int e = rowptr[i]; e < rowptr[i + 1]; ++e) {
+                const double2 *w = W + (size_t)b * nbeta + col[e];
+                double2 p = make_double2(0.0, 0.0);
 #pragma unroll 4
-            for (int z = 0; z < S; ++z) p = cadd(p, w[(size_t)z * total]);
-            s.x += val[e] * p.x;
-            s.y += val[e] * p.y;
+                for (int z = l8; z < S; z += 8) p = cadd(p, w[(size_t)z * total]);
+                s.x += val[e] * p.x;
+                s.y += val[e] * p.y;
+            }
         }
-        P2[t] = s;
+        for (int o = 4; o > 0; o >>= 1) {
+            s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
+            s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
+        }
+        if (t < total && l8 == 0) P2[t] = s;
     }
 }
 
@@ -475,12 +488,15 @@ template cudaError_t gemm_nn<float>(int64_t, int, int, const void *, int64_t, co
 template cudaError_t gemm_nn<double>(int64_t, int, int, const void *, int64_t, const double2 *, int64_t, void *, int64_t,
                                      int, cudaStream_t, int);
 
+size_t project_ws_bytes(int64_t K, int nbeta, int nb) {
+    return (size_t)zplan(K, nbeta, nb, true, 0, true).S * nbeta * nb * sizeof(double2);
+}
 cudaError_t project_dcsr(int64_t K, int nbeta, int nb, const double2 *beta, const double2 *psi, int64_t ldp, const int *rowptr,
                          const int *col, const double *val, double2 *P2, void *ws, cudaStream_t st) {
-    const ZPlan p = zplan(K, nbeta, nb, true, 0);
+    const ZPlan p = zplan(K, nbeta, nb, true, 0, true);
     cudaError_t e = launch_zgemm<true>(p, K, nbeta, nb, beta, K, psi, ldp, (double2 *)ws, 0, 0, 0, 0, 0, st);
     if (e != cudaSuccess) return e;
-    k_dcsr_splits<<<blocks_for((size_t)nbeta * nb), 256, 0, st>>>(nbeta, nb, rowptr, col, val, (const double2 *)ws, p.S, P2);
+    k_dcsr_splits<<<blocks_for((size_t)nbeta * nb * 8), 256, 0, st>>>(nbeta, nb, rowptr, col, val, (const double2 *)ws, p.S, P2);
     return cudaGetLastError();
 }
 cudaError_t apply_dcsr(int nbeta, int nb, const int *rowptr, const int *col, const double *val, const double2 *P,

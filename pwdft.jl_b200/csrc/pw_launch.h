@@ -34,6 +34,7 @@ struct FftLaunch {
     FftDim dx, dy, dz;
     const void *twx, *twy, *twz;  // twiddle tables of the launch precision
     int Cg;                       // columns per CTA in the z passes
+    int Cg_set = 0;               // Cg if the caller set it (pw_tuning.z_columns), else 0
     int Jc;                       // y lines per x chunk in the plane passes
     int bpc = 1;                  // bands of one z-plane per CTA in the FP32 plane pass (1..3)
     int bpc_set = 0;              // bpc if the caller set it (pw_tuning.plane_bands), else 0
@@ -105,7 +106,8 @@ template <typename T>
 cudaError_t gemm_nn(int64_t M, int n, int k, const void *A, int64_t lda, const double2 *B, int64_t ldb, void *C,
                     int64_t ldc, int accumulate, cudaStream_t, int tri = 0);
 // P2 = D (beta^H psi) in FP64 (beta K x nbeta with ld K; CSR D; P2 nbeta x nb,
-// ld = nbeta); ws as gemm_tn's (gemm_tn_ws_bytes(8, K, nbeta, nb))
+// ld = nbeta); ws: project_ws_bytes
+size_t project_ws_bytes(int64_t K, int nbeta, int nb);
 cudaError_t project_dcsr(int64_t K, int nbeta, int nb, const double2 *beta, const double2 *psi, int64_t ldp, const int *rowptr,
                          const int *col, const double *val, double2 *P2, void *ws, cudaStream_t);
 // P2[i][b] = sum_j D[i][j] P[j][b]  (CSR D; P, P2 are nbeta x nb, ld = nbeta)

@@ -491,17 +491,19 @@ __global__ void k_finalize(const float2 *__restrict__ W, int S, int m, int n, CT
 __global__ void k_dcsr_prep(const float2 *__restrict__ W, int S, int nbeta, int nb, const int *__restrict__ rowptr,
                             const int *__restrict__ col, const double *__restrict__ val, int Kp,
                             __nv_bfloat16 *__restrict__ hi, __nv_bfloat16 *__restrict__ lo) {
-    const int kp2 = Kp / 2;
+    const int kp2 = Kp / 2, l8 = threadIdx.x & 7;   // eight lanes share an element's splits
     const size_t total = (size_t)kp2 * nb, wz = (size_t)nbeta * nb;
-    for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
+    for (size_t t0 = (blockIdx.x * (size_t)blockDim.x + (threadIdx.x & ~31)) >> 3; t0 < total;
+         t0 += ((size_t)gridDim.x * blockDim.x) >> 3) {
+        const size_t t = t0 + ((threadIdx.x & 31) >> 3);
         const int b = (int)(t / kp2), i = (int)(t - (size_t)b * kp2);
         double re = 0.0, im = 0.0;
-        if (i < nbeta)
+        if (t < total && i < nbeta)
             for (int e = rowptr[i]; e < rowptr[i + 1]; ++e) {
                 const float2 *w = W + (size_t)b * nbeta + col[e];
                 double pr = 0.0, pi = 0.0;
 #pragma unroll 4
-                for (int z = 0; z < S; ++z) {
+                for (int z = l8; z < S; z += 8) {
                     const float2 v = w[z * wz];
                     pr += (double)v.x;
                     pi += (double)v.y;
@@ -509,6 +511,11 @@ __global__ void k_dcsr_prep(const float2 *__restrict__ W, int S, int nbeta, int 
                 re += val[e] * pr;
                 im += val[e] * pi;
             }
+        for (int o = 4; o > 0; o >>= 1) {
+            re += __shfl_xor_sync(0xffffffffu, re, o);
+            im += __shfl_xor_sync(0xffffffffu, im, o);
+        }
+        if (t >= total || l8) continue;
         __nv_bfloat16 a[2], c[2];
         splitn<2>((float)re, a);
         splitn<2>((float)im, c);
@@ -654,7 +661,7 @@ cudaError_t umma_dcsr_prep(const float *ws, int S, int nbeta, int nb, const int 
                            UmmaOperand &op, cudaStream_t st) {
     op.rows = nb;
     op.Kp = umma_kpad(nbeta);
-    k_dcsr_prep<<<blocks_for((size_t)op.Kp / 2 * nb), 256, 0, st>>>((const float2 *)ws, S, nbeta, nb, rowptr, col, val, op.Kp, op.hi,
+    k_dcsr_prep<<<blocks_for((size_t)op.Kp / 2 * nb * 8), 256, 0, st>>>((const float2 *)ws, S, nbeta, nb, rowptr, col, val, op.Kp, op.hi,
                                                                    op.lo);
     return cudaGetLastError();
 }
