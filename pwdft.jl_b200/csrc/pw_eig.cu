@@ -10,10 +10,11 @@
 //   4. C = Linv T Linv^H                two FP64 complex GEMMs
 //   5. C = Q Tr Q^H                     Householder tridiagonalisation (LAPACK
 //                                       zhetd2 conventions: H = I - tau v v^H,
-//                                       real tridiagonal Tr): columns in
-//                                       registers up to n = 1024, above that
-//                                       in L2 with one grid barrier per
-//                                       column (cooperative kernels)
+//                                       real tridiagonal Tr): the last 256
+//                                       columns in one cluster's registers,
+//                                       those before in registers across the
+//                                       grid (n <= 1024) or in L2 with one grid
+//                                       barrier per column
 //   6. lowest k eigenvalues of Tr       multisection on Sturm counts, one warp
 //                                       per eigenvalue; the block reflectors
 //                                       of step 8 meanwhile
@@ -367,7 +368,7 @@ __global__ void __launch_bounds__(COOP_THREADS) k_chol_inv(double2 *A, double2 *
 // between two buffers so that a CTA running ahead into the next phase M
 // cannot overwrite values a slower CTA still reads.
 __global__ void __launch_bounds__(COOP_THREADS)
-k_tridiag(double2 *C, int n, double *d, double *e, double2 *tau, double2 *ybuf, unsigned *ctr, int *err) {
+k_tridiag(double2 *C, int n, int jend, double *d, double *e, double2 *tau, double2 *ybuf, unsigned *ctr, int *err) {
     extern __shared__ __align__(16) unsigned char sm[];
     double2 *vc = reinterpret_cast<double2 *>(sm);  // v_j         [n]
     double2 *vp = vc + n;                           // v_{j-1}     [n]
@@ -413,7 +414,7 @@ k_tridiag(double2 *C, int n, double *d, double *e, double2 *tau, double2 *ybuf, 
     if (blockIdx.x == 0 && threadIdx.x == 0) d[0] = vc[0].x;
     if (n >= 2) tj = householder(0);
 
-    for (int j = 0; j < n - 1; ++j) {
+    for (int j = 0; j < jend; ++j) {
         double2 *yb = ybuf + (size_t)(j & 1) * n;
         // ---- phase M: update owned columns i > j with (v_{j-1}, w_{j-1}), y_i = col_i^H v_j
         for (int i = j + 1 + blockIdx.x + gridDim.x * warp; i < n; i += gridDim.x * nw) {
@@ -507,7 +508,19 @@ k_tridiag(double2 *C, int n, double *d, double *e, double2 *tau, double2 *ybuf, 
         }
         __syncthreads();
         if (blockIdx.x == 0 && threadIdx.x == 0) d[c1] = vc[c1].x;
-        if (c1 < n - 1) tj = householder(c1);
+        if (c1 < jend) tj = householder(c1);
+    }
+    // the trailing matrix from column jend on, with the last step's update, for
+    // the next kernel
+    if (jend < n - 1) {
+        gsync(ctr, tgt, err);   // everyone has read column jend
+        for (int i = jend + blockIdx.x; i < n; i += gridDim.x) {
+            const double2 cw = make_double2(wp[i].x, -wp[i].y), cv = make_double2(vp[i].x, -vp[i].y);
+            for (int r = jend + threadIdx.x; r < n; r += blockDim.x) {
+                const double2 p = cmul_d(vp[r], cw), q = cmul_d(wp[r], cv), a = __ldcg(&C[(size_t)i * n + r]);
+                C[(size_t)i * n + r] = make_double2(a.x - (p.x + q.x), a.y - (p.y + q.y));
+            }
+        }
     }
 }
 
@@ -553,7 +566,7 @@ __device__ __forceinline__ double half_sums(double2 v, int lane) {
 
 template <int NR, int W, int CPW>
 __global__ void __launch_bounds__(32 * W)
-k_tridiag_r(double2 *C, int n, double *d, double *e, double2 *tau, double2 *ybuf, int *err) {
+k_tridiag_r(double2 *C, int n, int jend, double *d, double *e, double2 *tau, double2 *ybuf, int *err) {
     constexpr int TH = 32 * W, EPT = 32 * NR / TH, NN = 32 * NR;
     static_assert(EPT * TH == NN, "every row has a thread");
     extern __shared__ __align__(16) unsigned char sm[];
@@ -629,7 +642,7 @@ k_tridiag_r(double2 *C, int n, double *d, double *e, double2 *tau, double2 *ybuf
 
     if (blockIdx.x == 0 && tid == 0) d[0] = x[0].x;
     if (n >= 2) tj = householder(0);
-    for (int j = 0; j < n - 1; ++j) {
+    for (int j = 0; j < jend; ++j) {
         const int c1 = j + 1;
         double2 *yb = ybuf + (size_t)j * ldy * 2;
         // ---- the warp's column: rank-2 update with (v_{j-1}, w_{j-1}), then y = column^H v_j
@@ -742,8 +755,259 @@ k_tridiag_r(double2 *C, int n, double *d, double *e, double2 *tau, double2 *ybuf
             x[u].y -= p.y + w.y;
             if (row(u) == c1 && blockIdx.x == 0) d[c1] = x[u].x;
         }
+        if (c1 < jend) tj = householder(c1);
+    }
+    // the trailing matrix from column jend on, with the last step's update, for
+    // the next kernel
+    __syncthreads();
+#pragma unroll
+    for (int c = 0; c < CPW; ++c)
+        if (jend < n - 1 && ci[c] >= jend && ci[c] < n) {
+            const double2 cw = make_double2(wp[ci[c]].x, -wp[ci[c]].y), cv = make_double2(vp[ci[c]].x, -vp[ci[c]].y);
+#pragma unroll
+            for (int u = 0; u < NR; ++u) {
+                const int r = lane + 32 * u;
+                if (r >= jend && r < n) {
+                    const double2 p = cmul_d(vp[r], cw), q = cmul_d(wp[r], cv);
+                    C[(size_t)ci[c] * n + r] = make_double2(a[c][u].x - (p.x + q.x), a[c][u].y - (p.y + q.y));
+                }
+            }
+        }
+}
+
+// The same for n <= 256 (or the last 256 columns of a larger matrix, leading
+// dimension ld) inside one thread-block cluster of 16 CTAs: every warp owns
+// CPW columns in registers, and the pairs (y_i, entry of row j + 1) go straight
+// into every CTA's shared memory (st.async), whose mbarrier counts their bytes: a
+// column costs a distributed-shared-memory store instead of a trip through L2
+// that other SMs poll.  Two exchange buffers suffice: a CTA publishes step j + 1
+// only after it has read step j, and nobody publishes step j + 2 before having
+// everyone's step j + 1.  Waits are bounded by polls of the mbarrier; when one
+// runs out the CTA sets *err and waits no more, and the cluster barrier at the
+// end keeps every CTA's shared memory alive until all have finished.  n = 160 /
+// 250 take 0.34 / 0.58 ms (k_tridiag_r 0.54 / 0.93, k_tridiag 0.77 / 1.27); with
+// 32 columns a CTA, n = 480, the update bounds it: 2.20 ms, k_tridiag_r 1.92.
+constexpr int TRC = 16;   // CTAs of the cluster
+template <int NR, int W, int CPW> constexpr size_t tridiag_c_smem() {
+    constexpr int SL = W * CPW;
+    return ((size_t)3 * 32 * NR + 2 * (size_t)TRC * SL * 2 + 2 * SL) * sizeof(double2);
+}
+template <int NR, int W, int CPW>
+__global__ void __launch_bounds__(32 * W, 1)
+k_tridiag_c(double2 *C, int n, int ld, double *d, double *e, double2 *tau, int *err) {
+    constexpr int TH = 32 * W, NN = 32 * NR, EPT = NN / TH, SL = W * CPW;
+    static_assert(TRC * SL >= NN, "every column has a warp");
+    static_assert(EPT * TH == NN, "every row has a thread");
+    extern __shared__ __align__(16) unsigned char sm[];
+    double2 *vc = reinterpret_cast<double2 *>(sm), *vp = vc + NN, *wp = vp + NN;   // v_j, v_{j-1}, w_{j-1}
+    double2 *ex = wp + NN;                       // exchange buffers [2][TRC][SL][2]
+    double2 *ysm = ex + 2 * TRC * SL * 2;        // this CTA's pairs [SL][2]
+    __shared__ double2 red[2][W + 1];
+    __shared__ __align__(8) unsigned long long bar[2];
+    __shared__ int failed;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    unsigned rank;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    const bool mute = (int)rank == g_gsync_withhold;
+    const long long lim = g_gsync_limit;
+    const unsigned bar0 = (unsigned)__cvta_generic_to_shared(&bar[0]), ex0 = (unsigned)__cvta_generic_to_shared(ex);
+    if (tid == 0) {
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar0));
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar0 + 8));
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        failed = 0;
+    }
+    int ci[CPW];
+    double2 a[CPW][NR];
+#pragma unroll
+    for (int c = 0; c < CPW; ++c) {
+        ci[c] = 1 + (int)rank + TRC * (warp + W * c);
+#pragma unroll
+        for (int u = 0; u < NR; ++u) {
+            const int r = lane + 32 * u;
+            a[c][u] = ci[c] < n && r < n ? __ldcg(&C[(size_t)ci[c] * ld + r]) : make_double2(0.0, 0.0);
+        }
+    }
+    auto row = [&](int u) { return tid + TH * u; };
+    double2 x[EPT], v[EPT];
+    int pos[EPT];
+#pragma unroll
+    for (int u = 0; u < EPT; ++u) {
+        x[u] = row(u) < n ? __ldcg(&C[row(u)]) : make_double2(0.0, 0.0);
+        const int i = max(row(u) - 1, 0);
+        pos[u] = 2 * ((i % TRC) * SL + i / TRC);
+    }
+    double2 tj = make_double2(0.0, 0.0);
+    // every mbarrier is ready, and everyone has read column 0
+    asm volatile("barrier.cluster.arrive.aligned;\n barrier.cluster.wait.aligned;" ::: "memory");
+
+    auto householder = [&](int j) {
+        double s2 = 0.0;
+#pragma unroll
+        for (int u = 0; u < EPT; ++u) {
+            if (row(u) > j + 1) s2 += x[u].x * x[u].x + x[u].y * x[u].y;
+            if (row(u) == j + 1) red[1][W] = x[u];
+        }
+        for (int o = 16; o > 0; o >>= 1) s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+        if (lane == 0) red[1][warp].x = s2;
+        __syncthreads();
+        s2 = 0.0;
+#pragma unroll
+        for (int w = 0; w < W; ++w) s2 += red[1][w].x;
+        const double2 alpha = red[1][W];
+        double2 t = make_double2(0.0, 0.0), scal = t;
+        double beta = alpha.x;
+        if (s2 != 0.0 || alpha.y != 0.0) {
+            beta = -copysign(sqrt(alpha.x * alpha.x + alpha.y * alpha.y + s2), alpha.x);
+            const double ib = 1.0 / beta;
+            t = make_double2((beta - alpha.x) * ib, -alpha.y * ib);
+            const double ar = alpha.x - beta, ai = alpha.y, den = 1.0 / (ar * ar + ai * ai);
+            scal = make_double2(ar * den, -ai * den);
+        }
+#pragma unroll
+        for (int u = 0; u < EPT; ++u) {
+            v[u] = row(u) <= j ? make_double2(0.0, 0.0) : row(u) == j + 1 ? make_double2(1.0, 0.0) : cmul_d(x[u], scal);
+            vc[row(u)] = v[u];
+        }
+        if (rank == 0 && tid == 0) {
+            e[j] = beta;
+            tau[j] = t;
+        }
+        __syncthreads();
+        return t;
+    };
+
+    if (rank == 0 && tid == 0) d[0] = x[0].x;
+    if (n >= 2) tj = householder(0);
+    for (int j = 0; j < n - 1; ++j) {
+        const int c1 = j + 1, b = j & 1;
+        // this CTA's mbarrier of the step expects 32 bytes a column i > j
+        const bool dead = *(volatile int *)&failed;   // a wait ran out: no more exchange
+        if (tid == 0 && !dead)
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar0 + 8 * b),
+                         "r"((unsigned)(n - 1 - j) * 32u)
+                         : "memory");
+        // ---- the warp's columns: rank-2 update with (v_{j-1}, w_{j-1}), then y = column^H v_j
+        double2 cw[CPW], cv[CPW], acc[CPW];
+        bool any = false;
+#pragma unroll
+        for (int c = 0; c < CPW; ++c) {
+            const bool on = ci[c] > j && ci[c] < n;
+            any |= on;
+            cw[c] = cv[c] = acc[c] = make_double2(0.0, 0.0);
+            if (on && j > 0) {
+                cw[c] = make_double2(wp[ci[c]].x, -wp[ci[c]].y);
+                cv[c] = make_double2(vp[ci[c]].x, -vp[ci[c]].y);
+            }
+        }
+        if (any) {
+#pragma unroll
+            for (int u = 0; u < NR; ++u) {
+                const int r = lane + 32 * u;
+                if (32 * u + 31 > j && 32 * u < n) {
+                    const double2 pv = vp[r], pw = wp[r], pc = vc[r];
+#pragma unroll
+                    for (int c = 0; c < CPW; ++c) {
+                        double2 t = a[c][u];
+                        if (j > 0) {
+                            t.x = fma(-pv.x, cw[c].x, fma(pv.y, cw[c].y, fma(-pw.x, cv[c].x, fma(pw.y, cv[c].y, t.x))));
+                            t.y = fma(-pv.x, cw[c].y, fma(-pv.y, cw[c].x, fma(-pw.x, cv[c].y, fma(-pw.y, cv[c].x, t.y))));
+                            a[c][u] = t;
+                        }
+                        if (r == c1) ysm[2 * (warp + W * c) + 1] = make_double2(t.x, -t.y);
+                        if (r > j) {
+                            acc[c].x = fma(t.x, pc.x, fma(t.y, pc.y, acc[c].x));
+                            acc[c].y = fma(t.x, pc.y, fma(-t.y, pc.x, acc[c].y));
+                        }
+                    }
+                }
+            }
+#pragma unroll
+            for (int c = 0; c < CPW; ++c) {
+                const double h = half_sums(acc[c], lane);
+                if ((lane & 15) == 0) (lane ? ysm[2 * (warp + W * c)].y : ysm[2 * (warp + W * c)].x) = h;
+            }
+        }
+        __syncthreads();
+        // ---- the CTA's pairs to every CTA of the cluster
+        for (int q = tid; q < TRC * 2 * SL; q += TH) {
+            const int it = q % (2 * SL), dst = q / (2 * SL), i = 1 + (int)rank + TRC * (it >> 1);
+            if (i > j && i < n && !mute && !dead) {
+                const double2 val = ysm[it];
+                unsigned ra, rb;
+                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+                             : "=r"(ra)
+                             : "r"(ex0 + 16u * (unsigned)(b * TRC * SL * 2 + (int)rank * 2 * SL + it)), "r"(dst));
+                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rb) : "r"(bar0 + 8 * b), "r"(dst));
+                asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f64 [%0], {%1, %2}, [%3];" ::"r"(ra),
+                             "d"(val.x), "d"(val.y), "r"(rb)
+                             : "memory");
+            }
+        }
+        // ---- everyone's pairs have arrived
+        {
+            const unsigned ph = (unsigned)((j >> 1) & 1);
+            for (long long it = 0; !*(volatile int *)&failed; ++it) {
+                unsigned ok;
+                asm volatile(
+                    "{\n .reg .pred p;\n mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+                    : "=r"(ok)
+                    : "r"(bar0 + 8 * b), "r"(ph)
+                    : "memory");
+                if (ok) break;
+                if (it > lim) {
+                    failed = 1;
+                    atomicExch(err, 1);
+                }
+            }
+        }
+        double2 y[EPT];
+#pragma unroll
+        for (int u = 0; u < EPT; ++u) {
+            const bool in = row(u) > j && row(u) < n;
+            const double2 *p = ex + (size_t)b * TRC * SL * 2 + pos[u];
+            y[u] = in ? p[0] : make_double2(0.0, 0.0);
+            x[u] = in ? p[1] : make_double2(0.0, 0.0);
+        }
+        // v_j to its place in C (all of column j has been read: every CTA has published this step)
+        if ((j % TRC) == (int)rank) {
+#pragma unroll
+            for (int u = 0; u < EPT; ++u)
+                if (row(u) > c1 && row(u) < n) C[(size_t)j * ld + row(u)] = v[u];
+        }
+        // w_j = tau y + alpha v_j, alpha = -tau/2 (tau y)^H v_j
+        double2 yv = make_double2(0.0, 0.0);
+#pragma unroll
+        for (int u = 0; u < EPT; ++u) {
+            y[u] = cmul_d(tj, y[u]);
+            const double2 q = cmulc_d(y[u], v[u]);
+            yv.x += q.x;
+            yv.y += q.y;
+            if (row(u) == c1) red[0][W] = y[u];
+        }
+        const double h = half_sums(yv, lane);
+        if ((lane & 15) == 0) (lane ? red[0][warp].y : red[0][warp].x) = h;
+        __syncthreads();   // also: every warp is done with vp, wp of this column's update
+        yv = make_double2(0.0, 0.0);
+#pragma unroll
+        for (int w = 0; w < W; ++w) yv = cadd(yv, red[0][w]);
+        const double2 al = cmul_d(make_double2(-0.5 * tj.x, -0.5 * tj.y), yv);
+        // column j+1 given the step-j update: x -= v conj(w_{j+1}) + w (v_{j+1} = 1)
+        const double2 wc = cadd(red[0][W], al), cw1 = make_double2(wc.x, -wc.y);
+#pragma unroll
+        for (int u = 0; u < EPT; ++u) {
+            const double2 w = cadd(y[u], cmul_d(al, v[u])), p = cmul_d(v[u], cw1);
+            vp[row(u)] = v[u];
+            wp[row(u)] = w;
+            x[u].x -= p.x + w.x;
+            x[u].y -= p.y + w.y;
+            if (row(u) == c1 && rank == 0) d[c1] = x[u].x;
+        }
         if (c1 < n - 1) tj = householder(c1);
     }
+    // no CTA leaves while another may still store into its shared memory
+    if (failed) __nanosleep(20000);
+    asm volatile("barrier.cluster.arrive.aligned;\n barrier.cluster.wait.aligned;" ::: "memory");
 }
 
 // Number of eigenvalues of a tridiagonal matrix below x from the signs of the
@@ -1285,22 +1549,45 @@ cudaError_t hegv_lowest(double2 *T, double2 *G, int n, int k, double *lam_out, d
         if ((e_ = gemm_nn<double>(n, n, n, M1, n, G, n, T, n, 0, st, 2)) != cudaSuccess) return e_;
         k_herm_upper<<<nb, 256, 0, st>>>(T, n);
     }
-    if (n <= 1024) {
-        // register-resident columns: few CTAs keep the exchange short, few
-        // columns a CTA the update (n = 160, us a column: 20 CTAs of 8 columns
-        // 3.4, 10 of 16 3.6; n = 480: 120 of 4 4.1, 60 of 8 4.5, 30 of 16 5.4)
-        const void *fn = n <= 256 ? (const void *)k_tridiag_r<8, 8, 1>
-                                  : n <= 512 ? (const void *)k_tridiag_r<16, 4, 1> : (const void *)k_tridiag_r<32, 8, 1>;
-        const int W = n <= 256 || n > 512 ? 8 : 4, sl = W;
-        const int nblk = std::max(1, (n - 1 + sl - 1) / sl);
-        if ((e_ = cudaMemsetAsync(ybuf, 0xff, (size_t)n * 2 * nblk * sl * sizeof(double2), st)) != cudaSuccess) return e_;
-        const size_t smem = 3 * (size_t)(n <= 256 ? 256 : n <= 512 ? 512 : 1024) * sizeof(double2);
-        if (smem > 48 * 1024 - 4096 &&
-            (e_ = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
-            return e_;
-        void *args[] = {(void *)&Cm, (void *)&n, (void *)&d, (void *)&e, (void *)&tau, (void *)&ybuf, (void *)&err};
+    // The last (or only) 256 columns, what one cluster holds in registers, go to
+    // it, those before them to the grid: in registers up to n = 1024, through L2
+    // above that.  At 2.3 against 4.0 us a column the whole reduced problem goes
+    // from 2.94 to 2.65 ms at n = 480, from 1.14 to 0.75 at 160 (k = n / 3); with
+    // 384 columns in a cluster of 384 threads a CTA it spills, 2.73 at 480.
+    constexpr int NC = 256;
+    const auto fc = k_tridiag_c<8, 8, 2>;
+    constexpr size_t smem_c = tridiag_c_smem<8, 8, 2>();
+    cudaLaunchConfig_t cf = {};
+    cudaLaunchAttribute at;
+    cf.gridDim = TRC;
+    cf.blockDim = 256;
+    cf.dynamicSmemBytes = smem_c;
+    cf.stream = st;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = TRC;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cf.attrs = &at;
+    cf.numAttrs = 1;
+    if ((e_ = cudaFuncSetAttribute(fc, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) != cudaSuccess) return e_;
+    static_assert(smem_c <= 48 << 10, "no opt-in");
+    // no room for 16 neighbouring SMs (a partitioned device): the grid does all
+    int ncl = 0;
+    if (cudaOccupancyMaxActiveClusters(&ncl, fc, &cf) != cudaSuccess) {
+        cudaGetLastError();
+        ncl = 0;
+    }
+    const int jend = ncl < 1 ? n - 1 : std::max(0, n - NC);
+    if ((jend > 0 || ncl < 1) && n <= 1024) {
+        // few CTAs keep the exchange short, few columns a CTA the update (n =
+        // 480, us a column: 120 CTAs of 4 columns 4.1, 60 of 8 4.5, 30 of 16 5.4)
+        const void *fn = n <= 512 ? (const void *)k_tridiag_r<16, 4, 1> : (const void *)k_tridiag_r<32, 8, 1>;
+        const int W = n > 512 ? 8 : 4, nblk = std::max(1, (n - 1 + W - 1) / W);
+        if ((e_ = cudaMemsetAsync(ybuf, 0xff, (size_t)jend * 2 * nblk * W * sizeof(double2), st)) != cudaSuccess) return e_;
+        const size_t smem = 3 * (size_t)(n <= 512 ? 512 : 1024) * sizeof(double2);
+        if ((e_ = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess) return e_;
+        void *args[] = {(void *)&Cm, (void *)&n, (void *)&jend, (void *)&d, (void *)&e, (void *)&tau, (void *)&ybuf, (void *)&err};
         if ((e_ = cudaLaunchCooperativeKernel(fn, nblk, 32 * W, args, smem, st)) != cudaSuccess) return e_;
-    } else {
+    } else if (jend > 0) {
         const size_t smem = (size_t)(3 * n + 32) * sizeof(double2);
         int nblk = 0;
         if ((e_ = coop_blocks((const void *)k_tridiag, smem, &nblk)) != cudaSuccess) return e_;
@@ -1308,8 +1595,13 @@ cudaError_t hegv_lowest(double2 *T, double2 *G, int n, int k, double *lam_out, d
         // the per-column barrier cheap for small n
         nblk = std::max(1, std::min(nblk, (n + 7) / 8));
         if ((e_ = cudaMemsetAsync(ctr, 0, sizeof(unsigned), st)) != cudaSuccess) return e_;
-        void *args[] = {(void *)&Cm, (void *)&n, (void *)&d, (void *)&e, (void *)&tau, (void *)&xg, (void *)&ctr, (void *)&err};
+        void *args[] = {(void *)&Cm, (void *)&n, (void *)&jend, (void *)&d, (void *)&e, (void *)&tau, (void *)&xg, (void *)&ctr, (void *)&err};
         if ((e_ = cudaLaunchCooperativeKernel((const void *)k_tridiag, nblk, COOP_THREADS, args, smem, st)) != cudaSuccess)
+            return e_;
+    }
+    if (ncl >= 1) {
+        if ((e_ = cudaLaunchKernelEx(&cf, fc, Cm + (size_t)jend * (n + 1), n - jend, n, d + jend, e + jend, tau + jend, err)) !=
+            cudaSuccess)
             return e_;
     }
     // a non-finite T or G reaches the tridiagonal matrix: report it (the

@@ -54,6 +54,13 @@ def test_orders(ctx, n, k):
     check(ctx, herm(n, n), k)
 
 
+@pytest.mark.parametrize("n,k", [(16, 16), (17, 3), (255, 80), (256, 256), (258, 70), (512, 40), (1024, 9), (1025, 9)])
+def test_last_columns_in_one_cluster(ctx, n, k):
+    """The last 256 columns of the tridiagonalisation go to one cluster, those
+    before them to the grid (registers up to 1024, L2 above)."""
+    check(ctx, herm(n, n), k)
+
+
 @pytest.mark.parametrize("n,k", [(1, 1), (33, 11), (100, 100), (480, 160), (545, 300)])
 def test_generalized(ctx, n, k):
     r = np.random.default_rng(n + 1)
