@@ -924,7 +924,14 @@ int apply_multi_T(pw_ctx *c, int nk, const int *iks, int ispin, void *const *psi
     if (vnl && c->nbeta > 2048) return fail(c, PW_ERR_UNSUPPORTED, "the batched op_V_Ps_nloc takes at most 2048 projectors");
     std::vector<MkK> tab(nk);
     std::vector<int> band_k;
-    std::vector<int2> groups;   // (k-point entry, first band) of each 16 bands: the nonlocal part's CTAs
+    // (k-point entry, first band) of the nonlocal part's CTAs: 16 bands each if
+    // that gives one to every SM and does not only add empty columns, else 8
+    // (Al4, FP32 op_H, 172 k-points x 4 bands: 431 us with 16, 392 with 8; with few
+    // k-points 16 were slower than one band a CTA, 125 us against 109)
+    std::vector<int2> groups;
+    int n16 = 0, n8 = 0;
+    for (int i = 0; i < nk; ++i) n16 += (nb[i] + 15) / 16, n8 += (nb[i] + 7) / 8;
+    const int gbands = n16 < 148 || n8 == n16 ? 8 : 16;
     size_t aoff = 0;
     int maxcol = 0, maxnb = 0, kx = iks[0];
     for (int i = 0; i < nk; ++i) {
@@ -942,7 +949,7 @@ int apply_multi_T(pw_ctx *c, int nk, const int *iks, int ispin, void *const *psi
         K.nb = nb[i];
         aoff += (size_t)nb[i] * c->N3 * kd.Ncol;
         band_k.insert(band_k.end(), nb[i], i);
-        for (int b = 0; b < nb[i]; b += 16) groups.push_back(make_int2(i, b));
+        for (int b = 0; b < nb[i]; b += gbands) groups.push_back(make_int2(i, b));
         maxcol = std::max(maxcol, kd.Ncol);
         maxnb = std::max(maxnb, nb[i]);
         if (kd.Nxa > c->k[kx].Nxa) kx = iks[i];
@@ -1000,7 +1007,7 @@ int apply_multi_T(pw_ctx *c, int nk, const int *iks, int ispin, void *const *psi
         }
         nlaunch = vnl ? 4 : 3;
         return launch_multik<T>(L, d_tab, d_bk, nk, nbands, maxnb, maxcol, V, c->A.p, flags, c->d_Drow, c->d_Dcol,
-                                c->d_Dval, vnl ? c->nbeta : 0, d_gr, (int)groups.size(), st);
+                                c->d_Dval, vnl ? c->nbeta : 0, d_gr, (int)groups.size(), gbands, st);
     };
     CK(c, run(c->stream));
     c->launches += nlaunch;

@@ -998,28 +998,30 @@ __device__ __forceinline__ void vnl_body(const MkK *__restrict__ ks, const int *
     }
 }
 
-// The same for up to 16 bands of one k-point per CTA on the FP64 tensor cores
+// The same for up to 8 NT bands of one k-point per CTA on the FP64 tensor cores
 // (m8n8k4: exact FP64 products and sums, FP32 operands converted in
 // registers): P = betaNL' psi with the G+k range split over the warps (three
-// 8 x 8 projector x band tiles by two a warp, then a sum over the warps), P2 =
-// D P, Hpsi += betaNL P2 with 8 G+k rows x 16 bands a warp.  Operand fragments
+// 8 x 8 projector x band tiles by NT a warp, then a sum over the warps), P2 =
+// D P, Hpsi += betaNL P2 with 8 G+k rows x 8 NT bands a warp.  gridDim.y CTAs
+// share a group's rows of the last step (each forms P for itself).  Operand fragments
 // come straight from global memory (runs of 4 or 8 values).  One CTA per band
 // (vnl_body) reads betaNL once a band and projector and converts each value
 // again for each; here a k-point's bands share both.  Bound by the FP64 pipe
 // (10 of 16 bands used: Al4, 260 k-points, 10 bands each: op_H 672 -> 576 us).
-constexpr int VT_BANDS = 16, VT_PB = VT_BANDS + 2, VT_J = 24;   // pitch 18: fragment reads hit 8 banks of 16 bytes
-inline size_t vnl_t_smem(int nbeta) {
-    return ((size_t)2 * ((nbeta + 7) / 8 * 8) * VT_PB + 8 * VT_J * VT_BANDS) * sizeof(double2);
+constexpr int VT_J = 24;
+inline size_t vnl_t_smem(int nbeta, int NT) {
+    return ((size_t)2 * ((nbeta + 7) / 8 * 8) * (8 * NT + 2) + 8 * VT_J * 8 * NT) * sizeof(double2);
 }
 __device__ __forceinline__ void vt_dmma(double (&c)[2], double a, double b) {
     asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
                  : "+d"(c[0]), "+d"(c[1])
                  : "d"(a), "d"(b));
 }
-template <typename T>
+template <typename T, int NT>
 __global__ void __launch_bounds__(256)
 mk_vnl_t(const MkK *__restrict__ ks, const int2 *__restrict__ groups, const int *__restrict__ Drow,
          const int *__restrict__ Dcol, const double *__restrict__ Dval, int nbeta) {
+    constexpr int VT_BANDS = 8 * NT, VT_PB = VT_BANDS + 2;   // pitch 10 or 18: fragment reads hit 8 banks of 16 bytes
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int nbr = (nbeta + 7) / 8 * 8;
     double2 *P = reinterpret_cast<double2 *>(smem_raw), *P2 = P + (size_t)nbr * VT_PB, *red = P2 + (size_t)nbr * VT_PB;
@@ -1032,24 +1034,24 @@ mk_vnl_t(const MkK *__restrict__ ks, const int2 *__restrict__ groups, const int 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
     const Cx<T> zero = cmake((T)0, (T)0);
     for (int j0 = 0; j0 < nbeta; j0 += VT_J) {
-        double re[3][2][2], im[3][2][2];
+        double re[3][NT][2], im[3][NT][2];
 #pragma unroll
         for (int i = 0; i < 3; ++i)
 #pragma unroll
-            for (int n = 0; n < 2; ++n) re[i][n][0] = re[i][n][1] = im[i][n][0] = im[i][n][1] = 0.0;
+            for (int n = 0; n < NT; ++n) re[i][n][0] = re[i][n][1] = im[i][n][0] = im[i][n][1] = 0.0;
 #pragma unroll 2
         for (int k0 = 4 * warp; k0 < ngw; k0 += 32) {
             const int gk = k0 + t;
-            Cx<T> a[3], b[2];
+            Cx<T> a[3], b[NT];
 #pragma unroll
             for (int i = 0; i < 3; ++i) {
                 const int j = j0 + 8 * i + g;
                 a[i] = gk < ngw && j < nbeta ? beta[(size_t)j * ngw + gk] : zero;
             }
 #pragma unroll
-            for (int n = 0; n < 2; ++n) b[n] = gk < ngw && 8 * n + g < nbl ? ps[(size_t)(8 * n + g) * K.ld + gk] : zero;
+            for (int n = 0; n < NT; ++n) b[n] = gk < ngw && 8 * n + g < nbl ? ps[(size_t)(8 * n + g) * K.ld + gk] : zero;
 #pragma unroll
-            for (int n = 0; n < 2; ++n) {
+            for (int n = 0; n < NT; ++n) {
                 const double br = b[n].x, bi = b[n].y;
 #pragma unroll
                 for (int i = 0; i < 3; ++i) {
@@ -1064,7 +1066,7 @@ mk_vnl_t(const MkK *__restrict__ ks, const int2 *__restrict__ groups, const int 
 #pragma unroll
         for (int i = 0; i < 3; ++i)
 #pragma unroll
-            for (int n = 0; n < 2; ++n)
+            for (int n = 0; n < NT; ++n)
 #pragma unroll
                 for (int q = 0; q < 2; ++q)
                     red[(warp * VT_J + 8 * i + g) * VT_BANDS + 8 * n + 2 * t + q] = make_double2(re[i][n][q], im[i][n][q]);
@@ -1090,24 +1092,26 @@ mk_vnl_t(const MkK *__restrict__ ks, const int2 *__restrict__ groups, const int 
         P2[i * VT_PB + b] = sum;
     }
     __syncthreads();
-    for (int m0 = 8 * warp; m0 < ngw; m0 += 64) {
+    for (int m0 = 8 * (warp + 8 * blockIdx.y); m0 < ngw; m0 += 64 * gridDim.y) {
         const int gk = m0 + g;
-        Cx<T> h[2][2];
+        Cx<T> h[NT][2];
 #pragma unroll
-        for (int n = 0; n < 2; ++n)
+        for (int n = 0; n < NT; ++n)
 #pragma unroll
             for (int q = 0; q < 2; ++q) {
                 const int b = 8 * n + 2 * t + q;
                 h[n][q] = gk < ngw && b < nbl ? hs[(size_t)b * K.ld + gk] : zero;
             }
-        double re[2][2] = {{0.0, 0.0}, {0.0, 0.0}}, im[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+        double re[NT][2], im[NT][2];
+#pragma unroll
+        for (int n = 0; n < NT; ++n) re[n][0] = re[n][1] = im[n][0] = im[n][1] = 0.0;
 #pragma unroll 4
         for (int j0 = 0; j0 < nbeta; j0 += 4) {
             const int j = j0 + t;
             const Cx<T> a = gk < ngw && j < nbeta ? beta[(size_t)j * ngw + gk] : zero;
             const double ar = a.x, ai = a.y;
 #pragma unroll
-            for (int n = 0; n < 2; ++n) {
+            for (int n = 0; n < NT; ++n) {
                 const double2 b = P2[j * VT_PB + 8 * n + g];
                 vt_dmma(re[n], ar, b.x);
                 vt_dmma(im[n], ar, b.y);
@@ -1116,7 +1120,7 @@ mk_vnl_t(const MkK *__restrict__ ks, const int2 *__restrict__ groups, const int 
             }
         }
 #pragma unroll
-        for (int n = 0; n < 2; ++n)
+        for (int n = 0; n < NT; ++n)
 #pragma unroll
             for (int q = 0; q < 2; ++q) {
                 const int b = 8 * n + 2 * t + q;
@@ -1417,7 +1421,7 @@ static cudaError_t launch_plane_rho64_x(const FftLaunch &L, const void *A, int n
 template <typename T>
 cudaError_t launch_multik(const FftLaunch &L, const MkK *ks, const int *band_k, int nk, int nbands, int max_nb,
                           int max_ncol, const void *Vr, void *A, int flags, const int *Drow, const int *Dcol,
-                          const double *Dval, int nbeta, const int2 *groups, int ngroups, cudaStream_t st) {
+                          const double *Dval, int nbeta, const int2 *groups, int ngroups, int gbands, cudaStream_t st) {
     const KPlan &kp = L.kp;
     if (kp.N1 != kp.N2 || kp.N2 != kp.N3) return cudaErrorNotSupported;
     const int Cg = L.Cg;
@@ -1463,11 +1467,19 @@ cudaError_t launch_multik(const FftLaunch &L, const MkK *ks, const int *band_k, 
 #undef PW_CASE
     if (e != cudaSuccess) return e;
     if (nbeta > 0) {
-        // 16 bands of a k-point a CTA where P and P2 of that many fit in shared
-        // memory with two CTAs an SM; one band a CTA beyond
-        if (vnl_t_smem(nbeta) <= 113 * 1024) {
-            if ((e = set_smem<T>((const void *)mk_vnl_t<T>, vnl_t_smem(nbeta))) != cudaSuccess) return e;
-            mk_vnl_t<T><<<ngroups, 256, vnl_t_smem(nbeta), st>>>(ks, groups, Drow, Dcol, Dval, nbeta);
+        // gbands (8 or 16) bands of a k-point a CTA where P and P2 of that many fit
+        // in shared memory with two CTAs an SM; one band a CTA beyond.  Few
+        // groups: up to four CTAs share a group's rows.
+        const int NT = gbands / 8;
+        const size_t tsm = vnl_t_smem(nbeta, NT);
+        if (tsm <= 113 * 1024) {
+            const dim3 grid(ngroups, std::max(1, std::min(4, 148 / ngroups)));
+            const void *fn = NT == 2 ? (const void *)mk_vnl_t<T, 2> : (const void *)mk_vnl_t<T, 1>;
+            if ((e = set_smem<T>(fn, tsm)) != cudaSuccess) return e;
+            if (NT == 2)
+                mk_vnl_t<T, 2><<<grid, 256, tsm, st>>>(ks, groups, Drow, Dcol, Dval, nbeta);
+            else
+                mk_vnl_t<T, 1><<<grid, 256, tsm, st>>>(ks, groups, Drow, Dcol, Dval, nbeta);
             return cudaGetLastError();
         }
         const size_t vsm = 2 * (size_t)nbeta * sizeof(double2);
@@ -1665,7 +1677,7 @@ cudaError_t launch_zero(void *p, int Ngw, int nb, int64_t ld, cudaStream_t st) {
                                                      const double *, int, unsigned *, int *, cudaStream_t);         \
     template cudaError_t launch_multik<T>(const FftLaunch &, const MkK *, const int *, int, int, int, int,           \
                                           const void *, void *, int, const int *, const int *, const double *, int,  \
-                                          const int2 *, int, cudaStream_t);                                                             \
+                                          const int2 *, int, int, cudaStream_t);                                                             \
     template cudaError_t launch_plane_rho<T>(const FftLaunch &, const void *, int, int, int, const double *, void *, \
                                              cudaStream_t);                                                          \
     template cudaError_t launch_rho_reduce<T>(const void *, int, size_t, double *, int, cudaStream_t);              \

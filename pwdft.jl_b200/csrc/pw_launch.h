@@ -71,7 +71,7 @@ cudaError_t launch_build_beta(const double *gk, int ngw, const ProjCol *cols, in
 template <typename T>
 cudaError_t launch_multik(const FftLaunch &L, const MkK *ks, const int *band_k, int nk, int nbands, int max_nb,
                           int max_ncol, const void *Vr, void *A, int flags, const int *Drow, const int *Dcol,
-                          const double *Dval, int nbeta, const int2 *groups, int ngroups, cudaStream_t st);
+                          const double *Dval, int nbeta, const int2 *groups, int ngroups, int gbands, cudaStream_t st);
 template <typename T>
 cudaError_t launch_multik_persistent(const FftLaunch &L, const MkK *ks, const int *band_k, int nbands, int max_ncol,
                                      const void *Vr, void *A, int flags, const int *Drow, const int *Dcol,

@@ -68,6 +68,24 @@ def test_apply_multi_matches_oracle_and_per_k(al4, prec):
     ctx.check_device()
 
 
+@pytest.mark.parametrize("prec", ["c128", "c64"])
+@pytest.mark.parametrize("nk,bands", [(2, (3, 1)), (36, (8, 5, 1)), (180, (7, 8)), (180, (1, 8, 9, 16, 17))])
+def test_apply_multi_band_groups(al4, prec, nk, bands):
+    """Few and many entries, with 8 or 16 bands a CTA of the nonlocal part."""
+    import torch
+    Ho, ctx, psis = al4
+    dt = torch.complex128 if prec == "c128" else torch.complex64
+    iks = [i % len(psis) for i in range(nk)]
+    X = _dev([np.tile(psis[ik], (1, 2))[:, i % 3:i % 3 + bands[i % len(bands)]] for i, ik in enumerate(iks)], dt)
+    HX = [torch.empty_like(x) for x in X]
+    ctx.apply_multi(iks, 0, X, HX)
+    for i, ik in enumerate(iks):
+        one = torch.empty_like(X[i])
+        ctx.apply(ik, 0, X[i], one)
+        assert _rel(HX[i].cpu().numpy(), one.cpu().numpy()) < (1e-13 if prec == "c128" else 1e-6), i
+    ctx.check_device()
+
+
 def test_apply_multi_accumulate_subset_and_graph(al4):
     import torch
     import pwb200
