@@ -33,7 +33,7 @@
 // values, 2-3 stage TMA -> MMA pipeline on mbarriers, split-K over gridDim.z
 // into an FP32 workspace, then a finalize kernel that sums the splits and
 // writes the complex result (FP32 or FP64, overwrite or add); a single split
-// goes through shared memory straight into C.
+// goes through shared memory straight into C.  Persistent CTAs, one an SM.
 // Warp roles: warp 0 = TMA producer, warp 1 = TMEM owner + MMA issuer,
 // warps 2..5 = epilogue of Re C, warps 6..9 of Im C (TMEM -> registers ->
 // global).  Every mbarrier wait is bounded; on expiry the CTA records an error
@@ -53,6 +53,7 @@ constexpr int TILE_A_BYTES = BM * BK * 2;   // 16 KB per A operand tile
 constexpr int THREADS = 320;
 constexpr long long WAIT_LIMIT = 1ll << 26;
 constexpr int MAX_STAGES = 3;
+constexpr int EC = 32;                      // output columns that the epilogue writes at a time
 
 // NS = number of BF16 pieces per FP32 value: 2 (hi, lo: 3 products, ~2^-17)
 // or 3 (hi, mid, lo: 6 products, ~2^-24, for products with heavy
@@ -64,8 +65,11 @@ template <int NS, int BN> struct Cfg {
     static constexpr int STAGE_BYTES = NS * (TILE_A_BYTES + TILE_B_BYTES);
     static constexpr int STAGES = (225 * 1024) / STAGE_BYTES < MAX_STAGES ? (225 * 1024) / STAGE_BYTES : MAX_STAGES;
     static_assert(STAGES >= 2, "at least a double-buffered pipeline");
-    // the epilogue's copy of the tile (BN columns of BM + 1 complex values) reuses the stages
-    static_assert((size_t)BN * (BM + 1) * 8 <= (size_t)STAGES * STAGE_BYTES, "output tile fits the stages");
+    // the epilogue's copy of EC columns (of BM + 1 complex values) has its own
+    // place where it fits beside the stages; else a CTA runs one tile and
+    // reuses them
+    static constexpr bool OWN_E = 1024 + STAGES * STAGE_BYTES + EC * (BM + 1) * 8 + 256 <= 227 * 1024;
+    static constexpr int E_BYTES = OWN_E ? EC * (BM + 1) * 8 : 0;
     // Re and Im accumulators, double-buffered, each from a multiple of 32
     // columns on; allocation a power of two >= 32
     static constexpr int ACC = (BN + 31) / 32 * 32;
@@ -85,7 +89,7 @@ struct __align__(8) Bars {
     int failed;
 };
 template <int NS, int BN> constexpr size_t smem_bytes() {
-    return 1024 + (size_t)Cfg<NS, BN>::STAGES * Cfg<NS, BN>::STAGE_BYTES + sizeof(Bars);
+    return 1024 + (size_t)Cfg<NS, BN>::STAGES * Cfg<NS, BN>::STAGE_BYTES + Cfg<NS, BN>::E_BYTES + sizeof(Bars);
 }
 
 __device__ __forceinline__ uint32_t su32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -147,37 +151,74 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
 }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
+// EC columns of a tile from shared memory (T2, columns of BM + 1) to C: thread
+// (r, h) writes row r of every other column, UB old values loaded together.
+template <typename E>
+__device__ __forceinline__ void store_columns(E *C, int64_t ld, const float2 *T2, int m0, int n0, int M, int N, int cols,
+                                              bool add, bool up) {
+    constexpr int UB = sizeof(E) == 16 ? 4 : 8;
+    const int t = threadIdx.x - 64, r = t & (BM - 1), h = t >> 7, i = m0 + r;
+#pragma unroll 1
+    for (int c = h; c < cols; c += 2 * UB) {
+        E o[UB];
+#pragma unroll
+        for (int u = 0; u < UB; ++u) {
+            const int n = n0 + c + 2 * u;
+            o[u].x = o[u].y = 0;
+            if (add && i < M && n < N && !(up && i > n)) o[u] = C[(size_t)n * ld + i];
+        }
+#pragma unroll
+        for (int u = 0; u < UB; ++u) {
+            const int n = n0 + c + 2 * u;
+            if (i < M && n < N && !(up && i > n)) {
+                const float2 v = T2[(c + 2 * u) * (BM + 1) + r];
+                o[u].x += v.x;
+                o[u].y += v.y;
+                C[(size_t)n * ld + i] = o[u];
+            }
+        }
+    }
+}
+
 // C (m x n complex) = sum over the split's k-blocks of the piece products
 //   NS = 2:  A0 B0 + A0 B1 + A1 B0
 //   NS = 3:  A0 B0 + A0 B1 + A1 B0 + A0 B2 + A1 B1 + A2 B0
 // written to W[z][n][m] (float2, column-major, ld = m), or, with a single
-// split (gridDim.z == 1) and C given, into the result C (element (i, j) at
+// split (S == 1) and C given, into the result C (element (i, j) at
 // C[j ldc + i]; cdouble: C is complex128; accumulate: C += D; upper: only
 // i <= j written).
+// A CTA runs the tiles blockIdx.x, + gridDim.x, ... of the (split, row block,
+// column block) list, the column block fastest: the CTAs that share a row block
+// of a tall A run together, so that A comes from DRAM once, and the products of
+// a CTA's next tile run while its epilogue writes the last one.  (betaNL D P of 64
+// atoms, 160 bands 118 -> 63 us against one tile a CTA, row blocks fastest, of
+// 216 atoms, 480 bands 1.51 -> 1.07 ms, there bound by the tensor pipe at 57 % of
+// its rate; Q U of 480 bands 1.36 -> 1.27 ms.)
 template <int NS, int BN>
 __global__ void __launch_bounds__(THREADS, 1)
 k_umma_gemm(const __grid_constant__ CUtensorMap tA0, const __grid_constant__ CUtensorMap tA1,
             const __grid_constant__ CUtensorMap tA2, const __grid_constant__ CUtensorMap tB0,
             const __grid_constant__ CUtensorMap tB1, const __grid_constant__ CUtensorMap tB2, int M, int N, int KB,
             int kb_per, float2 *__restrict__ W, int *__restrict__ err, int upper, int lolo, void *__restrict__ C,
-            int64_t ldc, int cdouble, int accumulate) {
+            int64_t ldc, int cdouble, int accumulate, int S) {
     using CF = Cfg<NS, BN>;
     constexpr int STAGES = CF::STAGES;
     constexpr int STAGE_BYTES = CF::STAGE_BYTES;
     constexpr int TB = CF::TILE_B_BYTES;
     constexpr int TA = TILE_A_BYTES;
-    const int m0 = blockIdx.x * BM, n0 = blockIdx.y * BN;
+    const int mt = (M + BM - 1) / BM, nt = (N + BN - 1) / BN, tiles = mt * nt * S;
     // upper: C = Z^H W is Hermitian and only its upper triangle is read; a
-    // tile whose rows all lie below its columns is skipped before any barrier
-    // or TMEM allocation
-    if (upper && m0 > n0 + BN - 1) return;
+    // tile whose rows all lie below its columns is skipped (with one tile a CTA
+    // before any barrier or TMEM allocation)
+    auto skipped = [&](int t) { return upper && (t / nt % mt) * BM > (t % nt) * BN + BN - 1; };
+    if ((int)gridDim.x >= tiles && skipped(blockIdx.x)) return;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char *smem = (unsigned char *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    Bars *bars = reinterpret_cast<Bars *>(smem + (size_t)STAGES * STAGE_BYTES);
+    Bars *bars = reinterpret_cast<Bars *>(smem + (size_t)STAGES * STAGE_BYTES + CF::E_BYTES);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int kb0 = blockIdx.z * kb_per;
-    const int kb1 = min(KB, kb0 + kb_per);
-    const int nkb = max(0, kb1 - kb0);
+    // the tile's k-blocks [kb0, kb0 + count)
+    auto first_kb = [&](int t) { return t / (nt * mt) * kb_per; };
+    auto count_kb = [&](int t) { return max(0, min(KB - first_kb(t), kb_per)); };
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < STAGES; ++s) {
@@ -203,28 +244,35 @@ k_umma_gemm(const __grid_constant__ CUtensorMap tA0, const __grid_constant__ CUt
 
     if (warp == 0 && lane == 0) {
         // ---------------- TMA producer
-        for (int i = 0; i < nkb; ++i) {
-            const int s = i % STAGES;
-            const uint32_t ph = (uint32_t)((i / STAGES) & 1);
-            if (!mbar_wait(&bars->empty[s], ph ^ 1)) {
-                bars->failed = 1;
-                break;
+        int i = 0;   // k-blocks of all tiles so far
+        bool ok = true;
+        for (int t = blockIdx.x; ok && t < tiles; t += gridDim.x) {
+            if (skipped(t)) continue;
+            const int m0 = (t / nt % mt) * BM, n0 = (t % nt) * BN, kb0 = first_kb(t), nkb = count_kb(t);
+            for (int k = 0; k < nkb; ++k, ++i) {
+                const int s = i % STAGES;
+                const uint32_t ph = (uint32_t)((i / STAGES) & 1);
+                if (!mbar_wait(&bars->empty[s], ph ^ 1)) {
+                    bars->failed = 1;
+                    ok = false;
+                    break;
+                }
+                unsigned char *st = smem + (size_t)s * STAGE_BYTES;
+                mbar_expect_tx(&bars->full[s], STAGE_BYTES);
+                const int kc = (kb0 + k) * BK;
+                // stage layout: A pieces 0..NS-1, then B pieces 0..NS-1
+                tma_load_2d(st, &tA0, &bars->full[s], kc, m0);
+                tma_load_2d(st + TA, &tA1, &bars->full[s], kc, m0);
+                if constexpr (NS == 3) tma_load_2d(st + 2 * TA, &tA2, &bars->full[s], kc, m0);
+                tma_load_2d(st + NS * TA, &tB0, &bars->full[s], kc, n0);
+                tma_load_2d(st + NS * TA + TB, &tB1, &bars->full[s], kc, n0);
+                if constexpr (NS == 3) tma_load_2d(st + NS * TA + 2 * TB, &tB2, &bars->full[s], kc, n0);
             }
-            unsigned char *st = smem + (size_t)s * STAGE_BYTES;
-            mbar_expect_tx(&bars->full[s], STAGE_BYTES);
-            const int kc = (kb0 + i) * BK;
-            // stage layout: A pieces 0..NS-1, then B pieces 0..NS-1
-            tma_load_2d(st, &tA0, &bars->full[s], kc, m0);
-            tma_load_2d(st + TA, &tA1, &bars->full[s], kc, m0);
-            if constexpr (NS == 3) tma_load_2d(st + 2 * TA, &tA2, &bars->full[s], kc, m0);
-            tma_load_2d(st + NS * TA, &tB0, &bars->full[s], kc, n0);
-            tma_load_2d(st + NS * TA + TB, &tB1, &bars->full[s], kc, n0);
-            if constexpr (NS == 3) tma_load_2d(st + NS * TA + 2 * TB, &tB2, &bars->full[s], kc, n0);
         }
         // wait (bounded) for the loads still in flight before leaving
-        for (int i = max(0, nkb - STAGES); i < nkb; ++i) {
-            const int s = i % STAGES;
-            if (!mbar_wait(&bars->full[s], (uint32_t)((i / STAGES) & 1))) bars->failed = 1;
+        for (int j = max(0, i - STAGES); j < i; ++j) {
+            const int s = j % STAGES;
+            if (!mbar_wait(&bars->full[s], (uint32_t)((j / STAGES) & 1))) bars->failed = 1;
         }
     } else if (warp == 1 && lane == 0) {
         // ---------------- MMA issuer: every k-block accumulates into a fresh
@@ -233,6 +281,9 @@ k_umma_gemm(const __grid_constant__ CUtensorMap tA0, const __grid_constant__ CUt
         // touches each value only a few times; the epilogue sums the tiles
         // with round-to-nearest adds (chains of 2 to 8 k-blocks gain at most
         // 6 % and bias the Gram diagonal by -6e-7 to -3e-6, one by -1e-7)
+        int nkb = 0;   // of all tiles
+        for (int t = blockIdx.x; t < tiles; t += gridDim.x)
+            if (!skipped(t)) nkb += count_kb(t);
         for (int i = 0; i < nkb; ++i) {
             const int s = i % STAGES;
             const uint32_t ph = (uint32_t)((i / STAGES) & 1);
@@ -278,92 +329,74 @@ k_umma_gemm(const __grid_constant__ CUtensorMap tA0, const __grid_constant__ CUt
         // tiles summed in registers
         const int q = warp & 3, part = warp >= 6 ? 1 : 0;
         const int ml = 32 * q + lane;
-        // the values to add to, on their way to L2 while the products run (the
-        // epilogue has no other CTA on its SM to hide behind: betaNL P of 216
-        // atoms took 1.51 ms with plain loads at the end)
-        const bool direct = gridDim.z == 1 && C;
-        if (direct && accumulate) {
-            const int es = cdouble ? 16 : 8, rows = 128 / es, lines = BM / rows;
-            for (int e = threadIdx.x - 64; e < BN * lines; e += 256) {
-                const int n = n0 + e / lines, i = m0 + (e % lines) * rows;
-                if (n < N && i < M)
-                    asm volatile("prefetch.global.L2 [%0];" ::"l"((const char *)C + ((size_t)n * ldc + i) * es));
-            }
-        }
-        float acc[BN];
-#pragma unroll
-        for (int t = 0; t < BN; ++t) acc[t] = 0.f;
+        const bool direct = S == 1 && C;
         bool ok = true;
-        for (int i = 0; i < nkb; ++i) {
-            const int b = i & 1;
-            const uint32_t tu = (uint32_t)((i >> 1) & 1);
-            if (!mbar_wait(&bars->tfull[b], tu)) {
-                ok = false;
-                break;
-            }
-            fence_after();
-            const uint32_t ta = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)((2 * b + part) * CF::ACC);
-            // two 16-column loads in flight
-#pragma unroll
-            for (int c = 0; c < BN / 16; c += 2) {
-                uint32_t r0[16], r1[16];
-                tmem_ld16(ta + 16 * c, r0);
-                if (c + 1 < BN / 16) tmem_ld16(ta + 16 * (c + 1), r1);
-                tmem_wait_ld();
-#pragma unroll
-                for (int t = 0; t < 16; ++t) acc[16 * c + t] += __uint_as_float(r0[t]);
-                if (c + 1 < BN / 16) {
-#pragma unroll
-                    for (int t = 0; t < 16; ++t) acc[16 * (c + 1) + t] += __uint_as_float(r1[t]);
+        int it = 0;   // k-blocks of all tiles so far
+        for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
+            if (skipped(t)) continue;
+            const int m0 = (t / nt % mt) * BM, n0 = (t % nt) * BN, nkb = count_kb(t);
+            // the values to add to, on their way to L2 while the products run
+            // (betaNL P of 216 atoms took 1.51 ms with plain loads at the end)
+            if (direct && accumulate) {
+                const int es = cdouble ? 16 : 8, rows = 128 / es, lines = BM / rows;
+                for (int e = threadIdx.x - 64; e < BN * lines; e += 256) {
+                    const int n = n0 + e / lines, i = m0 + (e % lines) * rows;
+                    if (n < N && i < M)
+                        asm volatile("prefetch.global.L2 [%0];" ::"l"((const char *)C + ((size_t)n * ldc + i) * es));
                 }
             }
-            fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&bars->tempty[b]);
+            float acc[BN];
+#pragma unroll
+            for (int c = 0; c < BN; ++c) acc[c] = 0.f;
+            for (int k = 0; k < nkb; ++k, ++it) {
+                const int b = it & 1;
+                const uint32_t tu = (uint32_t)((it >> 1) & 1);
+                // (after a wait ran out: no more waits, but every barrier below)
+                ok = ok && mbar_wait(&bars->tfull[b], tu);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                fence_after();
+                const uint32_t ta = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)((2 * b + part) * CF::ACC);
+                // two 16-column loads in flight
+#pragma unroll
+                for (int c = 0; c < BN / 16; c += 2) {
+                    uint32_t r0[16], r1[16];
+                    tmem_ld16(ta + 16 * c, r0);
+                    if (c + 1 < BN / 16) tmem_ld16(ta + 16 * (c + 1), r1);
+                    tmem_wait_ld();
+#pragma unroll
+                    for (int u = 0; u < 16; ++u) acc[16 * c + u] += __uint_as_float(r0[u]);
+                    if (c + 1 < BN / 16) {
+#pragma unroll
+                        for (int u = 0; u < 16; ++u) acc[16 * (c + 1) + u] += __uint_as_float(r1[u]);
+                    }
+                }
+                fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&bars->tempty[b]);
+            }
+            // through shared memory (with one tile a CTA maybe the stages: every
+            // MMA has completed), so that complex values leave in runs along the rows
+            float *T = reinterpret_cast<float *>(smem + (CF::OWN_E ? (size_t)STAGES * STAGE_BYTES : 0));
+#pragma unroll
+            for (int c0 = 0; c0 < BN; c0 += EC) {
+                constexpr int LAST = BN % EC ? BN % EC : EC;
+                const int cols = c0 + EC <= BN ? EC : LAST;
+#pragma unroll
+                for (int c = 0; c < EC; ++c)
+                    if (c0 + c < BN) T[2 * (c * (BM + 1) + ml) + part] = acc[c0 + c];
+                asm volatile("bar.sync 1, 256;" ::: "memory");   // the eight epilogue warps
+                const float2 *T2 = reinterpret_cast<const float2 *>(T);
+                if (!direct)
+                    store_columns(W + (size_t)(t / (nt * mt)) * M * (size_t)N, M, T2, m0, n0 + c0, M, N, cols, false, false);
+                else if (cdouble)
+                    store_columns((double2 *)C, ldc, T2, m0, n0 + c0, M, N, cols, accumulate != 0, upper != 0);
+                else
+                    store_columns((float2 *)C, ldc, T2, m0, n0 + c0, M, N, cols, accumulate != 0, upper != 0);
+                asm volatile("bar.sync 1, 256;" ::: "memory");
+            }
         }
         if (!ok) atomicExch(err, 2);
-        // the tile through shared memory (every MMA has completed: the stages
-        // are free), so that complex values leave in runs along the rows
-        float *T = reinterpret_cast<float *>(smem);
-#pragma unroll
-        for (int t = 0; t < BN; ++t) T[2 * (t * (BM + 1) + ml) + part] = acc[t];
-        asm volatile("bar.sync 1, 256;" ::: "memory");   // the eight epilogue warps
-        const float2 *T2 = reinterpret_cast<const float2 *>(smem);
-        float2 *Wz = W + (size_t)blockIdx.z * M * (size_t)N;
-        // eight values a thread and round, the old ones loaded together
-        static_assert(BN * BM % (256 * 8) == 0, "whole rounds");
-#pragma unroll 1
-        for (int e0 = threadIdx.x - 64; e0 < BN * BM; e0 += 256 * 8) {
-            float2 v[8], o[8];
-            double2 od[8];
-            size_t at[8];
-            bool in[8];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const int e = e0 + 256 * u, i = m0 + e % BM, n = n0 + e / BM;
-                v[u] = T2[(e / BM) * (BM + 1) + e % BM];
-                in[u] = i < M && n < N && !(direct && upper && i > n);
-                at[u] = (size_t)n * (direct ? ldc : (int64_t)M) + i;
-                o[u] = make_float2(0.f, 0.f);
-                od[u] = make_double2(0.0, 0.0);
-                if (direct && accumulate && in[u]) {
-                    if (cdouble)
-                        od[u] = ((const double2 *)C)[at[u]];
-                    else
-                        o[u] = ((const float2 *)C)[at[u]];
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                if (!in[u]) continue;
-                if (!direct)
-                    Wz[at[u]] = v[u];
-                else if (cdouble)
-                    ((double2 *)C)[at[u]] = make_double2(od[u].x + (double)v[u].x, od[u].y + (double)v[u].y);
-                else
-                    ((float2 *)C)[at[u]] = make_float2(o[u].x + v[u].x, o[u].y + v[u].y);
-            }
-        }
     }
     fence_before();
     __syncthreads();
@@ -645,15 +678,18 @@ size_t umma_ws_bytes(int64_t M, int N, int Kp, int splits, int upper) {
 }
 
 template <int NS, int BN>
-static cudaError_t launch_umma(const CUtensorMap *mA, const CUtensorMap *mB, dim3 grid, int M, int n, int KB, int kb_per,
+static cudaError_t launch_umma(const CUtensorMap *mA, const CUtensorMap *mB, int tiles, int M, int n, int KB, int kb_per,
                                float *ws, int *err, int upper, int lolo, void *C, int64_t ldc, int cdouble, int accumulate,
-                               cudaStream_t st) {
+                               int S, cudaStream_t st) {
     cudaError_t e = cudaFuncSetAttribute(k_umma_gemm<NS, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)smem_bytes<NS, BN>());
     if (e != cudaSuccess) return e;
+    // one CTA fits on an SM; a Hermitian product's tiles, half of them skipped,
+    // go out one a CTA
+    const int grid = !Cfg<NS, BN>::OWN_E || upper ? tiles : std::min(tiles, 148);
     k_umma_gemm<NS, BN><<<grid, THREADS, smem_bytes<NS, BN>(), st>>>(mA[0], mA[1], mA[2], mB[0], mB[1], mB[2], M, n, KB,
                                                                       kb_per, (float2 *)ws, err, upper, lolo, C, ldc, cdouble,
-                                                                      accumulate);
+                                                                      accumulate, S);
     return cudaGetLastError();
 }
 
@@ -685,15 +721,15 @@ cudaError_t umma_gemm(const UmmaOperand &A, const UmmaOperand &B, int m, int n, 
     const int KB = A.Kp / BK;
     const int S = umma_splits(A.rows, n, A.Kp, splits, upper);
     const int kb_per = (KB + S - 1) / S;
-    dim3 grid((unsigned)((A.rows + BM - 1) / BM), (n + bn - 1) / bn, S);
+    const int tiles = (int)((A.rows + BM - 1) / BM) * ((n + bn - 1) / bn) * S;
     // one split: the epilogue writes or adds into C itself, no workspace pass
     void *Cd = (S == 1 && upper != 2) ? C : nullptr;
     const int cd = sizeof(CT) == 16 ? 1 : 0;
     e = cudaErrorInvalidValue;
 #define PW_U(BN)                                                                                                     \
     if (bn == BN)                                                                                                    \
-        e = ns == 3 ? launch_umma<3, BN>(mA, mB, grid, m, n, KB, kb_per, ws, err, upper, 0, Cd, ldc, cd, accumulate, st) \
-                    : launch_umma<2, BN>(mA, mB, grid, m, n, KB, kb_per, ws, err, upper, lolo, Cd, ldc, cd, accumulate, st);
+        e = ns == 3 ? launch_umma<3, BN>(mA, mB, tiles, m, n, KB, kb_per, ws, err, upper, 0, Cd, ldc, cd, accumulate, S, st) \
+                    : launch_umma<2, BN>(mA, mB, tiles, m, n, KB, kb_per, ws, err, upper, lolo, Cd, ldc, cd, accumulate, S, st);
     PW_U(128)
     PW_U(96)
     PW_U(80)

@@ -70,3 +70,13 @@ def test_rotate_edges(ctx, M, n, k, pad):
     X.copy_(X0)
     ctx.rotate(A, U, X, accumulate=True)
     assert ((X - ref - X0).abs() <= bound + 4e-7 * (ref.abs() + X0.abs())).all()
+
+
+@pytest.mark.parametrize("M,n,k", [(40001, 20, 33), (19001, 50, 40), (40001, 70, 5), (33333, 90, 70), (20001, 250, 100)])
+def test_several_tiles_a_cta(ctx, M, n, k):
+    """More output tiles than SMs, at every tile width."""
+    test_rotate_edges(ctx, M, n, k, 0)
+
+
+def test_several_gram_tiles_a_cta(ctx):
+    test_gram_edges(ctx, 70, 1600, 1500, 1)
