@@ -219,7 +219,8 @@ k_zgemm(int64_t K, int64_t m, int n, const double2 *__restrict__ A, int64_t lda,
 // (about 2400 bytes a clock) and the reduction's launch (4000 clocks).
 // (480 x 480 over K = 23,871: 48 x 80 tiles, 0 % padding, against 14 % with
 // 64 x 64.)  Splitting stops at four CTAs an SM, which also bounds the workspace
-// (592 tiles: 49 MB).
+// (592 tiles: 49 MB).  Few values are split too (betaNL' psi of 8 bands over
+// about 730 plane waves: 35.8 us on one CTA, 5.0 in 23 parts).
 struct ZPlan {
     int wm, wn, S;
     int64_t kchunk;
@@ -238,10 +239,11 @@ ZPlan zplan(int64_t K, int64_t m, int n, bool tn, int upper, bool fused = false)
                 tiles = 0;
                 for (int64_t c = 0; c < tc; ++c) tiles += (double)std::min<int64_t>(tm, (c * 16 * wn + 16 * wn - 1) / (16 * wm) + 1);
             }
-            // splits that fill whole rounds of the 148 SMs
+            // splits that fill whole rounds of the 148 SMs, or as many as
+            // leave 32 values each
             for (int w = 0; w <= (tn ? 4 : 0); ++w) {
-                const int S = w == 0 ? 1 : (int)(148.0 * w / tiles);
-                if (w > 0 && (S < 2 || (int64_t)S * 64 > K)) continue;
+                const int S = w == 0 ? 1 : (int)std::min<int64_t>((int64_t)(148.0 * w / tiles), K / 32);
+                if (w > 0 && S < 2) continue;
                 const double kc = (double)((K + S - 1) / S);
                 const double per = std::ceil(tiles * S / 148.0);
                 double t = std::max(per * 16.0 * wm * wn * (per < 1.5 ? 1.15 : 1.0), 45.0) * (kc + 32.0);
