@@ -11,6 +11,8 @@
 // 92 us, of 32 atoms (75 x 75 x 40, 81 bands, FP64) 546 -> 490 us (z passes),
 // density and op_H on 36- to 108-point boxes 2.0 to 3.2 times faster.
 #pragma once
+#include <type_traits>
+
 #include <algorithm>
 
 #include "pw_fft_fused.cuh"
@@ -24,7 +26,10 @@ namespace any {
     X(96) X(100) X(108) X(120) X(125) X(128)
 
 constexpr int THREADS = 256, NW = THREADS / 32;
-constexpr int TWN = 64;   // twiddle entries kept per direction (2 R0 <= 54)
+// Twiddle entries kept per direction: in FP32 all N, in FP64 w^j, from which a
+// lane forms its powers (2 R0 <= 54).
+template <typename T> constexpr int TWN = sizeof(T) == 4 ? 128 : 64;
+template <typename T> using Tw = std::conditional_t<sizeof(T) == 4, pwf::FullTw<T>, const Cx<T> *>;
 
 // What the host chooses for a launch.
 struct Shape {
@@ -47,8 +52,8 @@ template <typename T> struct Sm {
     __device__ __forceinline__ Sm(const Shape &h, int nsub, int Nxa, int N2) {
         extern __shared__ __align__(16) unsigned char smem_raw[];
         tx = reinterpret_cast<Cx<T> *>(smem_raw);
-        ty = tx + TWN;
-        S = ty + TWN;
+        ty = tx + TWN<T>;
+        S = ty + TWN<T>;
         Cx<T> *x = S + (size_t)nsub * Nxa * h.LD;
         Xw = x + (threadIdx.x >> 5) * h.xw;
         P = reinterpret_cast<T *>(x + NW * h.xw);
@@ -61,7 +66,7 @@ template <typename T> struct Sm {
 // accesses stay shared-memory ones.
 template <typename T, int N2> __device__ __noinline__ void y_pass(Shape h, int nsub, int Nxa, int nl, int sign) {
     const Sm<T> m(h, nsub, Nxa, N2);
-    pwf::lines<T, N2, true, (pwf::fp_pad<N2>() > 0)>(m.S, nl, 1, h.LD, m.ty, sign);   // ends with __syncthreads
+    pwf::lines<T, N2, true, (pwf::fp_pad<N2>() > 0)>(m.S, nl, 1, h.LD, Tw<T>{m.ty}, sign);   // ends with __syncthreads
 }
 
 // Active-x rows of the elements a lane reads in the first inverse x stage (and
@@ -125,7 +130,7 @@ __device__ __noinline__ void x_vloc(Shape h, int Nxa, int N2, int nbh, const T *
             const int ia = rows.at(iax, x, r);
             if (ia >= 0) Sb[ia * LD] = v;
         };
-        pwf::group_fft_vpair<T, N1>(m.Xw, nl, m.tx, lane, ld_s, vsc, st_s);
+        pwf::group_fft_vpair<T, N1>(m.Xw, nl, Tw<T>{m.tx}, lane, ld_s, vsc, st_s);
     }
 }
 
@@ -149,12 +154,12 @@ __device__ __noinline__ void x_rho(Shape h, int Nxa, int N2, T *__restrict__ rp,
             T *p = RS ? &Rs[(g0 + line) * h.vst + x] : &rp[(g0 + line) * N1 + x];
             *p += wb * (v.x * v.x + v.y * v.y);
         };
-        pwf::group_fft<T, N1>(m.Xw, nl, m.tx, +1, lane, ld_s, st_r);
+        pwf::group_fft<T, N1>(m.Xw, nl, Tw<T>{m.tx}, +1, lane, ld_s, st_r);
     }
 }
 
 template <typename T> size_t sm_bytes(const Shape &h, int nsub, int Nxa, int N1, int N2) {
-    return ((size_t)2 * TWN + (size_t)nsub * Nxa * h.LD + (size_t)NW * h.xw) * sizeof(Cx<T>) + (size_t)N2 * h.vst * sizeof(T) +
+    return ((size_t)2 * TWN<T> + (size_t)nsub * Nxa * h.LD + (size_t)NW * h.xw) * sizeof(Cx<T>) + (size_t)N2 * h.vst * sizeof(T) +
            N1 * sizeof(short);
 }
 
@@ -203,8 +208,11 @@ template <typename T>
 __device__ __forceinline__ void setup(const KPlan &kp, const Shape &h, const Sm<T> &m, const Cx<T> *__restrict__ twx,
                                       const Cx<T> *__restrict__ twy) {
     for (int i = threadIdx.x; i < kp.N1; i += THREADS) m.iax[i] = -1;
-    for (int i = threadIdx.x; i < h.R0x; i += THREADS) m.tx[h.R0x + i] = twx[i];   // exp(-2 pi i j / N), j < R0
-    for (int i = threadIdx.x; i < h.R0y; i += THREADS) m.ty[h.R0y + i] = twy[i];
+    // entry r R0 + j: exp(-2 pi i r j / N), 1 <= r < R1 (FP64: r = 1), j < R0
+    // (one-stage plans: R0 = 0, no twiddles)
+    const int nx = sizeof(T) == 4 && h.R0x ? kp.N1 : 2 * h.R0x, ny = sizeof(T) == 4 && h.R0y ? kp.N2 : 2 * h.R0y;
+    for (int i = h.R0x + threadIdx.x; i < nx; i += THREADS) m.tx[i] = twx[i / h.R0x * (i % h.R0x)];
+    for (int i = h.R0y + threadIdx.x; i < ny; i += THREADS) m.ty[i] = twy[i / h.R0y * (i % h.R0y)];
 }
 // S := the plane's columns (zeros elsewhere), nbh bands
 template <typename T>

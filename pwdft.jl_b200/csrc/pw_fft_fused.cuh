@@ -281,6 +281,23 @@ template <typename T, int R> __device__ __forceinline__ void tw_pow(Cx<T> w1, Cx
 // Twiddles of butterfly jm of stage S (conjugated for the inverse, sign > 0)
 // applied to v[1 .. R).  Only the second stage of a two-stage plan has any;
 // its table entry tw_at(1, jm) is exp(-2 pi i jm / N).
+// With a whole table (FullTw) every power is read instead: in FP32 the powers
+// lose about a bit against entries that were rounded once (density of 8 bands, 32 /
+// 60 points: relative error 2.7e-7 / 1.3e-7 against 1.8e-7 / 1.0e-7; op_H of 8
+// atoms 69.7 against 70.1 us).
+template <typename T> struct FullTw {
+    const Cx<T> *p;
+    __device__ __forceinline__ operator const Cx<T> *() const { return p; }
+};
+template <typename T, int N, int S, int R>
+__device__ __forceinline__ void apply_tw(Cx<T> (&v)[R], FullTw<T> tw, int jm, int sign) {
+#pragma unroll
+    for (int r = 1; r < R; ++r) {
+        Cx<T> w = tw.p[tw_at<N, S>(r, jm)];
+        if (sign > 0) w.y = -w.y;
+        v[r] = cmul(v[r], w);
+    }
+}
 template <typename T, int N, int S, int R>
 __device__ __forceinline__ void apply_tw(Cx<T> (&v)[R], const Cx<T> *tw, int jm, int sign) {
     Cx<T> w1 = tw[tw_at<N, S>(1, jm)];
@@ -293,8 +310,8 @@ __device__ __forceinline__ void apply_tw(Cx<T> (&v)[R], const Cx<T> *tw, int jm,
 
 // PAD: elements at fp_pos(x) (es must be 1, two-stage plans): stage 0 writes
 // block j of R0 elements, stage 1 touches element j < R0 of block r
-template <typename T, int N, int S, bool JFAST, bool PAD>
-__device__ __forceinline__ void fstage(Cx<T> *buf, int l0, int nl, int es, int ls, const Cx<T> *tw, int sign, int lane) {
+template <typename T, int N, int S, bool JFAST, bool PAD, class TW>
+__device__ __forceinline__ void fstage(Cx<T> *buf, int l0, int nl, int es, int ls, TW tw, int sign, int lane) {
     constexpr int R = FPlan<N>::r(S);
     constexpr int NS = fp_ns<N>(S);
     constexpr int NBF = N / R;
@@ -352,8 +369,8 @@ __device__ __forceinline__ void fstage(Cx<T> *buf, int l0, int nl, int es, int l
 }
 
 // All lines [0, nlines) of length N; ends with __syncthreads().
-template <typename T, int N, bool JFAST, bool PAD = false>
-__device__ __forceinline__ void lines(Cx<T> *buf, int nlines, int es, int ls, const Cx<T> *tw, int sign) {
+template <typename T, int N, bool JFAST, bool PAD = false, class TW = const Cx<T> *>
+__device__ __forceinline__ void lines(Cx<T> *buf, int nlines, int es, int ls, TW tw, int sign) {
     constexpr int G = fp_group<N>();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     for (int l0 = warp * G; l0 < nlines; l0 += nw * G) {
@@ -373,8 +390,8 @@ namespace pwf {
 // butterfly it sits in): the first stage of a line can read its input
 // straight from another layout, the last can scale or scatter its output,
 // with no extra pass.
-template <typename T, int N, int S, class LD, class ST>
-__device__ __forceinline__ void fstage_io(int nl, const Cx<T> *tw, int sign, int lane, LD &ld, ST &st) {
+template <typename T, int N, int S, class TW, class LD, class ST>
+__device__ __forceinline__ void fstage_io(int nl, TW tw, int sign, int lane, LD &ld, ST &st) {
     constexpr int R = FPlan<N>::r(S);
     constexpr int NS = fp_ns<N>(S);
     constexpr int NBF = N / R;
@@ -410,8 +427,8 @@ __device__ __forceinline__ void fstage_io(int nl, const Cx<T> *tw, int sign, int
 // Whole N-point FFT of nl <= fp_group<N>() lines held by one warp in buf
 // (line stride fp_xs, padded positions): the first stage reads through ld0,
 // the last writes through stl, the stages between use buf.
-template <typename T, int N, class LD0, class STL>
-__device__ __forceinline__ void group_fft(Cx<T> *buf, int nl, const Cx<T> *tw, int sign, int lane, LD0 &ld0, STL &stl) {
+template <typename T, int N, class TW, class LD0, class STL>
+__device__ __forceinline__ void group_fft(Cx<T> *buf, int nl, TW tw, int sign, int lane, LD0 &ld0, STL &stl) {
     constexpr int XS = fp_xs<N>();
     // stage 0 writes element r of block (x - r) / R0, stage 1 reads element x - r R0 of block r
     auto bld = [&](int line, int x, int r) { return buf[line * XS + x + r * fp_pad<N>()]; };
@@ -435,8 +452,8 @@ __device__ __forceinline__ void group_fft(Cx<T> *buf, int nl, const Cx<T> *tw, i
 // stay in registers and one shared-memory exchange (buf) precedes the
 // radix-R0 DFTs, whose outputs go out through st(line, x, r, v).  One-stage
 // plans (one line per lane) never touch buf.
-template <typename T, int N, class LD0, class VS, class ST>
-__device__ __forceinline__ void group_fft_vpair(Cx<T> *buf, int nl, const Cx<T> *tw, int lane, LD0 &ld0, VS &vsc,
+template <typename T, int N, class TW, class LD0, class VS, class ST>
+__device__ __forceinline__ void group_fft_vpair(Cx<T> *buf, int nl, TW tw, int lane, LD0 &ld0, VS &vsc,
                                                 ST &st) {
     constexpr int NST = FPlan<N>::nst;
     static_assert(NST == 1 || NST == 2, "fused plans have one or two stages");
