@@ -283,7 +283,7 @@ template <typename T, int R> __device__ __forceinline__ void tw_pow(Cx<T> w1, Cx
 // its table entry tw_at(1, jm) is exp(-2 pi i jm / N).
 // With a whole table (FullTw) every power is read instead: in FP32 the powers
 // lose about a bit against entries that were rounded once (density of 8 bands, 32 /
-// 60 points: relative error 2.7e-7 / 1.3e-7 against 1.8e-7 / 1.0e-7; op_H of 8
+// 60 points: relative error 2.7e-7 / 1.3e-7 against 1.4e-7 / 0.8e-7; op_H of 8
 // atoms 69.7 against 70.1 us).
 template <typename T> struct FullTw {
     const Cx<T> *p;
