@@ -35,6 +35,7 @@
 
 #include "pw_eig.h"
 #include "pw_launch.h"
+#include "pw_tri.h"
 
 namespace pwk {
 namespace eig {
@@ -780,14 +781,14 @@ k_tridiag_r(double2 *C, int n, int jend, double *d, double *e, double2 *tau, dou
 // CPW columns in registers, and the pairs (y_i, entry of row j + 1) go straight
 // into every CTA's shared memory (st.async), whose mbarrier counts their bytes: a
 // column costs a distributed-shared-memory store instead of a trip through L2
-// that other SMs poll.  Two exchange buffers suffice: a CTA publishes step j + 1
-// only after it has read step j, and nobody publishes step j + 2 before having
-// everyone's step j + 1.  Waits are bounded by polls of the mbarrier; when one
+// that other SMs poll.  Two exchange buffers suffice, because a CTA leaves the
+// column loop, and is sent to no more, after its own last column (pw_tri.h); the
+// owner of column n - 1, which stays to the end, records d, e and tau.  Waits are
+// bounded by polls of the mbarrier; when one
 // runs out the CTA sets *err and waits no more, and the cluster barrier at the
 // end keeps every CTA's shared memory alive until all have finished.  n = 160 /
 // 250 take 0.34 / 0.58 ms (k_tridiag_r 0.54 / 0.93, k_tridiag 0.77 / 1.27); with
 // 32 columns a CTA, n = 480, the update bounds it: 2.20 ms, k_tridiag_r 1.92.
-constexpr int TRC = 16;   // CTAs of the cluster
 template <int NR, int W, int CPW> constexpr size_t tridiag_c_smem() {
     constexpr int SL = W * CPW;
     return ((size_t)3 * 32 * NR + 2 * (size_t)TRC * SL * 2 + 2 * SL) * sizeof(double2);
@@ -795,8 +796,9 @@ template <int NR, int W, int CPW> constexpr size_t tridiag_c_smem() {
 template <int NR, int W, int CPW>
 __global__ void __launch_bounds__(32 * W, 1)
 k_tridiag_c(double2 *C, int n, int ld, double *d, double *e, double2 *tau, int *err) {
-    constexpr int TH = 32 * W, NN = 32 * NR, EPT = NN / TH, SL = W * CPW;
+    constexpr int TH = 32 * W, NN = 32 * NR, EPT = NN / TH, SL = W * CPW, SR = TRC * 2 * SL / TH;
     static_assert(TRC * SL >= NN, "every column has a warp");
+    static_assert(SR * TH == TRC * 2 * SL, "a thread sends the same number of pairs");
     static_assert(EPT * TH == NN, "every row has a thread");
     extern __shared__ __align__(16) unsigned char sm[];
     double2 *vc = reinterpret_cast<double2 *>(sm), *vp = vc + NN, *wp = vp + NN;   // v_j, v_{j-1}, w_{j-1}
@@ -809,6 +811,11 @@ k_tridiag_c(double2 *C, int n, int ld, double *d, double *e, double2 *tau, int *
     unsigned rank;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
     const bool mute = (int)rank == g_gsync_withhold;
+    const int steps = tri_steps(n, (int)rank);   // this CTA takes part in the steps j < steps
+    const bool rec = (int)rank == tri_last_rank(n);
+    int to[SR];                                  // steps of the CTAs that this thread's pairs go to
+#pragma unroll
+    for (int u = 0; u < SR; ++u) to[u] = tri_steps(n, (tid + TH * u) / (2 * SL));
     const long long lim = g_gsync_limit;
     const unsigned bar0 = (unsigned)__cvta_generic_to_shared(&bar[0]), ex0 = (unsigned)__cvta_generic_to_shared(ex);
     if (tid == 0) {
@@ -869,7 +876,7 @@ k_tridiag_c(double2 *C, int n, int ld, double *d, double *e, double2 *tau, int *
             v[u] = row(u) <= j ? make_double2(0.0, 0.0) : row(u) == j + 1 ? make_double2(1.0, 0.0) : cmul_d(x[u], scal);
             vc[row(u)] = v[u];
         }
-        if (rank == 0 && tid == 0) {
+        if (rec && tid == 0) {
             e[j] = beta;
             tau[j] = t;
         }
@@ -877,15 +884,15 @@ k_tridiag_c(double2 *C, int n, int ld, double *d, double *e, double2 *tau, int *
         return t;
     };
 
-    if (rank == 0 && tid == 0) d[0] = x[0].x;
-    if (n >= 2) tj = householder(0);
-    for (int j = 0; j < n - 1; ++j) {
+    if (rec && tid == 0) d[0] = x[0].x;
+    if (steps > 0) tj = householder(0);
+    for (int j = 0; j < steps; ++j) {
         const int c1 = j + 1, b = j & 1;
         // this CTA's mbarrier of the step expects 32 bytes a column i > j
         const bool dead = *(volatile int *)&failed;   // a wait ran out: no more exchange
         if (tid == 0 && !dead)
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar0 + 8 * b),
-                         "r"((unsigned)(n - 1 - j) * 32u)
+                         "r"(tri_bytes(n, j))
                          : "memory");
         // ---- the warp's columns: rank-2 update with (v_{j-1}, w_{j-1}), then y = column^H v_j
         double2 cw[CPW], cv[CPW], acc[CPW];
@@ -929,10 +936,11 @@ k_tridiag_c(double2 *C, int n, int ld, double *d, double *e, double2 *tau, int *
             }
         }
         __syncthreads();
-        // ---- the CTA's pairs to every CTA of the cluster
-        for (int q = tid; q < TRC * 2 * SL; q += TH) {
-            const int it = q % (2 * SL), dst = q / (2 * SL), i = 1 + (int)rank + TRC * (it >> 1);
-            if (i > j && i < n && !mute && !dead) {
+        // ---- the CTA's pairs to every CTA that takes part in the step
+#pragma unroll
+        for (int u = 0; u < SR; ++u) {
+            const int q = tid + TH * u, it = q % (2 * SL), dst = q / (2 * SL), i = 1 + (int)rank + TRC * (it >> 1);
+            if (i > j && i < n && j < to[u] && !mute && !dead) {
                 const double2 val = ysm[it];
                 unsigned ra, rb;
                 asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
@@ -970,7 +978,7 @@ k_tridiag_c(double2 *C, int n, int ld, double *d, double *e, double2 *tau, int *
             x[u] = in ? p[1] : make_double2(0.0, 0.0);
         }
         // v_j to its place in C (all of column j has been read: every CTA has published this step)
-        if ((j % TRC) == (int)rank) {
+        if (tri_writer(j) == (int)rank) {
 #pragma unroll
             for (int u = 0; u < EPT; ++u)
                 if (row(u) > c1 && row(u) < n) C[(size_t)j * ld + row(u)] = v[u];
@@ -1001,9 +1009,9 @@ k_tridiag_c(double2 *C, int n, int ld, double *d, double *e, double2 *tau, int *
             wp[row(u)] = w;
             x[u].x -= p.x + w.x;
             x[u].y -= p.y + w.y;
-            if (row(u) == c1 && rank == 0) d[c1] = x[u].x;
+            if (row(u) == c1 && rec) d[c1] = x[u].x;
         }
-        if (c1 < n - 1) tj = householder(c1);
+        if (c1 < steps) tj = householder(c1);
     }
     // no CTA leaves while another may still store into its shared memory
     if (failed) __nanosleep(20000);
