@@ -1,12 +1,14 @@
 """Failure detection on the device, without faulting or hanging the GPU.
 
   - Bounded waits: the cooperative kernels of the FP64 eigensolver
-    (pw_eigh: Cholesky, triangular inverse, tridiagonalisation) synchronise
+    (pw_eigh: Cholesky with its inverse, tridiagonalisation) synchronise
     with a grid barrier whose waits give up after a poll limit, record an
     error word and let the kernel run to completion.  A test-only hook
     shortens the limit and makes one CTA withhold its arrivals: the others'
     waits run out, pw_eigh reports PW_ERR_TIMEOUT, and once the hook is
-    cleared the same context solves the next problem correctly.
+    cleared the same context solves the next problem correctly.  The
+    tridiagonalisation's own waits (polled words of the register kernel, the
+    mbarriers of the cluster kernel) are made to expire in the same way.
   - Non-finite values: a NaN in the density, the wavefunctions or a LOBPCG
     block is reported as PW_ERR_NAN by the FP64 reductions that meet it
     (pw_update, pw_band_energies; pw_lobpcg reports it from its Ritz values
@@ -73,6 +75,29 @@ def test_eigh_barrier_timeout_is_reported_and_context_recovers(fcc):
     lam, S = ctx.eigh(dev(T), dev(G), k=k)
     ref = sla.eigh(T, G, eigvals_only=True)[:k]
     assert np.abs(lam.cpu().numpy() - ref).max() < 1e-10 * np.abs(ref).max()
+    ctx.check_device()
+
+
+# without G there is no Cholesky, whose barrier would expire first.  CTA 0 of the
+# cluster (n = 192: only the cluster kernel runs), CTA 20 of the grid (n = 480:
+# the register kernel; the cluster has 16 CTAs, which no hook holds there)
+@pytest.mark.parametrize("n,cta", [(192, 0), (480, 20)])
+def test_tridiagonalisation_wait_expires(fcc, n, cta):
+    import torch
+    import pwb200
+    ctx = fcc.ctx
+    T, _ = _pencil(n, n)
+    dev = lambda M: torch.from_numpy(np.ascontiguousarray(M.T)).cuda()
+    try:
+        _hook(1 << 14, cta)
+        with pytest.raises(pwb200.PWError) as e:
+            ctx.eigh(dev(T), None, k=40)
+        assert e.value.status == pwb200._lib.PW_ERR_TIMEOUT
+    finally:
+        _hook(0, -1)
+    lam, _ = ctx.eigh(dev(T), None, k=40)
+    ref = np.linalg.eigvalsh(T)[:40]
+    assert np.abs(lam.cpu().numpy() - ref).max() < 1e-12 * np.abs(ref).max()
     ctx.check_device()
 
 
