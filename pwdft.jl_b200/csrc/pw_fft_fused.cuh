@@ -21,23 +21,64 @@ template <typename T> struct Dft<T, 4> { static __host__ __device__ __forceinlin
 template <typename T> struct Dft<T, 5> { static __host__ __device__ __forceinline__ void run(Cx<T> *v, T s, const Cx<T> *, int) { SmallDft<T, 5>::run(v, s); } };
 template <typename T> struct Dft<T, 8> { static __host__ __device__ __forceinline__ void run(Cx<T> *v, T s, const Cx<T> *, int) { SmallDft<T, 8>::run(v, s); } };
 
-// exp(-2 pi i m / R) evaluated at compile time: Taylor series of sin and
-// cos about 0 after reduction to [-pi, pi] (30 terms: below 1e-17 there).
-__host__ __device__ constexpr double ce_trig(double x, bool sine) {
-    constexpr double PI = 3.14159265358979323846264338327950288;
-    while (x > PI) x -= 2 * PI;
-    while (x < -PI) x += 2 * PI;
-    double term = sine ? x : 1.0, sum = term;
-    for (int k = 1; k < 30; ++k) {
-        const int a = sine ? 2 * k : 2 * k - 1, b = sine ? 2 * k + 1 : 2 * k;
-        term *= -x * x / ((double)a * (double)b);
-        sum += term;
+// exp(-2 pi i m / R) at compile time, rounded once: the angle is reduced to
+// [0, pi/4] as a fraction of a turn, and the Taylor series of sin and cos is summed
+// in pairs of doubles (the sum of a pair is exact to about 2^-100).  A series in
+// plain doubles on [-pi, pi] was off by up to 4e-16: lines of 36 to 125 points with
+// a radix of 9, 16, 25 or 27 lost up to 1.3 times the error of a rounded table.
+struct Pair {
+    double h, l;
+};
+__host__ __device__ constexpr Pair two_sum(double a, double b) {
+    const double s = a + b, t = s - a;
+    return {s, (a - (s - t)) + (b - t)};
+}
+__host__ __device__ constexpr Pair two_prod(double a, double b) {   // Dekker: 26-bit halves
+    const double ca = 134217729.0 * a, ah = ca - (ca - a), al = a - ah;
+    const double cb = 134217729.0 * b, bh = cb - (cb - b), bl = b - bh, p = a * b;
+    return {p, ((ah * bh - p) + ah * bl + al * bh) + al * bl};
+}
+__host__ __device__ constexpr Pair operator+(Pair a, Pair b) {
+    const Pair s = two_sum(a.h, b.h);
+    return two_sum(s.h, s.l + a.l + b.l);
+}
+__host__ __device__ constexpr Pair operator*(Pair a, Pair b) {
+    const Pair p = two_prod(a.h, b.h);
+    return two_sum(p.h, p.l + a.h * b.l + a.l * b.h);
+}
+__host__ __device__ constexpr Pair operator/(Pair a, double d) {
+    const double q = a.h / d;
+    const Pair p = two_prod(q, -d), r = Pair{a.h, a.l} + p;
+    return two_sum(q, r.h / d);
+}
+// cos or sin of 2 pi p / q for 0 <= p / q <= 1/8
+__host__ __device__ constexpr double ce_octant(int p, int q, bool sine) {
+    const Pair x = Pair{6.283185307179586, 2.4492935982947064e-16} * Pair{(double)p, 0.0} / (double)q;
+    const Pair x2 = x * x;
+    Pair term = sine ? x : Pair{1.0, 0.0}, sum = term;
+    for (int k = 1; k < 16; ++k) {
+        const int a = sine ? 2 * k : 2 * k - 1;
+        term = Pair{-x2.h, -x2.l} * term / (double)(a * (a + 1));
+        sum = sum + term;
     }
-    return sum;
+    return sum.h;
+}
+__host__ __device__ constexpr double ce_trig(int p, int q, bool sine) {   // 0 <= p < q
+    double sign = 1.0;
+    if (2 * p > q) {   // past half a turn: -p
+        p = q - p;
+        if (sine) sign = -sign;
+    }
+    if (4 * p > q) {   // past a quarter: half a turn less
+        p = q - 2 * p;
+        q *= 2;
+        if (!sine) sign = -sign;
+    }
+    if (8 * p > q) return sign * ce_octant(q - 4 * p, 4 * q, !sine);
+    return sign * ce_octant(p, q, sine);
 }
 template <int M, int R> struct Root {
-    static constexpr double ang = -2.0 * 3.14159265358979323846264338327950288 * (double)(M % R) / (double)R;
-    static constexpr double c = ce_trig(ang, false), s = ce_trig(ang, true);
+    static constexpr double c = ce_trig(M % R, R, false), s = -ce_trig(M % R, R, true);
 };
 
 // compile-time loop: f(std::integral_constant<int, I>) for I in [I0, I1)
