@@ -11,8 +11,6 @@
 // 92 us, of 32 atoms (75 x 75 x 40, 81 bands, FP64) 546 -> 490 us (z passes),
 // density and op_H on 36- to 108-point boxes 2.0 to 3.2 times faster.
 #pragma once
-#include <type_traits>
-
 #include <algorithm>
 
 #include "pw_fft_fused.cuh"
@@ -26,10 +24,12 @@ namespace any {
     X(96) X(100) X(108) X(120) X(125) X(128)
 
 constexpr int THREADS = 256, NW = THREADS / 32;
-// Twiddle entries kept per direction: in FP32 all N, in FP64 w^j, from which a
-// lane forms its powers (2 R0 <= 54).
-template <typename T> constexpr int TWN = sizeof(T) == 4 ? 128 : 64;
-template <typename T> using Tw = std::conditional_t<sizeof(T) == 4, pwf::FullTw<T>, const Cx<T> *>;
+// Twiddles: all N entries of a direction, in both precisions (powers formed in
+// registers cost accuracy, see pwf::FullTw).
+constexpr int TWN = 128;
+template <typename T> using Tw = pwf::FullTw<T>;
+// entry i = r R0 + j of the table, 1 <= r < R1, j < R0: exp(-2 pi i r j / N)
+__host__ __device__ __forceinline__ int tw_entry(int i, int R0) { return i / R0 * (i % R0); }
 
 // What the host chooses for a launch.
 struct Shape {
@@ -52,8 +52,8 @@ template <typename T> struct Sm {
     __device__ __forceinline__ Sm(const Shape &h, int nsub, int Nxa, int N2) {
         extern __shared__ __align__(16) unsigned char smem_raw[];
         tx = reinterpret_cast<Cx<T> *>(smem_raw);
-        ty = tx + TWN<T>;
-        S = ty + TWN<T>;
+        ty = tx + TWN;
+        S = ty + TWN;
         Cx<T> *x = S + (size_t)nsub * Nxa * h.LD;
         Xw = x + (threadIdx.x >> 5) * h.xw;
         P = reinterpret_cast<T *>(x + NW * h.xw);
@@ -159,7 +159,7 @@ __device__ __noinline__ void x_rho(Shape h, int Nxa, int N2, T *__restrict__ rp,
 }
 
 template <typename T> size_t sm_bytes(const Shape &h, int nsub, int Nxa, int N1, int N2) {
-    return ((size_t)2 * TWN<T> + (size_t)nsub * Nxa * h.LD + (size_t)NW * h.xw) * sizeof(Cx<T>) + (size_t)N2 * h.vst * sizeof(T) +
+    return ((size_t)2 * TWN + (size_t)nsub * Nxa * h.LD + (size_t)NW * h.xw) * sizeof(Cx<T>) + (size_t)N2 * h.vst * sizeof(T) +
            N1 * sizeof(short);
 }
 
@@ -208,11 +208,10 @@ template <typename T>
 __device__ __forceinline__ void setup(const KPlan &kp, const Shape &h, const Sm<T> &m, const Cx<T> *__restrict__ twx,
                                       const Cx<T> *__restrict__ twy) {
     for (int i = threadIdx.x; i < kp.N1; i += THREADS) m.iax[i] = -1;
-    // entry r R0 + j: exp(-2 pi i r j / N), 1 <= r < R1 (FP64: r = 1), j < R0
     // (one-stage plans: R0 = 0, no twiddles)
-    const int nx = sizeof(T) == 4 && h.R0x ? kp.N1 : 2 * h.R0x, ny = sizeof(T) == 4 && h.R0y ? kp.N2 : 2 * h.R0y;
-    for (int i = h.R0x + threadIdx.x; i < nx; i += THREADS) m.tx[i] = twx[i / h.R0x * (i % h.R0x)];
-    for (int i = h.R0y + threadIdx.x; i < ny; i += THREADS) m.ty[i] = twy[i / h.R0y * (i % h.R0y)];
+    const int nx = h.R0x ? kp.N1 : 0, ny = h.R0y ? kp.N2 : 0;
+    for (int i = h.R0x + threadIdx.x; i < nx; i += THREADS) m.tx[i] = twx[tw_entry(i, h.R0x)];
+    for (int i = h.R0y + threadIdx.x; i < ny; i += THREADS) m.ty[i] = twy[tw_entry(i, h.R0y)];
 }
 // S := the plane's columns (zeros elsewhere), nbh bands
 template <typename T>

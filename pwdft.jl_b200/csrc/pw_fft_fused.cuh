@@ -272,7 +272,7 @@ template <int N> __host__ __device__ constexpr int fp_xs() {
 static_assert(fp_xs<120>() == 120 && fp_pad<120>() == 0, "the 120-point plan is unpadded");
 
 // twiddle of element r of stage-S butterfly jm (jm < N_S, the stage's span)
-template <int N, int S> __device__ __forceinline__ int tw_at(int r, int jm) {
+template <int N, int S> __host__ __device__ __forceinline__ int tw_at(int r, int jm) {
     if constexpr (FPlan<N>::nst == 2 && S == 1) {
         constexpr int R0 = FPlan<N>::r(0);
         return R0 + (r - 1) * R0 + jm;
@@ -312,7 +312,7 @@ template <int NBF, int G> struct LaneMap {
 
 // w[r] = w1^r for r < R, w[r] = w[r / 2] w[r - r / 2] (about log2(r) + 1
 // roundings): the stage twiddles of one butterfly from a single table read.
-template <typename T, int R> __device__ __forceinline__ void tw_pow(Cx<T> w1, Cx<T> (&w)[R]) {
+template <typename T, int R> __host__ __device__ __forceinline__ void tw_pow(Cx<T> w1, Cx<T> (&w)[R]) {
     w[0] = cmake((T)1, (T)0);
     if constexpr (R > 1) w[1] = w1;
 #pragma unroll
@@ -322,16 +322,18 @@ template <typename T, int R> __device__ __forceinline__ void tw_pow(Cx<T> w1, Cx
 // Twiddles of butterfly jm of stage S (conjugated for the inverse, sign > 0)
 // applied to v[1 .. R).  Only the second stage of a two-stage plan has any;
 // its table entry tw_at(1, jm) is exp(-2 pi i jm / N).
-// With a whole table (FullTw) every power is read instead: in FP32 the powers
-// lose about a bit against entries that were rounded once (density of 8 bands, 32 /
-// 60 points: relative error 2.7e-7 / 1.3e-7 against 1.4e-7 / 0.8e-7; op_H of 8
-// atoms 69.7 against 70.1 us).
+// With a whole table (FullTw) every power is read instead: the powers lose up to
+// a bit against entries that were rounded once.  FP32 density of 8 bands, 32 / 60
+// points: relative error 2.7e-7 / 1.3e-7 against 1.4e-7 / 0.8e-7 (op_H of 8 atoms
+// 69.7 against 70.1 us); FP64 density of 4 bands, 40 / 64 / 72 points: 3.3e-16 /
+// 4.4e-16 / 4.5e-16 against 2.5e-16 / 3.1e-16 / 2.4e-16 (op_H and density of 40
+// bands on 22 boxes at most 3 % longer, 5 % at 72 points; 81 points 3 % shorter).
 template <typename T> struct FullTw {
     const Cx<T> *p;
-    __device__ __forceinline__ operator const Cx<T> *() const { return p; }
+    __host__ __device__ __forceinline__ operator const Cx<T> *() const { return p; }
 };
 template <typename T, int N, int S, int R>
-__device__ __forceinline__ void apply_tw(Cx<T> (&v)[R], FullTw<T> tw, int jm, int sign) {
+__host__ __device__ __forceinline__ void apply_tw(Cx<T> (&v)[R], FullTw<T> tw, int jm, int sign) {
 #pragma unroll
     for (int r = 1; r < R; ++r) {
         Cx<T> w = tw.p[tw_at<N, S>(r, jm)];
@@ -340,7 +342,7 @@ __device__ __forceinline__ void apply_tw(Cx<T> (&v)[R], FullTw<T> tw, int jm, in
     }
 }
 template <typename T, int N, int S, int R>
-__device__ __forceinline__ void apply_tw(Cx<T> (&v)[R], const Cx<T> *tw, int jm, int sign) {
+__host__ __device__ __forceinline__ void apply_tw(Cx<T> (&v)[R], const Cx<T> *tw, int jm, int sign) {
     Cx<T> w1 = tw[tw_at<N, S>(1, jm)];
     if (sign > 0) w1.y = -w1.y;
     Cx<T> w[R];

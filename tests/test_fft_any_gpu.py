@@ -2,8 +2,10 @@
 length with a fused plan taking each direction once, against dense FFTs in
 double precision; one band, an odd block, and each setting of plane_bands.
 
-Bounds: FP64 1e-13, FP32 4e-6 of the largest value (a line of n points rounds
-about log2 n times; 6 lines a value, eps 6e-8)."""
+Bounds, largest difference over the largest value and 2-norm over 2-norm: about
+twice the largest of the 32 boxes (density: FP64 1.4e-15 and 6.6e-16, FP32 4.5e-7
+and 2.4e-7; the dense FP64 FFTs are themselves as far from extended precision
+as the FP64 kernels)."""
 import numpy as np
 import pytest
 
@@ -25,13 +27,13 @@ def test_box(Ns):
     idx = np.nonzero(r2.ravel() < 0.2 ** 2)[0]
     idx = idx[rng.permutation(len(idx))][:max(1, len(idx) - 5)]        # unordered, a few columns ragged
     N = N1 * N2 * N3
-    gk2 = rng.uniform(0, 30, len(idx))
+    gk2 = rng.uniform(0, 1, len(idx))          # small: rounding of the transforms, not of K, is seen
     V = rng.standard_normal(N)
     ctx = pwb200.Context(Ns, 100.0, [idx], [gk2])
     ctx.set_vloc(V)
     t = torch.from_numpy(idx).cuda()
     Vt = torch.from_numpy(V).cuda().view(N3, N2, N1)
-    for dt, tol in ((torch.complex128, 1e-13), (torch.complex64, 4e-6)):
+    for dt, tol, tol2 in ((torch.complex128, 3e-15, 1.3e-15), (torch.complex64, 9e-7, 5e-7)):
         for nb, pb in ((1, 0), (5, 0), (5, 1), (5, 2), (4, 3)):
             g = torch.Generator(device="cuda").manual_seed(nb)
             x = torch.randn((nb, len(idx)), dtype=torch.complex128, device="cuda", generator=g).to(dt)
@@ -44,6 +46,7 @@ def test_box(Ns):
             ref = torch.fft.fftn(u * Vt, dim=(1, 2, 3)).reshape(nb, N)[:, t]
             ref = ref + 0.5 * torch.from_numpy(gk2).cuda() * x.to(torch.complex128)
             assert (y - ref).abs().max() <= tol * ref.abs().max(), (dt, nb, pb)
+            assert torch.linalg.vector_norm(y - ref) <= tol2 * torch.linalg.vector_norm(ref), (dt, nb, pb)
             if pb:
                 continue
             w = rng.uniform(0.1, 2.0, nb)
@@ -51,4 +54,5 @@ def test_box(Ns):
             ctx.calc_rhoe(0, x, w, rho)
             rr = (torch.from_numpy(w).cuda()[:, None] * (u.abs() ** 2).reshape(nb, N)).sum(dim=0) * N * N / 100.0
             assert (rho - rr).abs().max() <= tol * rr.abs().max(), (dt, nb)
+            assert torch.linalg.vector_norm(rho - rr) <= tol2 * torch.linalg.vector_norm(rr), (dt, nb)
     ctx.close()
