@@ -109,14 +109,15 @@ struct pw_ctx {
     // vectors of the density sphere, 3 x Ng, for grad rho and div h)
     int xc = PW_XC_VWN;
     double *d_xcG = nullptr;
-    // batched op_H over k-points: device tables (MkK per k-point, band ->
-    // k-point map), and the CUDA graph of the last call made with PW_GRAPH
     // symmetrize_rhoe!: orbits of the density sphere (nshell x nsym sphere
     // indices and phases e^{i G.ft})
     int *d_sym_isg = nullptr;
     double2 *d_sym_ph = nullptr;
     int sym_nshell = 0, sym_nsym = 0;
-    DevBuf mk_tab;
+    // batched op_H over k-points: device tables (MkK per k-point, band ->
+    // k-point map, band groups) of the direct launches and of the CUDA graph of
+    // the last call made with PW_GRAPH
+    DevBuf mk_tab, mk_gtab;
     uint64_t mk_key = 0;
     cudaGraphExec_t mk_exec = nullptr;
     int mk_nlaunch = 0;
@@ -962,33 +963,42 @@ int apply_multi_T(pw_ctx *c, int nk, const int *iks, int ispin, void *const *psi
     const size_t bk_off = (tab_bytes + 255) / 256 * 256;
     const size_t ctr_off = (bk_off + bk_bytes + 255) / 256 * 256;   // grid-barrier counter of the persistent launch
     const size_t gr_off = ctr_off + 256, gr_bytes = groups.size() * sizeof(int2);
-    if ((s = ensure(c, c->mk_tab, gr_off + gr_bytes))) return s;
+    // the graph reads its tables at every replay: they have a buffer of their own,
+    // and whatever is about to change it forgets the graph first
+    const bool graph = (ops & PW_GRAPH) != 0;
+    DevBuf &tb = graph ? c->mk_gtab : c->mk_tab;
+    if (graph && tb.bytes < gr_off + gr_bytes) c->mk_key = 0;
+    if ((s = ensure(c, tb, gr_off + gr_bytes))) return s;
+    char *const tp = (char *)tb.p;
     const void *V = sizeof(T) == 8 ? (const void *)(c->d_V64 + (size_t)ispin * c->N)
                                    : (const void *)(c->d_V32 + (size_t)ispin * c->N);
     const int flags = ((o & PW_OP_K) ? 2 : 0) | ((ops & PW_ACCUMULATE) ? 4 : 0);
     const FftLaunch L = make_launch<T>(c, kx);
-    const MkK *d_tab = (const MkK *)c->mk_tab.p;
-    const int *d_bk = (const int *)((const char *)c->mk_tab.p + bk_off);
-    unsigned *d_ctr = (unsigned *)((char *)c->mk_tab.p + ctr_off);
-    const int2 *d_gr = (const int2 *)((const char *)c->mk_tab.p + gr_off);
+    const MkK *d_tab = (const MkK *)tp;
+    const int *d_bk = (const int *)(tp + bk_off);
+    unsigned *d_ctr = (unsigned *)(tp + ctr_off);
+    const int2 *d_gr = (const int2 *)(tp + gr_off);
     // graph replay: same blocks, k-points, flags and buffers as the captured call
     uint64_t key = 1469598103934665603ull;
     key = fnv(key, tab.data(), tab_bytes);
     key = fnv(key, &V, sizeof(V));
     key = fnv(key, &c->A.p, sizeof(void *));
-    key = fnv(key, &c->mk_tab.p, sizeof(void *));
+    key = fnv(key, &tb.p, sizeof(void *));
+    const void *const D[3] = {vnl ? c->d_Drow : nullptr, vnl ? c->d_Dcol : nullptr, vnl ? c->d_Dval : nullptr};
+    key = fnv(key, D, sizeof(D));
     key = fnv(key, &flags, sizeof(flags));
     const unsigned pflag = ops & PW_PERSISTENT;
     key = fnv(key, &pflag, sizeof(pflag));
     key = fnv(key, &nbands, sizeof(nbands));
-    if ((ops & PW_GRAPH) && c->mk_exec && key == c->mk_key) {
+    if (graph && c->mk_exec && key == c->mk_key) {
         CK(c, cudaGraphLaunch(c->mk_exec, c->stream));
         c->launches += c->mk_nlaunch;
         return PW_OK;
     }
-    CK(c, cudaMemcpyAsync(c->mk_tab.p, tab.data(), tab_bytes, cudaMemcpyHostToDevice, c->stream));
-    CK(c, cudaMemcpyAsync((char *)c->mk_tab.p + bk_off, band_k.data(), bk_bytes, cudaMemcpyHostToDevice, c->stream));
-    CK(c, cudaMemcpyAsync((char *)c->mk_tab.p + gr_off, groups.data(), gr_bytes, cudaMemcpyHostToDevice, c->stream));
+    if (graph) c->mk_key = 0;
+    CK(c, cudaMemcpyAsync(tp, tab.data(), tab_bytes, cudaMemcpyHostToDevice, c->stream));
+    CK(c, cudaMemcpyAsync(tp + bk_off, band_k.data(), bk_bytes, cudaMemcpyHostToDevice, c->stream));
+    CK(c, cudaMemcpyAsync(tp + gr_off, groups.data(), gr_bytes, cudaMemcpyHostToDevice, c->stream));
     // one persistent cooperative launch for every stage (the per-stage
     // launches when it does not fit or a stream capture refuses it)
     bool persistent = (ops & PW_PERSISTENT) != 0;
@@ -1011,14 +1021,13 @@ int apply_multi_T(pw_ctx *c, int nk, const int *iks, int ispin, void *const *psi
     };
     CK(c, run(c->stream));
     c->launches += nlaunch;
-    if (ops & PW_GRAPH) {
+    if (graph) {
         // capture the same launches for replay (the tables stay resident)
         CK(c, cudaStreamSynchronize(c->stream));
         if (!c->cap_stream) CK(c, cudaStreamCreateWithFlags(&c->cap_stream, cudaStreamNonBlocking));
         if (c->mk_exec) {
             CK(c, cudaGraphExecDestroy(c->mk_exec));
             c->mk_exec = nullptr;
-            c->mk_key = 0;
         }
         cudaGraph_t g = nullptr;
         CK(c, cudaStreamBeginCapture(c->cap_stream, cudaStreamCaptureModeRelaxed));

@@ -117,6 +117,44 @@ def test_apply_multi_accumulate_subset_and_graph(al4):
     ctx.check_device()
 
 
+@pytest.mark.parametrize("persistent", [False, True])
+def test_graph_replay_between_other_calls(al4, persistent):
+    """A captured call is replayed after direct calls on other blocks, after
+    another graph, and after D has changed: each time its own result."""
+    import torch
+    import pwb200
+    Ho, ctx, psis = al4
+
+    def check(iks, X, HX):
+        for j, ik in enumerate(iks):
+            one = torch.empty_like(X[j])
+            ctx.apply(ik, 0, X[j], one)
+            assert _rel(HX[j].cpu().numpy(), one.cpu().numpy()) < 1e-13, j
+    A, B = [3, 0, 17, 35], [5, 1, 2]
+    XA, XB = _dev([psis[i] for i in A], torch.complex128), _dev([psis[i][:, :7] for i in B], torch.complex128)
+    HA, HB = [torch.zeros_like(x) for x in XA], [torch.zeros_like(x) for x in XB]
+    ctx.apply_multi(A, 0, XA, HA, graph=True, persistent=persistent)
+    for other in (False, True):
+        for h in HA + HB:
+            h.zero_()
+        ctx.apply_multi(B, 0, XB, HB, graph=other)
+        HBc = [h.clone() for h in HB]
+        ctx.apply_multi(A, 0, XA, HA, graph=True, persistent=persistent)
+        check(A, XA, HA)
+        check(B, XB, HB)
+        assert all(torch.equal(h, k) for h, k in zip(HB, HBc))
+    try:
+        for f in (1.5, 0.5, 2.0):
+            ctx.set_nonlocal_coef([(i, j, f * h) for i, j, h in Ho.nl_triplets])
+            spare = [torch.zeros(n, dtype=torch.uint8, device="cuda") for n in (64, 256, 1024, 4096)]
+            ctx.apply_multi(A, 0, XA, HA, graph=True, persistent=persistent)
+            check(A, XA, HA)
+            del spare
+    finally:
+        ctx.set_nonlocal_coef(Ho.nl_triplets)
+    ctx.check_device()
+
+
 @pytest.mark.parametrize("prec", ["c128", "c64"])
 def test_apply_multi_persistent_matches_oracle(al4, prec):
     """PW_PERSISTENT: every stage in one cooperative launch (bounded grid
