@@ -493,7 +493,7 @@ int apply_T(pw_ctx *c, int ik, int ispin, const void *psi, void *Hpsi, int64_t l
             if ((s = ensure(c, c->um_ws, umma_ws_bytes(kd.beta_nn.rows, nb, kd.beta_nn.Kp, c->gemm_splits)))) return s;
             CK(c, umma_gemm<float2>(kd.beta_nn, P2op, kd.Ngw, nb, Hpsi, ld, 1, (float *)c->um_ws.p, c->d_err, st, 0, 0,
                                     c->gemm_splits));
-            c->launches += 2;
+            c->launches += umma_splits(kd.beta_nn.rows, nb, kd.beta_nn.Kp, c->gemm_splits) > 1 ? 2 : 1;
         } else {
             CK(c, gemm_nn<T>(kd.Ngw, nb, c->nbeta, beta, kd.Ngw, (const double2 *)c->P2.p, c->nbeta, Hpsi, ld, 1, st));
             c->launches += 1;
@@ -1159,7 +1159,7 @@ extern "C" int pw_gram(pw_ctx *c, int dtype, int64_t K, int m, int n, const void
         CK(c, gemm_tn<double>(K, m, n, A, lda, B, ldb, (double2 *)C, ldc, accumulate, c->gemm_ws.p, c->stream, same));
     else
         CK(c, gemm_tn<float>(K, m, n, A, lda, B, ldb, (double2 *)C, ldc, accumulate, c->gemm_ws.p, c->stream));
-    c->launches += 2;
+    c->launches += gemm_tn_launches(dtype == PW_C128 ? 8 : 4, K, m, n, same);
     return PW_OK;
 }
 
@@ -1180,7 +1180,7 @@ int pwk_gram_upper(pw_ctx *c, int dtype, int64_t K, int m, const void *A, int64_
         CK(c, gemm_tn<double>(K, m, m, A, lda, B, ldb, (double2 *)C, ldc, 0, c->gemm_ws.p, c->stream, 1));
     else
         CK(c, gemm_tn<float>(K, m, m, A, lda, B, ldb, (double2 *)C, ldc, 0, c->gemm_ws.p, c->stream, 1));
-    c->launches += 2;
+    c->launches += gemm_tn_launches(dtype == PW_C128 ? 8 : 4, K, m, m, 1);
     return PW_OK;
 }
 
@@ -1367,7 +1367,7 @@ int pwk_beta_dot(pw_ctx *c, int ik, int dtype, const void *psi, int64_t ld, int 
             CK(c, (gemm_tn<double>(kd.Ngw, c->nbeta, nb, beta, kd.Ngw, psi, ld, out, c->nbeta, 0, c->gemm_ws.p, st)));
         else
             CK(c, (gemm_tn<float>(kd.Ngw, c->nbeta, nb, beta, kd.Ngw, psi, ld, out, c->nbeta, 0, c->gemm_ws.p, st)));
-        c->launches += 2;
+        c->launches += gemm_tn_launches(dtype == PW_C128 ? 8 : 4, kd.Ngw, c->nbeta, nb);
     }
     return PW_OK;
 }

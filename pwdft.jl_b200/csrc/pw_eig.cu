@@ -1516,7 +1516,7 @@ __global__ void k_check_finite(const double *__restrict__ d, const double *__res
 }
 
 cudaError_t hegv_lowest(double2 *T, double2 *G, int n, int k, double *lam_out, double2 *S, void *work, size_t work_bytes,
-                        void *gemm_ws, int *d_status, cudaStream_t st) {
+                        int *launches, int *d_status, cudaStream_t st) {
     if (n <= 0 || k <= 0 || k > n || work_bytes < eig_work_bytes(n, k)) return cudaErrorInvalidValue;
     unsigned char *p = (unsigned char *)work;
     auto take = [&](size_t bytes) {
@@ -1545,9 +1545,11 @@ cudaError_t hegv_lowest(double2 *T, double2 *G, int n, int k, double *lam_out, d
     if ((e_ = cudaMemsetAsync(gb, 0, sizeof(GridBar), st)) != cudaSuccess) return e_;
     if ((e_ = cudaMemsetAsync(err, 0, sizeof(int) * 4, st)) != cudaSuccess) return e_;
     const int nb = blocks_for(nn);
+    int nl = 1;   // kernels launched
     k_herm_upper<<<nb, 256, 0, st>>>(T, n);
     double2 *Cm = T;
     if (G) {
+        nl += 6;
         k_herm_upper<<<nb, 256, 0, st>>>(G, n);
         if ((e_ = chol_and_inverse(G, n, Linv, ctr, err, st)) != cudaSuccess) return e_;
         // C = Linv T Linv^H: Linv lower triangular, only C's upper triangle
@@ -1595,6 +1597,7 @@ cudaError_t hegv_lowest(double2 *T, double2 *G, int n, int k, double *lam_out, d
         if ((e_ = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess) return e_;
         void *args[] = {(void *)&Cm, (void *)&n, (void *)&jend, (void *)&d, (void *)&e, (void *)&tau, (void *)&ybuf, (void *)&err};
         if ((e_ = cudaLaunchCooperativeKernel(fn, nblk, 32 * W, args, smem, st)) != cudaSuccess) return e_;
+        nl += 1;
     } else if (jend > 0) {
         const size_t smem = (size_t)(3 * n + 32) * sizeof(double2);
         int nblk = 0;
@@ -1606,11 +1609,13 @@ cudaError_t hegv_lowest(double2 *T, double2 *G, int n, int k, double *lam_out, d
         void *args[] = {(void *)&Cm, (void *)&n, (void *)&jend, (void *)&d, (void *)&e, (void *)&tau, (void *)&xg, (void *)&ctr, (void *)&err};
         if ((e_ = cudaLaunchCooperativeKernel((const void *)k_tridiag, nblk, COOP_THREADS, args, smem, st)) != cudaSuccess)
             return e_;
+        nl += 1;
     }
     if (ncl >= 1) {
         if ((e_ = cudaLaunchKernelEx(&cf, fc, Cm + (size_t)jend * (n + 1), n - jend, n, d + jend, e + jend, tau + jend, err)) !=
             cudaSuccess)
             return e_;
+        nl += 1;
     }
     // a non-finite T or G reaches the tridiagonal matrix: report it (the
     // Sturm counts would otherwise turn it into finite, meaningless values)
@@ -1622,6 +1627,7 @@ cudaError_t hegv_lowest(double2 *T, double2 *G, int n, int k, double *lam_out, d
             (e_ = cudaFuncSetAttribute((const void *)k_bisect, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
             return e_;
         k_bisect<<<nwy + (k + per - 1) / per, BIS_THREADS, smem, st>>>(d, e, n, k, lam, nrm, Cm, tau, nwy, Tw);
+        nl += 2;
     }
     if ((e_ = cudaMemcpyAsync(lam_out, lam, k * sizeof(double), cudaMemcpyDeviceToDevice, st)) != cudaSuccess) return e_;
     if (S) {
@@ -1649,7 +1655,9 @@ cudaError_t hegv_lowest(double2 *T, double2 *G, int n, int k, double *lam_out, d
             // S = Linv^H Z  (Linv^H sits in G)
             if ((e_ = gemm_nn<double>(n, k, n, G, n, Z, n, S, n, 0, st, 3)) != cudaSuccess) return e_;
         }
+        nl += G ? 3 : 2;
     }
+    *launches = nl;
     if ((e_ = cudaGetLastError()) != cudaSuccess) return e_;
     // status: [0] barrier expiry, [1] Cholesky breakdown column (1-based),
     // [2] non-finite tridiagonal matrix

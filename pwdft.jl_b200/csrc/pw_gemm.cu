@@ -437,9 +437,13 @@ int splitk_count(int64_t K, int m, int n) {
 
 }  // namespace
 
-size_t gemm_tn_ws_bytes(int dtype, int64_t K, int m, int n, int upper) {
-    const size_t S = dtype == 8 ? zplan(K, m, n, true, upper).S : splitk_count(K, m, n);
-    return S * m * n * sizeof(double2);
+int gemm_tn_launches(int real_bytes, int64_t K, int m, int n, int upper) {
+    return real_bytes == 8 && upper != 2 && zplan(K, m, n, true, upper).S == 1 ? 1 : 2;
+}
+
+size_t gemm_tn_ws_bytes(int real_bytes, int64_t K, int m, int n, int upper) {
+    const size_t S = real_bytes == 8 ? zplan(K, m, n, true, upper).S : splitk_count(K, m, n);
+    return gemm_tn_launches(real_bytes, K, m, n, upper) == 1 ? 0 : S * m * n * sizeof(double2);
 }
 
 template <typename T>

@@ -92,6 +92,8 @@ cudaError_t launch_polarize(int Ngw, int nb, const void *psi, const void *lam, i
 // ws: split-K workspace of at least gemm_tn_ws_bytes() bytes (real_bytes =
 // sizeof(T), same K, m, n, upper).
 size_t gemm_tn_ws_bytes(int real_bytes, int64_t K, int m, int n, int upper = 0);
+// kernels that it launches (1: C is written directly, no workspace)
+int gemm_tn_launches(int real_bytes, int64_t K, int m, int n, int upper = 0);
 template <typename T>
 // upper: 1 = only C[i][j] with i <= j is formed and written (Hermitian
 // products whose consumer reads the upper triangle); tiles strictly below

@@ -92,14 +92,15 @@ struct Run {
 
 // lowest k eigenpairs of (T, G) (G may be null) of order n; T, G overwritten
 int eig(Run &r, double2 *T, double2 *G, int n, int k, double *lam_dev, double2 *S) {
-    CKR(r.c, pwk::hegv_lowest(T, G, n, k, lam_dev, S, r.eigw, r.eigw_bytes, nullptr, r.eigstat, r.st));
+    int nl = 0;
+    CKR(r.c, pwk::hegv_lowest(T, G, n, k, lam_dev, S, r.eigw, r.eigw_bytes, &nl, r.eigstat, r.st));
+    pwk_count_launches(r.c, nl);
     int h[3] = {0, 0, 0};
     CKR(r.c, cudaMemcpyAsync(h, r.eigstat, sizeof(h), cudaMemcpyDeviceToHost, r.st));
     CKR(r.c, cudaStreamSynchronize(r.st));
     if (h[0]) return pwk_fail(r.c, PW_ERR_TIMEOUT, "a bounded grid barrier of the eigensolver expired");
     if (h[1]) return pwk_fail(r.c, PW_ERR_NOT_POSDEF, "overlap matrix not positive definite (Cholesky)");
     if (h[2]) return pwk_fail(r.c, PW_ERR_NAN, "non-finite value in the eigenproblem");
-    pwk_count_launches(r.c, 10);
     return PW_OK;
 }
 
@@ -179,7 +180,7 @@ int chol_rinv(Run &r, double2 *C, int n, double2 *Rinv) {
     CKR(r.c, cudaStreamSynchronize(r.st));
     if (h[0]) return pwk_fail(r.c, PW_ERR_TIMEOUT, "a bounded grid barrier of the Cholesky expired");
     if (h[1]) return pwk_fail(r.c, PW_ERR_NOT_POSDEF, "cholesky(Hermitian(C)) failed: C not positive definite");
-    pwk_count_launches(r.c, 4);
+    pwk_count_launches(r.c, 3);
     return PW_OK;
 }
 }  // namespace
