@@ -1463,17 +1463,23 @@ int blocks_for(size_t total) {
     return b < 1 ? 1 : (int)b;
 }
 
-cudaError_t coop_blocks(const void *fn, size_t smem, int *nblk) {
+// CTAs of fn that are resident at once on the current device; one_per_sm: at
+// most that many
+cudaError_t resident_ctas(const void *fn, int threads, size_t smem, int *n, bool one_per_sm = false) {
     int dev = 0, sms = 0, per = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
     if (smem > 48 * 1024 && (e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess)
         return e;
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, COOP_THREADS, smem)) != cudaSuccess) return e;
-    if (per < 1) return cudaErrorCooperativeLaunchTooLarge;
-    *nblk = sms * std::min(per, 1);  // one CTA per SM keeps the barrier cheap
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, fn, threads, smem)) != cudaSuccess) return e;
+    *n = sms * (one_per_sm ? std::min(per, 1) : per);
     return cudaSuccess;
+}
+
+cudaError_t coop_blocks(const void *fn, size_t smem, int *nblk) {
+    const cudaError_t e = resident_ctas(fn, COOP_THREADS, smem, nblk, true);   // one CTA per SM keeps the barrier cheap
+    return e != cudaSuccess ? e : *nblk < 1 ? cudaErrorCooperativeLaunchTooLarge : cudaSuccess;
 }
 
 }  // namespace eig
@@ -1564,8 +1570,8 @@ cudaError_t hegv_lowest(double2 *T, double2 *G, int n, int k, double *lam_out, d
     // above that.  At 2.3 against 4.0 us a column the whole reduced problem goes
     // from 2.94 to 2.65 ms at n = 480, from 1.14 to 0.75 at 160 (k = n / 3); with
     // 384 columns in a cluster of 384 threads a CTA it spills, 2.73 at 480.
-    constexpr int NC = 256;
     const auto fc = k_tridiag_c<8, 8, 2>;
+    static_assert(32 * 8 == TRI_NC, "the cluster's columns");
     constexpr size_t smem_c = tridiag_c_smem<8, 8, 2>();
     cudaLaunchConfig_t cf = {};
     cudaLaunchAttribute at;
@@ -1586,17 +1592,19 @@ cudaError_t hegv_lowest(double2 *T, double2 *G, int n, int k, double *lam_out, d
         cudaGetLastError();
         ncl = 0;
     }
-    const int jend = ncl < 1 ? n - 1 : std::max(0, n - NC);
-    if ((jend > 0 || ncl < 1) && n <= 1024) {
-        // few CTAs keep the exchange short, few columns a CTA the update (n =
-        // 480, us a column: 120 CTAs of 4 columns 4.1, 60 of 8 4.5, 30 of 16 5.4)
-        const void *fn = n <= 512 ? (const void *)k_tridiag_r<16, 4, 1> : (const void *)k_tridiag_r<32, 8, 1>;
-        const int W = n > 512 ? 8 : 4, nblk = std::max(1, (n - 1 + W - 1) / W);
-        if ((e_ = cudaMemsetAsync(ybuf, 0xff, (size_t)jend * 2 * nblk * W * sizeof(double2), st)) != cudaSuccess) return e_;
-        const size_t smem = 3 * (size_t)(n <= 512 ? 512 : 1024) * sizeof(double2);
-        if ((e_ = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess) return e_;
+    // few CTAs keep the exchange short, few columns a CTA the update (n =
+    // 480, us a column: 120 CTAs of 4 columns 4.1, 60 of 8 4.5, 30 of 16 5.4)
+    const void *fn = n <= 512 ? (const void *)k_tridiag_r<16, 4, 1> : (const void *)k_tridiag_r<32, 8, 1>;
+    const size_t smem_r = 3 * (size_t)(n <= 512 ? 512 : 1024) * sizeof(double2);
+    const int W = tri_r_warps(n), ctas_r = tri_r_ctas(n);
+    int res_r = 0;
+    if (n <= 1024 && (n > TRI_NC || ncl < 1) && (e_ = resident_ctas(fn, 32 * W, smem_r, &res_r)) != cudaSuccess) return e_;
+    const TriRoute route = tri_route(n, res_r, ncl);
+    const int jend = route.jend;
+    if ((jend > 0 || !route.cluster) && route.registers) {
+        if ((e_ = cudaMemsetAsync(ybuf, 0xff, (size_t)jend * 2 * ctas_r * W * sizeof(double2), st)) != cudaSuccess) return e_;
         void *args[] = {(void *)&Cm, (void *)&n, (void *)&jend, (void *)&d, (void *)&e, (void *)&tau, (void *)&ybuf, (void *)&err};
-        if ((e_ = cudaLaunchCooperativeKernel(fn, nblk, 32 * W, args, smem, st)) != cudaSuccess) return e_;
+        if ((e_ = cudaLaunchCooperativeKernel(fn, ctas_r, 32 * W, args, smem_r, st)) != cudaSuccess) return e_;
         nl += 1;
     } else if (jend > 0) {
         const size_t smem = (size_t)(3 * n + 32) * sizeof(double2);
@@ -1611,7 +1619,7 @@ cudaError_t hegv_lowest(double2 *T, double2 *G, int n, int k, double *lam_out, d
             return e_;
         nl += 1;
     }
-    if (ncl >= 1) {
+    if (route.cluster) {
         if ((e_ = cudaLaunchKernelEx(&cf, fc, Cm + (size_t)jend * (n + 1), n - jend, n, d + jend, e + jend, tau + jend, err)) !=
             cudaSuccess)
             return e_;

@@ -4,7 +4,8 @@ the ranks' step counts compiled into a host program that runs the protocol
 the others can go on without it, and in random order.  A store into a buffer
 whose earlier step has not been read yet, a step that never completes, or a
 writer that has already left fails.  The same program with every rank receiving
-to the end (the form that needs luck in timing) has to be caught."""
+to the end (the form that needs luck in timing) has to be caught.  And the choice
+of the kernel for the columns before the cluster's, on devices with few SMs."""
 import os
 import shutil
 import subprocess
@@ -92,6 +93,23 @@ int main() {
             return 1;
         }
     }
+    // the register kernel of the grid is taken only where all its CTAs are resident:
+    // a whole B200 (148 SMs; 4 and 1 CTAs an SM up to and past n = 512, at the
+    // least), an eighth of one, and no device at all
+    for (int n = 1; n <= 2000; ++n)
+        for (int sms : {148, 18, 0})
+            for (int per : {4, 1})
+                for (int clusters : {9, 0}) {
+                    const TriRoute t = tri_route(n, sms * per, clusters);
+                    ok &= t.cluster == (clusters > 0) && t.jend == (clusters ? n > 256 ? n - 256 : 0 : n - 1);
+                    ok &= !t.registers || (n <= 1024 && tri_r_ctas(n) <= sms * per);
+                    ok &= tri_r_ctas(n) * tri_r_warps(n) >= n - 1;
+                    if (sms == 148) ok &= t.registers == (n <= 1024);
+                }
+    if (!ok) {
+        std::printf("route\n");
+        return 1;
+    }
     to_end = true;
     for (int n : {12, 17, 160, 256}) {
         bool caught = false;
@@ -108,7 +126,7 @@ int main() {
 
 
 @pytest.mark.skipif(shutil.which("g++") is None, reason="g++ not available")
-def test_late_ranks_read_every_step(tmp_path):
+def test_late_ranks_and_the_route(tmp_path):
     src = tmp_path / "tri.cpp"
     src.write_text(PROG)
     exe = tmp_path / "tri"
