@@ -274,11 +274,7 @@ __global__ void k_zero(Cx<T> *p, int Ngw, int nb, int64_t ld) {
 template <typename T, int N, bool JF, bool PAD = false>
 __device__ __forceinline__ void line_fft(Cx<T> *buf, int nl, int es, int ls, const Cx<T> *tw, int sign) {
     static_assert(!PAD || sizeof(T) == 4, "padded lines are FP32 only");
-    // 27, 75 and 120 points: powers of one entry (as in their plane kernels)
-    constexpr bool POW = N == 27 || N == 75 || N == 120;
-    if constexpr (sizeof(T) == 4 && POW)
-        pwf::lines<T, N, JF, PAD>(buf, nl, es, ls, tw, sign);
-    else if constexpr (sizeof(T) == 4)
+    if constexpr (sizeof(T) == 4)
         pwf::lines<T, N, JF, PAD>(buf, nl, es, ls, pwf::FullTw<T>{tw}, sign);
     else
         pwt::lines<T, N, MaxV<T>::v, JF>(buf, nl, es, ls, tw, sign);
