@@ -1265,9 +1265,9 @@ static cudaError_t set_smem(const void *fn, size_t bytes) {
     X(20) X(24) X(25) X(27) X(30) X(32) X(36) X(40) X(45) X(48) X(50) X(54) X(60) X(64) X(72) X(75) X(80) X(81) X(90) \
     X(96) X(100) X(108) X(120) X(125) X(128)
 
-// Columns per CTA of the z passes: the tuned or default width, halved (down to 8)
-// while the CTAs do not fill the GPU once (8 bands of a 27-point grid: 16 CTAs
-// of 64 columns, the passes 9 and 12 us long).
+// Columns per CTA of the z passes: the tuned or default width, halved while it is
+// above 8 (so 5 to 8 at the least) and the CTAs do not fill the GPU once (8 bands
+// of a 27-point grid: 16 CTAs of 64 columns, the passes 9 and 12 us long).
 static int z_columns(const FftLaunch &L, int nb) {
     int Cg = L.Cg;
     if (!L.Cg_set)

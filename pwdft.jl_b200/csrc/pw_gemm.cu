@@ -218,9 +218,11 @@ k_zgemm(int64_t K, int64_t m, int n, const double2 *__restrict__ A, int64_t lda,
 // most CTAs decides; a split adds the partial sums' trip through L2
 // (about 2400 bytes a clock) and the reduction's launch (4000 clocks).
 // (480 x 480 over K = 23,871: 48 x 80 tiles, 0 % padding, against 14 % with
-// 64 x 64.)  Splitting stops at four CTAs an SM, which also bounds the workspace
-// (592 tiles: 49 MB).  Few values are split too (betaNL' psi of 8 bands over
-// about 730 plane waves: 35.8 us on one CTA, 5.0 in 23 parts).
+// 64 x 64.)  Splitting stops at four CTAs an SM, which also bounds the workspace: 592
+// tiles, 49 MB, and up to about twice that for a triangular product, where only the
+// formed tiles count but every split has room for all.  Few values are split too
+// (betaNL' psi of 8 bands over about 730 plane waves: 35.8 us on one CTA, 5.0 in 23
+// parts).
 struct ZPlan {
     int wm, wn, S;
     int64_t kchunk;
