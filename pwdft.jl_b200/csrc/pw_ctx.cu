@@ -14,6 +14,7 @@
 
 #include "../../include/pwb200.h"
 #include "pw_launch.h"
+#include "pw_rho.h"
 #include "pw_umma.h"
 
 using namespace pwk;
@@ -43,6 +44,7 @@ struct KData {
     UmmaOperand beta_tn;  // split-BF16 betaNL for betaNL' psi   (tensor-core path)
     UmmaOperand beta_nn;  // split-BF16 betaNL^H for betaNL * P  (tensor-core path)
     double *d_gk = nullptr;  // (G+k) vectors, 3 x Ngw (forces)
+    int rho_per_sm[2] = {0, 0};  // CTAs of the density pass that an SM holds, FP32 and FP64 (0: not asked yet)
 };
 
 constexpr int kMaxV64 = 8;  // complex values per thread per round in the FP64 FFT stages
@@ -502,26 +504,13 @@ int apply_T(pw_ctx *c, int ik, int ispin, const void *psi, void *Hpsi, int64_t l
     return PW_OK;
 }
 
-// Band groups of the density pass: each of the N3 G CTAs takes one z-plane of
-// ceil(cnt / G) bands, two (FP32) or one (FP64) to an SM, so the time goes with
-// waves x bands per group, plus about 0.3 of a band for a CTA's set-up and
-// plane and 0.1 a group for the reduction.  (75-point grid, 41 FP64 bands: 7
-// groups run 4 x 6 bands deep, 4 groups, "enough CTAs to fill the GPU twice",
-// 3 x 11, their third wave nearly empty: 128 bands 882 -> 812 us.)
+// CTAs of the density pass that an SM holds at k-point ik (asked once)
 template <typename T>
-int rho_groups(const pw_ctx *c, int cnt) {
-    const int slots = sizeof(T) == 4 ? 2 * 148 : 148;
-    int best = 1;
-    double tbest = 1e300;
-    for (int G = 1; G <= std::min(cnt, 16); ++G) {
-        const int waves = (c->N3 * G + slots - 1) / slots, Bg = (cnt + G - 1) / G;
-        const double t = waves * (Bg + 0.3) + 0.1 * G;
-        if (t < tbest) {
-            tbest = t;
-            best = G;
-        }
-    }
-    return best;
+int rho_per_sm(pw_ctx *c, int ik, const FftLaunch &L, int *per_sm) {
+    int &p = c->k[ik].rho_per_sm[sizeof(T) == 8];
+    if (p <= 0) CK(c, launch_plane_rho<T>(L, nullptr, 0, 0, 0, nullptr, nullptr, c->stream, &p));
+    *per_sm = p;
+    return PW_OK;
 }
 
 template <typename T>
@@ -533,8 +522,9 @@ int rhoe_T(pw_ctx *c, int ik, const void *psi, int64_t ld, int nb, const double 
     const int nbc = band_chunk(c, ik, es, nb);
     int s;
     if ((s = ensure(c, c->A, (size_t)nbc * c->N3 * kd.Ncol * es))) return s;
-    int G = 1;
-    for (int b0 = 0; b0 < nb; b0 += nbc) G = std::max(G, rho_groups<T>(c, std::min(nbc, nb - b0)));
+    int G = 1, per_sm = 0;
+    if ((s = rho_per_sm<T>(c, ik, L, &per_sm))) return s;
+    for (int b0 = 0; b0 < nb; b0 += nbc) G = std::max(G, rho_groups(c->N3, std::min(nbc, nb - b0), per_sm));
     if ((s = ensure(c, c->rho_part, (size_t)G * c->N * sizeof(T)))) return s;
     if ((s = ensure(c, c->w, (size_t)nb * sizeof(double)))) return s;
     std::vector<double> wv(w_host, w_host + nb);
@@ -542,7 +532,7 @@ int rhoe_T(pw_ctx *c, int ik, const void *psi, int64_t ld, int nb, const double 
     CK(c, cudaMemcpyAsync(c->w.p, wv.data(), nb * sizeof(double), cudaMemcpyHostToDevice, st));
     for (int b0 = 0; b0 < nb; b0 += nbc) {
         const int cnt = std::min(nbc, nb - b0);
-        const int Gc = rho_groups<T>(c, cnt);
+        const int Gc = rho_groups(c->N3, cnt, per_sm);
         const int Bg = (cnt + Gc - 1) / Gc;
         const int Gu = (cnt + Bg - 1) / Bg;
         const char *pin = (const char *)psi + (size_t)b0 * ld * es;

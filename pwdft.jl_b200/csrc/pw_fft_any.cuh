@@ -380,7 +380,8 @@ cudaError_t plane_vloc(const FftLaunch &L, const void *Vr, void *A, int nb, cuda
 }
 
 template <typename T>
-cudaError_t plane_rho(const FftLaunch &L, const void *A, int nb, int G, int Bg, const double *w, void *rho_part, cudaStream_t st) {
+cudaError_t plane_rho(const FftLaunch &L, const void *A, int nb, int G, int Bg, const double *w, void *rho_part, cudaStream_t st,
+                      int *per_sm) {
     const KPlan &kp = L.kp;
     Shape h;
     Line lx, ly;
@@ -391,6 +392,7 @@ cudaError_t plane_rho(const FftLaunch &L, const void *A, int nb, int G, int Bg, 
     const void *fn = h.vst ? (const void *)ka_plane_rho<T, true> : (const void *)ka_plane_rho<T, false>;
     cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (e != cudaSuccess) return e;
+    if (per_sm) return cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, fn, THREADS, smem);
     const dim3 grid(kp.N3, G);
     const Cx<T> *twx = (const Cx<T> *)L.twx, *twy = (const Cx<T> *)L.twy;
     if (h.vst)

@@ -1255,6 +1255,10 @@ static cudaError_t set_smem(const void *fn, size_t bytes) {
     return cudaSuccess;
 }
 
+template <class K> static cudaError_t ctas_per_sm(K *fn, size_t smem, int *n) {
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(n, fn, FFT_THREADS, smem);
+}
+
 // Line lengths of the cube-grid plane and batched kernels (the grids of the
 // Si2/Al4 (27), Si64 (75) and Si216 (120) systems).
 #define FIXED_SIZES(X) X(27) X(75) X(120)
@@ -1381,7 +1385,7 @@ static cudaError_t launch_plane_vloc64_x(const FftLaunch &L, const void *Vr, voi
 }
 template <int NN>
 static cudaError_t launch_plane_rho_x(const FftLaunch &L, const void *A, int nb, int G, int Bg, const double *w,
-                                      void *rho_part, cudaStream_t st) {
+                                      void *rho_part, cudaStream_t st, int *per_sm) {
     const KPlan &kp = L.kp;
     constexpr bool RS = NN * NN * 4 <= 32 * 1024;
     PlaneXSmem ps{NN, NN, kp.Nxa, FFT_THREADS / 32, pwf::fp_group<NN>(), RS ? NN * NN : 0};
@@ -1389,6 +1393,7 @@ static cudaError_t launch_plane_rho_x(const FftLaunch &L, const void *A, int nb,
     const size_t smem = ps.elems() * sizeof(float2);
     cudaError_t e = set_smem<float>((const void *)kx_plane_rho<NN, NN, RS>, smem);
     if (e != cudaSuccess) return e;
+    if (per_sm) return ctas_per_sm(kx_plane_rho<NN, NN, RS>, smem, per_sm);
     dim3 grid(kp.N3, G);
     kx_plane_rho<NN, NN, RS><<<grid, FFT_THREADS, smem, st>>>(kp, (const float2 *)L.twx, (const float2 *)L.twy,
                                                              (const float2 *)A, nb, Bg, w, (float *)rho_part);
@@ -1399,7 +1404,7 @@ static cudaError_t launch_plane_rho_x(const FftLaunch &L, const void *A, int nb,
 // shared memory when it takes at most 48 KB, else the global partial sums
 template <int NN>
 static cudaError_t launch_plane_rho64_x(const FftLaunch &L, const void *A, int nb, int G, int Bg, const double *w,
-                                        void *rho_part, cudaStream_t st) {
+                                        void *rho_part, cudaStream_t st, int *per_sm) {
     const KPlan &kp = L.kp;
     constexpr bool RS = NN * NN * 8 <= 48 * 1024;
     PlaneXSmem ps{NN, NN, kp.Nxa, FFT_THREADS / 32, pwf::fp_group<NN>(), RS ? NN * NN : 0};
@@ -1408,6 +1413,7 @@ static cudaError_t launch_plane_rho64_x(const FftLaunch &L, const void *A, int n
     if (smem > 227 * 1024) return cudaErrorNotSupported;   // the caller takes the plane-wide kernel
     cudaError_t e = set_smem<double>((const void *)kx_plane_rho64<NN, NN, RS>, smem);
     if (e != cudaSuccess) return e;
+    if (per_sm) return ctas_per_sm(kx_plane_rho64<NN, NN, RS>, smem, per_sm);
     dim3 grid(kp.N3, G);
     kx_plane_rho64<NN, NN, RS><<<grid, FFT_THREADS, smem, st>>>(kp, (const double2 *)L.twx, (const double2 *)L.twy,
                                                                (const double2 *)A, nb, Bg, w, (double *)rho_part);
@@ -1593,22 +1599,22 @@ cudaError_t launch_plane_vloc(const FftLaunch &L, const void *Vr, void *A, int n
 
 template <typename T>
 cudaError_t launch_plane_rho(const FftLaunch &L, const void *A, int nb, int G, int Bg, const double *w, void *rho_part,
-                             cudaStream_t st) {
+                             cudaStream_t st, int *per_sm) {
     const KPlan &kp = L.kp;
     if constexpr (sizeof(T) == 4) {
         if (kp.N1 == kp.N2) {
 #define PW_CASE(NN) \
-    if (kp.N1 == NN) return launch_plane_rho_x<NN>(L, A, nb, G, Bg, w, rho_part, st);
+    if (kp.N1 == NN) return launch_plane_rho_x<NN>(L, A, nb, G, Bg, w, rho_part, st, per_sm);
             FIXED_SIZES(PW_CASE)
 #undef PW_CASE
         }
     } else if (kp.N1 == kp.N2 && (kp.N1 == 75 || kp.N1 == 120)) {
-        const cudaError_t e = kp.N1 == 75 ? launch_plane_rho64_x<75>(L, A, nb, G, Bg, w, rho_part, st)
-                                          : launch_plane_rho64_x<120>(L, A, nb, G, Bg, w, rho_part, st);
+        const cudaError_t e = kp.N1 == 75 ? launch_plane_rho64_x<75>(L, A, nb, G, Bg, w, rho_part, st, per_sm)
+                                          : launch_plane_rho64_x<120>(L, A, nb, G, Bg, w, rho_part, st, per_sm);
         if (e != cudaErrorNotSupported) return e;
     }
     if (!(kp.N1 == 27 && kp.N2 == 27)) {
-        const cudaError_t e = launch_any_plane_rho<T>(L, A, nb, G, Bg, w, rho_part, st);
+        const cudaError_t e = launch_any_plane_rho<T>(L, A, nb, G, Bg, w, rho_part, st, per_sm);
         if (e != cudaErrorNotSupported) return e;
     }
     PlaneSmem ps{kp.N1, kp.N2, kp.Nxa, L.Jc};
@@ -1619,6 +1625,7 @@ cudaError_t launch_plane_rho(const FftLaunch &L, const void *A, int nb, int G, i
     if (kp.N1 == NN && kp.N2 == NN) {                                                                                \
         cudaError_t e = set_smem<T>((const void *)kf_plane_rho<T, NN, NN>, smem);                                    \
         if (e != cudaSuccess) return e;                                                                              \
+        if (per_sm) return ctas_per_sm(kf_plane_rho<T, NN, NN>, smem, per_sm);                                       \
         kf_plane_rho<T, NN, NN><<<grid, FFT_THREADS, smem, st>>>(kp, (const Cx<T> *)L.twx, (const Cx<T> *)L.twy,     \
                                                                  (const Cx<T> *)A, nb, Bg, w, (T *)rho_part, L.Jc);  \
         return cudaGetLastError();                                                                                   \
@@ -1628,6 +1635,7 @@ cudaError_t launch_plane_rho(const FftLaunch &L, const void *A, int nb, int G, i
     }
     cudaError_t e = set_smem<T>((const void *)k_plane_rho<T>, smem);
     if (e != cudaSuccess) return e;
+    if (per_sm) return ctas_per_sm(k_plane_rho<T>, smem, per_sm);
     dim3 grid(kp.N3, G);
     k_plane_rho<T><<<grid, FFT_THREADS, smem, st>>>(kp, L.dx, L.dy, (const Cx<T> *)L.twx, (const Cx<T> *)L.twy,
                                                     (const Cx<T> *)A, nb, Bg, w, (T *)rho_part, L.Jc);
@@ -1679,7 +1687,7 @@ cudaError_t launch_zero(void *p, int Ngw, int nb, int64_t ld, cudaStream_t st) {
                                           const void *, void *, int, const int *, const int *, const double *, int,  \
                                           const int2 *, int, int, cudaStream_t);                                                             \
     template cudaError_t launch_plane_rho<T>(const FftLaunch &, const void *, int, int, int, const double *, void *, \
-                                             cudaStream_t);                                                          \
+                                             cudaStream_t, int *);                                                          \
     template cudaError_t launch_rho_reduce<T>(const void *, int, size_t, double *, int, cudaStream_t);              \
     template cudaError_t launch_opK<T>(int, int, const double *, const void *, void *, int64_t, int, cudaStream_t); \
     template cudaError_t launch_kprec<T>(int, int, const double *, const void *, void *, int64_t, cudaStream_t);    \

@@ -51,13 +51,15 @@ template <typename T> cudaError_t launch_plane_vloc(const FftLaunch &, const voi
 template <typename T> cudaError_t launch_any_plane_vloc(const FftLaunch &, const void *Vr, void *A, int nb, cudaStream_t);
 template <typename T>
 cudaError_t launch_any_plane_rho(const FftLaunch &, const void *A, int nb, int G, int Bg, const double *w, void *rho_part,
-                                 cudaStream_t);
+                                 cudaStream_t, int *per_sm);
 template <> cudaError_t launch_any_plane_vloc<float>(const FftLaunch &, const void *, void *, int, cudaStream_t);
 template <> cudaError_t launch_any_plane_vloc<double>(const FftLaunch &, const void *, void *, int, cudaStream_t);
 template <>
-cudaError_t launch_any_plane_rho<float>(const FftLaunch &, const void *, int, int, int, const double *, void *, cudaStream_t);
+cudaError_t launch_any_plane_rho<float>(const FftLaunch &, const void *, int, int, int, const double *, void *, cudaStream_t,
+                                        int *);
 template <>
-cudaError_t launch_any_plane_rho<double>(const FftLaunch &, const void *, int, int, int, const double *, void *, cudaStream_t);
+cudaError_t launch_any_plane_rho<double>(const FftLaunch &, const void *, int, int, int, const double *, void *, cudaStream_t,
+                                         int *);
 // One projector column of betaNL (PsPotNL.jl:147-195 order): its atom,
 // angular momentum l, m in [-l, l], radial index i (1-based), r_l and the
 // normalisation of eval_proj_G.
@@ -77,8 +79,9 @@ cudaError_t launch_multik_persistent(const FftLaunch &L, const MkK *ks, const in
                                      const void *Vr, void *A, int flags, const int *Drow, const int *Dcol,
                                      const double *Dval, int nbeta, unsigned *ctr, int *err, cudaStream_t st);
 template <typename T>
+// per_sm != nullptr: nothing is launched, *per_sm = CTAs of the pass that an SM holds
 cudaError_t launch_plane_rho(const FftLaunch &, const void *A, int nb, int G, int Bg, const double *w, void *rho_part,
-                             cudaStream_t);
+                             cudaStream_t, int *per_sm = nullptr);
 template <typename T> cudaError_t launch_rho_reduce(const void *part, int G, size_t N, double *rho, int acc, cudaStream_t);
 template <typename T>
 cudaError_t launch_opK(int Ngw, int nb, const double *Gk2, const void *psi, void *Hpsi, int64_t ld, int acc, cudaStream_t);
