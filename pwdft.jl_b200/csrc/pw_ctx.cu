@@ -448,16 +448,15 @@ int apply_T(pw_ctx *c, int ik, int ispin, const void *psi, void *Hpsi, int64_t l
             c->launches += 3;
         } else {
             if ((s = ensure(c, c->P2, pb))) return s;
-            if ((s = ensure(c, c->gemm_ws, sizeof(T) == 8 ? project_ws_bytes(kd.Ngw, c->nbeta, nb)
-                                                          : gemm_tn_ws_bytes((int)sizeof(T), kd.Ngw, c->nbeta, nb))))
-                return s;
             if (sizeof(T) == 8) {
+                if ((s = ensure(c, c->gemm_ws, project_ws_bytes(kd.Ngw, c->nbeta, nb)))) return s;
                 CK(c, project_dcsr(kd.Ngw, c->nbeta, nb, kd.d_beta64, (const double2 *)psi, ld, c->d_Drow, c->d_Dcol, c->d_Dval,
                                    (double2 *)c->P2.p, c->gemm_ws.p, st));
                 c->launches += 2;
             } else {
-                if ((s = ensure(c, c->P, pb))) return s;
-                CK(c, (gemm_tn<T>(kd.Ngw, c->nbeta, nb, beta, kd.Ngw, psi, ld, (double2 *)c->P.p, c->nbeta, 0, c->gemm_ws.p, st)));
+                const TnPlan p = gemm_tn_plan((int)sizeof(T), kd.Ngw, c->nbeta, nb);
+                if ((s = ensure(c, c->gemm_ws, p.ws_bytes)) || (s = ensure(c, c->P, pb))) return s;
+                CK(c, (gemm_tn<T>(p, kd.Ngw, c->nbeta, nb, beta, kd.Ngw, psi, ld, (double2 *)c->P.p, c->nbeta, 0, c->gemm_ws.p, st)));
                 CK(c, apply_dcsr(c->nbeta, nb, c->d_Drow, c->d_Dcol, c->d_Dval, (const double2 *)c->P.p, (double2 *)c->P2.p, st));
                 c->launches += 3;
             }
@@ -1144,12 +1143,13 @@ extern "C" int pw_gram(pw_ctx *c, int dtype, int64_t K, int m, int n, const void
     if (dtype == PW_C64 && c->use_umma) return umma_tn<double2>(c, K, m, n, A, lda, B, ldb, C, ldc, accumulate);
     // A^H A: one triangle is formed, the other is its conjugate
     const int same = dtype == PW_C128 && A == B && lda == ldb && m == n ? 2 : 0;
-    if ((s = ensure(c, c->gemm_ws, gemm_tn_ws_bytes(dtype == PW_C128 ? 8 : 4, K, m, n, same)))) return s;
+    const TnPlan p = gemm_tn_plan(dtype == PW_C128 ? 8 : 4, K, m, n, same);
+    if ((s = ensure(c, c->gemm_ws, p.ws_bytes))) return s;
     if (dtype == PW_C128)
-        CK(c, gemm_tn<double>(K, m, n, A, lda, B, ldb, (double2 *)C, ldc, accumulate, c->gemm_ws.p, c->stream, same));
+        CK(c, gemm_tn<double>(p, K, m, n, A, lda, B, ldb, (double2 *)C, ldc, accumulate, c->gemm_ws.p, c->stream, same));
     else
-        CK(c, gemm_tn<float>(K, m, n, A, lda, B, ldb, (double2 *)C, ldc, accumulate, c->gemm_ws.p, c->stream));
-    c->launches += gemm_tn_launches(dtype == PW_C128 ? 8 : 4, K, m, n, same);
+        CK(c, gemm_tn<float>(p, K, m, n, A, lda, B, ldb, (double2 *)C, ldc, accumulate, c->gemm_ws.p, c->stream));
+    c->launches += p.launches;
     return PW_OK;
 }
 
@@ -1165,12 +1165,13 @@ int pwk_gram_upper(pw_ctx *c, int dtype, int64_t K, int m, const void *A, int64_
     if (!A || !B || !C || K <= 0 || m <= 0 || lda < K || ldb < K || ldc < m) return fail(c, PW_ERR_ARG, "bad gram arguments");
     CK(c, cudaSetDevice(c->device));
     if (dtype == PW_C64 && c->use_umma) return umma_tn<double2>(c, K, m, m, A, lda, B, ldb, C, ldc, 0, 1);
-    if ((s = ensure(c, c->gemm_ws, gemm_tn_ws_bytes(dtype == PW_C128 ? 8 : 4, K, m, m, 1)))) return s;
+    const TnPlan p = gemm_tn_plan(dtype == PW_C128 ? 8 : 4, K, m, m, 1);
+    if ((s = ensure(c, c->gemm_ws, p.ws_bytes))) return s;
     if (dtype == PW_C128)
-        CK(c, gemm_tn<double>(K, m, m, A, lda, B, ldb, (double2 *)C, ldc, 0, c->gemm_ws.p, c->stream, 1));
+        CK(c, gemm_tn<double>(p, K, m, m, A, lda, B, ldb, (double2 *)C, ldc, 0, c->gemm_ws.p, c->stream, 1));
     else
-        CK(c, gemm_tn<float>(K, m, m, A, lda, B, ldb, (double2 *)C, ldc, 0, c->gemm_ws.p, c->stream, 1));
-    c->launches += gemm_tn_launches(dtype == PW_C128 ? 8 : 4, K, m, m, 1);
+        CK(c, gemm_tn<float>(p, K, m, m, A, lda, B, ldb, (double2 *)C, ldc, 0, c->gemm_ws.p, c->stream, 1));
+    c->launches += p.launches;
     return PW_OK;
 }
 
@@ -1352,12 +1353,13 @@ int pwk_beta_dot(pw_ctx *c, int ik, int dtype, const void *psi, int64_t ld, int 
         CK(c, umma_gemm<double2>(kd.beta_tn, B, c->nbeta, nb, out, c->nbeta, 0, (float *)c->um_ws.p, c->d_err, st));
         c->launches += 2 + (umma_splits(kd.beta_tn.rows, nb, kd.beta_tn.Kp) > 1 ? 1 : 0);
     } else {
-        if ((s = ensure(c, c->gemm_ws, gemm_tn_ws_bytes(dtype == PW_C128 ? 8 : 4, kd.Ngw, c->nbeta, nb)))) return s;
+        const TnPlan p = gemm_tn_plan(dtype == PW_C128 ? 8 : 4, kd.Ngw, c->nbeta, nb);
+        if ((s = ensure(c, c->gemm_ws, p.ws_bytes))) return s;
         if (dtype == PW_C128)
-            CK(c, (gemm_tn<double>(kd.Ngw, c->nbeta, nb, beta, kd.Ngw, psi, ld, out, c->nbeta, 0, c->gemm_ws.p, st)));
+            CK(c, (gemm_tn<double>(p, kd.Ngw, c->nbeta, nb, beta, kd.Ngw, psi, ld, out, c->nbeta, 0, c->gemm_ws.p, st)));
         else
-            CK(c, (gemm_tn<float>(kd.Ngw, c->nbeta, nb, beta, kd.Ngw, psi, ld, out, c->nbeta, 0, c->gemm_ws.p, st)));
-        c->launches += gemm_tn_launches(dtype == PW_C128 ? 8 : 4, kd.Ngw, c->nbeta, nb);
+            CK(c, (gemm_tn<float>(p, kd.Ngw, c->nbeta, nb, beta, kd.Ngw, psi, ld, out, c->nbeta, 0, c->gemm_ws.p, st)));
+        c->launches += p.launches;
     }
     return PW_OK;
 }

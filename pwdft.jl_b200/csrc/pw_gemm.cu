@@ -98,7 +98,8 @@ __device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
 
 // k range of the CTA: [kbeg, kend).  direct: C is written (or added to)
 // here, else the partial sums go to C[z][n][m] (ld m) for k_splitk_reduce.
-// upper (TN): tiles strictly below the diagonal are skipped.  tri (NN):
+// upper (TN): tiles strictly below the diagonal are skipped; 2: with direct, the
+// other triangle gets the conjugates.  tri (NN):
 // triangular structure the caller guarantees (the k-loop skips the zero
 // blocks, whole tiles are skipped where no needed output lies):
 //   1  A lower triangular (A[g][l] = 0 for l > g)
@@ -203,9 +204,13 @@ k_zgemm(int64_t K, int64_t m, int n, const double2 *__restrict__ A, int64_t lda,
                 const int nn = n0 + wn + 8 * j + 2 * t + q;
                 if (mm < m && nn < n) {
                     double2 *p = direct ? &C[(size_t)nn * ldc + mm] : &C[(size_t)nn * m + mm];
-                    double2 v = make_double2(re[i][j][q], im[i][j][q]);
-                    if (direct && accumulate) v = cadd(*p, v);
-                    if (!(direct && upper && mm > nn)) *p = v;
+                    const double2 v = make_double2(re[i][j][q], im[i][j][q]);
+                    if (!(direct && upper && mm > nn)) *p = direct && accumulate ? cadd(*p, v) : v;
+                    if (direct && upper == 2 && mm < nn) {
+                        double2 *h = &C[(size_t)mm * ldc + nn];
+                        const double2 cv = make_double2(v.x, -v.y);
+                        *h = accumulate ? cadd(*h, cv) : cv;
+                    }
                 }
             }
     }
@@ -223,13 +228,9 @@ k_zgemm(int64_t K, int64_t m, int n, const double2 *__restrict__ A, int64_t lda,
 // formed tiles count but every split has room for all.  Few values are split too
 // (betaNL' psi of 8 bands over about 730 plane waves: 35.8 us on one CTA, 5.0 in 23
 // parts).
-struct ZPlan {
-    int wm, wn, S;
-    int64_t kchunk;
-};
 // fused: the caller's next pass sums the splits.
-ZPlan zplan(int64_t K, int64_t m, int n, bool tn, int upper, bool fused = false) {
-    ZPlan best{2, 2, 1, K};
+TnPlan zplan(int64_t K, int64_t m, int n, bool tn, int upper, bool fused = false) {
+    TnPlan best{2, 2, 1, K, 0, 1};
     double tbest = 1e300;
     for (int wm = 2; wm <= 4; ++wm)
         for (int wn = 1; wn <= 5; ++wn) {
@@ -252,7 +253,7 @@ ZPlan zplan(int64_t K, int64_t m, int n, bool tn, int upper, bool fused = false)
                 if (S > 1) t += (fused ? 0.0 : 4000.0) + (double)S * m * n * 32.0 / 2400.0;
                 if (t < tbest * (1.0 - 1e-9)) {
                     tbest = t;
-                    best = ZPlan{wm, wn, S, K};
+                    best = TnPlan{wm, wn, S, K, 0, 1};
                 }
             }
         }
@@ -262,7 +263,7 @@ ZPlan zplan(int64_t K, int64_t m, int n, bool tn, int upper, bool fused = false)
 }
 
 template <int WM, int WN, bool TN>
-cudaError_t launch_z(const ZPlan &p, int64_t K, int64_t m, int n, const double2 *A, int64_t lda, const double2 *B,
+cudaError_t launch_z(const TnPlan &p, int64_t K, int64_t m, int n, const double2 *A, int64_t lda, const double2 *B,
                      int64_t ldb, double2 *C, int64_t ldc, int direct, int accumulate, int upper, int tri, cudaStream_t st) {
     constexpr size_t smem = zgemm_smem<WM, WN, TN>();
     if (smem > 48 * 1024) {
@@ -274,7 +275,7 @@ cudaError_t launch_z(const ZPlan &p, int64_t K, int64_t m, int n, const double2 
     return cudaGetLastError();
 }
 template <bool TN>
-cudaError_t launch_zgemm(const ZPlan &p, int64_t K, int64_t m, int n, const void *A, int64_t lda, const void *B, int64_t ldb,
+cudaError_t launch_zgemm(const TnPlan &p, int64_t K, int64_t m, int n, const void *A, int64_t lda, const void *B, int64_t ldb,
                          double2 *C, int64_t ldc, int direct, int accumulate, int upper, int tri, cudaStream_t st) {
     const double2 *a = (const double2 *)A, *b = (const double2 *)B;
 #define PW_Z(WM, WN)               \
@@ -294,6 +295,15 @@ cudaError_t launch_zgemm(const ZPlan &p, int64_t K, int64_t m, int n, const void
 // C[j ldc + i] (+)= sum over the S partial sums W[z][j][i].  upper: 1 = only
 // i <= j is formed and written, 2 = only i <= j was formed and the other
 // triangle gets its conjugate transpose (A^H A).
+__device__ __forceinline__ void put_sum(double2 *C, int64_t ldc, int mm, int nn, double2 s, int accumulate, int upper) {
+    double2 *p = &C[(size_t)nn * ldc + mm];
+    *p = accumulate ? cadd(*p, s) : s;
+    if (upper == 2 && mm < nn) {
+        double2 *q = &C[(size_t)mm * ldc + nn];
+        const double2 h = make_double2(s.x, -s.y);
+        *q = accumulate ? cadd(*q, h) : h;
+    }
+}
 __global__ void k_splitk_reduce(const double2 *__restrict__ W, int S, int m, int n, double2 *__restrict__ C, int64_t ldc,
                                 int accumulate, int upper) {
     const size_t total = (size_t)m * n;
@@ -303,13 +313,31 @@ __global__ void k_splitk_reduce(const double2 *__restrict__ W, int S, int m, int
         double2 s = make_double2(0.0, 0.0);
 #pragma unroll 4
         for (int z = 0; z < S; ++z) s = cadd(s, W[(size_t)z * total + t]);
-        double2 *p = &C[(size_t)nn * ldc + mm];
-        *p = accumulate ? cadd(*p, s) : s;
-        if (upper == 2 && mm < nn) {
-            double2 *q = &C[(size_t)mm * ldc + nn];
-            const double2 h = make_double2(s.x, -s.y);
-            *q = accumulate ? cadd(*q, h) : h;
+        put_sum(C, ldc, mm, nn, s, accumulate, upper);
+    }
+}
+// The same with eight lanes to an element, for many parts and few elements (4 x 4
+// values over 24,000 in FP64, 148 parts: the product 41 us with one thread an
+// element, 14 with eight).
+__global__ void k_splitk_reduce8(const double2 *__restrict__ W, int S, int m, int n, double2 *__restrict__ C, int64_t ldc,
+                                 int accumulate, int upper) {
+    const size_t total = (size_t)m * n;
+    const int l8 = threadIdx.x & 7;
+    for (size_t t0 = (blockIdx.x * (size_t)blockDim.x + (threadIdx.x & ~31)) >> 3; t0 < total;
+         t0 += ((size_t)gridDim.x * blockDim.x) >> 3) {
+        const size_t t = t0 + ((threadIdx.x & 31) >> 3);
+        const int nn = (int)(t / m), mm = (int)(t - (size_t)nn * m);
+        const bool in = t < total && !(upper && mm > nn);
+        double2 s = make_double2(0.0, 0.0);
+        if (in) {
+#pragma unroll 4
+            for (int z = l8; z < S; z += 8) s = cadd(s, W[(size_t)z * total + t]);
         }
+        for (int o = 4; o > 0; o >>= 1) {
+            s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
+            s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
+        }
+        if (in && l8 == 0) put_sum(C, ldc, mm, nn, s, accumulate, upper);
     }
 }
 
@@ -439,37 +467,42 @@ int splitk_count(int64_t K, int m, int n) {
 
 }  // namespace
 
-int gemm_tn_launches(int real_bytes, int64_t K, int m, int n, int upper) {
-    return real_bytes == 8 && upper != 2 && zplan(K, m, n, true, upper).S == 1 ? 1 : 2;
-}
-
-size_t gemm_tn_ws_bytes(int real_bytes, int64_t K, int m, int n, int upper) {
-    const size_t S = real_bytes == 8 ? zplan(K, m, n, true, upper).S : splitk_count(K, m, n);
-    return gemm_tn_launches(real_bytes, K, m, n, upper) == 1 ? 0 : S * m * n * sizeof(double2);
+TnPlan gemm_tn_plan(int real_bytes, int64_t K, int m, int n, int upper) {
+    if (real_bytes == 8) {
+        TnPlan p = zplan(K, m, n, true, upper);
+        if (p.S > 1) {
+            p.ws_bytes = (size_t)p.S * m * n * sizeof(double2);
+            p.launches = 2;
+        }
+        return p;
+    }
+    TnPlan p{0, 0, splitk_count(K, m, n), 0, 0, 2};
+    p.kchunk = ((K + p.S - 1) / p.S + TN_BK - 1) / TN_BK * TN_BK;
+    p.ws_bytes = (size_t)p.S * m * n * sizeof(double2);
+    return p;
 }
 
 template <typename T>
-cudaError_t gemm_tn(int64_t K, int m, int n, const void *A, int64_t lda, const void *B, int64_t ldb, double2 *C,
-                    int64_t ldc, int accumulate, void *ws, cudaStream_t st, int upper) {
+cudaError_t gemm_tn(const TnPlan &p, int64_t K, int m, int n, const void *A, int64_t lda, const void *B, int64_t ldb,
+                    double2 *C, int64_t ldc, int accumulate, void *ws, cudaStream_t st, int upper) {
     if (m <= 0 || n <= 0) return cudaSuccess;
-    int S;
+    const int S = p.S;
     cudaError_t e;
     if constexpr (sizeof(T) == 8) {
-        const ZPlan p = zplan(K, m, n, true, upper);
-        S = p.S;
-        const int direct = S == 1 && upper != 2;
+        const int direct = p.ws_bytes == 0;
         e = launch_zgemm<true>(p, K, m, n, A, lda, B, ldb, direct ? C : (double2 *)ws, ldc, direct, accumulate, upper, 0, st);
         if (e != cudaSuccess || direct) return e;
     } else {
-        S = splitk_count(K, m, n);
-        int64_t kchunk = (K + S - 1) / S;
-        kchunk = ((kchunk + TN_BK - 1) / TN_BK) * TN_BK;
         dim3 grid((m + TN_BM - 1) / TN_BM, (n + TN_BN - 1) / TN_BN, S);
-        k_gemm_tn<T><<<grid, 256, 0, st>>>(K, m, n, (const Cx<T> *)A, lda, (const Cx<T> *)B, ldb, (double2 *)ws, kchunk, upper);
+        k_gemm_tn<T><<<grid, 256, 0, st>>>(K, m, n, (const Cx<T> *)A, lda, (const Cx<T> *)B, ldb, (double2 *)ws, p.kchunk, upper);
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
-    k_splitk_reduce<<<blocks_for((size_t)m * n), 256, 0, st>>>((const double2 *)ws, S, m, n, C, ldc, accumulate, upper);
+    const size_t total = (size_t)m * n;
+    if (S >= 16 && total <= 65536)
+        k_splitk_reduce8<<<blocks_for(total * 8), 256, 0, st>>>((const double2 *)ws, S, m, n, C, ldc, accumulate, upper);
+    else
+        k_splitk_reduce<<<blocks_for(total), 256, 0, st>>>((const double2 *)ws, S, m, n, C, ldc, accumulate, upper);
     return cudaGetLastError();
 }
 
@@ -487,9 +520,9 @@ cudaError_t gemm_nn(int64_t M, int n, int k, const void *A, int64_t lda, const d
     }
 }
 
-template cudaError_t gemm_tn<float>(int64_t, int, int, const void *, int64_t, const void *, int64_t, double2 *, int64_t,
+template cudaError_t gemm_tn<float>(const TnPlan &, int64_t, int, int, const void *, int64_t, const void *, int64_t, double2 *, int64_t,
                                     int, void *, cudaStream_t, int);
-template cudaError_t gemm_tn<double>(int64_t, int, int, const void *, int64_t, const void *, int64_t, double2 *, int64_t,
+template cudaError_t gemm_tn<double>(const TnPlan &, int64_t, int, int, const void *, int64_t, const void *, int64_t, double2 *, int64_t,
                                      int, void *, cudaStream_t, int);
 template cudaError_t gemm_nn<float>(int64_t, int, int, const void *, int64_t, const double2 *, int64_t, void *, int64_t,
                                     int, cudaStream_t, int);
@@ -501,7 +534,7 @@ size_t project_ws_bytes(int64_t K, int nbeta, int nb) {
 }
 cudaError_t project_dcsr(int64_t K, int nbeta, int nb, const double2 *beta, const double2 *psi, int64_t ldp, const int *rowptr,
                          const int *col, const double *val, double2 *P2, void *ws, cudaStream_t st) {
-    const ZPlan p = zplan(K, nbeta, nb, true, 0, true);
+    const TnPlan p = zplan(K, nbeta, nb, true, 0, true);
     cudaError_t e = launch_zgemm<true>(p, K, nbeta, nb, beta, K, psi, ldp, (double2 *)ws, 0, 0, 0, 0, 0, st);
     if (e != cudaSuccess) return e;
     k_dcsr_splits<<<blocks_for((size_t)nbeta * nb * 8), 256, 0, st>>>(nbeta, nb, rowptr, col, val, (const double2 *)ws, p.S, P2);

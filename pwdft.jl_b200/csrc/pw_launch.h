@@ -92,18 +92,22 @@ template <typename T>
 cudaError_t launch_polarize(int Ngw, int nb, const void *psi, const void *lam, int64_t ld, void *out, cudaStream_t);
 
 // C (m x n, double2, ldc) (+)= A^H B with A (K x m), B (K x n) of element Cx<T>.
-// ws: split-K workspace of at least gemm_tn_ws_bytes() bytes (real_bytes =
-// sizeof(T), same K, m, n, upper).
-size_t gemm_tn_ws_bytes(int real_bytes, int64_t K, int m, int n, int upper = 0);
-// kernels that it launches (1: C is written directly, no workspace)
-int gemm_tn_launches(int real_bytes, int64_t K, int m, int n, int upper = 0);
+// plan: of gemm_tn_plan() for sizeof(T) and the same K, m, n, upper; ws: its
+// workspace.
+struct TnPlan {
+    int wm, wn, S;      // tile 16 wm x 16 wn (FP64), parts of the sum
+    int64_t kchunk;     // K values a part
+    size_t ws_bytes;    // workspace (0: C is written directly)
+    int launches;
+};
+TnPlan gemm_tn_plan(int real_bytes, int64_t K, int m, int n, int upper = 0);
 template <typename T>
 // upper: 1 = only C[i][j] with i <= j is formed and written (Hermitian
 // products whose consumer reads the upper triangle); tiles strictly below
 // the diagonal are skipped.  2 (T = double, A = B) = the same work, the other
 // triangle filled with its conjugate transpose.
-cudaError_t gemm_tn(int64_t K, int m, int n, const void *A, int64_t lda, const void *B, int64_t ldb, double2 *C,
-                    int64_t ldc, int accumulate, void *ws, cudaStream_t, int upper = 0);
+cudaError_t gemm_tn(const TnPlan &plan, int64_t K, int m, int n, const void *A, int64_t lda, const void *B, int64_t ldb,
+                    double2 *C, int64_t ldc, int accumulate, void *ws, cudaStream_t, int upper = 0);
 // C (M x n, Cx<T>, ldc) (+)= A (M x k, Cx<T>) * B (k x n, double2); tri: 1 = A
 // lower triangular, 2 = B upper triangular and only C's upper triangle
 // needed, 3 = A upper triangular (zero blocks skipped)

@@ -51,6 +51,14 @@ def test_gram_edges(ctx, K, m, n, pad):
     assert ((S - 2 * refS).abs() <= 4 * K * EPS * (A.abs() @ A.abs().T) + 8 * EPS).all()
 
 
+@pytest.mark.parametrize("K,m,n", [(30, 5, 5), (24007, 1, 1), (24007, 3, 11), (40009, 33, 33), (9001, 256, 256),
+                                   (9001, 257, 256)])
+def test_few_values_in_many_parts(ctx, K, m, n):
+    """Sums without parts, with one thread and with eight lanes an element (up to
+    65,536 elements), both triangles; bound as above."""
+    test_gram_edges(ctx, K, m, n, 0)
+
+
 @pytest.mark.parametrize("M,n,k,pad", [(1, 1, 1, 0), (17, 3, 7, 1), (63, 16, 8, 0), (65, 33, 9, 2), (1009, 48, 50, 0),
                                        (5003, 81, 161, 3), (12007, 161, 480, 0)])
 def test_rotate_edges(ctx, M, n, k, pad):
