@@ -395,9 +395,10 @@ int umma_tn(pw_ctx *c, int64_t K, int m, int n, const void *Z, int64_t ldz, cons
         if ((s = umma_scratch(c, c->um_b_hi, c->um_b_lo, n, K, B))) return s;
         CK(c, umma_prep_tn<float2>(Wm, ldw, K, n, B, c->stream));
     }
-    if ((s = ensure(c, c->um_ws, umma_ws_bytes(A.rows, n, A.Kp, c->gemm_splits, upper)))) return s;
-    CK(c, umma_gemm<CT>(A, B, m, n, C, ldc, acc, (float *)c->um_ws.p, c->d_err, c->stream, upper, same, c->gemm_splits));
-    c->launches += (same ? 2 : 3) + (upper == 2 || umma_splits(A.rows, n, A.Kp, c->gemm_splits, upper) > 1 ? 1 : 0);
+    const UmmaPlan plan = umma_plan(A.rows, n, A.Kp, c->gemm_splits, upper);
+    if (plan.passes > 1 && (s = ensure(c, c->um_ws, plan.ws_bytes))) return s;
+    CK(c, umma_gemm<CT>(plan, A, B, m, n, C, ldc, acc, (float *)c->um_ws.p, c->d_err, c->stream, upper, same));
+    c->launches += (same ? 1 : 2) + plan.passes;
     return PW_OK;
 }
 
@@ -411,10 +412,10 @@ int umma_nn(pw_ctx *c, int64_t M, int n, int k, const void *A, int64_t lda, cons
     c->launches += 1;
     if ((s = umma_scratch(c, c->um_b_hi, c->um_b_lo, n, k, B))) return s;
     CK(c, umma_prep_tn<double2>(U, ldu, k, n, B, c->stream));
-    if ((s = ensure(c, c->um_ws, umma_ws_bytes(Ao.rows, n, Ao.Kp, c->gemm_splits)))) return s;
-    CK(c, umma_gemm<float2>(Ao, B, (int)M, n, C, ldc, acc, (float *)c->um_ws.p, c->d_err, c->stream, 0, 0,
-                            c->gemm_splits));
-    c->launches += 2 + (umma_splits(Ao.rows, n, Ao.Kp, c->gemm_splits) > 1 ? 1 : 0);
+    const UmmaPlan plan = umma_plan(Ao.rows, n, Ao.Kp, c->gemm_splits);
+    if (plan.passes > 1 && (s = ensure(c, c->um_ws, plan.ws_bytes))) return s;
+    CK(c, umma_gemm<float2>(plan, Ao, B, (int)M, n, C, ldc, acc, (float *)c->um_ws.p, c->d_err, c->stream));
+    c->launches += 1 + plan.passes;
     return PW_OK;
 }
 
@@ -440,10 +441,11 @@ int apply_T(pw_ctx *c, int ik, int ispin, const void *psi, void *Hpsi, int64_t l
             UmmaOperand B;
             if ((s = umma_scratch(c, c->um_b_hi, c->um_b_lo, nb, kd.Ngw, B, &c->um_b_lo2))) return s;
             CK(c, umma_prep_tn<float2>(psi, ld, kd.Ngw, nb, B, st));
-            if ((s = ensure(c, c->um_ws, umma_ws_bytes(kd.beta_tn.rows, nb, kd.beta_tn.Kp)))) return s;
-            CK(c, umma_gemm<double2>(kd.beta_tn, B, c->nbeta, nb, nullptr, 0, 0, (float *)c->um_ws.p, c->d_err, st));
+            const UmmaPlan plan = umma_plan(kd.beta_tn.rows, nb, kd.beta_tn.Kp);
+            if ((s = ensure(c, c->um_ws, plan.ws_bytes))) return s;
+            CK(c, umma_gemm<double2>(plan, kd.beta_tn, B, c->nbeta, nb, nullptr, 0, 0, (float *)c->um_ws.p, c->d_err, st));
             if ((s = umma_scratch(c, c->um_b_hi, c->um_b_lo, nb, c->nbeta, P2op))) return s;
-            CK(c, umma_dcsr_prep((const float *)c->um_ws.p, umma_splits(kd.beta_tn.rows, nb, kd.beta_tn.Kp), c->nbeta, nb,
+            CK(c, umma_dcsr_prep((const float *)c->um_ws.p, plan.S, c->nbeta, nb,
                                  c->d_Drow, c->d_Dcol, c->d_Dval, P2op, st));
             c->launches += 3;
         } else {
@@ -491,10 +493,10 @@ int apply_T(pw_ctx *c, int ik, int ispin, const void *psi, void *Hpsi, int64_t l
     if (o & PW_OP_VNL) {
         if (sizeof(T) == 4 && c->use_umma) {
             int s;
-            if ((s = ensure(c, c->um_ws, umma_ws_bytes(kd.beta_nn.rows, nb, kd.beta_nn.Kp, c->gemm_splits)))) return s;
-            CK(c, umma_gemm<float2>(kd.beta_nn, P2op, kd.Ngw, nb, Hpsi, ld, 1, (float *)c->um_ws.p, c->d_err, st, 0, 0,
-                                    c->gemm_splits));
-            c->launches += umma_splits(kd.beta_nn.rows, nb, kd.beta_nn.Kp, c->gemm_splits) > 1 ? 2 : 1;
+            const UmmaPlan plan = umma_plan(kd.beta_nn.rows, nb, kd.beta_nn.Kp, c->gemm_splits);
+            if (plan.passes > 1 && (s = ensure(c, c->um_ws, plan.ws_bytes))) return s;
+            CK(c, umma_gemm<float2>(plan, kd.beta_nn, P2op, kd.Ngw, nb, Hpsi, ld, 1, (float *)c->um_ws.p, c->d_err, st));
+            c->launches += plan.passes;
         } else {
             CK(c, gemm_nn<T>(kd.Ngw, nb, c->nbeta, beta, kd.Ngw, (const double2 *)c->P2.p, c->nbeta, Hpsi, ld, 1, st));
             c->launches += 1;
@@ -1349,9 +1351,10 @@ int pwk_beta_dot(pw_ctx *c, int ik, int dtype, const void *psi, int64_t ld, int 
         UmmaOperand B;
         if ((s = umma_scratch(c, c->um_b_hi, c->um_b_lo, nb, kd.Ngw, B, &c->um_b_lo2))) return s;
         CK(c, umma_prep_tn<float2>(psi, ld, kd.Ngw, nb, B, st));
-        if ((s = ensure(c, c->um_ws, umma_ws_bytes(kd.beta_tn.rows, nb, kd.beta_tn.Kp)))) return s;
-        CK(c, umma_gemm<double2>(kd.beta_tn, B, c->nbeta, nb, out, c->nbeta, 0, (float *)c->um_ws.p, c->d_err, st));
-        c->launches += 2 + (umma_splits(kd.beta_tn.rows, nb, kd.beta_tn.Kp) > 1 ? 1 : 0);
+        const UmmaPlan plan = umma_plan(kd.beta_tn.rows, nb, kd.beta_tn.Kp);
+        if (plan.passes > 1 && (s = ensure(c, c->um_ws, plan.ws_bytes))) return s;
+        CK(c, umma_gemm<double2>(plan, kd.beta_tn, B, c->nbeta, nb, out, c->nbeta, 0, (float *)c->um_ws.p, c->d_err, st));
+        c->launches += 1 + plan.passes;
     } else {
         const TnPlan p = gemm_tn_plan(dtype == PW_C128 ? 8 : 4, kd.Ngw, c->nbeta, nb);
         if ((s = ensure(c, c->gemm_ws, p.ws_bytes))) return s;

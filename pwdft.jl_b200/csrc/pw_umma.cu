@@ -42,6 +42,9 @@
 #include <cuda_bf16.h>
 #include <cudaTypedefs.h>
 
+#include <algorithm>
+#include <cmath>
+
 #include "pw_launch.h"
 #include "pw_umma.h"
 
@@ -180,13 +183,27 @@ __device__ __forceinline__ void store_columns(E *C, int64_t ld, const float2 *T2
     }
 }
 
+// The same columns' conjugates to the other triangle of C (one split of Z^H Z,
+// complex128; the widest tile has no registers for it: 24 -> 40 bytes spilled).
+template <int BN> constexpr bool MIRROR_BN = BN < 128;
+__device__ __noinline__ void mirror_columns(double2 *C, int64_t ld, const float2 *T2, int m0, int n0, int N, int cols, bool add) {
+    for (int e = threadIdx.x - 64; e < cols * BM; e += 256) {
+        const int c = e / BM, r = e % BM, i = m0 + r, n = n0 + c;
+        if (i < n && n < N) {
+            double2 *h = C + (size_t)i * ld + n;
+            const float2 v = T2[c * (BM + 1) + r];
+            *h = make_double2((add ? h->x : 0.0) + v.x, (add ? h->y : 0.0) - v.y);
+        }
+    }
+}
+
 // C (m x n complex) = sum over the split's k-blocks of the piece products
 //   NS = 2:  A0 B0 + A0 B1 + A1 B0
 //   NS = 3:  A0 B0 + A0 B1 + A1 B0 + A0 B2 + A1 B1 + A2 B0
 // written to W[z][n][m] (float2, column-major, ld = m), or, with a single
 // split (S == 1) and C given, into the result C (element (i, j) at
 // C[j ldc + i]; cdouble: C is complex128; accumulate: C += D; upper: only
-// i <= j written).
+// i <= j formed, 2: the other triangle filled with its conjugate).
 // A CTA runs the tiles blockIdx.x, + gridDim.x, ... of the (split, row block,
 // column block) list, the column block fastest: the CTAs that share a row block
 // of a tall A run together, so that A comes from DRAM once, and the products of
@@ -389,9 +406,11 @@ k_umma_gemm(const __grid_constant__ CUtensorMap tA0, const __grid_constant__ CUt
                 const float2 *T2 = reinterpret_cast<const float2 *>(T);
                 if (!direct)
                     store_columns(W + (size_t)(t / (nt * mt)) * M * (size_t)N, M, T2, m0, n0 + c0, M, N, cols, false, false);
-                else if (cdouble)
+                else if (cdouble) {
                     store_columns((double2 *)C, ldc, T2, m0, n0 + c0, M, N, cols, accumulate != 0, upper != 0);
-                else
+                    if constexpr (MIRROR_BN<BN>)
+                        if (upper == 2) mirror_columns((double2 *)C, ldc, T2, m0, n0 + c0, N, cols, accumulate != 0);
+                } else
                     store_columns((float2 *)C, ldc, T2, m0, n0 + c0, M, N, cols, accumulate != 0, upper != 0);
                 asm volatile("bar.sync 1, 256;" ::: "memory");
             }
@@ -495,6 +514,15 @@ __global__ void k_prep_nn_a(const CT *__restrict__ A, int64_t lda, int64_t M, in
 // formed and written, 2 = only i <= j was formed (Z^H Z) and the other
 // triangle gets its conjugate.
 template <typename CT>
+__device__ __forceinline__ void put_sum(CT *C, int64_t ldc, size_t i, size_t j, double re, double im, int accumulate, int upper) {
+    auto put = [&](CT *p, double y) {
+        p->x = accumulate ? re + (double)p->x : re;
+        p->y = accumulate ? y + (double)p->y : y;
+    };
+    put(C + j * ldc + i, im);
+    if (upper == 2 && i < j) put(C + i * ldc + j, -im);
+}
+template <typename CT>
 __global__ void k_finalize(const float2 *__restrict__ W, int S, int m, int n, CT *__restrict__ C, int64_t ldc, int accumulate,
                            int upper) {
     const size_t total = (size_t)m * n;
@@ -508,12 +536,35 @@ __global__ void k_finalize(const float2 *__restrict__ W, int S, int m, int n, CT
             re += (double)w.x;
             im += (double)w.y;
         }
-        auto put = [&](CT *p, double y) {
-            p->x = accumulate ? re + (double)p->x : re;
-            p->y = accumulate ? y + (double)p->y : y;
-        };
-        put(C + j * ldc + i, im);
-        if (upper == 2 && i < j) put(C + i * ldc + j, -im);
+        put_sum(C, ldc, i, j, re, im, accumulate, upper);
+    }
+}
+// The same with eight lanes to an element, for many parts and few elements: 8 x 8
+// values in 64 parts 17 us with one thread an element, 240 x 240 (one triangle) in
+// 47 parts 16 us against 10; 480 x 480 in 9 parts 6.5, here slower.
+template <typename CT>
+__global__ void k_finalize8(const float2 *__restrict__ W, int S, int m, int n, CT *__restrict__ C, int64_t ldc, int accumulate,
+                            int upper) {
+    const size_t total = (size_t)m * n;
+    const int l8 = threadIdx.x & 7;
+    for (size_t t0 = (blockIdx.x * (size_t)blockDim.x + (threadIdx.x & ~31)) >> 3; t0 < total;
+         t0 += ((size_t)gridDim.x * blockDim.x) >> 3) {
+        const size_t t = t0 + ((threadIdx.x & 31) >> 3), j = t / m, i = t - j * m;
+        const bool in = t < total && !(upper && i > j);
+        double re = 0.0, im = 0.0;
+        if (in) {
+#pragma unroll 4
+            for (int z = l8; z < S; z += 8) {
+                const float2 w = W[(size_t)z * total + t];
+                re += (double)w.x;
+                im += (double)w.y;
+            }
+        }
+        for (int o = 4; o > 0; o >>= 1) {
+            re += __shfl_xor_sync(0xffffffffu, re, o);
+            im += __shfl_xor_sync(0xffffffffu, im, o);
+        }
+        if (in && l8 == 0) put_sum(C, ldc, i, j, re, im, accumulate, upper);
     }
 }
 
@@ -621,60 +672,55 @@ cudaError_t umma_prep_nn_a(const void *A, int64_t lda, int64_t M, int k, UmmaOpe
     return cudaGetLastError();
 }
 
-// Output tile width for n complex columns: the one with the least padded
-// width, a column of a tile narrower than 128 counted dearer because the MMA
-// then waits for its operands (A's 128 rows and B's BN rows come from shared
-// memory at 128 bytes a clock: (128 + BN) / (2 BN) clocks a column).
-static int pick_bn(int n) {
-    int best = 128;
+// Tile width and split-K count of a product of M x N complex values: the pair with
+// the shortest modelled time, in units of about 1.2 us.  One CTA fits on an SM (222 KB
+// of shared memory), so the active tiles (those on or above the diagonal for a
+// Hermitian product) x splits run in waves of 148; a k-block takes 0.73 to 0.83
+// whatever the tile's width (the chain TMA, MMA, TMEM read), a tile 1.8 for its
+// pipeline and 0.23 for each 32 columns of its epilogue; split sums take a launch and
+// their trip through memory.  Splits: as many as fill whole waves, or as the split
+// sums' cost allows.  The numbers are a fit to 176 products (1 to 1440 columns, K =
+// 62 to 80,000) with each width and 5 to 15 split counts measured: the choice is 0.6 %
+// from the best of a product on average.  The width with the least padding and at
+// most 64 splits was up to 65 % off (8 x 8 values over 80,000: 68 us in 64 parts, 41
+// in 148; 100 x 100 over 200: 28.8 us in one tile, 19.2 in four narrow ones x 7).
+// Accuracy does not depend on either: every k-block is its own accumulation chain in
+// TMEM.
+UmmaPlan umma_plan(int64_t M, int N, int Kp, int splits, int upper) {
+    const int KB = Kp / BK, mt = (int)((M + BM - 1) / BM);
+    UmmaPlan best{128, 1, 1, 0};
     double tbest = 1e300;
     for (int bn : {128, 96, 80, 64, 32}) {
-        const double t = (double)((n + bn - 1) / bn) * std::max(1.0 * bn, 0.5 * (128 + bn));
-        if (t < tbest * (1.0 - 1e-9)) {
-            tbest = t;
-            best = bn;
+        if (bn > 32 && N <= (bn > 96 ? 96 : bn > 64 ? 64 : 32)) continue;   // a narrower tile holds all columns
+        const int nt = (N + bn - 1) / bn;
+        int active = mt * nt;
+        if (upper) {
+            active = 0;
+            for (int c = 0; c < nt; ++c) active += std::min(mt, (c * bn + bn - 1) / BM + 1);
+        }
+        const double sum = 2.9e-6 * (double)M * (double)N;   // a split's values
+        const int smax = splits > 0 ? std::min(splits, KB) : std::max(1, std::min(KB, std::max(64, 148 / active)));
+        const int even = smax > 1 ? (int)std::sqrt(KB / sum) : 1;
+        const int wmax = active > 64 ? 12 : 4;   // waves that the parts may fill
+        for (int w = 0, last = 0; w <= wmax + 1; ++w) {
+            int S = splits > 0 ? smax : w == 0 ? 1 : w > wmax ? even : (int)std::min<int64_t>((int64_t)148 * w / active, KB);
+            S = std::max(1, std::min(S, smax));
+            if (S == last) continue;
+            last = S;
+            const int per = (KB + S - 1) / S;
+            if (splits <= 0) S = (KB + per - 1) / per;
+            const double waves = (double)(((int64_t)active * S + 147) / 148);
+            double t = waves * (per * (0.73 + 0.0008 * bn) + 1.8 + 0.23 * bn / 32.0);
+            const bool two = S > 1 || (upper == 2 && bn == 128);   // passes
+            if (two) t += 0.9 + S * sum;
+            if (t < tbest * (1.0 - 1e-9)) {
+                tbest = t;
+                best = UmmaPlan{bn, S, two ? 2 : 1, (size_t)S * M * N * sizeof(float2)};
+            }
+            if (splits > 0) break;
         }
     }
     return best;
-}
-
-// Split-K count.  One CTA fits on an SM (222 KB of shared memory); the
-// count minimises a model of the run time in k-block units: waves of the
-// active tiles (those on or above the diagonal for a Hermitian product) x
-// splits over 148 SMs, times the k-blocks per split plus ~5 for a CTA's
-// pipeline fill and epilogue, plus the split-K workspace pass.  (Measured:
-// the Si64 betaNL' psi at 5 tiles x 60 splits ran as 2 waves plus 4 CTAs;
-// the Si216 Gram, 115 active tiles, was slower unsplit than at 2 splits.)
-// Accuracy does not depend on it: every k-block is its own
-// accumulation chain in TMEM.
-int umma_splits(int64_t M, int N, int Kp, int splits, int upper) {
-    const int KB = Kp / BK;
-    if (splits > 0) return std::max(1, std::min(splits, KB));
-    const int bn = pick_bn(N);
-    const int mt = (int)((M + BM - 1) / BM), nt = (N + bn - 1) / bn;
-    int active = mt * nt;
-    if (upper) {
-        active = 0;
-        for (int by = 0; by < nt; ++by)
-            for (int bx = 0; bx < mt; ++bx) active += bx * BM > by * bn + bn - 1 ? 0 : 1;
-    }
-    active = std::max(1, active);
-    const int smax = std::max(1, std::min(64, KB / 4));
-    int best = 1;
-    double tbest = 1e300;
-    for (int S = 1; S <= smax; ++S) {
-        const double waves = (double)((active * S + 147) / 148);
-        const double t = waves * ((double)(KB + S - 1) / S + 5.0) + (S > 1 ? (double)S * M * N / 1.3e6 : 0.0);
-        if (t < tbest * (1.0 - 1e-9)) {
-            tbest = t;
-            best = S;
-        }
-    }
-    return best;
-}
-
-size_t umma_ws_bytes(int64_t M, int N, int Kp, int splits, int upper) {
-    return (size_t)umma_splits(M, N, Kp, splits, upper) * M * N * sizeof(float2);
 }
 
 template <int NS, int BN>
@@ -703,14 +749,14 @@ cudaError_t umma_dcsr_prep(const float *ws, int S, int nbeta, int nb, const int 
 }
 
 template <typename CT>
-cudaError_t umma_gemm(const UmmaOperand &A, const UmmaOperand &B, int m, int n, void *C, int64_t ldc, int accumulate,
-                      float *ws, int *err, cudaStream_t st, int upper, int lolo, int splits) {
+cudaError_t umma_gemm(const UmmaPlan &plan, const UmmaOperand &A, const UmmaOperand &B, int m, int n, void *C, int64_t ldc,
+                      int accumulate, float *ws, int *err, cudaStream_t st, int upper, int lolo) {
     cudaError_t e = get_encoder();
     if (e != cudaSuccess) return e;
     if (A.Kp != B.Kp || A.rows != m || B.rows != n) return cudaErrorInvalidValue;
     // three BF16 pieces only when both operands carry them
     const int ns = (A.lo2 && B.lo2) ? 3 : 2;
-    const int bn = pick_bn(n);
+    const int bn = plan.bn;
     CUtensorMap mA[3], mB[3];
     const __nv_bfloat16 *pa[3] = {A.hi, A.lo, ns == 3 ? A.lo2 : A.lo};
     const __nv_bfloat16 *pb[3] = {B.hi, B.lo, ns == 3 ? B.lo2 : B.lo};
@@ -719,12 +765,12 @@ cudaError_t umma_gemm(const UmmaOperand &A, const UmmaOperand &B, int m, int n, 
         if ((e = make_map(&mB[q], pb[q], B.rows, B.Kp, bn)) != cudaSuccess) return e;
     }
     const int KB = A.Kp / BK;
-    const int S = umma_splits(A.rows, n, A.Kp, splits, upper);
+    const int S = plan.S;
     const int kb_per = (KB + S - 1) / S;
     const int tiles = (int)((A.rows + BM - 1) / BM) * ((n + bn - 1) / bn) * S;
     // one split: the epilogue writes or adds into C itself, no workspace pass
-    void *Cd = (S == 1 && upper != 2) ? C : nullptr;
     const int cd = sizeof(CT) == 16 ? 1 : 0;
+    void *Cd = plan.passes == 1 ? C : nullptr;
     e = cudaErrorInvalidValue;
 #define PW_U(BN)                                                                                                     \
     if (bn == BN)                                                                                                    \
@@ -737,16 +783,20 @@ cudaError_t umma_gemm(const UmmaOperand &A, const UmmaOperand &B, int m, int n, 
     PW_U(32)
 #undef PW_U
     if (e != cudaSuccess || Cd || !C) return e;
-    k_finalize<CT><<<blocks_for((size_t)m * n), 256, 0, st>>>((const float2 *)ws, S, m, n, (CT *)C, ldc, accumulate, upper);
+    const size_t total = (size_t)m * n;
+    if (S >= 16 && total <= 65536)
+        k_finalize8<CT><<<blocks_for(total * 8), 256, 0, st>>>((const float2 *)ws, S, m, n, (CT *)C, ldc, accumulate, upper);
+    else
+        k_finalize<CT><<<blocks_for(total), 256, 0, st>>>((const float2 *)ws, S, m, n, (CT *)C, ldc, accumulate, upper);
     return cudaGetLastError();
 }
 
 template cudaError_t umma_prep_tn<float2>(const void *, int64_t, int64_t, int, UmmaOperand &, cudaStream_t);
 template cudaError_t umma_prep_tn<double2>(const void *, int64_t, int64_t, int, UmmaOperand &, cudaStream_t);
 template cudaError_t umma_prep_nn_a<float2>(const void *, int64_t, int64_t, int, UmmaOperand &, cudaStream_t);
-template cudaError_t umma_gemm<float2>(const UmmaOperand &, const UmmaOperand &, int, int, void *, int64_t, int, float *,
-                                       int *, cudaStream_t, int, int, int);
-template cudaError_t umma_gemm<double2>(const UmmaOperand &, const UmmaOperand &, int, int, void *, int64_t, int, float *,
-                                        int *, cudaStream_t, int, int, int);
+template cudaError_t umma_gemm<float2>(const UmmaPlan &, const UmmaOperand &, const UmmaOperand &, int, int, void *, int64_t,
+                                       int, float *, int *, cudaStream_t, int, int);
+template cudaError_t umma_gemm<double2>(const UmmaPlan &, const UmmaOperand &, const UmmaOperand &, int, int, void *, int64_t,
+                                        int, float *, int *, cudaStream_t, int, int);
 
 }  // namespace pwk

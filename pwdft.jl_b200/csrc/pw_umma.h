@@ -21,11 +21,15 @@ struct UmmaOperand {
 
 int umma_kpad(int64_t K);                          // padded 2K (multiple of 64)
 size_t umma_operand_bytes(int64_t rows, int64_t K);  // hi + lo bytes for `rows` rows (one piece: half)
-// split-K count (splits > 0 overrides the automatic choice) and its
-// workspace; a single split writes the result directly (no finalize launch)
-// (upper: the product is Hermitian and only tiles on or above the diagonal run)
-int umma_splits(int64_t M, int N, int Kp, int splits = 0, int upper = 0);
-size_t umma_ws_bytes(int64_t M, int N, int Kp, int splits = 0, int upper = 0);
+// What a product of M x N complex values runs with.  splits > 0 overrides the
+// split-K count; upper: the product is Hermitian and only tiles on or above the
+// diagonal run (2: C is complex128).
+struct UmmaPlan {
+    int bn, S;         // tile width, parts of the sum
+    int passes;        // kernels of umma_gemm with C given: 1 (C written directly), or 2
+    size_t ws_bytes;   // the split sums, [S][N][M] complex (unused with 1 pass into C)
+};
+UmmaPlan umma_plan(int64_t M, int N, int Kp, int splits = 0, int upper = 0);
 
 // Operand builders (CT = float2 or double2 input element).
 //   tn:   m rows from Z (K x m)                for either operand of Z^H W
@@ -38,7 +42,8 @@ template <typename CT> cudaError_t umma_prep_nn_a(const void *A, int64_t lda, in
 cudaError_t umma_dcsr_prep(const float *ws, int S, int nbeta, int nb, const int *rowptr, const int *col, const double *val,
                            UmmaOperand &, cudaStream_t);
 
-// C (m x n complex of type CT, ldc) (+)= result; A.rows == m, B.rows == n.
+// C (m x n complex of type CT, ldc) (+)= result; A.rows == m, B.rows == n; plan: of
+// umma_plan(m, n, A.Kp, ..., upper).
 // C == nullptr: the split sums stay in ws ([split][n][m] complex).
 // err: device int set non-zero if a bounded wait in the kernel expired.
 template <typename CT>
@@ -46,7 +51,7 @@ template <typename CT>
 // 2 = the other triangle is filled with its conjugate as well.
 // lolo != 0 (two-piece operands from the same block, C = Z^H Z): add the
 // lo*lo product, whose omission biases the diagonal |z|^2 low.
-cudaError_t umma_gemm(const UmmaOperand &A, const UmmaOperand &B, int m, int n, void *C, int64_t ldc, int accumulate,
-                      float *ws, int *err, cudaStream_t, int upper = 0, int lolo = 0, int splits = 0);
+cudaError_t umma_gemm(const UmmaPlan &plan, const UmmaOperand &A, const UmmaOperand &B, int m, int n, void *C, int64_t ldc,
+                      int accumulate, float *ws, int *err, cudaStream_t, int upper = 0, int lolo = 0);
 
 }  // namespace pwk

@@ -54,6 +54,14 @@ def test_gram_edges(ctx, K, m, n, pad):
     assert ((S - 2 * refS).abs() <= 2 * boundS).all()
 
 
+@pytest.mark.parametrize("K,m,n", [(30, 5, 5), (30, 100, 100), (200, 100, 100), (80009, 3, 11), (40009, 33, 33), (9001, 256, 256),
+                                   (9001, 257, 256), (3001, 480, 480)])
+def test_tiles_and_parts(ctx, K, m, n):
+    """Narrow and wide tiles, unsplit (one pass, both triangles of A^H A) and in
+    many parts (eight lanes an element up to 65,536 of them)."""
+    test_gram_edges(ctx, K, m, n, 0)
+
+
 @pytest.mark.parametrize("M,n,k,pad", [(1, 1, 1, 0), (17, 3, 7, 1), (127, 32, 32, 0), (128, 33, 31, 1), (1009, 80, 65, 0),
                                        (5003, 97, 161, 3), (24001, 160, 320, 0)])
 def test_rotate_edges(ctx, M, n, k, pad):
