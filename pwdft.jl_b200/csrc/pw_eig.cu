@@ -1091,9 +1091,10 @@ __device__ void wy_panel(const double2 *__restrict__ C, const double2 *__restric
 #pragma unroll
         for (int v = 0; v < 4; ++v) S[(a0 + u) * LD + b0 + v] = acc[u][v];
     __syncthreads();
-    // T[:, i] = -tau_i T[0:i, 0:i] (V^H v_i)[0:i], T_ii = tau_i (Vs holds T)
-    for (int i = 0; i < WYB; ++i) {
-        const double2 ti = i < nv ? tau[j0 + i] : make_double2(0.0, 0.0);
+    // T[:, i] = -tau_i T[0:i, 0:i] (V^H v_i)[0:i], T_ii = tau_i (Vs holds T), zero
+    // past the panel's nv vectors
+    for (int i = 0; i < nv; ++i) {
+        const double2 ti = tau[j0 + i];
         if (tid < WYB) {
             double2 y = make_double2(0.0, 0.0);
             for (int q = tid; q < i; ++q) {
@@ -1106,7 +1107,8 @@ __device__ void wy_panel(const double2 *__restrict__ C, const double2 *__restric
         }
         __syncthreads();
     }
-    for (int e = tid; e < WYB * WYB; e += 128) T[e] = Vs[(e / WYB) * LD + e % WYB];
+    for (int e = tid; e < WYB * WYB; e += 128)
+        T[e] = e % WYB < nv ? Vs[(e / WYB) * LD + e % WYB] : make_double2(0.0, 0.0);
 }
 
 // lowest k eigenvalues of the real symmetric tridiagonal (d, e), ascending.
