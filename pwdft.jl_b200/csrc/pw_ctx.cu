@@ -15,6 +15,7 @@
 #include "../../include/pwb200.h"
 #include "pw_launch.h"
 #include "pw_rho.h"
+#include "pw_twiddle.h"
 #include "pw_umma.h"
 
 using namespace pwk;
@@ -199,8 +200,7 @@ int build_twiddles(pw_ctx *c, int n, int slot) {
     std::vector<double2> t64(n);
     std::vector<float2> t32(n);
     for (int m = 0; m < n; ++m) {
-        const double a = -2.0 * M_PI * (double)m / (double)n;
-        t64[m] = make_double2(std::cos(a), std::sin(a));
+        twiddle(m, n, t64[m].x, t64[m].y);
         t32[m] = make_float2((float)t64[m].x, (float)t64[m].y);
     }
     int s = upload(c, &c->tw64[slot], t64);
