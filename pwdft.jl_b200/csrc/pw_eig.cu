@@ -1479,6 +1479,55 @@ cudaError_t resident_ctas(const void *fn, int threads, size_t smem, int *n, bool
     return cudaSuccess;
 }
 
+// The last (or only) 256 columns of the tridiagonalisation, what one cluster holds in
+// registers, go to it, those before them to the grid: in registers up to n = 1024,
+// through L2 above that.  At 2.3 against 4.0 us a column the whole reduced problem goes
+// from 2.94 to 2.65 ms at n = 480, from 1.14 to 0.75 at 160 (k = n / 3); with 384
+// columns in a cluster of 384 threads a CTA it spills, 2.73 at 480.
+const auto tri_c = k_tridiag_c<8, 8, 2>;
+static_assert(32 * 8 == TRI_NC, "the cluster's columns");
+struct TriKernels {
+    TriRoute route;
+    const void *fn_r;           // the register kernel for n, and its shared memory
+    size_t smem_r;
+    cudaLaunchConfig_t cf;      // the cluster's launch
+    cudaLaunchAttribute at;
+};
+cudaError_t tri_kernels(int n, cudaStream_t st, TriKernels *k) {
+    cudaError_t e;
+    constexpr size_t smem_c = tridiag_c_smem<8, 8, 2>();
+    static_assert(smem_c <= 48 << 10, "no opt-in");
+    k->cf = {};
+    k->cf.gridDim = TRC;
+    k->cf.blockDim = 256;
+    k->cf.dynamicSmemBytes = smem_c;
+    k->cf.stream = st;
+    k->at.id = cudaLaunchAttributeClusterDimension;
+    k->at.val.clusterDim.x = TRC;
+    k->at.val.clusterDim.y = k->at.val.clusterDim.z = 1;
+    k->cf.attrs = &k->at;
+    k->cf.numAttrs = 1;
+    if ((e = cudaFuncSetAttribute(tri_c, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) != cudaSuccess) return e;
+    // no room for 16 neighbouring SMs (a partitioned device): the grid does all
+    int ncl = 0;
+    if (cudaOccupancyMaxActiveClusters(&ncl, tri_c, &k->cf) != cudaSuccess) {
+        cudaGetLastError();
+        ncl = 0;
+    }
+    // few CTAs keep the exchange short, few columns a CTA the update (n =
+    // 480, us a column: 120 CTAs of 4 columns 4.1, 60 of 8 4.5, 30 of 16 5.4)
+    k->fn_r = n <= 512 ? (const void *)k_tridiag_r<16, 4, 1> : (const void *)k_tridiag_r<32, 8, 1>;
+    k->smem_r = 3 * (size_t)(n <= 512 ? 512 : 1024) * sizeof(double2);
+    int res = 0;
+    if (n <= 1024 && (n > TRI_NC || ncl < 1)) {
+        // (48 KB and the static arrays need the opt-in, or none would be resident)
+        if ((e = cudaFuncSetAttribute(k->fn_r, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k->smem_r)) != cudaSuccess) return e;
+        if ((e = resident_ctas(k->fn_r, 32 * tri_r_warps(n), k->smem_r, &res)) != cudaSuccess) return e;
+    }
+    k->route = tri_route(n, res, ncl);
+    return cudaSuccess;
+}
+
 cudaError_t coop_blocks(const void *fn, size_t smem, int *nblk) {
     const cudaError_t e = resident_ctas(fn, COOP_THREADS, smem, nblk, true);   // one CTA per SM keeps the barrier cheap
     return e != cudaSuccess ? e : *nblk < 1 ? cudaErrorCooperativeLaunchTooLarge : cudaSuccess;
@@ -1567,42 +1616,12 @@ cudaError_t hegv_lowest(double2 *T, double2 *G, int n, int k, double *lam_out, d
         if ((e_ = gemm_nn<double>(n, n, n, M1, n, G, n, T, n, 0, st, 2)) != cudaSuccess) return e_;
         k_herm_upper<<<nb, 256, 0, st>>>(T, n);
     }
-    // The last (or only) 256 columns, what one cluster holds in registers, go to
-    // it, those before them to the grid: in registers up to n = 1024, through L2
-    // above that.  At 2.3 against 4.0 us a column the whole reduced problem goes
-    // from 2.94 to 2.65 ms at n = 480, from 1.14 to 0.75 at 160 (k = n / 3); with
-    // 384 columns in a cluster of 384 threads a CTA it spills, 2.73 at 480.
-    const auto fc = k_tridiag_c<8, 8, 2>;
-    static_assert(32 * 8 == TRI_NC, "the cluster's columns");
-    constexpr size_t smem_c = tridiag_c_smem<8, 8, 2>();
-    cudaLaunchConfig_t cf = {};
-    cudaLaunchAttribute at;
-    cf.gridDim = TRC;
-    cf.blockDim = 256;
-    cf.dynamicSmemBytes = smem_c;
-    cf.stream = st;
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = TRC;
-    at.val.clusterDim.y = at.val.clusterDim.z = 1;
-    cf.attrs = &at;
-    cf.numAttrs = 1;
-    if ((e_ = cudaFuncSetAttribute(fc, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) != cudaSuccess) return e_;
-    static_assert(smem_c <= 48 << 10, "no opt-in");
-    // no room for 16 neighbouring SMs (a partitioned device): the grid does all
-    int ncl = 0;
-    if (cudaOccupancyMaxActiveClusters(&ncl, fc, &cf) != cudaSuccess) {
-        cudaGetLastError();
-        ncl = 0;
-    }
-    // few CTAs keep the exchange short, few columns a CTA the update (n =
-    // 480, us a column: 120 CTAs of 4 columns 4.1, 60 of 8 4.5, 30 of 16 5.4)
-    const void *fn = n <= 512 ? (const void *)k_tridiag_r<16, 4, 1> : (const void *)k_tridiag_r<32, 8, 1>;
-    const size_t smem_r = 3 * (size_t)(n <= 512 ? 512 : 1024) * sizeof(double2);
-    const int W = tri_r_warps(n), ctas_r = tri_r_ctas(n);
-    int res_r = 0;
-    if (n <= 1024 && (n > TRI_NC || ncl < 1) && (e_ = resident_ctas(fn, 32 * W, smem_r, &res_r)) != cudaSuccess) return e_;
-    const TriRoute route = tri_route(n, res_r, ncl);
-    const int jend = route.jend;
+    TriKernels tk;
+    if ((e_ = tri_kernels(n, st, &tk)) != cudaSuccess) return e_;
+    const TriRoute route = tk.route;
+    const void *fn = tk.fn_r;
+    const size_t smem_r = tk.smem_r;
+    const int W = tri_r_warps(n), ctas_r = tri_r_ctas(n), jend = route.jend;
     if ((jend > 0 || !route.cluster) && route.registers) {
         if ((e_ = cudaMemsetAsync(ybuf, 0xff, (size_t)jend * 2 * ctas_r * W * sizeof(double2), st)) != cudaSuccess) return e_;
         void *args[] = {(void *)&Cm, (void *)&n, (void *)&jend, (void *)&d, (void *)&e, (void *)&tau, (void *)&ybuf, (void *)&err};
@@ -1622,7 +1641,7 @@ cudaError_t hegv_lowest(double2 *T, double2 *G, int n, int k, double *lam_out, d
         nl += 1;
     }
     if (route.cluster) {
-        if ((e_ = cudaLaunchKernelEx(&cf, fc, Cm + (size_t)jend * (n + 1), n - jend, n, d + jend, e + jend, tau + jend, err)) !=
+        if ((e_ = cudaLaunchKernelEx(&tk.cf, tri_c, Cm + (size_t)jend * (n + 1), n - jend, n, d + jend, e + jend, tau + jend, err)) !=
             cudaSuccess)
             return e_;
         nl += 1;
@@ -1692,6 +1711,15 @@ cudaError_t chol_inverse_upper(double2 *C, int n, double2 *Rinv, void *work, int
 }
 
 }  // namespace pwk
+
+// Test-only export (not in pwb200.h): the kernels that an order-n problem takes on
+// `device`: 1 the register kernel, 2 the cluster, 3 both, 0 the grid-barrier kernel
+// alone, negative on an error.
+extern "C" int pwk_test_tri_route(int device, int n) {
+    pwk::eig::TriKernels k;
+    if (cudaSetDevice(device) != cudaSuccess || pwk::eig::tri_kernels(n, nullptr, &k) != cudaSuccess) return -1;
+    return (k.route.registers && (k.route.jend > 0 || !k.route.cluster) ? 1 : 0) + (k.route.cluster ? 2 : 0);
+}
 
 // Test-only export (not in pwb200.h): sets the grid-barrier poll limit
 // (limit <= 0 restores the default) and the CTA that withholds its arrivals

@@ -61,6 +61,17 @@ def test_last_columns_in_one_cluster(ctx, n, k):
     check(ctx, herm(n, n), k)
 
 
+@pytest.mark.parametrize("n,want", [(1, 2), (256, 2), (257, 3), (480, 3), (512, 3), (513, 3), (700, 3), (1024, 3), (1025, 2)])
+def test_kernels_of_the_tridiagonalisation(n, want):
+    """On a whole B200: the register kernel (1) for the columns before the last 256
+    up to n = 1024, the cluster (2) for those."""
+    import ctypes as C
+    import pwb200
+    f = pwb200.lib().pwk_test_tri_route
+    f.restype, f.argtypes = C.c_int, [C.c_int, C.c_int]
+    assert f(0, n) == want
+
+
 @pytest.mark.parametrize("n,k", [(1, 1), (33, 11), (100, 100), (480, 160), (545, 300)])
 def test_generalized(ctx, n, k):
     r = np.random.default_rng(n + 1)
