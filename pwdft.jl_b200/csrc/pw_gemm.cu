@@ -74,13 +74,24 @@ k_gemm_tn(int64_t K, int m, int n, const Cx<T> *__restrict__ A, int64_t lda, con
 // cp.async stages.  Rows are padded to 12 (k-contiguous operands) or 16 WM + 2
 // (row-contiguous ones) complex values, which puts the eight lanes of each
 // 128-byte phase of a fragment read on different banks.
+// Sums: the 16 products of a step of eight k are summed from zero, then added to the
+// accumulator, which so is rounded once in eight values.  Every instruction
+// accumulating into the long sum (two roundings in four values, each of the long
+// sum's size) is 2 to 15 % faster and loses accuracy: against extended precision, 180
+// columns over 24,000 5.0e-15 against 4.8e-16 here and 1.7e-15 on CUDA cores; 480
+// columns times 480 x 160 1.0e-15, 3.0e-16, 7.4e-16.
 // TN: C = A^H B, A and B k-contiguous.  NN: C = A B, A row-contiguous.
 // Bound by the FP64 pipe (36.9 TFLOP/s measured for a loop of nothing else).
 // The 32 x 32 CUDA-core tiles before it were bound by shared-memory reads
 // (two 16-byte reads per complex multiply-add and thread).  Measured, 480
 // columns over K = 23,871 (Q'HQ, Q'Q and Q U of 160 bands together):
-// 6.66 -> 3.07 ms, 26 TFLOP/s; op_H of 32 atoms (81 bands) 664 -> 546 us.
+// 6.66 -> 3.01 ms, 27 TFLOP/s; op_H of 32 atoms (81 bands) 664 -> 546 us.
 constexpr int ZBK = 8, ZST = 3, ZKP = ZBK + 4;
+__device__ __forceinline__ void dmma0(double (&c)[2], double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%4, %4};"
+                 : "=d"(c[0]), "=d"(c[1])
+                 : "d"(a), "d"(b), "d"(0.0));
+}
 template <int WM, int WN, bool TN> constexpr size_t zgemm_smem() {
     return (size_t)ZST * ((TN ? 16 * WM * ZKP : ZBK * (16 * WM + 2)) + 16 * WN * ZKP) * sizeof(double2);
 }
@@ -172,24 +183,41 @@ k_zgemm(int64_t K, int64_t m, int n, const double2 *__restrict__ A, int64_t lda,
         if (it + ZST - 1 < nk) load(it + ZST - 1);
         asm volatile("cp.async.commit_group;" ::: "memory");
         const double2 *as = As + (it % ZST) * ASZ, *bs = Bs + (it % ZST) * BSZ;
+        double2 b[2][WN];
 #pragma unroll
-        for (int kk = 0; kk < ZBK; kk += 4) {
-            double2 a[WM], b[WN];
+        for (int j = 0; j < WN; ++j)
 #pragma unroll
-            for (int i = 0; i < WM; ++i)
-                a[i] = TN ? as[(wm + 8 * i + g) * ZKP + kk + t] : as[(kk + t) * AP + wm + 8 * i + g];
+            for (int h = 0; h < 2; ++h) b[h][j] = bs[(wn + 8 * j + g) * ZKP + 4 * h + t];
 #pragma unroll
-            for (int j = 0; j < WN; ++j) b[j] = bs[(wn + 8 * j + g) * ZKP + kk + t];
+        for (int i = 0; i < WM; ++i) {
+            double2 a[2];
 #pragma unroll
-            for (int i = 0; i < WM; ++i) {
-                const double an = -a[i].y;
+            for (int h = 0; h < 2; ++h)
+                a[h] = TN ? as[(wm + 8 * i + g) * ZKP + 4 * h + t] : as[(4 * h + t) * AP + wm + 8 * i + g];
 #pragma unroll
-                for (int j = 0; j < WN; ++j) {
-                    dmma(re[i][j], a[i].x, b[j].x);
-                    dmma(im[i][j], a[i].x, b[j].y);
-                    dmma(re[i][j], TN ? a[i].y : an, b[j].y);
-                    dmma(im[i][j], TN ? an : a[i].y, b[j].x);
-                }
+            for (int j0 = 0; j0 < WN; j0 += 2) {
+                double tr[2][2], ti[2][2];
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                    for (int p = 0; p < 4; ++p)
+#pragma unroll
+                        for (int u = 0; u < 2; ++u) {
+                            if (j0 + u >= WN) continue;
+                            const double2 bb = b[h][j0 + u];
+                            if (p == 0) h ? dmma(tr[u], a[h].x, bb.x) : dmma0(tr[u], a[h].x, bb.x);
+                            if (p == 1) h ? dmma(ti[u], a[h].x, bb.y) : dmma0(ti[u], a[h].x, bb.y);
+                            if (p == 2) dmma(tr[u], TN ? a[h].y : -a[h].y, bb.y);
+                            if (p == 3) dmma(ti[u], TN ? -a[h].y : a[h].y, bb.x);
+                        }
+#pragma unroll
+                for (int u = 0; u < 2; ++u)
+#pragma unroll
+                    for (int q = 0; q < 2; ++q)
+                        if (j0 + u < WN) {
+                            re[i][j0 + u][q] += tr[u][q];
+                            im[i][j0 + u][q] += ti[u][q];
+                        }
             }
         }
     }
@@ -218,12 +246,15 @@ k_zgemm(int64_t K, int64_t m, int n, const double2 *__restrict__ A, int64_t lda,
 
 // Tile and split-K count of a product: the candidate with the shortest
 // modelled time in clocks.  A CTA's tile costs 16 WM WN clocks of its SM's
-// FP64 pipe per k, but not less than 45 (the ring waits for L2: 350 clocks a step
-// of 8), plus about 32 k for filling the ring and storing; the SM with the
-// most CTAs decides; a split adds the partial sums' trip through L2
-// (about 2400 bytes a clock) and the reduction's launch (4000 clocks).
-// (480 x 480 over K = 23,871: 48 x 80 tiles, 0 % padding, against 14 % with
-// 64 x 64.)  Splitting stops at four CTAs an SM, which also bounds the workspace: 592
+// FP64 pipe per k, more by 0.8 (TN) or 0.3 (NN) times 1 / WM + 1 / WN for the
+// fragments it reads per product, but not less than 45 (the ring waits for L2: 350
+// clocks a step of 8), plus about 32 k for filling the ring and storing; the SM with
+// the most CTAs decides, its last ones alone at 1.3 (one left over) or 1.05 (two) times
+// their share; a split adds the partial sums' trip through L2 (about 2400 bytes a
+// clock) and the reduction's launch (4000 clocks).  The three factors are a fit to 16
+// products with each of the 15 tiles measured; the choice is within 5 % of the best
+// there (A^H A of 180 columns over 24,000: 173 us with 64 x 64 tiles, 289 with the 32 x
+// 16 ones that a model without them takes).  Splitting stops at four CTAs an SM, which also bounds the workspace: 592
 // tiles, 49 MB, and up to about twice that for a triangular product, where only the
 // formed tiles count but every split has room for all.  Few values are split too
 // (betaNL' psi of 8 bands over about 730 plane waves: 35.8 us on one CTA, 5.0 in 23
@@ -242,14 +273,17 @@ TnPlan zplan(int64_t K, int64_t m, int n, bool tn, int upper, bool fused = false
                 tiles = 0;
                 for (int64_t c = 0; c < tc; ++c) tiles += (double)std::min<int64_t>(tm, (c * 16 * wn + 16 * wn - 1) / (16 * wm) + 1);
             }
+            const double f = 1.0 + (tn ? 0.8 : 0.3) * (1.0 / wm + 1.0 / wn);
+            const int res = wm * wn >= 12 ? 2 : wm * wn >= 6 ? 3 : 4;   // CTAs that an SM holds
             // splits that fill whole rounds of the 148 SMs, or as many as
             // leave 32 values each
             for (int w = 0; w <= (tn ? 4 : 0); ++w) {
                 const int S = w == 0 ? 1 : (int)std::min<int64_t>((int64_t)(148.0 * w / tiles), K / 32);
                 if (w > 0 && S < 2) continue;
                 const double kc = (double)((K + S - 1) / S);
-                const double per = std::ceil(tiles * S / 148.0);
-                double t = std::max(per * 16.0 * wm * wn * (per < 1.5 ? 1.15 : 1.0), 45.0) * (kc + 32.0);
+                const int per = (int)std::ceil(tiles * S / 148.0), left = per % res;
+                const double busy = per + (left == 1 ? 0.3 : left == 2 ? 0.1 : 0.0);
+                double t = std::max(busy * 16.0 * wm * wn * f, 45.0) * (kc + 32.0);
                 if (S > 1) t += (fused ? 0.0 : 4000.0) + (double)S * m * n * 32.0 / 2400.0;
                 if (t < tbest * (1.0 - 1e-9)) {
                     tbest = t;
