@@ -1017,6 +1017,24 @@ __device__ __forceinline__ void vt_dmma(double (&c)[2], double a, double b) {
                  : "+d"(c[0]), "+d"(c[1])
                  : "d"(a), "d"(b));
 }
+// c += a b + d e over four k.  FP64: the eight products are summed first, so that the
+// long sum is rounded once (op_H of 32 k-points, 9 bands, against 64-bit results:
+// 2.4e-16, as with one band a CTA; 2.7e-16 where each product rounds the long sum;
+// 409 against 390 us, 419 with one band a CTA).  FP32 results don't see it.
+template <typename T> __device__ __forceinline__ void vt_add(double (&c)[2], double a, double b, double d, double e) {
+    if constexpr (sizeof(T) == 8) {
+        double t[2];
+        asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%4, %4};"
+                     : "=d"(t[0]), "=d"(t[1])
+                     : "d"(a), "d"(b), "d"(0.0));
+        vt_dmma(t, d, e);
+        c[0] += t[0];
+        c[1] += t[1];
+    } else {
+        vt_dmma(c, a, b);
+        vt_dmma(c, d, e);
+    }
+}
 template <typename T, int NT>
 __global__ void __launch_bounds__(256)
 mk_vnl_t(const MkK *__restrict__ ks, const int2 *__restrict__ groups, const int *__restrict__ Drow,
@@ -1056,10 +1074,8 @@ mk_vnl_t(const MkK *__restrict__ ks, const int2 *__restrict__ groups, const int 
 #pragma unroll
                 for (int i = 0; i < 3; ++i) {
                     const double ar = a[i].x, ai = a[i].y;
-                    vt_dmma(re[i][n], ar, br);
-                    vt_dmma(im[i][n], ar, bi);
-                    vt_dmma(re[i][n], ai, bi);
-                    vt_dmma(im[i][n], -ai, br);
+                    vt_add<T>(re[i][n], ar, br, ai, bi);
+                    vt_add<T>(im[i][n], ar, bi, -ai, br);
                 }
             }
         }
@@ -1113,10 +1129,8 @@ mk_vnl_t(const MkK *__restrict__ ks, const int2 *__restrict__ groups, const int 
 #pragma unroll
             for (int n = 0; n < NT; ++n) {
                 const double2 b = P2[j * VT_PB + 8 * n + g];
-                vt_dmma(re[n], ar, b.x);
-                vt_dmma(im[n], ar, b.y);
-                vt_dmma(re[n], -ai, b.y);
-                vt_dmma(im[n], ai, b.x);
+                vt_add<T>(re[n], ar, b.x, -ai, b.y);
+                vt_add<T>(im[n], ar, b.y, ai, b.x);
             }
         }
 #pragma unroll
